@@ -1,18 +1,17 @@
 // Selection attention backward, general geometry (bf16 / fp16, D in {64,128}):
 //   * inverted (block -> query groups) CSR index: histogram, per-(b,h) scan, scatter;
-//   * dQ kernel: one thread block per (b, group, h), same packed K/V tiles as the forward;
+//   * dQ kernel: one thread block per (b, group, h), the same ring of K/V tiles as the forward (sel_rows.cuh);
 //     computes delta = sum(O*dO) in its prologue and stores it for the dK/dV kernel;
-//   * dK/dV kernel: one thread block OWNS a 64-token tile of one (b, h, block) and walks the
+//   * dK/dV kernel: one thread block OWNS a tile of at most 32 tokens of one (b, h, block) and walks the
 //     block's bucket of query groups in ascending group order - no atomics, results are
 //     bit-reproducible from run to run.
-#include "sel_common.cuh"
+#include "sel_rows.cuh"
 
 namespace nsa {
 namespace {
 
 __host__ __device__ __forceinline__ int64_t min64(int64_t a, int64_t b) { return a < b ? a : b; }
 constexpr int kIdxThreads = 256;
-constexpr int kSortCap = 1024;   // bucket entries sorted in shared memory
 
 struct IdxParams {
   const int32_t* ids;
@@ -244,212 +243,158 @@ struct BwdParams {
   } tab;
 };
 
-template <typename T, int D>
-__global__ void __launch_bounds__(256) sel_bwd_dq_kernel(const BwdParams p) {
-  constexpr int PITCH = D + 8;
-  constexpr int ESZ = sizeof(T);
-  constexpr int KK = D / 16;
-  constexpr int DN = D / 8;
-  extern __shared__ __align__(16) char smem[];
-
-  const int g = blockIdx.x, h = blockIdx.y, b = blockIdx.z;
+// W warps of 16 query rows share one ring of K/V tiles; with W = 1 the list may be dealt out to KS warps.  Bounds as in
+// the forward, with 9 warps per SM (registers: Q and dO fragments and the accumulator).  32760 queries x 12 heads,
+// 15-query groups, 16 blocks of 30: 623 us (10142 us with one warp per thread block).
+template <typename T, int D, int W, int KS, bool TMA>
+__global__ void __launch_bounds__(32 * W * KS, W == 4 && D == 128 ? 3 : 1) sel_bwd_dq_rows_kernel(
+    const __grid_constant__ RingMaps maps, const BwdParams p, const int stages, int32_t* status) {
+  static_assert(W == 1 || KS == 1, "only single-warp groups are split");
+  constexpr int ESZ = sizeof(T), ROWS = 32;
+  extern __shared__ __align__(1024) uint8_t smem[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int gid = lane >> 2, t4 = lane & 3;
-  const int rows_pad = (blockDim.x >> 5) * 16;
-  const int64_t m0 = static_cast<int64_t>(g) * p.G;
-  const int n_q = static_cast<int>(p.M - m0 < p.G ? p.M - m0 : p.G);
-  const int q_chunk = static_cast<int>(m0 / p.chunk_size);
+  const int g = blockIdx.x, h = blockIdx.y, b = blockIdx.z;
+  const int64_t g0 = static_cast<int64_t>(g) * p.G;
+  const int row_warp = W > 1 ? warp : 0, part = KS > 1 ? warp : 0;
+  const int n_q = static_cast<int>(p.M - g0 < p.G ? p.M - g0 : p.G) - row_warp * 16;
+  const int64_t m0 = g0 + row_warp * 16;
 
-  T* tiles = reinterpret_cast<T*>(smem);                         // [2][2][64][PITCH]
-  T* sQ = tiles + 4 * kTileRows * PITCH;                          // [rows_pad][PITCH]
-  T* sdO = sQ + rows_pad * PITCH;
-  float* s_lse = reinterpret_cast<float*>(sdO + rows_pad * PITCH);
-  float* s_delta = s_lse + rows_pad;
-  const SlotTable st = carve_slot_table(reinterpret_cast<char*>(s_delta + rows_pad), p.T);
-  auto stageK = [&](int s) { return tiles + (s * 2) * kTileRows * PITCH; };
-  auto stageV = [&](int s) { return tiles + (s * 2 + 1) * kTileRows * PITCH; };
+  const uint32_t ring_bytes = static_cast<uint32_t>(stages) * 2 * kRingTile<D, ROWS>;
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + KS * ring_bytes);
+  int* words = reinterpret_cast<int*>(bars + KS * kRingBars);                          // abort, tile count
+  RingTile* list = reinterpret_cast<RingTile*>(words + 4);
+  if (warp == 0) {
+    const int count = ring_list<ESZ>(list, p.kv, p.ids, b * p.i_sb + g * p.i_sg + h * p.i_sh, p.i_st, p.T, b, h, D,
+                                     p.block_size, p.chunk_size, p.causal != 0, static_cast<int>(g0 / p.chunk_size));
+    if (lane == 0) { words[0] = 0; words[1] = count; }
+  }
+  Ring<D, ROWS, TMA> ring{smem_u32(smem) + part * ring_bytes, bars + part * kRingBars, words,
+                          0, stages, row_warp, W};
+  ring.init();
+  __syncthreads();
+  ring.count = KS > 1 ? (words[1] - part + KS - 1) / KS : words[1];
+  const RingSource src = kv_ring_source<ESZ>(p.kv, maps, p.B, b, h, D, p.block_size);
+  const auto tile_of = [&](int i) { return list[part + i * KS]; };
+  ring.start(src, tile_of);
 
-  const int total = build_slot_table<ESZ>(st, p.kv, p.ids, b * p.i_sb + g * p.i_sg + h * p.i_sh, p.i_st,
-                                          p.T, b, h, D, p.block_size, p.chunk_size, p.causal != 0, q_chunk);
-
-  const char* q_base = p.q + (b * p.q_sb + m0 * p.q_sm + h * p.q_sh) * ESZ;
-  const char* o_base = p.o + (b * p.o_sb + m0 * p.o_sm + h * p.o_sh) * ESZ;
-  const char* do_base = p.dO + (b * p.do_sb + m0 * p.do_sm + h * p.do_sh) * ESZ;
-  char* dq_base = p.dq + (b * p.dq_sb + m0 * p.dq_sm + h * p.dq_sh) * ESZ;
+  // delta = sum_d O * dO of this thread's rows (lo, hi), from the fragments of both
+  uint32_t q[D / 16][4], dO[D / 16][4];
+  float delta[2] = {0.f, 0.f}, lse2[2];
+  load_a_frag<D>(dO, p.dO + (b * p.do_sb + m0 * p.do_sm + h * p.do_sh) * ESZ, p.do_sm * ESZ, n_q);
+  load_a_frag<D>(q, p.o + (b * p.o_sb + m0 * p.o_sm + h * p.o_sh) * ESZ, p.o_sm * ESZ, n_q);
+#pragma unroll
+  for (int kk = 0; kk < D / 16; ++kk)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const float2 x = unpack2<T>(q[kk][e]), y = unpack2<T>(dO[kk][e]);
+      delta[e & 1] += x.x * y.x + x.y * y.y;
+    }
+  load_a_frag<D>(q, p.q + (b * p.q_sb + m0 * p.q_sm + h * p.q_sh) * ESZ, p.q_sm * ESZ, n_q);
   const int64_t bhm = (static_cast<int64_t>(b) * p.H + h) * p.M + m0;
+#pragma unroll
+  for (int r = 0; r < 2; ++r) {
+    delta[r] += __shfl_xor_sync(0xffffffffu, delta[r], 1);
+    delta[r] += __shfl_xor_sync(0xffffffffu, delta[r], 2);
+    const int row = gid + 8 * r;
+    lse2[r] = row < n_q ? p.lse[bhm + row] * kLog2e : INFINITY;
+    if (t4 == 0 && row < n_q && part == 0) p.delta[bhm + row] = delta[r];
+  }
 
-  // delta = sum_d O * dO (one warp per row), kept in shared memory and stored for dK/dV
-  for (int r = warp; r < rows_pad; r += (blockDim.x >> 5)) {
-    float acc = 0.f;
-    if (r < n_q) {
-      const T* orow = reinterpret_cast<const T*>(o_base + r * p.o_sm * ESZ);
-      const T* drow = reinterpret_cast<const T*>(do_base + r * p.do_sm * ESZ);
-      for (int d = lane * 2; d < D; d += 64) {
-        const float2 a = unpack2<T>(*reinterpret_cast<const uint32_t*>(orow + d));
-        const float2 c = unpack2<T>(*reinterpret_cast<const uint32_t*>(drow + d));
-        acc += a.x * c.x + a.y * c.y;
+  float dq[D / 8][4];
+#pragma unroll
+  for (int n = 0; n < D / 8; ++n) dq[n][0] = dq[n][1] = dq[n][2] = dq[n][3] = 0.f;
+  bool ok = true;
+  for (int i = 0; i < ring.count && ok; ++i) {
+    const int n = list[part + i * KS].n, brought = list[part + i * KS].clear;
+    const int n16 = (n + 15) >> 4;
+    float s[ROWS / 8][4], dp[ROWS / 8][4];
+#pragma unroll
+    for (int j = 0; j < ROWS / 8; ++j) {
+      s[j][0] = s[j][1] = s[j][2] = s[j][3] = 0.f;
+      dp[j][0] = dp[j][1] = dp[j][2] = dp[j][3] = 0.f;
+    }
+    if (!ring.template wait<0>()) { ok = false; break; }
+    mma_rows_t<T, D, ROWS>(s, q, ring.tile(0), n16);
+    if (!ring.template wait<1>()) { ok = false; break; }
+    mma_rows_t<T, D, ROWS>(dp, dO, ring.tile(1), n16);
+    // V can go; K is still wanted for dQ (a ring with several readers lets go of both at the end)
+    if (W == 1) ok = ring.template release<1>(i, src, tile_of);
+    uint32_t ds[ROWS / 16][4];
+#pragma unroll
+    for (int j = 0; j < ROWS / 8; ++j) {
+      float x[4];
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const float pe = fast_exp2(s[j][e] * p.scale_log2 - lse2[e >> 1]);
+        x[e] = 8 * j + 2 * t4 + (e & 1) < n ? pe * (dp[j][e] - delta[e >> 1]) * p.scale : 0.f;
       }
+      ds[j >> 1][(j & 1) * 2] = pack2<T>(x[0], x[1]);
+      ds[j >> 1][(j & 1) * 2 + 1] = pack2<T>(x[2], x[3]);
     }
-#pragma unroll
-    for (int d = 16; d; d >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, d);
-    if (lane == 0) {
-      s_delta[r] = acc;
-      s_lse[r] = r < n_q ? p.lse[bhm + r] * kLog2e : INFINITY;
-      if (r < n_q) p.delta[bhm + r] = acc;
-    }
+    if (TMA && n < brought) ring_clear_rows<D, ROWS>(ring.tile(0), n, brought);
+    mma_rows<T, D, ROWS>(dq, ds, ring.tile(0), n16);
+    if (TMA && n < brought) fence_async_shared();        // the cleared rows before the next copy into this tile
+    ok = (W == 1 ? ring.template release<0>(i, src, tile_of) : ring.template release<1>(i, src, tile_of)) && ok;
+    ring.step();
   }
+  if (!ok) atomicExch(status, NSA_ERR_CUDA);
 
-  if (total == 0) {
-    for (int i = threadIdx.x; i < n_q * (D / 8); i += blockDim.x) {
-      const int r = i / (D / 8), c = i % (D / 8);
-      *reinterpret_cast<uint4*>(dq_base + r * p.dq_sm * ESZ + c * 16) = make_uint4(0, 0, 0, 0);
-    }
-    return;
-  }
-
-  const int64_t k_row_bytes = kv_row_bytes(p.kv, false, D, ESZ);
-  const int64_t v_row_bytes = kv_row_bytes(p.kv, true, D, ESZ);
-  const int ntiles = (total + kTileRows - 1) / kTileRows;
-
-  issue_rows<T, D, PITCH>(sQ, q_base, p.q_sm * ESZ, n_q, rows_pad);
-  issue_rows<T, D, PITCH>(sdO, do_base, p.do_sm * ESZ, n_q, rows_pad);
-  issue_kv_tile<T, D, PITCH>(stageK(0), stageV(0), st, p.T, 0, total, k_row_bytes, v_row_bytes, p.q);
-  cp_async_commit();
-
-  float dq[DN][4];
+  __syncthreads();                                        // the rings are done with: their memory stages what follows
+  if constexpr (KS > 1) {
+    float4* part_mem = reinterpret_cast<float4*>(smem) + (warp - 1) * (D / 8 * 32);
+    if (warp > 0) {
 #pragma unroll
-  for (int n = 0; n < DN; ++n) { dq[n][0] = dq[n][1] = dq[n][2] = dq[n][3] = 0.f; }
-  const bool warp_active = warp * 16 < n_q;
-  const T* qa = sQ + (warp * 16 + (lane & 15)) * PITCH + (lane >> 4) * 8;
-  const T* da = sdO + (warp * 16 + (lane & 15)) * PITCH + (lane >> 4) * 8;
-
-  for (int i = 0; i < ntiles; ++i) {
-    if (i + 1 < ntiles) {
-      issue_kv_tile<T, D, PITCH>(stageK((i + 1) & 1), stageV((i + 1) & 1), st, p.T,
-                                 (i + 1) * kTileRows, total, k_row_bytes, v_row_bytes, p.q);
-      cp_async_commit();
-      cp_async_wait<1>();
-    } else {
-      cp_async_wait<0>();
+      for (int n = 0; n < D / 8; ++n) part_mem[n * 32 + lane] = make_float4(dq[n][0], dq[n][1], dq[n][2], dq[n][3]);
     }
     __syncthreads();
-    if (warp_active) {
-      const T* sK = stageK(i & 1);
-      const T* sV = stageV(i & 1);
-      const int nvalid = min(kTileRows, total - i * kTileRows);
-      const int nb_off = ((lane & 7) + ((lane >> 4) << 3)) * PITCH + ((lane >> 3) & 1) * 8;
-      float s[8][4], dp[8][4];
+    if (warp > 0) return;
+    for (int k = 0; k < KS - 1; ++k)
 #pragma unroll
-      for (int n = 0; n < 8; ++n) {
-        s[n][0] = s[n][1] = s[n][2] = s[n][3] = 0.f;
-        dp[n][0] = dp[n][1] = dp[n][2] = dp[n][3] = 0.f;
+      for (int n = 0; n < D / 8; ++n) {
+        const float4 x = reinterpret_cast<const float4*>(smem)[(k * (D / 8) + n) * 32 + lane];
+        dq[n][0] += x.x; dq[n][1] += x.y; dq[n][2] += x.z; dq[n][3] += x.w;
       }
-#pragma unroll
-      for (int kk = 0; kk < KK; ++kk) {
-        uint32_t aq[4], ad[4];
-        ldmatrix_x4(aq, qa + kk * 16);
-        ldmatrix_x4(ad, da + kk * 16);
-#pragma unroll
-        for (int n16 = 0; n16 < 4; ++n16) {
-          if (n16 * 16 < nvalid) {
-            uint32_t bf[4];
-            ldmatrix_x4(bf, sK + nb_off + n16 * 16 * PITCH + kk * 16);
-            mma16816<T>(s[2 * n16], aq, bf[0], bf[1]);
-            mma16816<T>(s[2 * n16 + 1], aq, bf[2], bf[3]);
-            ldmatrix_x4(bf, sV + nb_off + n16 * 16 * PITCH + kk * 16);
-            mma16816<T>(dp[2 * n16], ad, bf[0], bf[1]);
-            mma16816<T>(dp[2 * n16 + 1], ad, bf[2], bf[3]);
-          }
-        }
-      }
-      const float lse0 = s_lse[warp * 16 + gid], lse1 = s_lse[warp * 16 + gid + 8];
-      const float dl0 = s_delta[warp * 16 + gid], dl1 = s_delta[warp * 16 + gid + 8];
-      uint32_t dsa[4][4];
-#pragma unroll
-      for (int n = 0; n < 8; ++n) {
-        float ds[4];
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const int col = n * 8 + 2 * t4 + (e & 1);
-          const float l = (e >> 1) ? lse1 : lse0;
-          const float dl = (e >> 1) ? dl1 : dl0;
-          const float pe = (col < nvalid) ? fast_exp2(s[n][e] * p.scale_log2 - l) : 0.f;
-          ds[e] = pe * (dp[n][e] - dl) * p.scale;
-        }
-        dsa[n >> 1][(n & 1) * 2] = pack2<T>(ds[0], ds[1]);
-        dsa[n >> 1][(n & 1) * 2 + 1] = pack2<T>(ds[2], ds[3]);
-      }
-      const T* kb = sK + ((lane & 7) + ((lane >> 3) & 1) * 8) * PITCH + (lane >> 4) * 8;
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        if (j * 16 < nvalid) {
-#pragma unroll
-          for (int d16 = 0; d16 < D / 16; ++d16) {
-            uint32_t bf[4];
-            ldmatrix_x4_trans(bf, kb + j * 16 * PITCH + d16 * 16);
-            mma16816<T>(dq[2 * d16], dsa[j], bf[0], bf[1]);
-            mma16816<T>(dq[2 * d16 + 1], dsa[j], bf[2], bf[3]);
-          }
-        }
-      }
-    }
-    __syncthreads();
+    __syncwarp();
   }
-
-  if (warp_active) {
-#pragma unroll
-    for (int r = 0; r < 2; ++r) {
-      const int row = warp * 16 + gid + 8 * r;
-      if (row < n_q) {
-        char* drow = dq_base + row * p.dq_sm * ESZ;
-#pragma unroll
-        for (int n = 0; n < DN; ++n)
-          *reinterpret_cast<uint32_t*>(drow + (n * 8 + 2 * t4) * ESZ) =
-              pack2<T>(dq[n][2 * r], dq[n][2 * r + 1]);
-      }
-    }
-  }
+  if (n_q > 0)
+    store_rows<T, D>(dq, 1.f, 1.f, smem_u32(smem) + row_warp * 16 * (D * 2 + 16),
+                     p.dq + (b * p.dq_sb + m0 * p.dq_sm + h * p.dq_sh) * ESZ, p.dq_sm * ESZ, n_q);
 }
 
 // --------------------------------------------------------------------------------- dK / dV
-template <typename T, int D>
-__global__ void __launch_bounds__(128) sel_bwd_dkv_kernel(const BwdParams p, int tiles_per_block) {
-  constexpr int PITCH = D + 8;
-  constexpr int ESZ = sizeof(T);
-  constexpr int KK = D / 16;
-  constexpr int DN = D / 8;
-  constexpr int QT = 64;
-  extern __shared__ __align__(16) char smem[];
-
-  const int blk = blockIdx.x / tiles_per_block, kt = blockIdx.x % tiles_per_block;
-  const int h = blockIdx.y, b = blockIdx.z;
+// A thread block of TW warps owns at most 16 TW tokens of one (batch, head, block) tile, 16 per warp, keeps their K and
+// V rows in shared memory as A operands and streams the Q and dO rows (and LSE and delta) of the block's bucket, in
+// ascending group order, through the ring, 16 query rows at a time: S^T = K Q^T and dP^T = V dO^T, then dV += P^T dO
+// and dK += dS^T Q.  No atomics: results are bit-reproducible.  What bounds it is the length of a step (products,
+// exponentials, and the issue of the next copies: 3.5 k cycles, of them 1.8 k products) times the 12 warps per SM that
+// two accumulators of 16 x 128 allow.  32760 queries x 12 heads, 15-query groups, 16 blocks of 30: 971 us (3847 us with
+// 64-row tiles; two query tiles per step with 8 warps per SM: 1096 us).
+template <typename T, int D, int TW, bool TMA>
+__global__ void __launch_bounds__(32 * TW, (D == 128 ? 12 : 16) / TW)
+sel_bwd_dkv_rows_kernel(const __grid_constant__ RingMaps maps, const BwdParams p, const int tiles_per_block, const int stages,
+                        int32_t* status) {
+  constexpr int ESZ = sizeof(T), TROWS = 16 * TW, kList = 64;
+  extern __shared__ __align__(1024) uint8_t smem[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int gid = lane >> 2, t4 = lane & 3;
-
-  T* sK = reinterpret_cast<T*>(smem);            // [64][PITCH]
-  T* sV = sK + kTileRows * PITCH;
-  T* sQd = sV + kTileRows * PITCH;               // [2][2][QT][PITCH]  (stage, Q|dO)
-  float* s_lse = reinterpret_cast<float*>(sQd + 4 * QT * PITCH);   // [2][QT]
-  float* s_delta = s_lse + 2 * QT;                                  // [2][QT]
-  int* s_grp = reinterpret_cast<int*>(s_delta + 2 * QT);            // [kSortCap]
-  int* s_tmp = s_grp + kSortCap;                                    // [kSortCap]
-  auto stageQ = [&](int s) { return sQd + (s * 2) * QT * PITCH; };
-  auto stageD = [&](int s) { return sQd + (s * 2 + 1) * QT * PITCH; };
+  const int blk = blockIdx.x / tiles_per_block, kt = blockIdx.x - blk * tiles_per_block;
+  const int h = blockIdx.y, b = blockIdx.z;
 
   const int64_t t0 = static_cast<int64_t>(blk) * p.block_size;
   const int n_blk = p.tab.on ? p.block_size : static_cast<int>(min64(p.block_size, p.kv.n_tokens - t0));  // tokens that exist
-  const int row_lo = kt * kTileRows;                        // first block row of this tile
-  const int n_rows = max(0, min(kTileRows, n_blk - row_lo)); // rows this tile owns
-  if (n_rows == 0) return;
+  const int row_lo = kt * TROWS;                                  // first block row of this tile
+  const int n_rows = min(TROWS, n_blk - row_lo);                  // rows this tile owns
+  if (n_rows <= 0) return;
   const int64_t tok0 = t0 + row_lo;
-  char* dk_base = p.dk + ((static_cast<int64_t>(b) * p.kv.n_tokens + tok0) * p.H + h) * D * ESZ;
-  char* dv_base = p.dv + ((static_cast<int64_t>(b) * p.kv.n_tokens + tok0) * p.H + h) * D * ESZ;
   const int64_t out_row_bytes = static_cast<int64_t>(p.H) * D * ESZ;
+  char* dk_base = p.dk + (static_cast<int64_t>(b) * p.kv.n_tokens + tok0) * out_row_bytes + h * D * ESZ;
+  char* dv_base = p.dv + (static_cast<int64_t>(b) * p.kv.n_tokens + tok0) * out_row_bytes + h * D * ESZ;
 
-  const int64_t row = static_cast<int64_t>(b) * p.H + h;
-  const int32_t* offs = p.offsets + row * (p.NS + 1);
+  const int64_t bh = static_cast<int64_t>(b) * p.H + h;
+  const int32_t* offs = p.offsets + bh * (p.NS + 1);
   const int beg = offs[blk], n_ent = offs[blk + 1] - beg;
-  const int32_t* bucket = p.groups + row * static_cast<int64_t>(p.MG) * p.T + beg;
+  const int32_t* bucket = p.groups + bh * p.MG * p.T + beg;
 
   BlockRef br{nullptr, nullptr, 0};
   float* fdk = nullptr;
@@ -483,7 +428,7 @@ __global__ void __launch_bounds__(128) sel_bwd_dkv_kernel(const BwdParams p, int
     br = resolve_block<ESZ>(p.kv, b, h, blk, D, p.block_size, 1, false, 0);
   }
   if (n_ent == 0 || br.k == nullptr) {
-    for (int i = threadIdx.x; i < n_rows * (D / 8); i += blockDim.x) {
+    for (int i = threadIdx.x; i < n_rows * (D / 8); i += 32 * TW) {
       const int r = i / (D / 8), c = i % (D / 8);
       *reinterpret_cast<uint4*>(dk_base + r * out_row_bytes + c * 16) = make_uint4(0, 0, 0, 0);
       *reinterpret_cast<uint4*>(dv_base + r * out_row_bytes + c * 16) = make_uint4(0, 0, 0, 0);
@@ -491,244 +436,222 @@ __global__ void __launch_bounds__(128) sel_bwd_dkv_kernel(const BwdParams p, int
     return;
   }
 
-  // bucket -> ascending group order (rank sort; duplicates keep their arrival order)
-  const bool sorted = n_ent <= kSortCap;
-  if (sorted) {
-    for (int i = threadIdx.x; i < n_ent; i += blockDim.x) s_tmp[i] = bucket[i];
-    __syncthreads();
-    for (int i = threadIdx.x; i < n_ent; i += blockDim.x) {
-      const int v = s_tmp[i];
-      int rank = 0;
-      for (int j = 0; j < n_ent; ++j) {
-        const int w = s_tmp[j];
-        rank += (w < v) || (w == v && j < i);
-      }
-      s_grp[rank] = v;
-    }
-    __syncthreads();
-  }
-  auto entry = [&](int i) { return sorted ? s_grp[i] : bucket[i]; };
+  const uint32_t k_tile = smem_u32(smem), v_tile = k_tile + kRingTile<D, TROWS>;
+  const uint32_t ring_mem = v_tile + kRingTile<D, TROWS>;
+  const uint32_t ring_bytes = static_cast<uint32_t>(stages) * 2 * kRingTile<D, 16>;
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + 2 * kRingTile<D, TROWS> + ring_bytes);
+  int* words = reinterpret_cast<int*>(bars + kRingBars);
+  const float* rows32 = reinterpret_cast<const float*>(words + 4);         // [stage][LSE, delta][16]
+  int4* list = reinterpret_cast<int4*>(words + 4 + stages * 32);           // [2 kList] tiles: group, first row, rows, visible tokens
 
-  const int spg = (p.G + QT - 1) / QT;      // query sub-tiles per group
-  const int n_items = n_ent * spg;
-  const int64_t k_row_bytes = p.tab.on ? p.tab.s_bn * ESZ : kv_row_bytes(p.kv, false, D, ESZ);
-  const int64_t v_row_bytes = p.tab.on ? p.tab.s_bn * ESZ : kv_row_bytes(p.kv, true, D, ESZ);
-
-  auto issue_item = [&](int it, int stg) {
-    const int g = entry(it / spg), sub = it % spg;
-    const int64_t m0 = static_cast<int64_t>(g) * p.G + sub * QT;
-    int nq = static_cast<int>(min64(p.G, p.M - static_cast<int64_t>(g) * p.G)) - sub * QT;
-    nq = max(0, min(QT, nq));
-    issue_rows<T, D, PITCH>(stageQ(stg), p.q + (b * p.q_sb + m0 * p.q_sm + h * p.q_sh) * ESZ,
-                            p.q_sm * ESZ, nq, QT);
-    issue_rows<T, D, PITCH>(stageD(stg), p.dO + (b * p.do_sb + m0 * p.do_sm + h * p.do_sh) * ESZ,
-                            p.do_sm * ESZ, nq, QT);
-    if (threadIdx.x < QT) {
-      const int r = threadIdx.x;
-      const int64_t at = (static_cast<int64_t>(b) * p.H + h) * p.M + m0 + r;
-      s_lse[stg * QT + r] = r < nq ? p.lse[at] * kLog2e : INFINITY;
-      s_delta[stg * QT + r] = r < nq ? p.delta[at] : 0.f;
+  const int subs = (p.G + 15) / 16;                         // ring tiles per group
+  Ring<D, 16, TMA, true> ring{ring_mem, bars, words, n_ent * subs, stages, warp, TW, p.lse, p.delta, smem_u32(rows32)};
+  if (threadIdx.x == 0) words[0] = 0;
+  ring.init();
+  // tiles [from, from + kList) of the bucket
+  const auto list_tiles = [&](int from) {
+    for (int i = from + threadIdx.x; i < from + kList && i < ring.count; i += 32 * TW) {
+      const int e = i / subs, r0 = (i - e * subs) * 16, g = bucket[e];
+      const int64_t g0 = static_cast<int64_t>(g) * p.G;
+      // rows of the tile (a short last group may leave one empty); rows of this block that the group may see
+      const int n = max(0, min(16, static_cast<int>(min64(p.G, p.M - g0)) - r0));
+      int vis = n_rows;
+      if (p.causal) vis = static_cast<int>(min64(vis, (g0 / p.chunk_size + 1) * p.chunk_size - tok0));
+      list[i % (2 * kList)] = make_int4(g, r0, n, n > 0 ? vis : 0);
     }
   };
+  list_tiles(0);
+  __syncthreads();
+  const RingSource src{&maps, p.q_sm * ESZ, p.do_sm * ESZ, h, b, p.G, static_cast<int>(p.M / p.G), p.B == 1};
+  const int64_t bhm = bh * p.M;
+  const auto tile_of = [&](int i) {
+    const int4 w = list[i % (2 * kList)];
+    RingTile t;
+    t.unit = w.x;
+    t.r0 = w.y;
+    t.n = t.clear = w.z;
+    const int64_t m = w.z > 0 ? static_cast<int64_t>(w.x) * p.G + w.y : 0;
+    t.aux = bhm + m;
+    if (!TMA) {
+      t.a = reinterpret_cast<uint64_t>(p.q + (b * p.q_sb + m * p.q_sm + h * p.q_sh) * ESZ);
+      t.b = reinterpret_cast<uint64_t>(p.dO + (b * p.do_sb + m * p.do_sm + h * p.do_sh) * ESZ);
+    }
+    return t;
+  };
+  ring.start(src, tile_of);
 
-  issue_rows<T, D, PITCH>(sK, br.k + row_lo * k_row_bytes, k_row_bytes, n_rows, kTileRows);
-  issue_rows<T, D, PITCH>(sV, br.v + row_lo * v_row_bytes, v_row_bytes, n_rows, kTileRows);
-  issue_item(0, 0);
-  cp_async_commit();
+  // this block's K and V rows
+  {
+    const int64_t k_row = p.tab.on ? p.tab.s_bn * ESZ : kv_row_bytes(p.kv, false, D, ESZ);
+    const int64_t v_row = p.tab.on ? p.tab.s_bn * ESZ : kv_row_bytes(p.kv, true, D, ESZ);
+    const char* k_src = br.k + row_lo * k_row;
+    const char* v_src = br.v + row_lo * v_row;
+#pragma unroll 4
+    for (int i = threadIdx.x; i < TROWS * (D / 8); i += 32 * TW) {
+      const int r = i / (D / 8), c = i % (D / 8), bytes = r < n_rows ? 16 : 0;
+      const int64_t at = r < n_rows ? r : 0;
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(k_tile + ring_at<TROWS>(r, c)), "l"(k_src + at * k_row + c * 16), "r"(bytes) : "memory");
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(v_tile + ring_at<TROWS>(r, c)), "l"(v_src + at * v_row + c * 16), "r"(bytes) : "memory");
+    }
+    cp_async_commit();
+    cp_async_wait<0>();
+  }
+  __syncthreads();
 
-  float dk[DN][4], dv[DN][4];
+  float dk[D / 8][4], dv[D / 8][4];
 #pragma unroll
-  for (int n = 0; n < DN; ++n) {
+  for (int n = 0; n < D / 8; ++n) {
     dk[n][0] = dk[n][1] = dk[n][2] = dk[n][3] = 0.f;
     dv[n][0] = dv[n][1] = dv[n][2] = dv[n][3] = 0.f;
   }
-  const T* ka = sK + (warp * 16 + (lane & 15)) * PITCH + (lane >> 4) * 8;
-  const T* va = sV + (warp * 16 + (lane & 15)) * PITCH + (lane >> 4) * 8;
-  const int nb_off = ((lane & 7) + ((lane >> 4) << 3)) * PITCH + ((lane >> 3) & 1) * 8;
-  const int tb_off = ((lane & 7) + ((lane >> 3) & 1) * 8) * PITCH + (lane >> 4) * 8;
-  const bool warp_active = warp * 16 < n_rows;
-
-  for (int it = 0; it < n_items; ++it) {
-    if (it + 1 < n_items) {
-      issue_item(it + 1, (it + 1) & 1);
-      cp_async_commit();
-      cp_async_wait<1>();
-    } else {
-      cp_async_wait<0>();
+  bool ok = true;
+  for (int i = 0; i < ring.count; ++i) {
+    if (i % kList == 0 && i + kList < ring.count) {           // the copies run at most `stages` tiles ahead
+      __syncthreads();
+      list_tiles(i + kList);
+      __syncthreads();
     }
-    __syncthreads();
-    const int g = entry(it / spg), sub = it % spg;
-    int nq = static_cast<int>(min64(p.G, p.M - static_cast<int64_t>(g) * p.G)) - sub * QT;
-    nq = max(0, min(QT, nq));
-    // rows of this tile the group may see (causal: prefix of the block)
-    int vis = n_blk;
-    if (p.causal) {
-      const int64_t qc = (static_cast<int64_t>(g) * p.G) / p.chunk_size;
-      vis = static_cast<int>(min64(vis, (qc + 1) * p.chunk_size - t0));
+    const int4 w = list[i % (2 * kList)];
+    const int n = w.z, vis = w.w - warp * 16;                 // query rows; visible rows among this warp's
+    ok = ok && ring.template wait<0>();
+    if (ok && vis > 0) {
+      const uint32_t qt = ring.tile(0), dt = ring.tile(1);
+      float st[2][4], dp[2][4];
+#pragma unroll
+      for (int j = 0; j < 2; ++j) {
+        st[j][0] = st[j][1] = st[j][2] = st[j][3] = 0.f;
+        dp[j][0] = dp[j][1] = dp[j][2] = dp[j][3] = 0.f;
+      }
+      mma_rows_t2<T, D, TROWS>(st, k_tile, qt, dp, v_tile, dt, warp * 16);
+      const float2* lse = reinterpret_cast<const float2*>(rows32 + ring.stage * 32) + t4;
+      uint32_t pa[1][4], ds[1][4];
+#pragma unroll
+      for (int j = 0; j < 2; ++j) {
+        const int q0 = 8 * j + 2 * t4;                         // this thread's columns: query rows q0, q0 + 1
+        const float2 l = lse[j * 4], dl = lse[8 + j * 4];
+        const float dls[2] = {dl.x, dl.y};
+        // rows past the group's end: exp2(-inf) = 0
+        const float l2[2] = {q0 < n ? l.x * kLog2e : INFINITY, q0 + 1 < n ? l.y * kLog2e : INFINITY};
+#pragma unroll
+        for (int y = 0; y < 4; ++y) {
+          st[j][y] = fast_exp2(st[j][y] * p.scale_log2 - l2[y & 1]);
+          if (gid + 8 * (y >> 1) >= vis) st[j][y] = 0.f;
+        }
+        pa[0][j * 2] = pack2<T>(st[j][0], st[j][1]);
+        pa[0][j * 2 + 1] = pack2<T>(st[j][2], st[j][3]);
+        const float2 p01 = unpack2<T>(pa[0][j * 2]), p23 = unpack2<T>(pa[0][j * 2 + 1]);
+        ds[0][j * 2] = pack2<T>(p01.x * (dp[j][0] - dls[0]) * p.scale, p01.y * (dp[j][1] - dls[1]) * p.scale);
+        ds[0][j * 2 + 1] = pack2<T>(p23.x * (dp[j][2] - dls[0]) * p.scale, p23.y * (dp[j][3] - dls[1]) * p.scale);
+      }
+      mma_rows<T, D, 16>(dv, pa, dt, 1);
+      mma_rows<T, D, 16>(dk, ds, qt, 1);
     }
-    const int nkv = max(0, min(kTileRows, vis - row_lo));
-    if (warp_active && nq > 0 && warp * 16 < nkv) {
-      const T* sQ = stageQ(it & 1);
-      const T* sD = stageD(it & 1);
-      const float* lse2 = s_lse + (it & 1) * QT;
-      const float* dlt = s_delta + (it & 1) * QT;
-      float st[8][4];
-#pragma unroll
-      for (int n = 0; n < 8; ++n) { st[n][0] = st[n][1] = st[n][2] = st[n][3] = 0.f; }
-#pragma unroll
-      for (int kk = 0; kk < KK; ++kk) {
-        uint32_t a[4];
-        ldmatrix_x4(a, ka + kk * 16);
-#pragma unroll
-        for (int n16 = 0; n16 < 4; ++n16) {
-          if (n16 * 16 < nq) {
-            uint32_t bf[4];
-            ldmatrix_x4(bf, sQ + nb_off + n16 * 16 * PITCH + kk * 16);
-            mma16816<T>(st[2 * n16], a, bf[0], bf[1]);
-            mma16816<T>(st[2 * n16 + 1], a, bf[2], bf[3]);
-          }
-        }
-      }
-      uint32_t pa[4][4];
-#pragma unroll
-      for (int n = 0; n < 8; ++n) {
-        float pe[4];
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const int krow = warp * 16 + gid + 8 * (e >> 1);
-          const int col = n * 8 + 2 * t4 + (e & 1);
-          pe[e] = (krow < nkv && col < nq) ? fast_exp2(st[n][e] * p.scale_log2 - lse2[col]) : 0.f;
-        }
-        pa[n >> 1][(n & 1) * 2] = pack2<T>(pe[0], pe[1]);
-        pa[n >> 1][(n & 1) * 2 + 1] = pack2<T>(pe[2], pe[3]);
-      }
-      // dV += P^T dO
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        if (j * 16 < nq) {
-#pragma unroll
-          for (int d16 = 0; d16 < D / 16; ++d16) {
-            uint32_t bf[4];
-            ldmatrix_x4_trans(bf, sD + tb_off + j * 16 * PITCH + d16 * 16);
-            mma16816<T>(dv[2 * d16], pa[j], bf[0], bf[1]);
-            mma16816<T>(dv[2 * d16 + 1], pa[j], bf[2], bf[3]);
-          }
-        }
-      }
-      // dP^T = V dO^T
-#pragma unroll
-      for (int n = 0; n < 8; ++n) { st[n][0] = st[n][1] = st[n][2] = st[n][3] = 0.f; }
-#pragma unroll
-      for (int kk = 0; kk < KK; ++kk) {
-        uint32_t a[4];
-        ldmatrix_x4(a, va + kk * 16);
-#pragma unroll
-        for (int n16 = 0; n16 < 4; ++n16) {
-          if (n16 * 16 < nq) {
-            uint32_t bf[4];
-            ldmatrix_x4(bf, sD + nb_off + n16 * 16 * PITCH + kk * 16);
-            mma16816<T>(st[2 * n16], a, bf[0], bf[1]);
-            mma16816<T>(st[2 * n16 + 1], a, bf[2], bf[3]);
-          }
-        }
-      }
-      // dS^T = P^T (dP^T - delta) scale, packed back into the same A fragments
-#pragma unroll
-      for (int n = 0; n < 8; ++n) {
-        const int col = n * 8 + 2 * t4;
-        const float d0 = dlt[col], d1 = dlt[col + 1];
-        const float2 p01 = unpack2<T>(pa[n >> 1][(n & 1) * 2]);
-        const float2 p23 = unpack2<T>(pa[n >> 1][(n & 1) * 2 + 1]);
-        pa[n >> 1][(n & 1) * 2] =
-            pack2<T>(p01.x * (st[n][0] - d0) * p.scale, p01.y * (st[n][1] - d1) * p.scale);
-        pa[n >> 1][(n & 1) * 2 + 1] =
-            pack2<T>(p23.x * (st[n][2] - d0) * p.scale, p23.y * (st[n][3] - d1) * p.scale);
-      }
-      // dK += dS^T Q
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        if (j * 16 < nq) {
-#pragma unroll
-          for (int d16 = 0; d16 < D / 16; ++d16) {
-            uint32_t bf[4];
-            ldmatrix_x4_trans(bf, sQ + tb_off + j * 16 * PITCH + d16 * 16);
-            mma16816<T>(dk[2 * d16], pa[j], bf[0], bf[1]);
-            mma16816<T>(dk[2 * d16 + 1], pa[j], bf[2], bf[3]);
-          }
-        }
-      }
-    }
-    __syncthreads();
+    ok = ok && ring.template release<1>(i, src, tile_of);
+    ring.step();
   }
+  if (!ok) atomicExch(status, NSA_ERR_CUDA);
 
-  if (warp_active) {
+  __syncthreads();                                           // K and V tiles are done with: they stage the rows
+  const int mine_rows = n_rows - warp * 16;
+  if (mine_rows <= 0) return;
+  if (p.tab.on) {
 #pragma unroll
     for (int r = 0; r < 2; ++r) {
-      const int krow = warp * 16 + gid + 8 * r;
-      if (krow < n_rows && p.tab.on) {
-        float* kr = fdk + static_cast<int64_t>(krow) * p.tab.s_dbn;
-        float* vr = fdv + static_cast<int64_t>(krow) * p.tab.s_dbn;
+      const int row = gid + 8 * r;
+      if (row < mine_rows) {
+        float* kr = fdk + static_cast<int64_t>(warp * 16 + row) * p.tab.s_dbn;
+        float* vr = fdv + static_cast<int64_t>(warp * 16 + row) * p.tab.s_dbn;
 #pragma unroll
-        for (int n = 0; n < DN; ++n) {
+        for (int n = 0; n < D / 8; ++n) {
           *reinterpret_cast<float2*>(kr + n * 8 + 2 * t4) = make_float2(dk[n][2 * r], dk[n][2 * r + 1]);
           *reinterpret_cast<float2*>(vr + n * 8 + 2 * t4) = make_float2(dv[n][2 * r], dv[n][2 * r + 1]);
         }
-      } else if (krow < n_rows) {
-        char* kr = dk_base + krow * out_row_bytes;
-        char* vr = dv_base + krow * out_row_bytes;
-#pragma unroll
-        for (int n = 0; n < DN; ++n) {
-          *reinterpret_cast<uint32_t*>(kr + (n * 8 + 2 * t4) * ESZ) = pack2<T>(dk[n][2 * r], dk[n][2 * r + 1]);
-          *reinterpret_cast<uint32_t*>(vr + (n * 8 + 2 * t4) * ESZ) = pack2<T>(dv[n][2 * r], dv[n][2 * r + 1]);
-        }
       }
     }
+    return;
   }
+  const uint32_t stage = k_tile + warp * 16 * (D * 2 + 16);
+  store_rows<T, D>(dk, 1.f, 1.f, stage, dk_base + warp * 16 * out_row_bytes, out_row_bytes, mine_rows);
+  __syncwarp();
+  store_rows<T, D>(dv, 1.f, 1.f, stage, dv_base + warp * 16 * out_row_bytes, out_row_bytes, mine_rows);
 }
 
-size_t dq_smem(int rows_pad, int D, int T) {
-  return static_cast<size_t>(4 * kTileRows + 2 * rows_pad) * (D + 8) * 2 + 2 * rows_pad * 4 +
-         slot_table_bytes(T);
-}
-size_t dkv_smem(int D) {
-  return static_cast<size_t>(2 * kTileRows + 4 * 64) * (D + 8) * 2 + 4 * 64 * 4 + 2 * kSortCap * 4;
-}
-
-template <typename T, int D>
-int launch_dq(const BwdParams& p, cudaStream_t stream) {
-  const int nw = cdiv(p.G, 16);
-  const size_t smem_q = dq_smem(nw * 16, D, p.T);
-  NSA_REQUIRE(smem_q <= 220 * 1024, NSA_ERR_UNSUPPORTED, "sel_bwd: T=%d needs too much shared memory", p.T);
-  NSA_CUDA_OK(cudaFuncSetAttribute(sel_bwd_dq_kernel<T, D>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   static_cast<int>(smem_q)));
-  sel_bwd_dq_kernel<T, D><<<dim3(p.MG, p.H, p.B), nw * 32, smem_q, stream>>>(p);
-  NSA_LAUNCH_OK("sel_bwd_dq_kernel");
+template <typename T, int D, int W, int KS, bool TMA>
+int launch_dq_rows(const RingMaps& maps, const BwdParams& p, int32_t* status, cudaStream_t stream) {
+  const int tiles = p.T * cdiv(p.block_size, 32);
+  constexpr int stages = W <= 2 ? 1 : 3;                    // as in the forward
+  static_assert(W * 16 * (D * 2 + 16) <= stages * 2 * kRingTile<D, 32>, "the epilogue stages its rows in the ring");
+  static_assert((KS - 1) * (D / 8 * 512) <= KS * 2 * kRingTile<D, 32>, "the partial results are summed in the ring");
+  const size_t smem = static_cast<size_t>(KS) * stages * 2 * kRingTile<D, 32> + KS * kRingBars * 8 + 16 +
+                      static_cast<size_t>(tiles) * sizeof(RingTile);
+  NSA_REQUIRE(smem <= 220 * 1024, NSA_ERR_UNSUPPORTED, "sel_bwd: T=%d needs too much shared memory", p.T);
+  auto kernel = sel_bwd_dq_rows_kernel<T, D, W, KS, TMA>;
+  NSA_CUDA_OK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
+  kernel<<<dim3(p.MG, p.H, p.B), 32 * W * KS, smem, stream>>>(maps, p, stages, status);
+  NSA_LAUNCH_OK("sel_bwd_dq_rows_kernel");
   return NSA_OK;
 }
 
+template <typename T, int D, bool TMA>
+int launch_dq_loader(const RingMaps& maps, const BwdParams& p, int32_t* st, cudaStream_t s) {
+  if (p.G <= 16) {
+    // as many warps per list as still fit the chip at once (see the forward)
+    const int64_t units = static_cast<int64_t>(p.MG) * p.H * p.B, room = 148 * (D == 128 ? 10 : 16);
+    if (units * 4 <= room) return launch_dq_rows<T, D, 1, 4, TMA>(maps, p, st, s);
+    if (units * 2 <= room) return launch_dq_rows<T, D, 1, 2, TMA>(maps, p, st, s);
+    return launch_dq_rows<T, D, 1, 1, TMA>(maps, p, st, s);
+  }
+  if (p.G <= 32) return launch_dq_rows<T, D, 2, 1, TMA>(maps, p, st, s);
+  if (p.G <= 64) return launch_dq_rows<T, D, 4, 1, TMA>(maps, p, st, s);
+  return launch_dq_rows<T, D, 8, 1, TMA>(maps, p, st, s);
+}
+
 template <typename T, int D>
-int launch_dkv(const BwdParams& p, cudaStream_t stream) {
-  const size_t smem_kv = dkv_smem(D);
-  NSA_CUDA_OK(cudaFuncSetAttribute(sel_bwd_dkv_kernel<T, D>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   static_cast<int>(smem_kv)));
-  const int tpb = cdiv(p.block_size, kTileRows);
+int launch_dq(const nsa_kv_source* kv, const BwdParams& p, int32_t* st, cudaStream_t s) {
+  RingMaps maps{};
+  return make_ring_maps(kv, p.B, p.H, D, p.block_size, 32, &maps) ? launch_dq_loader<T, D, true>(maps, p, st, s)
+                                                          : launch_dq_loader<T, D, false>(maps, p, st, s);
+}
+
+template <typename T, int D, int TW, bool TMA>
+int launch_dkv_rows(const RingMaps& maps, const BwdParams& p, int32_t* status, cudaStream_t stream) {
+  const int tpb = cdiv(p.block_size, 16 * TW);
+  constexpr int stages = TW == 2 && D == 128 ? 1 : 2;   // where registers leave the room (measured 971 / 1008 us at TW = 2, D = 128; 653 / 642 us at D = 64)
+  constexpr size_t smem = 2 * kRingTile<D, 16 * TW> + static_cast<size_t>(stages) * (2 * kRingTile<D, 16> + 128) + kRingBars * 8 + 16 + 2 * 64 * 16;
+  static_assert(TW * 16 * (D * 2 + 16) <= 2 * kRingTile<D, 16 * TW>, "the epilogue stages its rows in the K and V tiles");
   const int64_t nblk = p.NS * tpb;
   NSA_REQUIRE(nblk <= 0x7fffffff, NSA_ERR_INVALID, "sel_bwd: too many K/V tiles");
-  if (nblk > 0) {
-    sel_bwd_dkv_kernel<T, D><<<dim3(static_cast<unsigned>(nblk), p.H, p.B), 128, smem_kv, stream>>>(p, tpb);
-    NSA_LAUNCH_OK("sel_bwd_dkv_kernel");
-  }
+  if (nblk == 0) return NSA_OK;
+  auto kernel = sel_bwd_dkv_rows_kernel<T, D, TW, TMA>;
+  NSA_CUDA_OK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
+  kernel<<<dim3(static_cast<unsigned>(nblk), p.H, p.B), 32 * TW, smem, stream>>>(maps, p, tpb, stages, status);
+  NSA_LAUNCH_OK("sel_bwd_dkv_rows_kernel");
   return NSA_OK;
 }
 
-template <bool DQ>
-int dispatch_bwd(const BwdParams& p, int dtype, int D, cudaStream_t s) {
+template <typename T, int D>
+int launch_dkv(const BwdParams& p, int32_t* st, cudaStream_t s) {
+  const int64_t qs[3] = {p.q_sb, p.q_sm, p.q_sh}, ds[3] = {p.do_sb, p.do_sm, p.do_sh};
+  RingMaps maps{};
+  const bool tma = make_unit_maps(&maps.a, &maps.a_tail, p.q, qs, p.B, p.M, p.H, D, p.G, 16) &&
+                   make_unit_maps(&maps.b, &maps.b_tail, p.dO, ds, p.B, p.M, p.H, D, p.G, 16);
+  // a block of more than 32 tokens is one tile of four warps: its bucket's rows are fetched once, not per 32 tokens
+  if (p.block_size > 32)
+    return tma ? launch_dkv_rows<T, D, 4, true>(maps, p, st, s) : launch_dkv_rows<T, D, 4, false>(maps, p, st, s);
+  return tma ? launch_dkv_rows<T, D, 2, true>(maps, p, st, s) : launch_dkv_rows<T, D, 2, false>(maps, p, st, s);
+}
+
+// kv: the source of the dQ kernel's K/V; nullptr: dK / dV
+int dispatch_bwd(const nsa_kv_source* kv, const BwdParams& p, int dtype, int D, cudaStream_t s) {
+  int32_t* st = nullptr;
+  const int rc = device_status_address(&st);
+  if (rc) return rc;
   if (dtype == NSA_BF16) {
-    if (D == 128) return DQ ? launch_dq<__nv_bfloat16, 128>(p, s) : launch_dkv<__nv_bfloat16, 128>(p, s);
-    return DQ ? launch_dq<__nv_bfloat16, 64>(p, s) : launch_dkv<__nv_bfloat16, 64>(p, s);
+    if (D == 128) return kv ? launch_dq<__nv_bfloat16, 128>(kv, p, st, s) : launch_dkv<__nv_bfloat16, 128>(p, st, s);
+    return kv ? launch_dq<__nv_bfloat16, 64>(kv, p, st, s) : launch_dkv<__nv_bfloat16, 64>(p, st, s);
   }
-  if (D == 128) return DQ ? launch_dq<__half, 128>(p, s) : launch_dkv<__half, 128>(p, s);
-  return DQ ? launch_dq<__half, 64>(p, s) : launch_dkv<__half, 64>(p, s);
+  if (D == 128) return kv ? launch_dq<__half, 128>(kv, p, st, s) : launch_dkv<__half, 128>(p, st, s);
+  return kv ? launch_dq<__half, 64>(kv, p, st, s) : launch_dkv<__half, 64>(p, st, s);
 }
 
 int run_inverted_index(const IdxParams& ip, int32_t* groups, int32_t* offsets, int32_t* counts,
@@ -931,7 +854,7 @@ extern "C" int nsa_sel_bwd_dq_pds(const void* q, const int64_t q_stride[3], cons
   p.G = group_size; p.MG = static_cast<int>(cdiv64(M, group_size)); p.M = M;
   p.NS = cdiv64(kv->n_tokens, block_size);
   p.scale = scale; p.scale_log2 = scale * kLog2e;
-  return dispatch_bwd<true>(p, dtype, D, static_cast<cudaStream_t>(stream));
+  return dispatch_bwd(kv, p, dtype, D, static_cast<cudaStream_t>(stream));
 }
 
 extern "C" int nsa_sel_bwd_dkv(const void* q, const int64_t q_stride[3], const nsa_kv_source* kv,
@@ -997,7 +920,7 @@ extern "C" int nsa_sel_bwd_dkv_pds(const void* q, const int64_t q_stride[3], con
   p.B = B; p.H = H; p.T = T; p.block_size = block_size; p.chunk_size = chunk_size; p.causal = causal;
   p.G = group_size; p.MG = static_cast<int>(cdiv64(M, group_size)); p.M = M; p.NS = cdiv64(N, block_size);
   p.scale = scale; p.scale_log2 = scale * kLog2e;
-  return dispatch_bwd<false>(p, dtype, D, s);
+  return dispatch_bwd(nullptr, p, dtype, D, s);
 }
 
 extern "C" int nsa_sel_bwd_dkv_ptr(const void* q, const int64_t q_stride[3], const int64_t* base_k,
@@ -1048,7 +971,7 @@ extern "C" int nsa_sel_bwd_dkv_ptr(const void* q, const int64_t q_stride[3], con
   p.tab.in_chunk_kv_bytes = in_chunk_block_bytes_kv; p.tab.in_chunk_dkv_bytes = in_chunk_block_bytes_dkv;
   p.tab.blocks_per_chunk = blocks_per_chunk;
   p.tab.s_bn = stride_bn; p.tab.s_dbn = stride_dbn;
-  return dispatch_bwd<false>(p, dtype, D, static_cast<cudaStream_t>(stream));
+  return dispatch_bwd(nullptr, p, dtype, D, static_cast<cudaStream_t>(stream));
 }
 
 extern "C" int nsa_sel_bwd(const void* q, const int64_t q_stride[3], const nsa_kv_source* kv,

@@ -1,9 +1,8 @@
-// Selection attention forward, general geometry (any block size, group size <= 128,
-// D in {64, 128}, bf16 / fp16): one thread block per (batch, query group, head); each warp
-// owns 16 query rows; selected tokens are packed into 64-row K/V tiles that stream through a
-// two-stage cp.async ring; S = Q K^T and O += P V run on mma.sync m16n8k16 with fp32
-// accumulation and an online softmax in the exp2 domain.
-#include "sel_common.cuh"
+// Selection attention forward, general geometry (any block size, group size <= 128, D in {64, 128}, bf16 / fp16):
+// a thread block is one (batch, query group, head); each of its warps owns 16 query rows and all of them read the
+// same ring of K/V tiles (sel_rows.cuh); S = Q K^T and O += P V run on mma.sync m16n8k16 with fp32 accumulation
+// and an online softmax in the exp2 domain.
+#include "sel_rows.cuh"
 
 namespace nsa {
 namespace {
@@ -22,182 +21,206 @@ struct FwdParams {
   float scale_log2;
 };
 
-template <typename T, int D>
-__global__ void __launch_bounds__(256) sel_fwd_kernel(const FwdParams p) {
-  constexpr int PITCH = D + 8;
-  constexpr int ESZ = sizeof(T);
-  constexpr int KK = D / 16;     // k-steps of S = Q K^T
-  constexpr int DN = D / 8;      // n8 tiles of O
-  extern __shared__ __align__(16) char smem[];
-
-  const int g = blockIdx.x, h = blockIdx.y, b = blockIdx.z;
+// W warps of 16 query rows each share one ring; with W = 1 the tiles of the list may be dealt out to KS warps
+// with rings of their own, whose partial results are merged at the end (few groups on many SMs).
+// What bounds it for small groups: the gathered K/V rows, which every list fetches for itself, through the L2 to SM
+// path.  32760 queries x 12 heads, 15-query groups, 16 blocks of 30 tokens: 397 us = 16 TB/s of rows against the
+// 18 TB/s that bulk copies reach here (5911 us with one warp per 70 KB thread block, 124 TF -> 243 TF of products).
+// One K/V stage and 12 warps per SM: 397 us; two stages and 7 warps: 661 us; 16- or 32-byte loads straight into
+// fragments, no shared memory: 780 us.
+template <typename T, int D, int W, int KS, bool TMA>
+__global__ void __launch_bounds__(32 * W * KS) sel_fwd_rows_kernel(const __grid_constant__ RingMaps maps, const FwdParams p,
+                                                                   const int stages, int32_t* status) {
+  static_assert(W == 1 || KS == 1, "only single-warp groups are split");
+  constexpr int ESZ = sizeof(T), ROWS = 32;
+  extern __shared__ __align__(1024) uint8_t smem[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int gid = lane >> 2, t4 = lane & 3;
-  const int64_t m0 = static_cast<int64_t>(g) * p.G;
-  const int n_q = static_cast<int>(p.M - m0 < p.G ? p.M - m0 : p.G);
-  const int q_chunk = static_cast<int>(m0 / p.chunk_size);
+  const int g = blockIdx.x, h = blockIdx.y, b = blockIdx.z;
+  const int64_t g0 = static_cast<int64_t>(g) * p.G;
+  const int row_warp = W > 1 ? warp : 0, part = KS > 1 ? warp : 0;
+  const int n_q = static_cast<int>(p.M - g0 < p.G ? p.M - g0 : p.G) - row_warp * 16;   // rows of this warp (may be <= 0)
+  const int64_t m0 = g0 + row_warp * 16;
 
-  T* tiles = reinterpret_cast<T*>(smem);                       // [2][2][64][PITCH]
-  const SlotTable st = carve_slot_table(smem + 4 * kTileRows * PITCH * ESZ, p.T);
-  auto stageK = [&](int s) { return tiles + (s * 2) * kTileRows * PITCH; };
-  auto stageV = [&](int s) { return tiles + (s * 2 + 1) * kTileRows * PITCH; };
-
-  const int total = build_slot_table<ESZ>(st, p.kv, p.ids, b * p.i_sb + g * p.i_sg + h * p.i_sh, p.i_st,
-                                          p.T, b, h, D, p.block_size, p.chunk_size, p.causal != 0, q_chunk);
-
-  char* out_row0 = p.out + (b * p.o_sb + m0 * p.o_sm + h * p.o_sh) * ESZ;
-  float* lse_row0 = p.lse + (static_cast<int64_t>(b) * p.H + h) * p.M + m0;
-  if (total == 0) {  // no visible key: O = 0, LSE = -inf
-    for (int i = threadIdx.x; i < n_q * (D / 8); i += blockDim.x) {
-      const int r = i / (D / 8), c = i % (D / 8);
-      *reinterpret_cast<uint4*>(out_row0 + r * p.o_sm * ESZ + c * 16) = make_uint4(0, 0, 0, 0);
-    }
-    for (int r = threadIdx.x; r < n_q; r += blockDim.x) lse_row0[r] = -INFINITY;
-    return;
+  const uint32_t ring_bytes = static_cast<uint32_t>(stages) * 2 * kRingTile<D, ROWS>;
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + KS * ring_bytes);
+  int* words = reinterpret_cast<int*>(bars + KS * kRingBars);                          // abort, tile count
+  RingTile* list = reinterpret_cast<RingTile*>(words + 4);
+  if (warp == 0) {
+    const int count = ring_list<ESZ>(list, p.kv, p.ids, b * p.i_sb + g * p.i_sg + h * p.i_sh, p.i_st, p.T, b, h, D,
+                                     p.block_size, p.chunk_size, p.causal != 0, static_cast<int>(g0 / p.chunk_size));
+    if (lane == 0) { words[0] = 0; words[1] = count; }
   }
-
-  const int64_t k_row_bytes = kv_row_bytes(p.kv, false, D, ESZ);
-  const int64_t v_row_bytes = kv_row_bytes(p.kv, true, D, ESZ);
-  const char* q_base = p.q + (b * p.q_sb + m0 * p.q_sm + h * p.q_sh) * ESZ;
-  const int ntiles = (total + kTileRows - 1) / kTileRows;
-  const int rows_pad = (blockDim.x >> 5) * 16;
-
-  // Q goes through stage 1 (128 rows) while tile 0 lands in stage 0.
-  issue_rows<T, D, PITCH>(stageK(1), q_base, p.q_sm * ESZ, n_q, rows_pad);
-  cp_async_commit();
-  issue_kv_tile<T, D, PITCH>(stageK(0), stageV(0), st, p.T, 0, total, k_row_bytes, v_row_bytes, p.q);
-  cp_async_commit();
-  cp_async_wait<1>();
+  Ring<D, ROWS, TMA> ring{smem_u32(smem) + part * ring_bytes, bars + part * kRingBars, words,
+                        0, stages, row_warp, W};
+  ring.init();
   __syncthreads();
+  ring.count = KS > 1 ? (words[1] - part + KS - 1) / KS : words[1];
+  const RingSource src = kv_ring_source<ESZ>(p.kv, maps, p.B, b, h, D, p.block_size);
+  const auto tile_of = [&](int i) { return list[part + i * KS]; };
+  ring.start(src, tile_of);
 
-  uint32_t qf[KK][4];
-  {
-    const T* sQ = stageK(1) + (warp * 16 + (lane & 15)) * PITCH + (lane >> 4) * 8;
+  float o[D / 8][4];
 #pragma unroll
-    for (int kk = 0; kk < KK; ++kk) ldmatrix_x4(qf[kk], sQ + kk * 16);
-  }
-  __syncthreads();
+  for (int n = 0; n < D / 8; ++n) o[n][0] = o[n][1] = o[n][2] = o[n][3] = 0.f;
+  float m_ref[2] = {-INFINITY, -INFINITY}, l_i[2] = {0.f, 0.f};
+  uint32_t q[D / 16][4];
+  load_a_frag<D>(q, p.q + (b * p.q_sb + m0 * p.q_sm + h * p.q_sh) * ESZ, p.q_sm * ESZ, n_q);
 
-  float o[DN][4];
+  bool ok = true;
+  for (int i = 0; i < ring.count && ok; ++i) {
+    const int n = list[part + i * KS].n, brought = list[part + i * KS].clear;
+    if (!ring.template wait<0>()) { ok = false; break; }
+    const int n16 = (n + 15) >> 4;
+    float s[4][4];
 #pragma unroll
-  for (int n = 0; n < DN; ++n) { o[n][0] = o[n][1] = o[n][2] = o[n][3] = 0.f; }
-  float m_i[2] = {-INFINITY, -INFINITY};
-  float l_i[2] = {0.f, 0.f};
-  const bool warp_active = warp * 16 < n_q;
-
-  for (int i = 0; i < ntiles; ++i) {
-    if (i + 1 < ntiles) {
-      issue_kv_tile<T, D, PITCH>(stageK((i + 1) & 1), stageV((i + 1) & 1), st, p.T,
-                                 (i + 1) * kTileRows, total, k_row_bytes, v_row_bytes, p.q);
-      cp_async_commit();
-      cp_async_wait<1>();
-    } else {
-      cp_async_wait<0>();
+    for (int j = 0; j < 4; ++j) s[j][0] = s[j][1] = s[j][2] = s[j][3] = 0.f;
+    mma_rows_t<T, D, ROWS>(s, q, ring.tile(0), n16);
+    ok = ring.template release<0>(i, src, tile_of);
+    if (n < ROWS) {
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+          if (8 * j + 2 * t4 + (e & 1) >= n) s[j][e] = -INFINITY;
     }
-    __syncthreads();
-    if (warp_active) {
-      const T* sK = stageK(i & 1);
-      const T* sV = stageV(i & 1);
-      const int nvalid = min(kTileRows, total - i * kTileRows);
-      float s[8][4];
-#pragma unroll
-      for (int n = 0; n < 8; ++n) { s[n][0] = s[n][1] = s[n][2] = s[n][3] = 0.f; }
-      const T* kb = sK + ((lane & 7) + ((lane >> 4) << 3)) * PITCH + ((lane >> 3) & 1) * 8;
-#pragma unroll
-      for (int kk = 0; kk < KK; ++kk) {
-#pragma unroll
-        for (int n16 = 0; n16 < 4; ++n16) {
-          if (n16 * 16 < nvalid) {
-            uint32_t bf[4];
-            ldmatrix_x4(bf, kb + n16 * 16 * PITCH + kk * 16);
-            mma16816<T>(s[2 * n16], qf[kk], bf[0], bf[1]);
-            mma16816<T>(s[2 * n16 + 1], qf[kk], bf[2], bf[3]);
-          }
-        }
-      }
-      // mask + online softmax (rows gid and gid + 8), exp2 domain
-      float mx[2] = {-INFINITY, -INFINITY};
-#pragma unroll
-      for (int n = 0; n < 8; ++n) {
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const int col = n * 8 + 2 * t4 + (e & 1);
-          const float v = (col < nvalid) ? s[n][e] * p.scale_log2 : -INFINITY;
-          s[n][e] = v;
-          mx[e >> 1] = fmaxf(mx[e >> 1], v);
-        }
-      }
-#pragma unroll
-      for (int r = 0; r < 2; ++r) {
-        mx[r] = fmaxf(mx[r], __shfl_xor_sync(0xffffffffu, mx[r], 1));
-        mx[r] = fmaxf(mx[r], __shfl_xor_sync(0xffffffffu, mx[r], 2));
-        const float m_new = fmaxf(m_i[r], mx[r]);   // finite: every tile has a valid column
-        const float corr = fast_exp2(m_i[r] - m_new);
-        m_i[r] = m_new;
-        l_i[r] *= corr;
-#pragma unroll
-        for (int n = 0; n < DN; ++n) { o[n][2 * r] *= corr; o[n][2 * r + 1] *= corr; }
-      }
-      uint32_t pa[4][4];
-#pragma unroll
-      for (int n = 0; n < 8; ++n) {
-        const float p0 = fast_exp2(s[n][0] - m_i[0]);
-        const float p1 = fast_exp2(s[n][1] - m_i[0]);
-        const float p2 = fast_exp2(s[n][2] - m_i[1]);
-        const float p3 = fast_exp2(s[n][3] - m_i[1]);
-        l_i[0] += p0 + p1;
-        l_i[1] += p2 + p3;
-        pa[n >> 1][(n & 1) * 2] = pack2<T>(p0, p1);
-        pa[n >> 1][(n & 1) * 2 + 1] = pack2<T>(p2, p3);
-      }
-      const T* vb = sV + ((lane & 7) + ((lane >> 3) & 1) * 8) * PITCH + (lane >> 4) * 8;
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        if (j * 16 < nvalid) {
-#pragma unroll
-          for (int d16 = 0; d16 < D / 16; ++d16) {
-            uint32_t bf[4];
-            ldmatrix_x4_trans(bf, vb + j * 16 * PITCH + d16 * 16);
-            mma16816<T>(o[2 * d16], pa[j], bf[0], bf[1]);
-            mma16816<T>(o[2 * d16 + 1], pa[j], bf[2], bf[3]);
-          }
-        }
-      }
-    }
-    __syncthreads();
-  }
-
-  if (warp_active) {
+    float mx[2];
 #pragma unroll
     for (int r = 0; r < 2; ++r) {
-      l_i[r] += __shfl_xor_sync(0xffffffffu, l_i[r], 1);
-      l_i[r] += __shfl_xor_sync(0xffffffffu, l_i[r], 2);
-      const int row = warp * 16 + gid + 8 * r;
-      if (row < n_q) {
-        const float inv = l_i[r] > 0.f ? 1.f / l_i[r] : 0.f;
-        char* orow = out_row0 + row * p.o_sm * ESZ;
+      mx[r] = -INFINITY;
 #pragma unroll
-        for (int n = 0; n < DN; ++n)
-          *reinterpret_cast<uint32_t*>(orow + (n * 8 + 2 * t4) * ESZ) =
-              pack2<T>(o[n][2 * r] * inv, o[n][2 * r + 1] * inv);
-        if (t4 == 0)
-          lse_row0[row] = l_i[r] > 0.f ? (m_i[r] + log2f(l_i[r])) * kLn2 : -INFINITY;
+      for (int j = 0; j < 4; ++j) mx[r] = fmaxf(mx[r], fmaxf(s[j][2 * r], s[j][2 * r + 1]) * p.scale_log2);
+      mx[r] = fmaxf(mx[r], __shfl_xor_sync(0xffffffffu, mx[r], 1));
+      mx[r] = fmaxf(mx[r], __shfl_xor_sync(0xffffffffu, mx[r], 2));
+    }
+    // the accumulator is rescaled only when a maximum has grown by more than 2^8 (and in the first step)
+    if (__any_sync(0xffffffffu, mx[0] > m_ref[0] + 8.f || mx[1] > m_ref[1] + 8.f)) {
+#pragma unroll
+      for (int r = 0; r < 2; ++r) {
+        const float m_new = fmaxf(m_ref[r], mx[r]);
+        const float corr = fast_exp2(m_ref[r] - m_new);
+        m_ref[r] = m_new;
+        l_i[r] *= corr;
+#pragma unroll
+        for (int d = 0; d < D / 8; ++d) { o[d][2 * r] *= corr; o[d][2 * r + 1] *= corr; }
       }
     }
+    uint32_t pa[2][4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      float e[4];
+#pragma unroll
+      for (int x = 0; x < 4; ++x) e[x] = fast_exp2(s[j][x] * p.scale_log2 - m_ref[x >> 1]);
+      l_i[0] += e[0] + e[1];
+      l_i[1] += e[2] + e[3];
+      pa[j >> 1][(j & 1) * 2] = pack2<T>(e[0], e[1]);
+      pa[j >> 1][(j & 1) * 2 + 1] = pack2<T>(e[2], e[3]);
+    }
+    ok = ring.template wait<1>() && ok;
+    if (!ok) break;
+    if (TMA && n < brought) ring_clear_rows<D, ROWS>(ring.tile(1), n, brought);
+    mma_rows<T, D, ROWS>(o, pa, ring.tile(1), n16);
+    if (TMA && n < brought) fence_async_shared();            // the cleared rows before the next copy into this tile
+    ok = ring.template release<1>(i, src, tile_of);
+    ring.step();
+  }
+  if (!ok) atomicExch(status, NSA_ERR_CUDA);
+
+#pragma unroll
+  for (int r = 0; r < 2; ++r) {
+    l_i[r] += __shfl_xor_sync(0xffffffffu, l_i[r], 1);
+    l_i[r] += __shfl_xor_sync(0xffffffffu, l_i[r], 2);
+  }
+  __syncthreads();                                        // the rings are done with: their memory stages what follows
+  if constexpr (KS > 1) {
+    // partial sums of warps 1 .. KS - 1 in fragment order: [D / 8][32 lanes] float4, then maxima and sums
+    float* part_mem = reinterpret_cast<float*>(smem) + (warp - 1) * (D / 8 * 128 + 128);
+    if (warp > 0) {
+#pragma unroll
+      for (int n = 0; n < D / 8; ++n)
+        reinterpret_cast<float4*>(part_mem)[n * 32 + lane] = make_float4(o[n][0], o[n][1], o[n][2], o[n][3]);
+      reinterpret_cast<float4*>(part_mem + D / 8 * 128)[lane] = make_float4(m_ref[0], m_ref[1], l_i[0], l_i[1]);
+    }
+    __syncthreads();
+    if (warp > 0) return;
+    for (int k = 0; k < KS - 1; ++k) {
+      const float* from = reinterpret_cast<const float*>(smem) + k * (D / 8 * 128 + 128);
+      const float4 ml = reinterpret_cast<const float4*>(from + D / 8 * 128)[lane];
+      const float m_new[2] = {fmaxf(m_ref[0], ml.x), fmaxf(m_ref[1], ml.y)};
+      float mine[2], theirs[2];
+#pragma unroll
+      for (int r = 0; r < 2; ++r) {
+        const float m = m_new[r] == -INFINITY ? 0.f : m_new[r];   // neither part saw a key: all sums are 0
+        mine[r] = fast_exp2(m_ref[r] - m);
+        theirs[r] = fast_exp2((r ? ml.y : ml.x) - m);
+        l_i[r] = l_i[r] * mine[r] + (r ? ml.w : ml.z) * theirs[r];
+        m_ref[r] = m_new[r];
+      }
+#pragma unroll
+      for (int n = 0; n < D / 8; ++n) {
+        const float4 x = reinterpret_cast<const float4*>(from)[n * 32 + lane];
+        o[n][0] = o[n][0] * mine[0] + x.x * theirs[0];
+        o[n][1] = o[n][1] * mine[0] + x.y * theirs[0];
+        o[n][2] = o[n][2] * mine[1] + x.z * theirs[1];
+        o[n][3] = o[n][3] * mine[1] + x.w * theirs[1];
+      }
+    }
+    __syncwarp();
+  }
+  if (n_q <= 0) return;
+  const float inv[2] = {l_i[0] > 0.f ? 1.f / l_i[0] : 0.f, l_i[1] > 0.f ? 1.f / l_i[1] : 0.f};
+  store_rows<T, D>(o, inv[0], inv[1], smem_u32(smem) + row_warp * 16 * (D * 2 + 16),
+                   p.out + (b * p.o_sb + m0 * p.o_sm + h * p.o_sh) * ESZ, p.o_sm * ESZ, n_q);
+  if (t4 == 0) {
+    float* lse = p.lse + (static_cast<int64_t>(b) * p.H + h) * p.M + m0;
+#pragma unroll
+    for (int r = 0; r < 2; ++r)
+      if (gid + 8 * r < n_q) lse[gid + 8 * r] = l_i[r] > 0.f ? (m_ref[r] + log2f(l_i[r])) * kLn2 : -INFINITY;
   }
 }
 
-template <typename T, int D>
-int launch(const FwdParams& p, int MG, cudaStream_t stream) {
-  const int nw = cdiv(p.G, 16);
-  const size_t smem = 4 * kTileRows * (D + 8) * sizeof(T) + slot_table_bytes(p.T);
-  NSA_REQUIRE(smem <= 200 * 1024, NSA_ERR_UNSUPPORTED, "sel_fwd: T=%d needs too much shared memory", p.T);
-  NSA_CUDA_OK(cudaFuncSetAttribute(sel_fwd_kernel<T, D>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   static_cast<int>(smem)));
-  dim3 grid(MG, p.H, p.B);
-  sel_fwd_kernel<T, D><<<grid, nw * 32, smem, stream>>>(p);
-  NSA_LAUNCH_OK("sel_fwd_kernel");
+template <typename T, int D, int W, int KS, bool TMA>
+int launch_rows(const RingMaps& maps, const FwdParams& p, int MG, int32_t* status, cudaStream_t stream) {
+  const int tiles = p.T * cdiv(p.block_size, 32);
+  // stages: two per ring of a single warp (the thread blocks that share an SM are the depth), three where several
+  // warps wait for the same ring; never less than the epilogue's staging needs
+  const int stages = W <= 2 ? 1 : 3;
+  static_assert(W * 16 * (D * 2 + 16) <= (W <= 2 ? 1 : 3) * 2 * kRingTile<D, 32>, "the epilogue stages its rows in the ring");
+  static_assert((KS - 1) * (D / 8 * 128 + 128) * 4 <= KS * 2 * kRingTile<D, 32>, "the partial results are merged in the ring");
+  const size_t smem = static_cast<size_t>(KS) * stages * 2 * kRingTile<D, 32> + KS * kRingBars * 8 + 16 +
+                      static_cast<size_t>(tiles) * sizeof(RingTile);
+  NSA_REQUIRE(smem <= 220 * 1024, NSA_ERR_UNSUPPORTED, "sel_fwd: T=%d needs too much shared memory", p.T);
+  auto kernel = sel_fwd_rows_kernel<T, D, W, KS, TMA>;
+  NSA_CUDA_OK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
+  kernel<<<dim3(MG, p.H, p.B), 32 * W * KS, smem, stream>>>(maps, p, stages, status);
+  NSA_LAUNCH_OK("sel_fwd_rows_kernel");
   return NSA_OK;
+}
+
+template <typename T, int D, bool TMA>
+int launch_loader(const RingMaps& maps, const FwdParams& p, int MG, int32_t* st, cudaStream_t s) {
+  if (p.G <= 16) {
+    // as many warps per list as still fit the chip at once: 12 warps per SM at D = 128 (registers), 16 at D = 64.
+    // Measured, D = 128, 16 blocks of 30, one / two / four warps per list: 384 lists 22.7 / 18.5 / 15.5 us,
+    // 768 lists 25.9 / 23.0 / 28.0 us, 1248 lists 31.6 / 40.8 / 41.0 us
+    const int64_t units = static_cast<int64_t>(MG) * p.H * p.B, room = 148 * (D == 128 ? 12 : 16);
+    if (units * 4 <= room) return launch_rows<T, D, 1, 4, TMA>(maps, p, MG, st, s);
+    if (units * 2 <= room) return launch_rows<T, D, 1, 2, TMA>(maps, p, MG, st, s);
+    return launch_rows<T, D, 1, 1, TMA>(maps, p, MG, st, s);
+  }
+  if (p.G <= 32) return launch_rows<T, D, 2, 1, TMA>(maps, p, MG, st, s);
+  if (p.G <= 64) return launch_rows<T, D, 4, 1, TMA>(maps, p, MG, st, s);
+  return launch_rows<T, D, 8, 1, TMA>(maps, p, MG, st, s);
+}
+
+template <typename T, int D>
+int launch(const nsa_kv_source* kv, const FwdParams& p, int MG, cudaStream_t s) {
+  int32_t* st = nullptr;
+  int rc = device_status_address(&st);
+  if (rc) return rc;
+  RingMaps maps{};
+  return make_ring_maps(kv, p.B, p.H, D, p.block_size, 32, &maps) ? launch_loader<T, D, true>(maps, p, MG, st, s)
+                                                              : launch_loader<T, D, false>(maps, p, MG, st, s);
 }
 
 }  // namespace
@@ -313,11 +336,11 @@ extern "C" int nsa_sel_fwd(const void* q, const int64_t q_stride[3], const nsa_k
     if (launched) return NSA_OK;
   }
   if (dtype == NSA_BF16) {
-    return D == 128 ? launch<__nv_bfloat16, 128>(p, static_cast<int>(MG), s)
-                    : launch<__nv_bfloat16, 64>(p, static_cast<int>(MG), s);
+    return D == 128 ? launch<__nv_bfloat16, 128>(kv, p, static_cast<int>(MG), s)
+                    : launch<__nv_bfloat16, 64>(kv, p, static_cast<int>(MG), s);
   }
-  return D == 128 ? launch<__half, 128>(p, static_cast<int>(MG), s)
-                  : launch<__half, 64>(p, static_cast<int>(MG), s);
+  return D == 128 ? launch<__half, 128>(kv, p, static_cast<int>(MG), s)
+                  : launch<__half, 64>(kv, p, static_cast<int>(MG), s);
 }
 
 extern "C" size_t nsa_range_fwd_workspace_bytes(int32_t B, int64_t M, int32_t H, int32_t D, int32_t n_blocks) {

@@ -18,7 +18,7 @@
 // 2^8 (the reference maximum is otherwise kept, which is exact because P and the row sum use the
 // same reference).  The epilogue normalises the O fragments, stages them with stmatrix in the dead
 // Q tile and writes them with TMA tile stores whose box holds one group's rows.
-#include "sel_common.cuh"
+#include "sel_rows.cuh"
 #include "tc_common.cuh"
 
 #include <cstdlib>
@@ -41,17 +41,21 @@ EncodeTiledFn encode_tiled_fn() {
   return fn;
 }
 
-int make_bf16_map(CUtensorMap* map, const void* base, int rank, const uint64_t* dims, const uint64_t* strides_bytes,
-                  const uint32_t* box) {
+CUresult encode_16bit_map(CUtensorMap* map, const void* base, int rank, const uint64_t* dims, const uint64_t* strides_bytes,
+                          const uint32_t* box) {
   EncodeTiledFn enc = encode_tiled_fn();
-  NSA_REQUIRE(enc != nullptr, NSA_ERR_CUDA, "cuTensorMapEncodeTiled is not available from the driver");
   cuuint64_t d[5], s[4];
   cuuint32_t bx[5], es[5];
   for (int i = 0; i < rank; ++i) { d[i] = dims[i]; bx[i] = box[i]; es[i] = 1; }
   for (int i = 0; i + 1 < rank; ++i) s[i] = strides_bytes[i];
-  const CUresult r = enc(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, rank, const_cast<void*>(base), d, s, bx, es,
-                         CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                         CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  return enc(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, rank, const_cast<void*>(base), d, s, bx, es,
+             CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+}
+int make_bf16_map(CUtensorMap* map, const void* base, int rank, const uint64_t* dims, const uint64_t* strides_bytes,
+                  const uint32_t* box) {
+  NSA_REQUIRE(encode_tiled_fn() != nullptr, NSA_ERR_CUDA, "cuTensorMapEncodeTiled is not available from the driver");
+  const CUresult r = encode_16bit_map(map, base, rank, dims, strides_bytes, box);
   NSA_REQUIRE(r == CUDA_SUCCESS, NSA_ERR_CUDA, "cuTensorMapEncodeTiled failed with code %d", static_cast<int>(r));
   return NSA_OK;
 }
@@ -510,6 +514,38 @@ int make_tile_maps(const void* q, const int64_t* q_stride, const nsa_kv_source* 
     if ((rc = tc::make_bf16_map(mapV, kv->v, 3, dims, st, box))) return rc;
   }
   return NSA_OK;
+}
+
+// Maps of the row kernels' rings (sel_rows.cuh): (column, head, row of the unit, unit, half or batch).  With one batch
+// element the last dimension is the 64-column half, so that one copy brings whole rows.  fp16 travels as bf16: a copy
+// does not look at the values.
+static bool unit_map(CUtensorMap* map, const void* base, int64_t head_stride, int64_t row_stride, int64_t batch_stride, int B,
+                     int H, int D, int64_t unit_rows, int64_t units, int rows) {
+  // a dimension of size 1 may carry any stride; the map wants a positive multiple of 16 bytes
+  auto st = [](int64_t s, int64_t size) { return size > 1 ? static_cast<uint64_t>(s) * 2 : 128ull; };
+  if (encode_tiled_fn() == nullptr || unit_rows <= 0 || units <= 0 || unit_rows > 0x7fffffff || units > 0x7fffffff) return false;
+  if ((H > 1 && head_stride <= 0) || (unit_rows * units > 1 && row_stride <= 0) || (B > 1 && batch_stride <= 0)) return false;
+  const uint64_t dims[5] = {static_cast<uint64_t>(B > 1 ? D : 64), static_cast<uint64_t>(H), static_cast<uint64_t>(unit_rows),
+                            static_cast<uint64_t>(units), static_cast<uint64_t>(B > 1 ? B : D / 64)};
+  const uint64_t s[4] = {st(head_stride, H), st(row_stride, unit_rows), st(row_stride * unit_rows, units),
+                         B > 1 ? static_cast<uint64_t>(batch_stride) * 2 : 128ull};
+  const uint32_t bx[5] = {64, 1, static_cast<uint32_t>(rows), 1, static_cast<uint32_t>(B > 1 ? 1 : D / 64)};
+  return tc::encode_16bit_map(map, base, 5, dims, s, bx) == CUDA_SUCCESS;
+}
+bool make_unit_maps(CUtensorMap* whole, CUtensorMap* tail, const void* base, const int64_t* stride, int B, int64_t N, int H,
+                    int D, int unit, int rows) {
+  if (N > 0x7fffffff) return false;
+  return (N / unit == 0 || unit_map(whole, base, stride[2], stride[1], stride[0], B, H, D, unit, N / unit, rows)) &&
+         (N % unit == 0 || unit_map(tail, base, stride[2], stride[1], stride[0], B, H, D, N, 1, rows));
+}
+bool make_ring_maps(const nsa_kv_source* kv, int B, int H, int D, int unit, int rows, RingMaps* m) {
+  if (kv->mode == NSA_KV_PAGED) {
+    const int64_t pages = kv->num_pages > 0 ? kv->num_pages : (1ll << 31) / unit;
+    return unit_map(&m->a, kv->k, 0, D, 0, 1, 1, D, unit, pages, rows) && unit_map(&m->b, kv->v, 0, D, 0, 1, 1, D, unit, pages, rows);
+  }
+  return kv->mode == NSA_KV_DENSE &&
+         make_unit_maps(&m->a, &m->a_tail, kv->k, kv->k_stride, B, kv->n_tokens, H, D, unit, rows) &&
+         make_unit_maps(&m->b, &m->b_tail, kv->v, kv->v_stride, B, kv->n_tokens, H, D, unit, rows);
 }
 
 // 4-D map of a [B,M,H,128] bf16 tensor whose box holds `box_rows` rows of one head (64 columns):
