@@ -164,6 +164,11 @@ int nsa_select_blocks(const void* q, const int64_t q_stride[3], const void* k,
  * the reference (it has no multi-GPU mode for this path). */
 int nsa_local_block_ids(const int32_t* ids, int64_t n, int32_t R, int32_t r, int32_t* out, void* stream);
 
+/* *flag = 1 if any of the n ids is >= limit (else it is left alone).  `flag` may be mapped pinned host
+ * memory: the host reads it once the launch has completed, with no copy (the range check of the
+ * reference's facade, nsa/ops/selection/__init__.py:36-44). */
+int nsa_check_block_ids(const int32_t* ids, int64_t n, int32_t limit, int32_t* flag, void* stream);
+
 /* Merge R candidate lists (idx/scores [R][rows][T], global ids) into the global top-k with
  * the same order rule.  New for block-sharded KV; the order rule is topk.cu:100-102 and the
  * packed-key merge it mirrors is topk.cu:442-471. */
@@ -327,6 +332,11 @@ int nsa_merge_packed_rows(const void* parts, int32_t R, int64_t rows, int32_t H,
  * Products and partial sums are rounded to `dtype` left to right, as the eager expression does. */
 int nsa_gate_combine(const void* g_logits, const void* o_cmp, const void* o_slc, const void* o_swa,
                      void* x, int64_t rows, int32_t D, int32_t softmax, int32_t dtype, void* stream);
+/* The same with the logits of token t's head h at g_logits + t * g_token_stride + h * 3 (elements): a
+ * view into a wider projection. */
+int nsa_gate_combine_strided(const void* g_logits, int64_t g_token_stride, const void* o_cmp, const void* o_slc,
+                             const void* o_swa, void* x, int64_t tokens, int32_t H, int32_t D, int32_t softmax,
+                             int32_t dtype, void* stream);
 /* Backward of nsa_gate_combine: d_o_i = g_i * dx (NULL = not wanted), d_g_logits [rows, 3]
  * (zero where a logit lies outside [-10, 10]).  D = 64, 128 or 256. */
 int nsa_gate_combine_bwd(const void* g_logits, const void* o_cmp, const void* o_slc,
@@ -419,6 +429,11 @@ int nsa_rope_apply(const void* x, const int64_t x_stride[2], int64_t S, int32_t 
  * Replaces dedup_run (block_kv_dedup.cu:16-120; block_kv_ops.h:26-31) and the host LRU touch
  * loop of nsa/ops/selection/padded_ptr/wrapper.py:253-362. */
 size_t nsa_cache_dedup_workspace_bytes(int64_t n_keys);
+/* The LRU touch alone, without the lists: same stamps and counters as nsa_cache_dedup_touch with a
+ * block table (ids [..,H,T], bpc == max_blocks), in one pass over the ids. */
+int nsa_cache_touch(const int32_t* block_indices, int64_t n_entries, int32_t H, int32_t T, int32_t max_blocks,
+                    int32_t* stamp, int32_t epoch, const int32_t* block_table, int64_t* page_stamp, int64_t epoch64,
+                    int64_t* counters, void* stream);
 int nsa_cache_dedup_touch(const int32_t* block_indices, int64_t n_entries, int32_t H, int32_t T,
                           int32_t max_blocks, int32_t bpc, int32_t* stamp, int32_t epoch32,
                           const int32_t* block_table, int64_t* page_stamp, int64_t epoch,
@@ -459,6 +474,27 @@ int nsa_cache_move_pages(int32_t direction, const int32_t* pages, const int32_t*
                          int64_t page_bytes, void* host_k, void* host_v, int32_t* block_table,
                          int32_t* page_owner, int64_t* page_stamp, int64_t epoch, int64_t* counters,
                          void* stream);
+
+/* One stop of a transformer layer's residual stream, rows of d elements (bf16 / fp16, d <= 2048):
+ *   x' = x                                  (y == NULL)
+ *   x' = x + y                              (no gate vector)
+ *   x' = x + (y * (gate_mod + gate_e))      (products and sums rounded to dtype, as the eager tensors are)
+ *   h  = norm(x') * (1 + scale) + shift     (modulated != 0), or norm(x') * scale + shift
+ * norm: layer norm in fp32; scale = scale_mod + scale_e and shift likewise, *_mod [d] in dtype and *_e [d]
+ * fp32, either NULL.  x' goes to x_out (with y), h to h_out (NULL: residual only).
+ * (causal_wan_nsa_model.py, the block's modulated norms and gated residuals around its sub-layers.) */
+int nsa_residual_norm(const void* x, const void* y, const void* gate_mod, const float* gate_e,
+                      const void* scale_mod, const float* scale_e, const void* shift_mod, const float* shift_e,
+                      int32_t modulated, void* x_out, void* h_out, int64_t rows, int32_t d, float eps,
+                      int32_t dtype, void* stream);
+/* x * rsqrt(mean(x^2) + eps) * weight over rows of d elements, fp32 inside; out contiguous. */
+int nsa_rms_rows(const void* x, int64_t row_stride, const void* weight, void* out, int64_t rows, int32_t d,
+                 float eps, int32_t dtype, void* stream);
+/* nsa_rms_rows over the H*D elements of every token of q and of k, rounded, then the rotary embedding of
+ * nsa_rope_apply: q, k rows row_stride elements apart -> q_out, k_out [S,H,D] contiguous. */
+int nsa_qk_norm_rope(const void* q, const void* k, int64_t row_stride, const void* q_weight, const void* k_weight,
+                     float eps, int64_t S, int32_t H, int32_t D, void* q_out, void* k_out, const nsa_rope* rope,
+                     int32_t dtype, void* stream);
 
 /* The reference's K1 and K2 entry points with their own contracts (block_kv_ops.h:12-24):
  * desc int64 SoA [src_k|src_v|dst_k|dst_v|pub_k|pub_v] x n_fetch then clear x n_clear;

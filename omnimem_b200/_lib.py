@@ -89,12 +89,14 @@ PROTOTYPES = {
     "nsa_sel_bwd_dkv_pds": (_i32, [_vp, _S3, C.POINTER(KVSource), _vp, _vp, _vp, _vp, _sz, _vp, _vp, _vp, _S3, _vp, _vp,
                                    _i32, _i64, _i32, _i32, _i32, _i32, _i32, _i32, _i32, _f32, _vp, _sz, _i32, _vp]),
     "nsa_local_block_ids": (_i32, [_vp, _i64, _i32, _i32, _vp, _vp]),
+    "nsa_check_block_ids": (_i32, [_vp, _i64, _i32, _vp, _vp]),
     "nsa_merge_partials": (_i32, [_vp, _vp, _i32, _i32, _i64, _i32, _i32, _vp, _vp, _i32, _vp]),
     "nsa_merge_packed_rows": (_i32, [_vp, _i32, _i64, _i32, _i32, _vp, _i32, _vp]),
     "nsa_sel_bwd_dkv_ptr": (_i32, [_vp, _S3, _vp, _vp, _vp, _vp, _S3, _i32, _vp, _i64, _i64, _i64, _i64, _i32, _i64,
                                    _i64, _vp, _vp, _i64, _vp, _vp, _vp, _S3, _i32, _i64, _i32, _i32, _i32, _i32, _i32,
                                    _f32, _i32, _vp]),
     "nsa_gate_combine": (_i32, [_vp, _vp, _vp, _vp, _vp, _i64, _i32, _i32, _i32, _vp]),
+    "nsa_gate_combine_strided": (_i32, [_vp, _i64, _vp, _vp, _vp, _vp, _i64, _i32, _i32, _i32, _i32, _vp]),
     "nsa_gate_combine_bwd": (_i32, [_vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _i64, _i32, _i32, _i32, _vp]),
     "nsa_build_ptr_table": (_i32, [_vp, _S3, _vp, _vp, _vp, _i32, _i32, _i32, _i32, _i32, _i64,
                                    _i32, _i64, _vp, _vp, _vp]),
@@ -104,11 +106,15 @@ PROTOTYPES = {
                                      _vp, _i32, _vp, _vp, _i64, _vp, _vp, _vp, _i32, C.POINTER(Rope), _vp]),
     "nsa_rope_apply": (_i32, [_vp, _S3, _i64, _i32, _i32, _vp, _i32, C.POINTER(Rope), _vp]),
     "nsa_cache_dedup_workspace_bytes": (_sz, [_i64]),
+    "nsa_cache_touch": (_i32, [_vp, _i64, _i32, _i32, _i32, _vp, _i32, _vp, _vp, _i64, _vp, _vp]),
     "nsa_cache_dedup_touch": (_i32, [_vp, _i64, _i32, _i32, _i32, _i32, _vp, _i32, _vp, _vp, _i64,
                                      _vp, _vp, _i32, _vp, _vp, _sz, _vp]),
     "nsa_cache_select_victims": (_i32, [_vp, _vp, _i32, _i32, _i32, _i64, _i32, _vp, _i32, _vp, _vp, _vp]),
     "nsa_cache_move_pages": (_i32, [_i32, _vp, _vp, _i32, _vp, _i32, _vp, _vp, _i64, _vp, _vp, _vp,
                                     _vp, _vp, _i64, _vp, _vp]),
+    "nsa_residual_norm": (_i32, [_vp] * 8 + [_i32, _vp, _vp, _i64, _i32, _f32, _i32, _vp]),
+    "nsa_rms_rows": (_i32, [_vp, _i64, _vp, _vp, _i64, _i32, _f32, _i32, _vp]),
+    "nsa_qk_norm_rope": (_i32, [_vp, _vp, _i64, _vp, _vp, _f32, _i64, _i32, _i32, _vp, _vp, C.POINTER(Rope), _i32, _vp]),
     "nsa_gather_publish_clear": (_i32, [_vp, _i64, _i64, _i64, _i32, _i32, C.POINTER(C.c_int64), _vp]),
     "nsa_block_range": (_i32, [_vp, _vp, _i32, _i64, _i64, _i64, _i64, _i64, _i64, _i64, _i64, _i32,
                                _i32, _i32, _vp]),
@@ -137,6 +143,29 @@ def load() -> C.CDLL:
             fn.argtypes = args
         _lib = lib
     return _lib
+
+
+def _host_or_raise():
+    try:
+        from . import _host
+    except ImportError as e:
+        raise NSABackendError(f"the native host path is missing ({e}): build it with `python -m omnimem_b200.build`. "
+                              "There is no fallback path.") from None
+    _host.set_error(NSABackendError)
+    return _host
+
+
+class _Host:
+    """The native host path (csrc/host.cpp), loaded on first use (importing the package needs no build)."""
+
+    def __getattr__(self, name):
+        load()
+        fn = getattr(_host_or_raise(), name)
+        setattr(self, name, fn)
+        return fn
+
+
+host = _Host()
 
 
 def call(name: str, *args) -> None:

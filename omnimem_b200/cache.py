@@ -27,7 +27,7 @@ from typing import Optional
 import torch
 
 from . import _lib, ops
-from ._lib import NSABackendError, call
+from ._lib import NSABackendError, call, host
 
 
 class RopeSpec:
@@ -40,17 +40,33 @@ class RopeSpec:
         if freqs.dtype != torch.complex128 or freqs.dim() != 2:
             raise NSABackendError("RopeSpec: freqs must be a complex128 [max_len, D/2] table")
         self.freqs, self.grid_hw, self.start_frame, self.pool = freqs, tuple(grid_hw), int(start_frame), tuple(pool)
-        self._tables = None
+        self._tables = self._native = None
 
-    def struct(self, device, D: int) -> _lib.Rope:
+    def _split(self, device, D: int):
         c = D // 2
         if self.freqs.shape[1] != c:
             raise NSABackendError(f"RopeSpec: freqs has {self.freqs.shape[1]} columns, head dim {D} needs {c}")
+        device = torch.device(device)
+        if device.index is None:
+            device = torch.device(device.type, torch.cuda.current_device())
         if self._tables is None or self._tables[0].device != device:
             parts = self.freqs.split([c - 2 * (c // 3), c // 3, c // 3], dim=1)
             self._tables = [torch.view_as_real(p.contiguous()).to(device).contiguous() for p in parts]
+            self._native = None
+        return self._tables
+
+    def native(self, device, D: int):
+        """The tables on `device` and the geometry, as the native host path takes them."""
+        if self._native is None or self._tables[0].device != device:
+            tables = self._split(device, D)
+            self._native = host.Rope(*tables, *self.grid_hw, *self.pool, self.start_frame)
+        return self._native
+
+    def struct(self, device, D: int) -> _lib.Rope:
+        c = D // 2
+        tables = self._split(device, D)
         s = _lib.Rope()
-        s.freqs_f, s.freqs_h, s.freqs_w = (t.data_ptr() for t in self._tables)
+        s.freqs_f, s.freqs_h, s.freqs_w = (t.data_ptr() for t in tables)
         s.c_f, s.c_h, s.c_w = c - 2 * (c // 3), c // 3, c // 3
         s.grid_h, s.grid_w = self.grid_hw
         s.pool_f, s.pool_h, s.pool_w = self.pool
@@ -63,14 +79,7 @@ def rope_apply(x: torch.Tensor, rope: RopeSpec) -> torch.Tensor:
     the query-side use of causal_reorder_rope_apply (causal_wan_nsa_model.py:72-105, 463-466)."""
     if not x.is_cuda or x.dim() != 3:
         raise NSABackendError("rope_apply: x must be a CUDA tensor [S,H,D]")
-    x = ops._rows16(x)
-    S, H, D = x.shape
-    out = torch.empty(S, H, D, dtype=x.dtype, device=x.device)
-    spec = rope.struct(x.device, D)
-    with torch.cuda.device(x.device):
-        call("nsa_rope_apply", x.data_ptr(), (C.c_int64 * 3)(x.stride(0), x.stride(1), 0), S, H, D, out.data_ptr(),
-             ops._dtype(x), C.byref(spec), torch.cuda.current_stream(x.device).cuda_stream)
-    return out
+    return host.rope_apply(x, rope.native(x.device, x.shape[-1]))
 
 
 class BlockKVCache:
@@ -85,6 +94,8 @@ class BlockKVCache:
         dev = torch.device(device)
         if dev.type != "cuda":
             raise NSABackendError("BlockKVCache lives on a CUDA device")
+        if dev.index is None:
+            dev = torch.device("cuda", torch.cuda.current_device())
         self.H, self.D, self.page_tokens = num_heads, head_dim, page_tokens
         self.num_pages, self.max_blocks = num_pages, max_blocks
         self.dtype, self.device = dtype, dev
@@ -115,6 +126,9 @@ class BlockKVCache:
         self._evicted_any = False
         self.page_bytes = page_tokens * head_dim * self.k_pool.element_size()
         self._dtype_code = ops._dtype(self.k_pool)
+        self._state = host.CacheState([self.k_pool, self.v_pool, self.block_table, self.page_owner, self.page_stamp,
+                                       self.k_pooled, self.v_pooled, self._stamp32, self.status, self.counters],
+                                      num_heads, head_dim, page_tokens, max_blocks)
         self.write_behind = bool(write_behind) and host_tier
         self._stage_k = self._stage_v = self._stage_keys = None
         self._drain_event = None                 # recorded behind the last copy from the staging buffer to the host
@@ -226,6 +240,29 @@ class BlockKVCache:
             self._move(1, victims, miss, 0, n_dev, cap)
         return uniq, miss
 
+    def _pages_for(self, first: int, n_touched: int, n_exist: int, n_new: int, protect_from: int):
+        """Makes the touched blocks that exist resident and finds pages for the new ones: int32
+        [H, n_touched], -1 where a block keeps its page (None: all of them do)."""
+        if n_exist and self._evicted_any:
+            if self.host_k is None:
+                raise NSABackendError("rewriting blocks after evictions needs the host tier (a dropped block "
+                                      "cannot be completed again)")
+            ids = torch.arange(first, first + n_exist, dtype=torch.int32, device=self.device).repeat_interleave(self.H)
+            self._make_resident(ids, 1, count=False, protect_from=protect_from)
+        need = n_new * self.H
+        if not need:
+            return None
+        new_pages = torch.full((self.H, n_touched), -1, dtype=torch.int32, device=self.device)
+        pages = self._select_victims(need, None, need, protect_from)
+        if self.write_behind:
+            self._evict_write_behind(pages, need)             # free pages pass through untouched
+        else:
+            self._move(0, pages, None, need, None, need)
+        new_pages[:, n_exist:] = pages.view(self.H, n_new)
+        if self.n_blocks * self.H + need > self.num_pages:
+            self._evicted_any = True
+        return new_pages
+
     # ------------------------------------------------------------------------------- append
     def append(self, k_new: torch.Tensor, v_new: torch.Tensor, pos0: Optional[int] = None,
                rope: Optional["RopeSpec"] = None) -> None:
@@ -256,35 +293,13 @@ class BlockKVCache:
         self.epoch += 1
         # pages for this call may only come from blocks in front of the ones it touches
         protect_from = max(min(first, self.n_blocks - self.protect_blocks), 0)
-        with torch.cuda.device(self.device):
-            if n_exist and self._evicted_any:
-                if self.host_k is None:
-                    raise NSABackendError("rewriting blocks after evictions needs the host tier (a dropped block "
-                                          "cannot be completed again)")
-                ids = torch.arange(first, first + n_exist, dtype=torch.int32, device=self.device).repeat_interleave(self.H)
-                self._make_resident(ids, 1, count=False, protect_from=protect_from)
-            new_pages = torch.full((self.H, n_touched), -1, dtype=torch.int32, device=self.device)
-            need = n_new * self.H
-            if need:
-                pages = self._select_victims(need, None, need, protect_from)
-                if self.write_behind:
-                    self._evict_write_behind(pages, need)             # free pages pass through untouched
-                else:
-                    self._move(0, pages, None, need, None, need)
-                new_pages[:, n_exist:] = pages.view(self.H, n_new)
-                if self.n_blocks * self.H + need > self.num_pages:
-                    self._evicted_any = True
-            args = (k_new.data_ptr(), v_new.data_ptr(),
-                    (C.c_int64 * 3)(k_new.stride(0), k_new.stride(1), 0), S, pos0, self.n_tokens, self.H, self.D,
-                    self.k_pool.data_ptr(), self.v_pool.data_ptr(), self.page_tokens, self.block_table.data_ptr(),
-                    self.max_blocks, new_pages.data_ptr(), n_touched, self.page_owner.data_ptr(),
-                    self.page_stamp.data_ptr(), self.epoch, self.k_pooled.data_ptr(), self.v_pooled.data_ptr(),
-                    self.status.data_ptr(), self._dtype_code)
-            if rope is None:
-                call("nsa_cache_append", *args, self._stream())
-            else:
-                spec = rope.struct(self.device, self.D)
-                call("nsa_cache_append_rope", *args, C.byref(spec), self._stream())
+        need = n_new * self.H
+        new_pages = None
+        if need or (n_exist and self._evicted_any):
+            with torch.cuda.device(self.device):
+                new_pages = self._pages_for(first, n_touched, n_exist, n_new, protect_from)
+        host.cache_append(self._state, k_new, v_new, pos0, self.n_tokens, self.epoch, new_pages,
+                          None if rope is None else rope.native(self.device, self.D))
         self.n_tokens = max(self.n_tokens, pos0 + S)
 
     # ------------------------------------------------------------------- selection residency
@@ -294,6 +309,10 @@ class BlockKVCache:
         ids = block_indices.contiguous().view(-1)
         T = block_indices.shape[-1]
         self.epoch += 1
+        if not return_lists and not (self._evicted_any and self.host_k is not None):
+            # nothing to fetch: stamps and counters only, no lists
+            host.cache_touch(self._state, ids, T, self.epoch)
+            return None
         with torch.cuda.device(self.device):
             uniq, miss = self._make_resident(ids, T, count=True)
         return (uniq, miss) if return_lists else None

@@ -3,6 +3,7 @@
 // and the reference's three block-KV entry points.  All byte / integer work, 16-byte
 // vectorised, no host synchronisation: data-dependent counts stay on the device.
 #include "common.cuh"
+#include "rope.cuh"
 
 namespace nsa {
 namespace {
@@ -13,7 +14,7 @@ __device__ __forceinline__ void copy16(char* dst, const char* src, int64_t bytes
 }
 
 // ------------------------------------------------------------------------------------ append
-struct AppendParams {
+struct AppendParams : RopeParams {        // (the rotary embedding of the new keys is optional)
   const char* k_new; const char* v_new;
   int64_t s_stride, h_stride;      // elements
   int64_t S, pos0;
@@ -25,36 +26,7 @@ struct AppendParams {
   int32_t* page_owner; int64_t* page_stamp; int64_t epoch;
   char* k_pooled; char* v_pooled;
   int32_t* status;
-  // optional rotary embedding of the new keys (causal_reorder_rope_apply,
-  // models/transformers/causal_wan_nsa_model.py:72-105): token t of the chunk, in the reordered
-  // order (f h w fs hs ws), sits at frame / row / column (fr, hr, wr) of the chunk's latent grid;
-  // complex pair j of a head takes its factor from the frame table (j < c_f, row start_frame + fr),
-  // the row table (next c_h pairs) or the column table (last c_w pairs); products in float64.
-  const double2* rope_f; const double2* rope_h; const double2* rope_w;
-  int c_f, c_h, c_w;
-  int grid_h, grid_w, pool_f, pool_h, pool_w, start_frame;
 };
-
-// frame / row / column of token t of a chunk stored in (f h w fs hs ws) order
-template <typename I>
-__device__ __forceinline__ void rope_position_t(const AppendParams& p, I t, int& fr, int& hr, int& wr) {
-  const I pw = static_cast<I>(p.pool_w), ph = static_cast<I>(p.pool_h), pf = static_cast<I>(p.pool_f);
-  const int ws = static_cast<int>(t % pw); t /= pw;
-  const int hs = static_cast<int>(t % ph); t /= ph;
-  const int fs = static_cast<int>(t % pf); t /= pf;
-  const I wq = static_cast<I>(p.grid_w / p.pool_w), hq = static_cast<I>(p.grid_h / p.pool_h);
-  const int wo = static_cast<int>(t % wq); t /= wq;
-  const int ho = static_cast<int>(t % hq); t /= hq;
-  fr = static_cast<int>(t) * p.pool_f + fs;
-  hr = ho * p.pool_h + hs;
-  wr = wo * p.pool_w + ws;
-}
-// (five divisions per call: in 32 bits whenever the token index allows, a 64-bit division costs
-// several times as many instructions and this runs once per row and thread)
-__device__ __forceinline__ void rope_position(const AppendParams& p, int64_t t, int& fr, int& hr, int& wr) {
-  if (static_cast<uint64_t>(t) <= 0xffffffffull) rope_position_t<uint32_t>(p, static_cast<uint32_t>(t), fr, hr, wr);
-  else rope_position_t<int64_t>(p, t, fr, hr, wr);
-}
 
 // One thread block per (touched block, group of `hc` neighbouring heads).  A thread owns one 16-byte
 // column piece of one head and one eighth of the block's rows, so that the block reads CONTIGUOUS
@@ -168,10 +140,7 @@ __global__ void __launch_bounds__(768) cache_append_kernel(const AppendParams p)
           for (int i = 0; i < VEC / 2; ++i) {
             const int at = tb_sel[i] == 0 ? pos[0] : tb_sel[i] == 1 ? pos[1] : pos[2];
             const double2 w = tb[i][static_cast<int64_t>(at) * tb_len[i]];
-            const double xr = static_cast<double>(to_f32<T>(e[2 * i])), xi = static_cast<double>(to_f32<T>(e[2 * i + 1]));
-            // float64 product, then float64 -> float32 -> T, as view_as_real(...).type_as(x) does
-            e[2 * i] = from_f32<T>(static_cast<float>(xr * w.x - xi * w.y));
-            e[2 * i + 1] = from_f32<T>(static_cast<float>(xr * w.y + xi * w.x));
+            rope_pair<T>(e[2 * i], e[2 * i + 1], w);
           }
         }
         *reinterpret_cast<uint4*>(kp + r * row_bytes) = kq[u];
@@ -260,15 +229,7 @@ __global__ void __launch_bounds__(256) rope_apply_kernel(const AppendParams p, c
 #pragma unroll
     for (int k = 0; k < VEC / 2; ++k) {
       const int j = cc * (VEC / 2) + k;
-      // one load through a selected table instead of three branches: a warp's threads sit in different tables
-      const bool in_f = j < p.c_f, in_h = j < p.c_f + p.c_h;
-      const double2* tbp = in_f ? p.rope_f + j : in_h ? p.rope_h + (j - p.c_f) : p.rope_w + (j - p.c_f - p.c_h);
-      const int len = in_f ? p.c_f : in_h ? p.c_h : p.c_w;
-      const int at = in_f ? p.start_frame + fr : in_h ? hr : wr;
-      const double2 w = tbp[static_cast<int64_t>(at) * len];
-      const double xr = static_cast<double>(to_f32<T>(e[2 * k])), xi = static_cast<double>(to_f32<T>(e[2 * k + 1]));
-      e[2 * k] = from_f32<T>(static_cast<float>(xr * w.x - xi * w.y));
-      e[2 * k + 1] = from_f32<T>(static_cast<float>(xr * w.y + xi * w.x));
+      rope_pair<T>(e[2 * k], e[2 * k + 1], rope_factor(p, j, fr, hr, wr));
     }
     *reinterpret_cast<uint4*>(out + ((t * p.H + h) * static_cast<int64_t>(p.D)) * sizeof(T) + cc * 16) = q;
   }
@@ -340,6 +301,35 @@ __global__ void __launch_bounds__(kTileKeys) dedup_compact_kernel(
   pm += __popc(mm & ((1u << lane) - 1));
   if (hit && ph < cap) out_unique[1 + ph] = static_cast<int32_t>(key);
   if (miss && out_missing && pm < cap) out_missing[1 + pm] = static_cast<int32_t>(key);
+}
+
+// Touch alone, for calls that need no lists: the first thread to mark a (head, block) this epoch stamps its page or
+// counts the miss.  One pass over the ids instead of mark, count, scan and compact over all keys.
+__global__ void __launch_bounds__(256) cache_touch_kernel(const int32_t* __restrict__ ids, int64_t n_entries, int H, int T,
+                                                          int max_blocks, int32_t* __restrict__ stamp, int32_t epoch,
+                                                          const int32_t* __restrict__ table, int64_t* __restrict__ page_stamp,
+                                                          int64_t epoch64, unsigned long long* counters) {
+  chain_release();
+  chain_wait();
+  const int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+  bool hit = false, miss = false;
+  if (i < n_entries) {
+    const int32_t bid = ids[i];
+    if (bid >= 0 && bid < max_blocks) {
+      const int64_t key = (i / T) % H * max_blocks + bid;
+      if (atomicExch(stamp + key, epoch) != epoch) {
+        const int page = table[key];
+        hit = page >= 0;
+        miss = page < 0;
+        if (hit) page_stamp[page] = epoch64;
+      }
+    }
+  }
+  const int hits = __syncthreads_count(hit), misses = __syncthreads_count(miss);
+  if (threadIdx.x == 0 && counters != nullptr) {
+    if (hits) atomicAdd(counters, static_cast<unsigned long long>(hits));
+    if (misses) atomicAdd(counters + 1, static_cast<unsigned long long>(misses));
+  }
 }
 
 // ------------------------------------------------------------------------- victim selection
@@ -744,11 +734,8 @@ __global__ void block_range_kernel(int64_t* __restrict__ table, int32_t* __restr
 }
 
 }  // namespace
-}  // namespace nsa
 
-using namespace nsa;
-
-static int set_rope(const nsa_rope* rope, int64_t S, int32_t D, AppendParams* p) {
+int set_rope(const nsa_rope* rope, int64_t S, int32_t D, RopeParams* p) {
   NSA_REQUIRE(rope->freqs_f && rope->freqs_h && rope->freqs_w, NSA_ERR_INVALID, "rope: null frequency table");
   NSA_REQUIRE(rope->c_f >= 0 && rope->c_h >= 0 && rope->c_w >= 0 && 2 * (rope->c_f + rope->c_h + rope->c_w) == D,
               NSA_ERR_INVALID, "rope: c_f + c_h + c_w must be D / 2");
@@ -764,6 +751,10 @@ static int set_rope(const nsa_rope* rope, int64_t S, int32_t D, AppendParams* p)
   p->pool_w = rope->pool_w; p->start_frame = rope->start_frame;
   return NSA_OK;
 }
+
+}  // namespace nsa
+
+using namespace nsa;
 
 static int cache_append_impl(const void* k_new, const void* v_new, const int64_t kv_stride[2],
                              int64_t S, int64_t pos0, int64_t n_tokens, int32_t H, int32_t D, void* k_pool,
@@ -791,7 +782,7 @@ static int cache_append_impl(const void* k_new, const void* v_new, const int64_t
   NSA_REQUIRE(aligned16(k_new) && aligned16(v_new) && (kv_stride[0] * esz) % 16 == 0 && (kv_stride[1] * esz) % 16 == 0,
               NSA_ERR_LAYOUT, "cache_append: new K/V rows must be 16-byte aligned");
   NSA_REQUIRE(static_cast<int64_t>(n_touched_blocks) * H <= 0x7fffffff, NSA_ERR_INVALID, "cache_append: too many blocks");
-  AppendParams p{static_cast<const char*>(k_new), static_cast<const char*>(v_new), kv_stride[0], kv_stride[1],
+  AppendParams p{{}, static_cast<const char*>(k_new), static_cast<const char*>(v_new), kv_stride[0], kv_stride[1],
                  S, pos0, n_tokens, H, D, page_tokens, max_blocks, n_touched_blocks, H, static_cast<char*>(k_pool),
                  static_cast<char*>(v_pool), block_table, new_pages, page_owner, page_stamp, epoch,
                  static_cast<char*>(k_pooled), static_cast<char*>(v_pooled), status};
@@ -878,6 +869,21 @@ extern "C" int nsa_rope_apply(const void* x, const int64_t x_stride[2], int64_t 
   if (dtype == NSA_BF16) rope_apply_kernel<__nv_bfloat16><<<blocks, 256, 0, s>>>(p, static_cast<char*>(out));
   else rope_apply_kernel<__half><<<blocks, 256, 0, s>>>(p, static_cast<char*>(out));
   NSA_LAUNCH_OK("rope_apply_kernel");
+  return NSA_OK;
+}
+
+extern "C" int nsa_cache_touch(const int32_t* block_indices, int64_t n_entries, int32_t H, int32_t T, int32_t max_blocks,
+                               int32_t* stamp, int32_t epoch, const int32_t* block_table, int64_t* page_stamp, int64_t epoch64,
+                               int64_t* counters, void* stream) {
+  NSA_REQUIRE(n_entries >= 0 && H > 0 && T > 0 && max_blocks > 0, NSA_ERR_INVALID, "cache_touch: bad size");
+  if (n_entries == 0) return NSA_OK;
+  NSA_REQUIRE(block_indices && stamp && block_table && page_stamp, NSA_ERR_INVALID, "cache_touch: null pointer");
+  const int64_t blocks = cdiv64(n_entries, 256);
+  NSA_REQUIRE(blocks <= 0x7fffffff, NSA_ERR_INVALID, "cache_touch: too many entries");
+  NSA_CUDA_OK(launch_chained(kChainSmall, cache_touch_kernel, dim3(static_cast<unsigned>(blocks)), dim3(256), 0,
+                             static_cast<cudaStream_t>(stream), block_indices, n_entries, H, T, max_blocks, stamp, epoch,
+                             block_table, page_stamp, epoch64, reinterpret_cast<unsigned long long*>(counters)));
+  NSA_LAUNCH_OK("cache_touch_kernel");
   return NSA_OK;
 }
 

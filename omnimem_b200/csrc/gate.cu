@@ -18,14 +18,18 @@ struct GateParams {
   char* dg;             // backward: [rows, 3] gradient of the logits
   int64_t rows;
   int D, softmax;
+  int H;                // logits of row r start at (r / H) * g_stride + (r % H) * 3
+  int64_t g_stride;
 };
 
 template <typename T>
 __device__ __forceinline__ void gates_of_row(const GateParams& p, int64_t row, float (&s)[3], bool (&inside)[3]) {
   float z[3];
+  const uint32_t token = static_cast<uint32_t>(row) / static_cast<uint32_t>(p.H);
+  const T* g = reinterpret_cast<const T*>(p.g) + token * p.g_stride + (static_cast<uint32_t>(row) - token * p.H) * 3;
 #pragma unroll
   for (int i = 0; i < 3; ++i) {
-    const float raw = to_f32<T>(reinterpret_cast<const T*>(p.g)[row * 3 + i]);
+    const float raw = to_f32<T>(g[i]);
     inside[i] = raw >= -10.f && raw <= 10.f;       // clamp passes the gradient on the closed interval
     z[i] = fminf(fmaxf(raw, -10.f), 10.f);
   }
@@ -137,6 +141,7 @@ int check_common(const char* what, const void* g, const void* o_cmp, const void*
                  int64_t rows, int D, int dtype) {
   NSA_REQUIRE(g != nullptr, NSA_ERR_INVALID, "%s: gate logits are null", what);
   NSA_REQUIRE(o_cmp != nullptr || o_slc != nullptr || o_swa != nullptr, NSA_ERR_INVALID, "%s: all three branches are null", what);
+  NSA_REQUIRE(rows <= 0xffffffffll, NSA_ERR_INVALID, "%s: too many rows", what);
   NSA_REQUIRE(rows >= 0 && D > 0 && D % 8 == 0, NSA_ERR_UNSUPPORTED, "%s: head dim %d must be a positive multiple of 8", what, D);
   NSA_REQUIRE(dtype == NSA_BF16 || dtype == NSA_F16, NSA_ERR_UNSUPPORTED, "%s: dtype %d (bf16 and fp16 only)", what, dtype);
   const void* ptrs[3] = {o_cmp, o_slc, o_swa};
@@ -152,6 +157,14 @@ using namespace nsa;
 
 extern "C" int nsa_gate_combine(const void* g_logits, const void* o_cmp, const void* o_slc, const void* o_swa,
                                 void* x, int64_t rows, int32_t D, int32_t softmax, int32_t dtype, void* stream) {
+  return nsa_gate_combine_strided(g_logits, 3, o_cmp, o_slc, o_swa, x, rows, 1, D, softmax, dtype, stream);
+}
+
+extern "C" int nsa_gate_combine_strided(const void* g_logits, int64_t g_token_stride, const void* o_cmp, const void* o_slc,
+                                        const void* o_swa, void* x, int64_t tokens, int32_t H, int32_t D, int32_t softmax,
+                                        int32_t dtype, void* stream) {
+  NSA_REQUIRE(H > 0 && tokens >= 0, NSA_ERR_INVALID, "gate_combine: bad size");
+  const int64_t rows = tokens * H;
   int rc;
   if ((rc = check_common("gate_combine", g_logits, o_cmp, o_slc, o_swa, rows, D, dtype))) return rc;
   NSA_REQUIRE(x != nullptr && aligned16(x), NSA_ERR_LAYOUT, "gate_combine: output must be non-null and 16-byte aligned");
@@ -159,7 +172,7 @@ extern "C" int nsa_gate_combine(const void* g_logits, const void* o_cmp, const v
   GateParams p{};
   p.g = static_cast<const char*>(g_logits);
   p.o[0] = static_cast<const char*>(o_cmp); p.o[1] = static_cast<const char*>(o_slc); p.o[2] = static_cast<const char*>(o_swa);
-  p.x = static_cast<char*>(x); p.rows = rows; p.D = D; p.softmax = softmax;
+  p.x = static_cast<char*>(x); p.rows = rows; p.D = D; p.softmax = softmax; p.H = H; p.g_stride = g_token_stride;
   const int64_t total = rows * (D / 8);
   NSA_REQUIRE(total <= 0xffffffffll, NSA_ERR_INVALID, "gate_combine: too many rows");
   const unsigned blocks = static_cast<unsigned>(cdiv64(total, 256));
@@ -187,7 +200,7 @@ extern "C" int nsa_gate_combine_bwd(const void* g_logits, const void* o_cmp, con
   p.dx = static_cast<const char*>(dx);
   for (int i = 0; i < 3; ++i) p.d_o[i] = static_cast<char*>(outs[i]);
   p.dg = static_cast<char*>(d_g_logits);
-  p.rows = rows; p.D = D; p.softmax = softmax;
+  p.rows = rows; p.D = D; p.softmax = softmax; p.H = 1; p.g_stride = 3;
   const int lpr = D / 8;
   const unsigned blocks = static_cast<unsigned>(cdiv64(rows * lpr, 256));
   cudaStream_t s = static_cast<cudaStream_t>(stream);

@@ -202,6 +202,30 @@ extern "C" int nsa_local_block_ids(const int32_t* ids, int64_t n, int32_t R, int
   return NSA_OK;
 }
 
+namespace nsa {
+namespace {
+__global__ void __launch_bounds__(256) check_block_ids_kernel(const int32_t* __restrict__ ids, int64_t n, int32_t limit, int32_t* flag) {
+  chain_release();
+  chain_wait();
+  bool bad = false;
+  for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += static_cast<int64_t>(gridDim.x) * blockDim.x)
+    bad |= ids[i] >= limit;
+  if (bad) *reinterpret_cast<volatile int32_t*>(flag) = 1;
+}
+}  // namespace
+}  // namespace nsa
+
+extern "C" int nsa_check_block_ids(const int32_t* ids, int64_t n, int32_t limit, int32_t* flag, void* stream) {
+  NSA_REQUIRE(n >= 0, NSA_ERR_INVALID, "check_block_ids: n < 0");
+  if (n == 0) return NSA_OK;
+  NSA_REQUIRE(ids && flag, NSA_ERR_INVALID, "check_block_ids: null pointer");
+  const int64_t want = cdiv64(n, 1024);
+  NSA_CUDA_OK(launch_chained(kChainSmall, nsa::check_block_ids_kernel, dim3(static_cast<unsigned>(want < 296 ? want : 296)), dim3(256), 0,
+                             static_cast<cudaStream_t>(stream), ids, n, limit, flag));
+  NSA_LAUNCH_OK("check_block_ids_kernel");
+  return NSA_OK;
+}
+
 extern "C" int nsa_build_ptr_table(const int32_t* block_indices, const int64_t idx_stride[4],
                                    const int64_t* base_k, const int64_t* base_v,
                                    const int32_t* n_blocks_per_head, int32_t B, int32_t MG, int32_t H,

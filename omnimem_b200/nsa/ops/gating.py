@@ -18,20 +18,7 @@ from typing import Optional
 import torch
 
 from ... import ops
-
-
-class _GatedSum(torch.autograd.Function):
-    @staticmethod
-    def forward(ctx, g_logits, o_cmp, o_slc, o_swa, gate_mode):
-        ctx.gate_mode = gate_mode
-        ctx.save_for_backward(g_logits, o_cmp, o_slc, o_swa)
-        return ops.gate_combine(g_logits, o_cmp, o_slc, o_swa, gate_mode)
-
-    @staticmethod
-    def backward(ctx, dx):
-        g_logits, o_cmp, o_slc, o_swa = ctx.saved_tensors
-        dg, da, db, dc = ops.gate_combine_bwd(g_logits, o_cmp, o_slc, o_swa, dx, ctx.gate_mode)
-        return dg, da, db, dc, None
+from ..._lib import host
 
 
 def gated_branch_sum(g_logits: torch.Tensor, o_cmp: Optional[torch.Tensor], o_slc: Optional[torch.Tensor],
@@ -42,4 +29,4 @@ def gated_branch_sum(g_logits: torch.Tensor, o_cmp: Optional[torch.Tensor], o_sl
         o_cmp = None
     elif skip_module == "slc":
         o_slc = None
-    return _GatedSum.apply(g_logits, o_cmp, o_slc, o_swa, gate_mode)
+    return host.gated_sum(g_logits, o_cmp, o_slc, o_swa, ops._softmax_gates(gate_mode))

@@ -3,7 +3,8 @@
 Every function runs on the current CUDA stream of its first tensor's device, allocates
 its outputs and scratch with torch's caching allocator, and never synchronises.  Inputs
 whose innermost stride is not 1 or whose rows are not 16-byte aligned are copied once
-(`_rows16`); everything else is passed by stride.
+(`_rows16`); everything else is passed by stride.  The functions on the hot paths are thin
+fronts of the native host path (csrc/host.cpp), which does all of that.
 """
 from __future__ import annotations
 
@@ -15,7 +16,7 @@ from typing import Optional, Tuple
 import torch
 
 from . import _lib
-from ._lib import NSABackendError, KVSource, TopkMask, call, strides3, strides4
+from ._lib import NSABackendError, KVSource, TopkMask, call, host, strides3, strides4
 
 _DTYPES = {torch.bfloat16: _lib.NSA_BF16, torch.float16: _lib.NSA_F16, torch.float32: _lib.NSA_F32}
 
@@ -59,15 +60,7 @@ def _i32(x, what: str) -> int:
 # ------------------------------------------------------------------------------------ pooling
 def pool_rows(x: torch.Tensor, size: int) -> torch.Tensor:
     """Mean over runs of `size` rows of dim 1 of x [B,N,H,D] -> [B,ceil(N/size),H,D]."""
-    _require_cuda(x)
-    B, N, H, D = x.shape
-    x = _rows16(x)
-    nb = (N + size - 1) // size
-    out = torch.empty(B, nb, H, D, dtype=x.dtype, device=x.device)
-    with torch.cuda.device(x.device):
-        call("nsa_pool_rows", x.data_ptr(), strides3(x), out.data_ptr(), strides3(out), B, N, H, D,
-             _i32(size, "size"), _dtype(x), _stream(x))
-    return out
+    return host.pool_rows(x, size)
 
 
 # -------------------------------------------------------------------------------------- top-k
@@ -86,26 +79,9 @@ def topk(q_pooled: torch.Tensor, k_pooled: torch.Tensor, topk: int, scale: float
          q_group_size: int = 1, id_base: int = 0, id_stride: int = 1, return_scores: bool = False):
     """int32 [B,MG,H,topk] block ids by (score desc, id asc), -1 padded; optionally the scores.
     `chunk_size` counts query tokens; a pooled row stands for `q_group_size` tokens."""
-    _require_cuda(q_pooled, k_pooled)
-    if q_pooled.dtype != k_pooled.dtype:
-        raise NSABackendError(f"topk: q and k must share a dtype, got {q_pooled.dtype} vs {k_pooled.dtype}")
-    B, MG, H, D = q_pooled.shape
-    NC = k_pooled.shape[1]
-    if k_pooled.shape[0] != B or k_pooled.shape[2] != H or k_pooled.shape[3] != D:
-        raise NSABackendError(f"topk: incompatible shapes q={tuple(q_pooled.shape)} k={tuple(k_pooled.shape)}")
-    q_pooled = q_pooled if q_pooled.stride(-1) == 1 else q_pooled.contiguous()
-    k_pooled = k_pooled if k_pooled.stride(-1) == 1 else k_pooled.contiguous()
-    dev = q_pooled.device
-    out = torch.empty(B, MG, H, topk, dtype=torch.int32, device=dev)
-    scores = torch.empty(B, MG, H, topk, dtype=torch.float32, device=dev) if return_scores else None
-    m = _mask(block_size, chunk_size, chunk_size_k, q_group_size, q_chunk_offset, ex_win, ex_sink,
-              causal, tf_mask, prog_excl, id_base, id_stride)
-    with torch.cuda.device(dev):
-        wsb = _lib.load().nsa_topk_workspace_bytes(B, MG, H, NC)
-        ws = torch.empty(max(wsb, 1), dtype=torch.uint8, device=dev)
-        call("nsa_topk", q_pooled.data_ptr(), strides3(q_pooled), k_pooled.data_ptr(), strides3(k_pooled),
-             B, MG, H, D, NC, _i32(topk, "topk"), float(scale), C.byref(m), out.data_ptr(), _ptr(scores),
-             ws.data_ptr(), wsb, _dtype(q_pooled), _stream(q_pooled))
+    out, scores = host.topk(q_pooled, k_pooled, topk, scale,
+                            (block_size, chunk_size, chunk_size_k, q_group_size, q_chunk_offset, ex_win, ex_sink,
+                             causal, tf_mask, prog_excl, id_base, id_stride), return_scores)
     return (out, scores) if return_scores else out
 
 
@@ -143,27 +119,9 @@ def select_blocks(q: torch.Tensor, k: torch.Tensor, topk: int, scale: float, blo
     """Block selection from the raw tensors in one call: q [B,M,H,D] pooled per query group, k
     [B,N,H,D] pooled per key block and scored in the same pass, top-k per (group, head).
     Returns (idx int32 [B,MG,H,topk], q_pooled, k_pooled[, scores])."""
-    _require_cuda(q, k)
-    if q.dtype != k.dtype:
-        raise NSABackendError(f"select_blocks: q and k must share a dtype, got {q.dtype} vs {k.dtype}")
-    B, M, H, D = q.shape
-    N = k.shape[1]
-    q, k = _rows16(q), _rows16(k)
-    MG = (M + group_size - 1) // group_size
-    NC = (N + block_size - 1) // block_size
-    dev = k.device
-    qp = torch.empty(B, MG, H, D, dtype=q.dtype, device=dev)
-    kp = torch.empty(B, NC, H, D, dtype=k.dtype, device=dev)
-    out = torch.empty(B, MG, H, topk, dtype=torch.int32, device=dev)
-    scores = torch.empty(B, MG, H, topk, dtype=torch.float32, device=dev) if return_scores else None
-    m = _mask(block_size, chunk_size, chunk_size_k, group_size, q_chunk_offset, ex_win, ex_sink,
-              causal, tf_mask, prog_excl, id_base, id_stride)
-    with torch.cuda.device(dev):
-        wsb = _lib.load().nsa_topk_workspace_bytes(B, MG, H, NC)
-        ws = torch.empty(max(wsb, 1), dtype=torch.uint8, device=dev)
-        call("nsa_select_blocks", q.data_ptr(), strides3(q), k.data_ptr(), strides3(k), B, M, H, D, N,
-             _i32(topk, "topk"), float(scale), C.byref(m), qp.data_ptr(), kp.data_ptr(), out.data_ptr(),
-             _ptr(scores), ws.data_ptr(), wsb, _dtype(k), _stream(k))
+    out, qp, kp, scores = host.select_blocks(q, k, topk, scale,
+                                             (block_size, chunk_size, chunk_size_k, group_size, q_chunk_offset, ex_win,
+                                              ex_sink, causal, tf_mask, prog_excl, id_base, id_stride), return_scores)
     return (out, qp, kp, scores) if return_scores else (out, qp, kp)
 
 
@@ -201,11 +159,16 @@ class DenseKV:
     """k, v [B,N,H,D] addressed by stride."""
 
     def __init__(self, k: torch.Tensor, v: torch.Tensor):
-        _require_cuda(k, v)
-        if k.shape != v.shape:
-            raise NSABackendError("k and v must have the same shape")
-        self.k, self.v = _rows16(k), _rows16(v)
+        self.native = host.dense(k, v)
         self.n_tokens = k.shape[1]
+
+    @property
+    def k(self) -> torch.Tensor:
+        return self.native.k
+
+    @property
+    def v(self) -> torch.Tensor:
+        return self.native.v
 
     def struct(self) -> KVSource:
         s = KVSource()
@@ -221,7 +184,7 @@ class PagedKV:
     """Fixed-page pool + block table (see omnimem_b200.cache.BlockKVCache)."""
 
     def __init__(self, k_pool, v_pool, block_table, n_tokens: int, page_tokens: int):
-        _require_cuda(k_pool, v_pool, block_table)
+        self.native = host.paged(k_pool, v_pool, block_table, int(n_tokens), int(page_tokens))
         self.k_pool, self.v_pool, self.block_table = k_pool, v_pool, block_table
         self.n_tokens, self.page_tokens = int(n_tokens), int(page_tokens)
 
@@ -248,6 +211,7 @@ class PtrKV:
         if ptr_k.shape != ptr_v.shape or ptr_k.stride() != ptr_v.stride():
             raise NSABackendError("ptr_k / ptr_v must be [B,MG,H,T] with identical layout")
         self.ptr_k, self.ptr_v, self.stride_bn = ptr_k, ptr_v, int(stride_bn)
+        self.native = host.pointers(ptr_k, ptr_v, self.stride_bn)
 
     def struct(self) -> KVSource:
         s = KVSource()
@@ -264,27 +228,7 @@ def sel_fwd(q: torch.Tensor, kv, block_indices: Optional[torch.Tensor], block_si
             out: Optional[torch.Tensor] = None) -> Tuple[torch.Tensor, torch.Tensor]:
     """(out [B,M,H,D] in q.dtype, lse fp32 [B,H,M]).  `out` may be given: a [B,M,H,D] tensor or
     view (innermost stride 1, 16-byte aligned rows) that the kernel writes in place."""
-    _require_cuda(q, block_indices)
-    B, M, H, D = q.shape
-    q = _rows16(q)
-    if out is None:
-        out = torch.empty(B, M, H, D, dtype=q.dtype, device=q.device)
-    elif out.shape != q.shape or out.dtype != q.dtype or _rows16(out) is not out:
-        raise NSABackendError("sel_fwd: `out` must have q's shape and dtype, unit innermost stride and 16-byte aligned rows")
-    lse = torch.empty(B, H, M, dtype=torch.float32, device=q.device)
-    table = kv.ptr_k if isinstance(kv, PtrKV) else block_indices
-    if table.dim() != 4:
-        raise NSABackendError("block_indices must be [B,MG,H,T]")
-    if block_indices is not None and block_indices.dtype != torch.int32:
-        raise NSABackendError("block_indices must be int32")
-    T = table.shape[-1]
-    src = kv.struct()
-    with torch.cuda.device(q.device):
-        call("nsa_sel_fwd", q.data_ptr(), strides3(q), C.byref(src), _ptr(block_indices), strides4(table),
-             out.data_ptr(), strides3(out), lse.data_ptr(), B, M, H, D, T, _i32(block_size, "block_size"),
-             _i32(chunk_size, "chunk_size"), int(bool(causal)), _i32(group_size, "group_size"), float(scale),
-             _dtype(q), _stream(q))
-    return out, lse
+    return host.sel_fwd(q, kv.native, block_indices, block_size, chunk_size, scale, causal, group_size, out)
 
 
 def range_fwd(q: torch.Tensor, kv, first_block: int, n_blocks: int, block_size: int, scale: float,
@@ -293,89 +237,32 @@ def range_fwd(q: torch.Tensor, kv, first_block: int, n_blocks: int, block_size: 
     causal: (out [B,M,H,D], lse fp32 [B,H,M]), what sel_fwd returns when every query group lists
     exactly those blocks.  Shapes the range kernel is not built for (anything but bf16, D = 128,
     64-token blocks, H > 1, dense or paged K/V, <= 1024 blocks) go to sel_fwd with the list spelt out."""
-    _require_cuda(q)
-    B, M, H, D = q.shape
-    first_block, n_blocks = _i32(first_block, "first_block"), _i32(n_blocks, "n_blocks")
     if first_block < 0 or n_blocks < 0:
         raise NSABackendError(f"range_fwd: first_block {first_block}, n_blocks {n_blocks}")
-    covered = (q.dtype == torch.bfloat16 and D == 128 and block_size == 64 and H > 1 and scale > 0
-               and isinstance(kv, (DenseKV, PagedKV)) and n_blocks <= 1024 and kv.n_tokens > 0
-               and os.environ.get("OMNIMEM_B200_RANGE_KERNEL", "") != "listed")   # test hook: always list the blocks
-    if not covered:
-        G = 64
-        ids = torch.arange(first_block, first_block + max(n_blocks, 1), dtype=torch.int32, device=q.device)
-        if n_blocks == 0:
-            ids = torch.full_like(ids, -1)
-        ids = ids.expand(B, -(-M // G), H, ids.numel())
-        return sel_fwd(q, kv, ids, block_size, 1, scale, False, G, out=out)
-    q = _rows16(q)
-    if out is None:
-        out = torch.empty(B, M, H, D, dtype=q.dtype, device=q.device)
-    elif out.shape != q.shape or out.dtype != q.dtype or _rows16(out) is not out:
-        raise NSABackendError("range_fwd: `out` must have q's shape and dtype, unit innermost stride and 16-byte aligned rows")
-    lse = torch.empty(B, H, M, dtype=torch.float32, device=q.device)
-    src = kv.struct()
-    with torch.cuda.device(q.device):
-        nbytes = _lib.load().nsa_range_fwd_workspace_bytes(B, M, H, D, n_blocks) if out.is_contiguous() else 0
-        ws = torch.empty(nbytes, dtype=torch.uint8, device=q.device) if nbytes else None
-        call("nsa_range_fwd", q.data_ptr(), strides3(q), C.byref(src), first_block, n_blocks, out.data_ptr(),
-             strides3(out), lse.data_ptr(), B, M, H, D, _i32(block_size, "block_size"), float(scale), _ptr(ws), nbytes,
-             _dtype(q), _stream(q))
-    return out, lse
+    done = host.range_fwd(q, kv.native, first_block, n_blocks, block_size, scale, out)
+    if done is not None:
+        return done
+    B, M, H, _ = q.shape
+    G = 64
+    ids = torch.arange(first_block, first_block + max(n_blocks, 1), dtype=torch.int32, device=q.device)
+    if n_blocks == 0:
+        ids = torch.full_like(ids, -1)
+    ids = ids.expand(B, -(-M // G), H, ids.numel())
+    return sel_fwd(q, kv, ids, block_size, 1, scale, False, G, out=out)
 
 
 def sel_bwd(q, kv, block_indices, out, lse, d_out, block_size: int, chunk_size: int, scale: float,
             causal: bool, group_size: int):
-    """(dq [B,M,H,D] q.dtype, dk, dv [B,N,H,D] k dtype, contiguous)."""
-    _require_cuda(q, block_indices, out, lse, d_out)
-    B, M, H, D = q.shape
-    q, out, d_out = _rows16(q), _rows16(out), _rows16(d_out)
-    lse = lse.contiguous()
-    if block_indices.dtype != torch.int32:
-        raise NSABackendError("block_indices must be int32")
-    N = kv.n_tokens
-    T = block_indices.shape[-1]
-    dev = q.device
-    dq = torch.empty(B, M, H, D, dtype=q.dtype, device=dev)
-    dk = torch.empty(B, N, H, D, dtype=q.dtype, device=dev)
-    dv = torch.empty(B, N, H, D, dtype=q.dtype, device=dev)
-    nbytes = stored_probabilities_bytes(q, kv, block_indices, block_size, group_size)
-    if nbytes:
-        # P and dS computed once: the dQ kernel stores them, the dK/dV kernel streams them
-        pds = torch.empty(nbytes, dtype=torch.uint8, device=dev)
-        NS = -(-N // block_size)
-        groups, offsets, slots = inverted_index(block_indices, NS, block_size, chunk_size, causal, group_size,
-                                                with_slots=True)
-        dq, delta, written = sel_bwd_dq(q, kv, block_indices, out, lse, d_out, block_size, chunk_size, scale, causal,
-                                        group_size, pds=pds)
-        dk, dv = sel_bwd_dkv(q, kv, groups, offsets, lse, delta, d_out, T, block_size, chunk_size, scale, causal,
-                             group_size, slots=slots if written else None, pds=pds if written else None)
-        return dq, dk, dv
-    src = kv.struct()
-    with torch.cuda.device(dev):
-        wsb = _lib.load().nsa_sel_bwd_workspace_bytes(B, M, H, N, T, block_size, group_size)
-        ws = torch.empty(max(wsb, 1), dtype=torch.uint8, device=dev)
-        call("nsa_sel_bwd", q.data_ptr(), strides3(q), C.byref(src), block_indices.data_ptr(),
-             strides4(block_indices), out.data_ptr(), strides3(out), lse.data_ptr(), d_out.data_ptr(),
-             strides3(d_out), dq.data_ptr(), strides3(dq), dk.data_ptr(), dv.data_ptr(), B, M, H, D, T,
-             _i32(block_size, "block_size"), _i32(chunk_size, "chunk_size"), int(bool(causal)),
-             _i32(group_size, "group_size"), float(scale), ws.data_ptr(), wsb, _dtype(q), _stream(q))
-    return dq, dk, dv
+    """(dq [B,M,H,D] q.dtype, dk, dv [B,N,H,D] k dtype, contiguous).  P and dS are computed once (the dQ
+    kernel stores them, the dK/dV kernel streams them) where stored_probabilities_bytes says so."""
+    return host.sel_bwd(q, kv.native, block_indices, out, lse, d_out, block_size, chunk_size, scale, causal, group_size)
 
 
 def stored_probabilities_bytes(q, kv, block_indices, block_size: int, group_size: int) -> int:
     """Size of the P / dS buffer when the backward of this call can compute them once (dQ kernel
     stores, dK/dV kernel streams), else 0.  The buffer holds 16 KiB per (query group, head, slot);
     OMNIMEM_B200_BWD_STORED_MB caps it (default 4096, 0 turns the path off)."""
-    cap_mb = int(os.environ.get("OMNIMEM_B200_BWD_STORED_MB", "4096"))
-    B, M, H, D = q.shape
-    T = block_indices.shape[-1]
-    if (cap_mb <= 0 or q.dtype != torch.bfloat16 or D != 128 or block_size != 64 or not 16 <= group_size <= 64
-            or H == 1 or T > 64 or not isinstance(kv, (DenseKV, PagedKV))):
-        return 0
-    with torch.cuda.device(q.device):
-        n = _lib.load().nsa_sel_bwd_pds_bytes(B, M, H, T, group_size)
-    return n if 0 < n <= cap_mb << 20 else 0
+    return host.stored_bytes(q, kv.native.mode, block_indices.shape[-1], block_size, group_size)
 
 
 def inverted_index(block_indices: torch.Tensor, NS: int, block_size: int, chunk_size: int, causal: bool,
@@ -553,54 +440,23 @@ def sel_bwd_dkv(q, kv, groups, offsets, lse, delta, d_out, T: int, block_size: i
     return dk, dv
 
 
-def _gate_args(g_logits, o_cmp, o_slc, o_swa):
-    present = [t for t in (o_cmp, o_slc, o_swa) if t is not None]
-    if not present:
-        raise ValueError("gate_combine: at least one branch is needed")
-    ref = present[0]
-    _require_cuda(g_logits, *present)
-    if g_logits.shape[-1] != 3 or tuple(g_logits.shape[:-1]) != tuple(ref.shape[:-1]):
-        raise ValueError(f"gate_combine: gate logits {tuple(g_logits.shape)} do not match branches {tuple(ref.shape)}")
-    for t in present:
-        if t.shape != ref.shape or t.dtype != ref.dtype:
-            raise ValueError("gate_combine: branches must share shape and dtype")
-    if g_logits.dtype != ref.dtype:
-        raise ValueError("gate_combine: gate logits must have the branches' dtype")
-    cont = lambda t: None if t is None else t.contiguous()
-    return g_logits.contiguous(), cont(o_cmp), cont(o_slc), cont(o_swa), ref
-
-
 def gate_combine(g_logits: torch.Tensor, o_cmp: Optional[torch.Tensor], o_slc: Optional[torch.Tensor],
                  o_swa: Optional[torch.Tensor], gate_mode: str = "sigmoid") -> torch.Tensor:
     """x = g_cmp*o_cmp + g_slc*o_slc + g_swa*o_swa with (g_cmp, g_slc, g_swa) = sigmoid / softmax of
-    clamp(g_logits, -10, 10); g_logits [..., H, 3], branches [..., H, D]; None skips a branch
-    (causal_wan_nsa_model.py:378-386, 541-546)."""
-    if gate_mode not in ("sigmoid", "softmax"):
-        raise NotImplementedError(f"gate_mode={gate_mode!r} not implemented")
-    g, a, b, c, ref = _gate_args(g_logits, o_cmp, o_slc, o_swa)
-    x = torch.empty_like(ref, memory_format=torch.contiguous_format)
-    D = ref.shape[-1]
-    with torch.cuda.device(ref.device):
-        call("nsa_gate_combine", g.data_ptr(), _ptr(a), _ptr(b), _ptr(c), x.data_ptr(), ref.numel() // D, D,
-             1 if gate_mode == "softmax" else 0, _dtype(ref), _stream(ref))
-    return x
+    clamp(g_logits, -10, 10); g_logits [..., H, 3] (may be a view into a wider projection), branches
+    [..., H, D]; None skips a branch (causal_wan_nsa_model.py:378-386, 541-546)."""
+    return host.gate_combine(g_logits, o_cmp, o_slc, o_swa, _softmax_gates(gate_mode))
 
 
 def gate_combine_bwd(g_logits, o_cmp, o_slc, o_swa, dx: torch.Tensor, gate_mode: str = "sigmoid"):
     """Gradients of gate_combine: (d_g_logits, d_o_cmp, d_o_slc, d_o_swa); None for skipped branches."""
+    return tuple(host.gate_combine_bwd(g_logits, o_cmp, o_slc, o_swa, dx, _softmax_gates(gate_mode)))
+
+
+def _softmax_gates(gate_mode: str) -> bool:
     if gate_mode not in ("sigmoid", "softmax"):
         raise NotImplementedError(f"gate_mode={gate_mode!r} not implemented")
-    g, a, b, c, ref = _gate_args(g_logits, o_cmp, o_slc, o_swa)
-    _require_cuda(dx)
-    dx = dx.contiguous()
-    dg = torch.empty_like(g)
-    outs = [None if t is None else torch.empty_like(t) for t in (a, b, c)]
-    D = ref.shape[-1]
-    with torch.cuda.device(ref.device):
-        call("nsa_gate_combine_bwd", g.data_ptr(), _ptr(a), _ptr(b), _ptr(c), dx.data_ptr(), dg.data_ptr(),
-             _ptr(outs[0]), _ptr(outs[1]), _ptr(outs[2]), ref.numel() // D, D,
-             1 if gate_mode == "softmax" else 0, _dtype(ref), _stream(ref))
-    return dg, outs[0], outs[1], outs[2]
+    return gate_mode == "softmax"
 
 
 def sel_bwd_dkv_ptr(q, base_k, base_v, base_dk, base_dv, n_blocks_per_head, groups, offsets, lse, delta, d_out,
