@@ -491,10 +491,11 @@ int nsa_residual_norm(const void* x, const void* y, const void* gate_mod, const 
 int nsa_rms_rows(const void* x, int64_t row_stride, const void* weight, void* out, int64_t rows, int32_t d,
                  float eps, int32_t dtype, void* stream);
 /* nsa_rms_rows over the H*D elements of every token of q and of k, rounded, then the rotary embedding of
- * nsa_rope_apply: q, k rows row_stride elements apart -> q_out, k_out [S,H,D] contiguous. */
+ * nsa_rope_apply: q, k rows row_stride elements apart -> q_out [S,H,D] contiguous, k_out rows k_out_stride
+ * elements apart (k_out == k with the same stride works in place). */
 int nsa_qk_norm_rope(const void* q, const void* k, int64_t row_stride, const void* q_weight, const void* k_weight,
-                     float eps, int64_t S, int32_t H, int32_t D, void* q_out, void* k_out, const nsa_rope* rope,
-                     int32_t dtype, void* stream);
+                     float eps, int64_t S, int32_t H, int32_t D, void* q_out, void* k_out, int64_t k_out_stride,
+                     const nsa_rope* rope, int32_t dtype, void* stream);
 
 /* The reference's K1 and K2 entry points with their own contracts (block_kv_ops.h:12-24):
  * desc int64 SoA [src_k|src_v|dst_k|dst_v|pub_k|pub_v] x n_fetch then clear x n_clear;

@@ -114,7 +114,7 @@ PROTOTYPES = {
                                     _vp, _vp, _i64, _vp, _vp]),
     "nsa_residual_norm": (_i32, [_vp] * 8 + [_i32, _vp, _vp, _i64, _i32, _f32, _i32, _vp]),
     "nsa_rms_rows": (_i32, [_vp, _i64, _vp, _vp, _i64, _i32, _f32, _i32, _vp]),
-    "nsa_qk_norm_rope": (_i32, [_vp, _vp, _i64, _vp, _vp, _f32, _i64, _i32, _i32, _vp, _vp, C.POINTER(Rope), _i32, _vp]),
+    "nsa_qk_norm_rope": (_i32, [_vp, _vp, _i64, _vp, _vp, _f32, _i64, _i32, _i32, _vp, _vp, _i64, C.POINTER(Rope), _i32, _vp]),
     "nsa_gather_publish_clear": (_i32, [_vp, _i64, _i64, _i64, _i32, _i32, C.POINTER(C.c_int64), _vp]),
     "nsa_block_range": (_i32, [_vp, _vp, _i32, _i64, _i64, _i64, _i64, _i64, _i64, _i64, _i64, _i32,
                                _i32, _i32, _vp]),

@@ -36,11 +36,13 @@ class RopeSpec:
     frame / row / column), `grid_hw` the latent rows and columns of a frame, `start_frame` the
     chunk's first frame, `pool` the (f, h, w) pooling window that defines the token order."""
 
-    def __init__(self, freqs: torch.Tensor, grid_hw, start_frame: int, pool=(1, 1, 1)):
+    def __init__(self, freqs: torch.Tensor, grid_hw, start_frame: int, pool=(1, 1, 1), like: Optional["RopeSpec"] = None):
+        """`like`: a RopeSpec over the same table, whose copies on the device are shared."""
         if freqs.dtype != torch.complex128 or freqs.dim() != 2:
             raise NSABackendError("RopeSpec: freqs must be a complex128 [max_len, D/2] table")
         self.freqs, self.grid_hw, self.start_frame, self.pool = freqs, tuple(grid_hw), int(start_frame), tuple(pool)
-        self._tables = self._native = None
+        self._tables = like._tables if like is not None and like.freqs is freqs else None
+        self._native = None
 
     def _split(self, device, D: int):
         c = D // 2

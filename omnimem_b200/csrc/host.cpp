@@ -600,17 +600,17 @@ Tensor rms_rows(const Tensor& x, const Tensor& weight, double eps) {
                                      static_cast<float>(eps), dtype_of(x), stream_of(x)));
   return out;
 }
-// q, k [S, H*D] views with a common row stride -> (q', k') [S,H,D]
-std::pair<Tensor, Tensor> qk_norm_rope(const Tensor& q, const Tensor& k, const Tensor& qw, const Tensor& kw, double eps, int64_t H, const Rope& rope) {
+// q, k [S, H*D] views with a common row stride -> q' [S,H,D]; k is overwritten with k'
+Tensor qk_norm_rope(const Tensor& q, const Tensor& k, const Tensor& qw, const Tensor& kw, double eps, int64_t H, const Rope& rope) {
   need_cuda({&q, &k});
   const c10::cuda::CUDAGuard guard(q.device());
   const int64_t S = q.size(0), D = q.size(1) / H;
   need(q.stride(0) == k.stride(0) && q.stride(1) == 1 && k.stride(1) == 1, "qk_norm_rope: q and k must share a row stride");
-  Tensor qo = at::empty({S, H, D}, q.options()), ko = at::empty({S, H, D}, q.options());
+  Tensor qo = at::empty({S, H, D}, q.options());
   const nsa_rope r = rope.c();
   check("nsa_qk_norm_rope", nsa_qk_norm_rope(q.data_ptr(), k.data_ptr(), q.stride(0), qw.data_ptr(), kw.data_ptr(), static_cast<float>(eps), S, H, D,
-                                             qo.data_ptr(), ko.data_ptr(), &r, dtype_of(q), stream_of(q)));
-  return {qo, ko};
+                                             qo.data_ptr(), k.data_ptr(), k.stride(0), &r, dtype_of(q), stream_of(q)));
+  return qo;
 }
 
 }  // namespace

@@ -156,7 +156,7 @@ struct QkParams : RopeParams {
   const char* q; const char* k;
   const void *qw, *kw;
   char* q_out; char* k_out;
-  int64_t S, row_stride;
+  int64_t S, row_stride, k_out_stride;
   int d, D;
   float eps;
 };
@@ -178,7 +178,7 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32) qk_norm_rope_kernel(const
 #pragma unroll
   for (int which = 0; which < 2; ++which) {
     const char* x = (which ? p.k : p.q) + t * p.row_stride * 2;
-    char* out = (which ? p.k_out : p.q_out) + t * p.d * 2;
+    char* out = which ? p.k_out + t * p.k_out_stride * 2 : p.q_out + t * p.d * 2;
     float v[C][8], sq = 0.f;
 #pragma unroll
     for (int c = 0; c < C; ++c) {
@@ -272,8 +272,8 @@ extern "C" int nsa_rms_rows(const void* x, int64_t row_stride, const void* weigh
 }
 
 extern "C" int nsa_qk_norm_rope(const void* q, const void* k, int64_t row_stride, const void* q_weight, const void* k_weight,
-                                float eps, int64_t S, int32_t H, int32_t D, void* q_out, void* k_out, const nsa_rope* rope,
-                                int32_t dtype, void* stream) {
+                                float eps, int64_t S, int32_t H, int32_t D, void* q_out, void* k_out, int64_t k_out_stride,
+                                const nsa_rope* rope, int32_t dtype, void* stream) {
   int rc;
   const int d = H * D;
   if ((rc = check_rows("qk_norm_rope", S, d, dtype))) return rc;
@@ -282,9 +282,9 @@ extern "C" int nsa_qk_norm_rope(const void* q, const void* k, int64_t row_stride
   if (S == 0) return NSA_OK;
   NSA_REQUIRE(q && k && q_weight && k_weight && q_out && k_out && rope, NSA_ERR_INVALID, "qk_norm_rope: null pointer");
   NSA_REQUIRE(aligned16(q) && aligned16(k) && aligned16(q_weight) && aligned16(k_weight) && aligned16(q_out) && aligned16(k_out) &&
-                  row_stride % 8 == 0, NSA_ERR_LAYOUT, "qk_norm_rope: rows must be 16-byte aligned");
+                  row_stride % 8 == 0 && k_out_stride % 8 == 0, NSA_ERR_LAYOUT, "qk_norm_rope: rows must be 16-byte aligned");
   QkParams p{{}, static_cast<const char*>(q), static_cast<const char*>(k), q_weight, k_weight, static_cast<char*>(q_out),
-             static_cast<char*>(k_out), S, row_stride, d, D, eps};
+             static_cast<char*>(k_out), S, row_stride, k_out_stride, d, D, eps};
   if ((rc = set_rope(rope, S, D, &p))) return rc;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   rc = with_pieces(d / 8, [&](auto c) -> int {

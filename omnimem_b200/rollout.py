@@ -13,11 +13,14 @@ attention over the last chunks, top-k block selection and selection attention ov
 history, gated sum, output projection.
 
 What runs where:
-  * linear layers, norms, cross-attention (SDPA), feed-forward: torch;
-  * key rotary embedding + pooling + page append (one kernel), query rotary embedding, query-group
-    pooling, scoring + top-k, LRU touch / evict / fetch, all THREE attention branches (the selection
-    forward kernel over the selected pages; the range forward kernel over the window's pages and
-    over the pooled history as a dense tensor), and the gated sum: this library.
+  * linear layers (the feed-forward's GELU in its epilogue), cross-attention (SDPA), embeddings: torch;
+  * residual add + layer norm + modulation (one kernel per stop of the residual stream), query / key norm +
+    rotary embedding (one kernel), pooling + page append (one kernel), query-group pooling, scoring + top-k,
+    LRU touch / evict / fetch, all THREE attention branches (the selection forward kernel over the selected
+    pages; the range forward kernel over the window's pages and over the pooled history as a dense tensor),
+    and the gated sum: this library.
+The fused form serves 16-bit activations without gradients, which is what a rollout is; anything else takes the
+eager form of the same layer.
 Tokens stay in (frame, row, column) order and a block is 64 consecutive tokens (the reference pools
 spatial tiles of 15 x 2 tokens; 64-token blocks cut across rows and chunk boundaries, which the block
 cache is built for).  The window starts at the block that holds its first token.
@@ -34,6 +37,7 @@ import torch.nn as nn
 import torch.nn.functional as F
 
 from . import ops
+from ._lib import host
 from .cache import BlockKVCache, RopeSpec, rope_apply
 from .nsa.ops.index_topk import should_use_selection_attention
 
@@ -140,6 +144,30 @@ class RMSNorm(nn.Module):
         return F.rms_norm(x.float(), (x.shape[-1],), self.weight.float(), self.eps).to(x.dtype)
 
 
+def _fused(x: torch.Tensor) -> bool:
+    """Whether the fused kernels serve activations x [.., d] (layer.cu): 16-bit, no gradients, rows they are built for."""
+    return x.is_cuda and x.dtype in (torch.bfloat16, torch.float16) and not torch.is_grad_enabled() \
+        and x.shape[-1] in (256, 512, 1024, 1536, 2048)
+
+
+class _MergedLinear:
+    """Several nn.Linear of one input as a single product: their weights one below the other, laid out once and
+    again whenever one of them has changed (new storage or an in-place update).  The outputs are padded to a
+    multiple of 64 columns so that every row keeps the alignment fast products want."""
+
+    def __init__(self, *mods: nn.Linear):
+        self.mods, self.key, self.weight, self.bias = mods, None, None, None
+
+    def __call__(self, x: torch.Tensor) -> torch.Tensor:
+        key = [(t.data_ptr(), t._version) for m in self.mods for t in (m.weight, m.bias)]
+        if key != self.key:
+            rows = sum(m.weight.shape[0] for m in self.mods)
+            w = torch.cat([m.weight.detach() for m in self.mods])
+            b = torch.cat([m.bias.detach() for m in self.mods])
+            self.weight, self.bias, self.key = F.pad(w, (0, 0, 0, -rows % 64)), F.pad(b, (0, -rows % 64)), key
+        return F.linear(x, self.weight, self.bias)
+
+
 class NSASelfAttention(nn.Module):
     """The rollout branch of CausalNSSelfAttention over a BlockKVCache."""
 
@@ -152,23 +180,37 @@ class NSASelfAttention(nn.Module):
         self.g_proj = nn.Linear(d, 3 * h)
         nn.init.normal_(self.g_proj.weight, mean=0.0, std=1e-3)     # gates start at 0.5 (initialize_gate, :164-168)
         nn.init.zeros_(self.g_proj.bias)
+        self._qkvg = _MergedLinear(self.q, self.k, self.v, self.g_proj)
 
     def forward(self, x, cache: BlockKVCache, rope: RopeSpec, start_token: int, timer=_NO_TIMER):
         p = self.plan
         _, S, _ = x.shape
         H, D = self.h, self.hd
-        with timer("qkv_gate_proj"):
-            q = self.norm_q(self.q(x)).view(S, H, D)
-            k = self.norm_k(self.k(x)).view(S, H, D)
-            v = self.v(x).view(S, H, D)
-            g = self.g_proj(x).view(1, S, H, 3)
         scale = D ** -0.5
-        # query rotary embedding; the keys receive theirs on the way into the pages, where they are also
-        # pooled: one kernel replaces rope + four cache updates + two poolings of the reference layer
-        with timer("rope_q"):
-            qr = rope_apply(q, rope).unsqueeze(0)
-        with timer("cache_append"):
-            cache.append(k, v, pos0=start_token, rope=rope)
+        if _fused(x) and 32 % (D // 8) == 0:
+            d = H * D
+            with timer("qkv_gate_proj"):
+                proj = self._qkvg(x[0])
+                q, k, v = proj[:, :d], proj[:, d:2 * d], proj[:, 2 * d:3 * d]
+                g = proj[:, 3 * d:3 * d + 3 * H].view(1, S, H, 3)
+            # norm and rotary embedding of queries and keys in one pass; the keys stay where they are
+            with timer("rope_q"):
+                qr = host.qk_norm_rope(q, k, self.norm_q.weight, self.norm_k.weight, self.norm_q.eps, H,
+                                       rope.native(x.device, D)).unsqueeze(0)
+            with timer("cache_append"):
+                cache.append(k.view(S, H, D), v.view(S, H, D), pos0=start_token)
+        else:
+            with timer("qkv_gate_proj"):
+                q = self.norm_q(self.q(x)).view(S, H, D)
+                k = self.norm_k(self.k(x)).view(S, H, D)
+                v = self.v(x).view(S, H, D)
+                g = self.g_proj(x).view(1, S, H, 3)
+            # query rotary embedding; the keys receive theirs on the way into the pages, where they are also
+            # pooled: one kernel replaces rope + four cache updates + two poolings of the reference layer
+            with timer("rope_q"):
+                qr = rope_apply(q, rope).unsqueeze(0)
+            with timer("cache_append"):
+                cache.append(k, v, pos0=start_token, rope=rope)
         nb = cache.n_blocks
         # compressed branch: attention over the pooled history, a dense [1, nb, H, D] view of the pooled
         # keys / values taken as one range of blocks
@@ -207,15 +249,26 @@ class CrossAttention(nn.Module):
         self.h, self.hd = h, d // h
         self.q, self.k, self.v, self.o = (nn.Linear(d, d) for _ in range(4))
         self.norm_q, self.norm_k = RMSNorm(d, shape.eps), RMSNorm(d, shape.eps)
+        self._kv = _MergedLinear(self.k, self.v)
 
     def forward(self, x, context):
-        B, S, _ = x.shape
+        B, S, d = x.shape
         L = context.shape[1]
+        if _fused(x):
+            heads = lambda t: t.unflatten(-1, (self.h, self.hd)).transpose(1, 2)
+            kv = self._kv(context)
+            q = heads(host.rms_rows(self.q(x), self.norm_q.weight, self.norm_q.eps))
+            k = heads(host.rms_rows(kv[..., :d], self.norm_k.weight, self.norm_k.eps))
+            y = F.scaled_dot_product_attention(q, k, heads(kv[..., d:2 * d]))
+            return self.o(y.transpose(1, 2).reshape(B, S, d))
         q = self.norm_q(self.q(x)).view(B, S, self.h, self.hd).transpose(1, 2)
         k = self.norm_k(self.k(context)).view(B, L, self.h, self.hd).transpose(1, 2)
         v = self.v(context).view(B, L, self.h, self.hd).transpose(1, 2)
         y = F.scaled_dot_product_attention(q, k, v)
         return self.o(y.transpose(1, 2).reshape(B, S, self.h * self.hd))
+
+
+_NO_VECTOR = (None, None)
 
 
 class Block(nn.Module):
@@ -228,6 +281,28 @@ class Block(nn.Module):
         self.cross_attn = CrossAttention(shape)
         self.ffn = nn.Sequential(nn.Linear(d, shape.ffn_dim), nn.GELU(approximate="tanh"), nn.Linear(shape.ffn_dim, d))
         self.modulation = nn.Parameter(torch.randn(1, 6, d) / d ** 0.5)
+
+    def fused(self, x, pending, e, context, cache, rope, start_token, timer=_NO_TIMER):
+        """forward() with the residual of the sub-layer in front still `pending` (its output and gate vector, or
+        None): returns (x, pending) for the next block.  e: the six fp32 rows of the time modulation."""
+        m = self.modulation[0].unbind(0)
+        vec = lambda i: (m[i], e[i])
+        y, gate = pending if pending is not None else (None, _NO_VECTOR)
+        with timer("norm_modulation"):
+            x, h = host.residual_norm(x, y, gate, vec(1), vec(0), True, True, self.eps)
+        y = self.self_attn(h, cache, rope, start_token, timer)
+        with timer("norm_modulation"):
+            x, h = host.residual_norm(x, y, vec(2), (self.norm3.weight, None), (self.norm3.bias, None), False, True,
+                                      self.norm3.eps)
+        with timer("cross_attn"):
+            y = self.cross_attn(h, context)
+        with timer("norm_modulation"):
+            x, h = host.residual_norm(x, y, _NO_VECTOR, vec(4), vec(3), True, True, self.eps)
+        with timer("ffn"):
+            up, down = self.ffn[0], self.ffn[2]
+            h = torch._addmm_activation(up.bias, h[0], up.weight.t(), use_gelu=True)     # tanh form, in the epilogue
+            y = F.linear(h, down.weight, down.bias).unsqueeze(0)
+        return x, (y, vec(5))
 
     def forward(self, x, e0, context, cache, rope, start_token, timer=_NO_TIMER):
         e = (self.modulation.float() + e0).unbind(1)                 # six [1, dim] rows (fp32, as the reference)
@@ -262,6 +337,7 @@ class CausalWanNSA(nn.Module):
         self.register_buffer("_dummy", torch.zeros(1), persistent=False)
         self.freqs = torch.cat([rope_table(1024, hd - 4 * (hd // 6)), rope_table(1024, 2 * (hd // 6)),
                                 rope_table(1024, 2 * (hd // 6))], dim=1)
+        self._rope = None                        # the last RopeSpec: its device tables serve the next forward
 
     def forward(self, latents, t, context_embedded, start_frame, caches: List[BlockKVCache], timer=_NO_TIMER):
         """latents [1, C, f, h, w]; t scalar timestep; returns the prediction in latent layout."""
@@ -273,13 +349,25 @@ class CausalWanNSA(nn.Module):
         temb = sinusoidal_embedding(sh.freq_dim, torch.full((1,), float(t), device=x.device)).to(x.dtype)
         e = self.time_embedding(temb)
         e0 = self.time_projection(e).float().view(1, 6, sh.dim)
-        rope = RopeSpec(self.freqs, (gh, gw), start_frame, (1, 1, 1))
+        rope = self._rope = RopeSpec(self.freqs, (gh, gw), start_frame, (1, 1, 1), like=self._rope)
         start_token = start_frame * gh * gw
+        if _fused(x):
+            pending, e_rows = None, e0[0].unbind(0)
+            for blk, cache in zip(self.blocks, caches):
+                x, pending = blk.fused(x, pending, e_rows, context_embedded, cache, rope, start_token, timer)
+            m, ef = self.head_modulation[0].unbind(0), e[0].float()
+            y, gate = pending if pending is not None else (None, _NO_VECTOR)
+            _, x = host.residual_norm(x, y, gate, (m[1], ef), (m[0], ef), True, True, self.head_norm_eps)
+            return self._unpatch(self.head(x), f, gh, gw)
         for blk, cache in zip(self.blocks, caches):
             x = blk(x, e0, context_embedded, cache, rope, start_token, timer)
         m = (self.head_modulation.float() + e.float().unsqueeze(1)).unbind(1)
         x = (F.layer_norm(x.float(), (sh.dim,), eps=self.head_norm_eps) * (1 + m[1]) + m[0]).to(x.dtype)
-        x = self.head(x)                                                # [1, S, out * pf*ph*pw]
+        return self._unpatch(self.head(x), f, gh, gw)
+
+    def _unpatch(self, x, f, gh, gw):
+        """[1, S, out * pf*ph*pw] -> latent layout"""
+        sh = self.shape
         pf, ph, pw = sh.patch
         x = x.view(1, f, gh, gw, pf, ph, pw, sh.out_dim).permute(0, 7, 1, 4, 2, 5, 3, 6)
         return x.reshape(1, sh.out_dim, f * pf, gh * ph, gw * pw)

@@ -1,0 +1,95 @@
+"""Row-wise kernels of a transformer layer (residual + norm + modulation, RMS norm, query / key norm + rotary embedding)
+against the eager expressions they replace, at rows of every built length."""
+import pytest
+import torch
+import torch.nn.functional as F
+
+from oracle import nsa_oracle as O
+
+pytestmark = pytest.mark.gpu
+
+# bf16 / fp16 results of fp32 arithmetic in another order: one unit in the last place of the largest terms
+ULP = {torch.bfloat16: 2.0 ** -7, torch.float16: 2.0 ** -10}
+
+
+def _close(got, want, dtype, terms=4.0):
+    tol = ULP[dtype] * terms
+    assert (got.float() - want.float()).abs().max() <= tol * max(1.0, want.float().abs().max().item())
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("rows,d", [(1, 8), (7, 248), (9, 256), (33, 520), (16, 1536), (5, 2048)])
+def test_residual_norm(dev, rows, d, dtype):
+    from omnimem_b200._lib import host
+    g = torch.Generator(device=dev).manual_seed(rows + d)
+    rand = lambda *s: torch.randn(*s, generator=g, device=dev)
+    x, y = rand(1, rows, d).to(dtype), rand(1, rows, d).to(dtype)
+    m, e = rand(3, d).to(dtype), rand(3, d)
+    eps, none = 1e-6, (None, None)
+    ln = lambda t: F.layer_norm(t.float(), (d,), eps=eps)
+    vec = lambda i: m[i].float() + e[i]
+    # no residual, modulated
+    got_x, got = host.residual_norm(x, None, none, (m[0], e[0]), (m[1], e[1]), True, True, eps)
+    assert torch.equal(got_x, x)
+    _close(got, (ln(x) * (1 + vec(0)) + vec(1)).to(dtype), dtype)
+    # gated residual, affine norm
+    x2 = x + (y.float() * vec(2)).to(dtype)
+    got_x, got = host.residual_norm(x, y, (m[2], e[2]), (m[0], None), (m[1], None), False, True, eps)
+    assert torch.equal(got_x, x2)
+    _close(got, F.layer_norm(x2, (d,), m[0], m[1], eps), dtype)
+    # plain residual without a norm
+    got_x, got = host.residual_norm(x, y, none, none, none, True, False, eps)
+    assert torch.equal(got_x, x + y) and got is None
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("H,D,grid", [(2, 128, (3, 5)), (4, 64, (4, 4)), (12, 128, (6, 7)), (8, 256, (1, 3))])
+def test_qk_norm_rope(dev, H, D, grid, dtype):
+    """Equal to the eager norm and the float64 rotary embedding up to the norm's last bit, keys in place."""
+    from omnimem_b200._lib import host
+    from omnimem_b200.cache import RopeSpec
+    from omnimem_b200.rollout import rope_table
+    d, frames, S = H * D, 2, 2 * grid[0] * grid[1]
+    g = torch.Generator(device=dev).manual_seed(d)
+    buf = torch.randn(S, 2 * d + 64, generator=g, device=dev).to(dtype)
+    qw, kw = (1 + 0.1 * torch.randn(2, d, generator=g, device=dev)).to(dtype).unbind(0)
+    freqs = torch.cat([rope_table(64, D - 4 * (D // 6)), rope_table(64, 2 * (D // 6)), rope_table(64, 2 * (D // 6))], 1)
+    rope = RopeSpec(freqs, grid, 3)
+    q, k = buf[:, :d], buf[:, d:2 * d]
+    rms = lambda t, w: F.rms_norm(t.float(), (d,), w.float(), 1e-6).to(dtype)
+    want = [O.reorder_rope_apply(rms(t, w).view(S, H, D).cpu(), (frames, *grid), freqs, 3, (1, 1, 1)) for t, w in ((q, qw), (k, kw))]
+    tail = buf[:, 2 * d:].clone()
+    got_q = host.qk_norm_rope(q, k, qw, kw, 1e-6, H, rope.native(dev, D))
+    _close(got_q.cpu(), want[0], dtype)
+    _close(k.reshape(S, H, D).cpu(), want[1], dtype)
+    assert torch.equal(buf[:, 2 * d:], tail)
+    _close(host.rms_rows(buf[:, :d], qw, 1e-6), rms(buf[:, :d], qw), dtype)
+
+
+def test_touch_without_lists_stamps_and_counts_like_the_lists(dev):
+    from omnimem_b200.cache import BlockKVCache
+    H, D, MB = 3, 128, 40
+    g = torch.Generator().manual_seed(2)
+    caches = [BlockKVCache(H, D, H * MB, MB, device=dev, host_tier=False) for _ in range(2)]
+    kv = torch.randn(20 * 64, H, D, generator=g).to(torch.bfloat16).to(dev)
+    ids = torch.randint(-1, 30, (1, 7, H, 5), generator=g, dtype=torch.int32).to(dev)       # some without a page, some -1
+    for c in caches:
+        c.append(kv, kv)
+    caches[0].touch(ids)
+    caches[1].touch(ids, return_lists=True)
+    assert torch.equal(caches[0].counters, caches[1].counters) and torch.equal(caches[0].page_stamp, caches[1].page_stamp)
+    assert caches[0].stats()["misses"] > 0 and caches[0].stats()["hits"] > 0
+
+
+def test_merged_projections_follow_their_modules(dev):
+    """The weights laid out for one product are laid out again when a module's weight changes."""
+    from omnimem_b200.rollout import _MergedLinear
+    a, b = (torch.nn.Linear(64, n, device=dev, dtype=torch.bfloat16) for n in (96, 20))
+    merged, x = _MergedLinear(a, b), torch.randn(5, 64, device=dev).to(torch.bfloat16)
+    with torch.no_grad():
+        for change in (lambda: None, lambda: a.weight.mul_(2), lambda: setattr(b, "bias", torch.nn.Parameter(torch.ones_like(b.bias)))):
+            change()
+            y = merged(x)
+            assert y.shape == (5, 128)
+            for got, want in ((y[:, :96], a(x)), (y[:, 96:116], b(x))):
+                assert (got.float() - want.float()).abs().max() <= 2 ** -6 * want.float().abs().max()
