@@ -145,31 +145,84 @@ class RMSNorm(nn.Module):
 
 
 def _fused(x: torch.Tensor) -> bool:
-    """Whether the fused kernels serve activations x [.., d] (layer.cu): 16-bit, no gradients, rows they are built for."""
+    """Whether the fused kernels serve activations x [.., d] (layer.cu): 16-bit, no gradients, no autocast, rows they are
+    built for."""
     return x.is_cuda and x.dtype in (torch.bfloat16, torch.float16) and not torch.is_grad_enabled() \
-        and x.shape[-1] in (256, 512, 1024, 1536, 2048)
+        and not torch.is_autocast_enabled("cuda") and x.shape[-1] in (256, 512, 1024, 1536, 2048)
 
 
-class _MergedLinear:
-    """Several nn.Linear of one input as a single product: their weights one below the other, laid out once and
-    again whenever one of them has changed (new storage or an in-place update).  The outputs are padded to a
-    multiple of 64 columns so that every row keeps the alignment fast products want."""
-
-    def __init__(self, *mods: nn.Linear):
-        self.mods, self.key, self.weight, self.bias = mods, None, None, None
-
-    def __call__(self, x: torch.Tensor) -> torch.Tensor:
-        key = [(t.data_ptr(), t._version) for m in self.mods for t in (m.weight, m.bias)]
-        if key != self.key:
-            rows = sum(m.weight.shape[0] for m in self.mods)
-            w = torch.cat([m.weight.detach() for m in self.mods])
-            b = torch.cat([m.bias.detach() for m in self.mods])
-            self.weight, self.bias, self.key = F.pad(w, (0, 0, 0, -rows % 64)), F.pad(b, (0, -rows % 64)), key
-        return F.linear(x, self.weight, self.bias)
+def _plain(dtype: torch.dtype, *mods: nn.Module) -> bool:
+    """Whether the parameters of `mods` may be used without calling them: the layers built here (not something a user
+    put in their place), no hooks, parameters of the activations' type."""
+    return all(type(m) in _PLAIN and not m._forward_hooks and not m._forward_pre_hooks and m.weight.dtype == dtype
+               for m in mods)
 
 
-class NSASelfAttention(nn.Module):
+_PLAIN = (nn.Linear, nn.LayerNorm, RMSNorm)
+
+
+class _Packed(nn.Module):
+    """A module whose linear layers of one input (`packed`) keep their weights one below the other in one storage, so
+    that a single product serves them.  The layers own their parameters as ever: updates in place are seen, and where
+    a parameter has moved to a storage of its own the product falls apart into one per layer.  The rows are padded to
+    a multiple of 64, so that every row of the output keeps the alignment that fast products want."""
+
+    packed: tuple = ()
+
+    def _apply(self, fn, *args, **kwargs):
+        super()._apply(fn, *args, **kwargs)
+        mods = [getattr(self, n) for n in self.packed]
+        if all(type(m) is nn.Linear and m.weight.is_cuda for m in mods) and self._joined(mods) is None \
+                and len({(m.weight.dtype, m.weight.device, m.in_features) for m in mods}) == 1:
+            rows = sum(m.out_features for m in mods)
+            weight = mods[0].weight.new_zeros(rows + -rows % 64, mods[0].in_features, requires_grad=False)
+            bias = weight.new_zeros(rows + -rows % 64)
+            at = 0
+            for m in mods:
+                for whole, t in ((weight, m.weight), (bias, m.bias)):
+                    part = whole[at:at + m.out_features]
+                    part.copy_(t.data)
+                    t.data = part
+                at += m.out_features
+        return self
+
+    @staticmethod
+    def _joined(mods):
+        """(weight, bias) of the layers as one, padded, or None if they do not lie so."""
+        out = []
+        for ts in ([m.weight for m in mods], [m.bias for m in mods]):
+            first = ts[0]
+            row = first.numel() // first.shape[0]
+            rows = sum(t.shape[0] for t in ts)
+            rows += -rows % 64
+            at, home = first.data_ptr(), first.untyped_storage()
+            if first.storage_offset() + rows * row > home.nbytes() // first.element_size():
+                return None
+            for t in ts:
+                if t.data_ptr() != at or not t.is_contiguous() or t.dtype != first.dtype \
+                        or t.untyped_storage().data_ptr() != home.data_ptr():
+                    return None
+                at += t.numel() * t.element_size()
+            out.append(first.detach().as_strided((rows,) + tuple(first.shape[1:]), first.stride()))
+        return out
+
+    def project(self, x: torch.Tensor):
+        """The layers' outputs of x [.., d] (views of one tensor where the weights lie together)."""
+        mods = [getattr(self, n) for n in self.packed]
+        joined = self._joined(mods)
+        if joined is None:
+            return [F.linear(x, m.weight, m.bias) for m in mods]
+        y, at, out = F.linear(x, *joined), 0, []
+        for m in mods:
+            out.append(y[..., at:at + m.out_features])
+            at += m.out_features
+        return out
+
+
+class NSASelfAttention(_Packed):
     """The rollout branch of CausalNSSelfAttention over a BlockKVCache."""
+
+    packed = ("q", "k", "v", "g_proj")
 
     def __init__(self, shape: WanShape, plan: RolloutPlan, layer_idx: int):
         super().__init__()
@@ -180,19 +233,17 @@ class NSASelfAttention(nn.Module):
         self.g_proj = nn.Linear(d, 3 * h)
         nn.init.normal_(self.g_proj.weight, mean=0.0, std=1e-3)     # gates start at 0.5 (initialize_gate, :164-168)
         nn.init.zeros_(self.g_proj.bias)
-        self._qkvg = _MergedLinear(self.q, self.k, self.v, self.g_proj)
 
     def forward(self, x, cache: BlockKVCache, rope: RopeSpec, start_token: int, timer=_NO_TIMER):
         p = self.plan
         _, S, _ = x.shape
         H, D = self.h, self.hd
         scale = D ** -0.5
-        if _fused(x) and 32 % (D // 8) == 0:
-            d = H * D
+        if _fused(x) and 32 % (D // 8) == 0 and \
+                _plain(x.dtype, self.q, self.k, self.v, self.g_proj, self.norm_q, self.norm_k):
             with timer("qkv_gate_proj"):
-                proj = self._qkvg(x[0])
-                q, k, v = proj[:, :d], proj[:, d:2 * d], proj[:, 2 * d:3 * d]
-                g = proj[:, 3 * d:3 * d + 3 * H].view(1, S, H, 3)
+                q, k, v, g = self.project(x[0])
+                g = g.view(1, S, H, 3)
             # norm and rotary embedding of queries and keys in one pass; the keys stay where they are
             with timer("rope_q"):
                 qr = host.qk_norm_rope(q, k, self.norm_q.weight, self.norm_k.weight, self.norm_q.eps, H,
@@ -242,24 +293,25 @@ class NSASelfAttention(nn.Module):
         return out
 
 
-class CrossAttention(nn.Module):
+class CrossAttention(_Packed):
+    packed = ("k", "v")
+
     def __init__(self, shape: WanShape):
         super().__init__()
         d, h = shape.dim, shape.num_heads
         self.h, self.hd = h, d // h
         self.q, self.k, self.v, self.o = (nn.Linear(d, d) for _ in range(4))
         self.norm_q, self.norm_k = RMSNorm(d, shape.eps), RMSNorm(d, shape.eps)
-        self._kv = _MergedLinear(self.k, self.v)
 
     def forward(self, x, context):
         B, S, d = x.shape
         L = context.shape[1]
-        if _fused(x):
+        if _fused(x) and _plain(x.dtype, self.k, self.v, self.norm_q, self.norm_k) and context.dtype == x.dtype:
             heads = lambda t: t.unflatten(-1, (self.h, self.hd)).transpose(1, 2)
-            kv = self._kv(context)
+            k, v = self.project(context)
             q = heads(host.rms_rows(self.q(x), self.norm_q.weight, self.norm_q.eps))
-            k = heads(host.rms_rows(kv[..., :d], self.norm_k.weight, self.norm_k.eps))
-            y = F.scaled_dot_product_attention(q, k, heads(kv[..., d:2 * d]))
+            k = heads(host.rms_rows(k, self.norm_k.weight, self.norm_k.eps))
+            y = F.scaled_dot_product_attention(q, k, heads(v))
             return self.o(y.transpose(1, 2).reshape(B, S, d))
         q = self.norm_q(self.q(x)).view(B, S, self.h, self.hd).transpose(1, 2)
         k = self.norm_k(self.k(context)).view(B, L, self.h, self.hd).transpose(1, 2)
@@ -281,6 +333,12 @@ class Block(nn.Module):
         self.cross_attn = CrossAttention(shape)
         self.ffn = nn.Sequential(nn.Linear(d, shape.ffn_dim), nn.GELU(approximate="tanh"), nn.Linear(shape.ffn_dim, d))
         self.modulation = nn.Parameter(torch.randn(1, 6, d) / d ** 0.5)
+
+    def fusable(self, dtype: torch.dtype) -> bool:
+        up, act, down = self.ffn if len(self.ffn) == 3 else (None, None, None)
+        return type(self) is Block and not self._forward_hooks and not self._forward_pre_hooks \
+            and type(act) is nn.GELU and act.approximate == "tanh" and not self.ffn._forward_hooks \
+            and not self.ffn._forward_pre_hooks and self.modulation.dtype == dtype and _plain(dtype, up, down, self.norm3)
 
     def fused(self, x, pending, e, context, cache, rope, start_token, timer=_NO_TIMER):
         """forward() with the residual of the sub-layer in front still `pending` (its output and gate vector, or
@@ -351,7 +409,7 @@ class CausalWanNSA(nn.Module):
         e0 = self.time_projection(e).float().view(1, 6, sh.dim)
         rope = self._rope = RopeSpec(self.freqs, (gh, gw), start_frame, (1, 1, 1), like=self._rope)
         start_token = start_frame * gh * gw
-        if _fused(x):
+        if _fused(x) and self.head_modulation.dtype == x.dtype and all(b.fusable(x.dtype) for b in self.blocks):
             pending, e_rows = None, e0[0].unbind(0)
             for blk, cache in zip(self.blocks, caches):
                 x, pending = blk.fused(x, pending, e_rows, context_embedded, cache, rope, start_token, timer)

@@ -81,15 +81,32 @@ def test_touch_without_lists_stamps_and_counts_like_the_lists(dev):
     assert caches[0].stats()["misses"] > 0 and caches[0].stats()["hits"] > 0
 
 
-def test_merged_projections_follow_their_modules(dev):
-    """The weights laid out for one product are laid out again when a module's weight changes."""
-    from omnimem_b200.rollout import _MergedLinear
-    a, b = (torch.nn.Linear(64, n, device=dev, dtype=torch.bfloat16) for n in (96, 20))
-    merged, x = _MergedLinear(a, b), torch.randn(5, 64, device=dev).to(torch.bfloat16)
+def test_packed_projections_follow_their_layers(dev):
+    """One product over layers whose weights lie together sees every way in which a parameter or a layer can change."""
+    from omnimem_b200.rollout import CrossAttention, WanShape, _plain
+    m = CrossAttention(WanShape(dim=256, num_heads=2)).to(device=dev, dtype=torch.bfloat16)
+    x = torch.randn(5, 256, device=dev).to(torch.bfloat16)
+
+    def same():
+        for got, layer in zip(m.project(x), (m.k, m.v)):
+            want = layer(x)
+            assert got.shape == want.shape and (got.float() - want.float()).abs().max() <= 2 ** -6 * want.float().abs().max()
+
+    state = {n: t.clone() for n, t in m.state_dict().items()}
+    fresh = lambda: torch.nn.Parameter(torch.randn_like(m.v.bias))
     with torch.no_grad():
-        for change in (lambda: None, lambda: a.weight.mul_(2), lambda: setattr(b, "bias", torch.nn.Parameter(torch.ones_like(b.bias)))):
+        assert m._joined((m.k, m.v)) is not None
+        changes = (lambda: m.k.weight.mul_(2), lambda: m.k.weight.data.copy_(torch.randn_like(m.k.weight)),
+                   lambda: m.load_state_dict(state), lambda: setattr(m.v, "bias", fresh()),
+                   lambda: m.to(dtype=torch.float32).to(dtype=torch.bfloat16), lambda: setattr(m.v, "bias", fresh()),
+                   lambda: setattr(m.v.weight, "data", torch.randn_like(m.v.weight)),
+                   lambda: m.load_state_dict(state, assign=True))
+        same()
+        for change in changes:
             change()
-            y = merged(x)
-            assert y.shape == (5, 128)
-            for got, want in ((y[:, :96], a(x)), (y[:, 96:116], b(x))):
-                assert (got.float() - want.float()).abs().max() <= 2 ** -6 * want.float().abs().max()
+            same()
+    assert _plain(torch.bfloat16, m.k, m.v) and not _plain(torch.float16, m.k)
+    m.k.register_forward_hook(lambda *a: None)
+    assert not _plain(torch.bfloat16, m.k)
+    m.v = torch.nn.Sequential(m.v)
+    assert not _plain(torch.bfloat16, m.v)
