@@ -340,7 +340,7 @@ void give_flag(const Flag& f) {
 // are out of range are skipped by the kernels, so a forward that was wrong to launch does no harm).
 struct IdCheck {
   Flag flag;
-  bool live = false;
+  bool live = false, waited = false;
   IdCheck(const Tensor& ids, int64_t limit) {
     if (ids.numel() == 0) return;
     flag = take_flag(ids.device().index());
@@ -357,10 +357,12 @@ struct IdCheck {
       e = cudaEventSynchronize(flag.event);
     }
     C10_CUDA_CHECK(e);
+    waited = true;
     return *static_cast<volatile int32_t*>(flag.word) != 0;
   }
   ~IdCheck() {
-    if (live) give_flag(flag);
+    // a forward that threw leaves the check in flight: its word serves no other call before it has run
+    if (live && (waited || cudaEventSynchronize(flag.event) == cudaSuccess)) give_flag(flag);
   }
   IdCheck(const IdCheck&) = delete;
 };
