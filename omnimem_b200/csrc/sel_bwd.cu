@@ -263,7 +263,7 @@ __global__ void __launch_bounds__(32 * W * KS, W == 4 && D == 128 ? 3 : 1) sel_b
   const uint32_t ring_bytes = static_cast<uint32_t>(stages) * 2 * kRingTile<D, ROWS>;
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + KS * ring_bytes);
   int* words = reinterpret_cast<int*>(bars + KS * kRingBars);                          // abort, tile count
-  RingTile* list = reinterpret_cast<RingTile*>(words + 4);
+  RingSlot* list = reinterpret_cast<RingSlot*>(words + 4);
   if (warp == 0) {
     const int count = ring_list<ESZ>(list, p.kv, p.ids, b * p.i_sb + g * p.i_sg + h * p.i_sh, p.i_st, p.T, b, h, D,
                                      p.block_size, p.chunk_size, p.causal != 0, static_cast<int>(g0 / p.chunk_size));
@@ -275,7 +275,8 @@ __global__ void __launch_bounds__(32 * W * KS, W == 4 && D == 128 ? 3 : 1) sel_b
   __syncthreads();
   ring.count = KS > 1 ? (words[1] - part + KS - 1) / KS : words[1];
   const RingSource src = kv_ring_source<ESZ>(p.kv, maps, p.B, b, h, D, p.block_size);
-  const auto tile_of = [&](int i) { return list[part + i * KS]; };
+  const int per_block = (p.block_size + ROWS - 1) / ROWS;
+  const auto tile_of = [&](int i) { return ring_tile(list, part + i * KS, per_block, src); };
   ring.start(src, tile_of);
 
   // delta = sum_d O * dO of this thread's rows (lo, hi), from the fragments of both
@@ -306,7 +307,8 @@ __global__ void __launch_bounds__(32 * W * KS, W == 4 && D == 128 ? 3 : 1) sel_b
   for (int n = 0; n < D / 8; ++n) dq[n][0] = dq[n][1] = dq[n][2] = dq[n][3] = 0.f;
   bool ok = true;
   for (int i = 0; i < ring.count && ok; ++i) {
-    const int n = list[part + i * KS].n, brought = list[part + i * KS].clear;
+    const RingTile now = tile_of(i);
+    const int n = now.n, brought = now.clear;
     const int n16 = (n + 15) >> 4;
     float s[ROWS / 8][4], dp[ROWS / 8][4];
 #pragma unroll
@@ -539,9 +541,8 @@ sel_bwd_dkv_rows_kernel(const __grid_constant__ RingMaps maps, const BwdParams p
         }
         pa[0][j * 2] = pack2<T>(st[j][0], st[j][1]);
         pa[0][j * 2 + 1] = pack2<T>(st[j][2], st[j][3]);
-        const float2 p01 = unpack2<T>(pa[0][j * 2]), p23 = unpack2<T>(pa[0][j * 2 + 1]);
-        ds[0][j * 2] = pack2<T>(p01.x * (dp[j][0] - dls[0]) * p.scale, p01.y * (dp[j][1] - dls[1]) * p.scale);
-        ds[0][j * 2 + 1] = pack2<T>(p23.x * (dp[j][2] - dls[0]) * p.scale, p23.y * (dp[j][3] - dls[1]) * p.scale);
+        ds[0][j * 2] = pack2<T>(st[j][0] * (dp[j][0] - dls[0]) * p.scale, st[j][1] * (dp[j][1] - dls[1]) * p.scale);
+        ds[0][j * 2 + 1] = pack2<T>(st[j][2] * (dp[j][2] - dls[0]) * p.scale, st[j][3] * (dp[j][3] - dls[1]) * p.scale);
       }
       mma_rows<T, D, 16>(dv, pa, dt, 1);
       mma_rows<T, D, 16>(dk, ds, qt, 1);
@@ -578,13 +579,12 @@ sel_bwd_dkv_rows_kernel(const __grid_constant__ RingMaps maps, const BwdParams p
 
 template <typename T, int D, int W, int KS, bool TMA>
 int launch_dq_rows(const RingMaps& maps, const BwdParams& p, int32_t* status, cudaStream_t stream) {
-  const int tiles = p.T * cdiv(p.block_size, 32);
   constexpr int stages = W <= 2 ? 1 : 3;                    // as in the forward
   static_assert(W * 16 * (D * 2 + 16) <= stages * 2 * kRingTile<D, 32>, "the epilogue stages its rows in the ring");
   static_assert((KS - 1) * (D / 8 * 512) <= KS * 2 * kRingTile<D, 32>, "the partial results are summed in the ring");
   const size_t smem = static_cast<size_t>(KS) * stages * 2 * kRingTile<D, 32> + KS * kRingBars * 8 + 16 +
-                      static_cast<size_t>(tiles) * sizeof(RingTile);
-  NSA_REQUIRE(smem <= 220 * 1024, NSA_ERR_UNSUPPORTED, "sel_bwd: T=%d needs too much shared memory", p.T);
+                      ring_list_bytes(p.T);
+  NSA_REQUIRE(smem <= 226 * 1024, NSA_ERR_UNSUPPORTED, "sel_bwd: T=%d needs too much shared memory", p.T);
   auto kernel = sel_bwd_dq_rows_kernel<T, D, W, KS, TMA>;
   NSA_CUDA_OK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
   kernel<<<dim3(p.MG, p.H, p.B), 32 * W * KS, smem, stream>>>(maps, p, stages, status);

@@ -45,7 +45,7 @@ __global__ void __launch_bounds__(32 * W * KS) sel_fwd_rows_kernel(const __grid_
   const uint32_t ring_bytes = static_cast<uint32_t>(stages) * 2 * kRingTile<D, ROWS>;
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + KS * ring_bytes);
   int* words = reinterpret_cast<int*>(bars + KS * kRingBars);                          // abort, tile count
-  RingTile* list = reinterpret_cast<RingTile*>(words + 4);
+  RingSlot* list = reinterpret_cast<RingSlot*>(words + 4);
   if (warp == 0) {
     const int count = ring_list<ESZ>(list, p.kv, p.ids, b * p.i_sb + g * p.i_sg + h * p.i_sh, p.i_st, p.T, b, h, D,
                                      p.block_size, p.chunk_size, p.causal != 0, static_cast<int>(g0 / p.chunk_size));
@@ -57,7 +57,8 @@ __global__ void __launch_bounds__(32 * W * KS) sel_fwd_rows_kernel(const __grid_
   __syncthreads();
   ring.count = KS > 1 ? (words[1] - part + KS - 1) / KS : words[1];
   const RingSource src = kv_ring_source<ESZ>(p.kv, maps, p.B, b, h, D, p.block_size);
-  const auto tile_of = [&](int i) { return list[part + i * KS]; };
+  const int per_block = (p.block_size + ROWS - 1) / ROWS;
+  const auto tile_of = [&](int i) { return ring_tile(list, part + i * KS, per_block, src); };
   ring.start(src, tile_of);
 
   float o[D / 8][4];
@@ -69,7 +70,8 @@ __global__ void __launch_bounds__(32 * W * KS) sel_fwd_rows_kernel(const __grid_
 
   bool ok = true;
   for (int i = 0; i < ring.count && ok; ++i) {
-    const int n = list[part + i * KS].n, brought = list[part + i * KS].clear;
+    const RingTile now = tile_of(i);
+    const int n = now.n, brought = now.clear;
     if (!ring.template wait<0>()) { ok = false; break; }
     const int n16 = (n + 15) >> 4;
     float s[4][4];
@@ -77,6 +79,11 @@ __global__ void __launch_bounds__(32 * W * KS) sel_fwd_rows_kernel(const __grid_
     for (int j = 0; j < 4; ++j) s[j][0] = s[j][1] = s[j][2] = s[j][3] = 0.f;
     mma_rows_t<T, D, ROWS>(s, q, ring.tile(0), n16);
     ok = ring.template release<0>(i, src, tile_of);
+    // scaled first, then masked: the scale may be zero or negative
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) s[j][e] *= p.scale_log2;
     if (n < ROWS) {
 #pragma unroll
       for (int j = 0; j < 4; ++j)
@@ -89,7 +96,7 @@ __global__ void __launch_bounds__(32 * W * KS) sel_fwd_rows_kernel(const __grid_
     for (int r = 0; r < 2; ++r) {
       mx[r] = -INFINITY;
 #pragma unroll
-      for (int j = 0; j < 4; ++j) mx[r] = fmaxf(mx[r], fmaxf(s[j][2 * r], s[j][2 * r + 1]) * p.scale_log2);
+      for (int j = 0; j < 4; ++j) mx[r] = fmaxf(mx[r], fmaxf(s[j][2 * r], s[j][2 * r + 1]));
       mx[r] = fmaxf(mx[r], __shfl_xor_sync(0xffffffffu, mx[r], 1));
       mx[r] = fmaxf(mx[r], __shfl_xor_sync(0xffffffffu, mx[r], 2));
     }
@@ -110,7 +117,7 @@ __global__ void __launch_bounds__(32 * W * KS) sel_fwd_rows_kernel(const __grid_
     for (int j = 0; j < 4; ++j) {
       float e[4];
 #pragma unroll
-      for (int x = 0; x < 4; ++x) e[x] = fast_exp2(s[j][x] * p.scale_log2 - m_ref[x >> 1]);
+      for (int x = 0; x < 4; ++x) e[x] = fast_exp2(s[j][x] - m_ref[x >> 1]);
       l_i[0] += e[0] + e[1];
       l_i[1] += e[2] + e[3];
       pa[j >> 1][(j & 1) * 2] = pack2<T>(e[0], e[1]);
@@ -181,15 +188,14 @@ __global__ void __launch_bounds__(32 * W * KS) sel_fwd_rows_kernel(const __grid_
 
 template <typename T, int D, int W, int KS, bool TMA>
 int launch_rows(const RingMaps& maps, const FwdParams& p, int MG, int32_t* status, cudaStream_t stream) {
-  const int tiles = p.T * cdiv(p.block_size, 32);
   // stages: two per ring of a single warp (the thread blocks that share an SM are the depth), three where several
   // warps wait for the same ring; never less than the epilogue's staging needs
   const int stages = W <= 2 ? 1 : 3;
   static_assert(W * 16 * (D * 2 + 16) <= (W <= 2 ? 1 : 3) * 2 * kRingTile<D, 32>, "the epilogue stages its rows in the ring");
   static_assert((KS - 1) * (D / 8 * 128 + 128) * 4 <= KS * 2 * kRingTile<D, 32>, "the partial results are merged in the ring");
   const size_t smem = static_cast<size_t>(KS) * stages * 2 * kRingTile<D, 32> + KS * kRingBars * 8 + 16 +
-                      static_cast<size_t>(tiles) * sizeof(RingTile);
-  NSA_REQUIRE(smem <= 220 * 1024, NSA_ERR_UNSUPPORTED, "sel_fwd: T=%d needs too much shared memory", p.T);
+                      ring_list_bytes(p.T);
+  NSA_REQUIRE(smem <= 226 * 1024, NSA_ERR_UNSUPPORTED, "sel_fwd: T=%d needs too much shared memory", p.T);
   auto kernel = sel_fwd_rows_kernel<T, D, W, KS, TMA>;
   NSA_CUDA_OK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
   kernel<<<dim3(MG, p.H, p.B), 32 * W * KS, smem, stream>>>(maps, p, stages, status);

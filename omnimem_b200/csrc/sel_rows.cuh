@@ -296,14 +296,21 @@ struct Ring {
   }
 };
 
-// The visible 32-row tiles of one (batch, group, head) list, in list order, written by one warp; returns their number.
+// A visible block of one (batch, group, head) list: its 32-row tiles are tiles [first, first of the next slot).
+struct RingSlot {
+  uint64_t a, b;       // addresses of row 0
+  int unit, n_vis;     // rows that count
+  int there, first;    // rows that a copy brings
+};
+inline size_t ring_list_bytes(int T) { return (static_cast<size_t>(T) + 1) * sizeof(RingSlot); }
+
+// The visible blocks of a list, in list order and with a sentinel at the end, written by one warp; returns their tiles.
 template <int ESZ>
-__device__ __forceinline__ int ring_list(RingTile* out, const KVSrc& kv, const int32_t* ids, int64_t ids_off, int64_t ids_st,
+__device__ __forceinline__ int ring_list(RingSlot* out, const KVSrc& kv, const int32_t* ids, int64_t ids_off, int64_t ids_st,
                                          int T, int b, int h, int D, int block_size, int chunk_size, bool causal, int q_chunk) {
   constexpr int ROWS = 32;
   const int lane = threadIdx.x & 31;
-  const int64_t k_row = kv_row_bytes(kv, false, D, ESZ), v_row = kv_row_bytes(kv, true, D, ESZ);
-  int count = 0;
+  int count = 0, slots = 0;
   for (int t0 = 0; t0 < T; t0 += 32) {
     BlockRef r{nullptr, nullptr, 0};
     int unit = 0;
@@ -330,23 +337,34 @@ __device__ __forceinline__ int ring_list(RingTile* out, const KVSrc& kv, const i
       const int y = __shfl_up_sync(0xffffffffu, upto, d);
       if (lane >= d) upto += y;
     }
-    for (int i = 0; i < mine; ++i) {
-      RingTile w;
-      w.a = reinterpret_cast<uint64_t>(r.k) + static_cast<int64_t>(i) * ROWS * k_row;
-      w.b = reinterpret_cast<uint64_t>(r.v) + static_cast<int64_t>(i) * ROWS * v_row;
-      w.unit = unit;
-      w.r0 = i * ROWS;
-      w.n = min(ROWS, r.n_vis - i * ROWS);
+    const uint32_t some = __ballot_sync(0xffffffffu, mine > 0);
+    if (mine > 0) {
       // (a cut-off last block of a dense tensor: what follows it is outside the tensor and arrives as zeros)
       const int64_t there = kv.mode == NSA_KV_DENSE ? kv.n_tokens - static_cast<int64_t>(unit) * block_size : block_size;
-      w.clear = min(ROWS, static_cast<int>(there < block_size ? there : block_size) - i * ROWS);
-      w.aux = 0;
-      out[count + upto - mine + i] = w;
+      out[slots + __popc(some & ((1u << lane) - 1))] =
+          RingSlot{reinterpret_cast<uint64_t>(r.k), reinterpret_cast<uint64_t>(r.v), unit, r.n_vis,
+                   static_cast<int>(there < block_size ? there : block_size), count + upto - mine};
     }
+    slots += __popc(some);
     count += __shfl_sync(0xffffffffu, upto, 31);
   }
+  if (lane == 0) out[slots].first = count;
   __syncwarp();
   return count;
+}
+
+// Tile i of a list: no block has more than `per_block` tiles and few (cut off, partly visible) have less, so the search
+// starts at slot i / per_block and hardly ever goes on.
+__device__ __forceinline__ const RingSlot& ring_slot(const RingSlot* list, int i, int per_block) {
+  if (per_block == 1) return list[i];
+  int s = i / per_block;
+  while (list[s + 1].first <= i) ++s;
+  return list[s];
+}
+__device__ __forceinline__ RingTile ring_tile(const RingSlot* list, int i, int per_block, const RingSource& src) {
+  const RingSlot& w = ring_slot(list, i, per_block);
+  const int r0 = (i - w.first) * 32;
+  return RingTile{w.a + r0 * src.a_row, w.b + r0 * src.b_row, w.unit, r0, min(32, w.n_vis - r0), min(32, w.there - r0), 0};
 }
 
 template <int ESZ>

@@ -95,3 +95,17 @@ def test_values_outside_the_list_do_not_leak(dev):
     out, lse = ops.sel_fwd(q, kv, ids, 30, 1, 128 ** -0.5, False, 15)
     grads = ops.sel_bwd(q, kv, ids, out, lse, do, 30, 1, 128 ** -0.5, False, 15)
     assert all(bool(torch.isfinite(t).all()) for t in (out, lse, *grads))
+
+
+@pytest.mark.parametrize("scale", [0.0, -0.1])
+def test_scales_that_are_not_positive(dev, scale):
+    """Masked columns stay masked whatever the sign of the scale (ragged tiles, causal limits inside a block)."""
+    from omnimem_b200 import ops
+    case = (1, 90, 250, 2, 128, 3, 30, 15, True, torch.bfloat16)
+    q, k, v, _, ids = _inputs(case, dev)
+    out, lse = ops.sel_fwd(q.to(dev), ops.DenseKV(k.to(dev), v.to(dev)), ids.to(dev), 30, 35, scale, True, 15)
+    o_ref, l_ref = O.selection_fwd(q.float(), k.float(), v.float(), ids, 30, 35, scale, True, 15)
+    fin = torch.isfinite(l_ref)
+    assert torch.equal(torch.isfinite(lse.cpu()), fin)
+    assert torch.allclose(lse.cpu()[fin], l_ref[fin], atol=2e-3, rtol=1e-4)
+    assert_close_bf16(out, o_ref, "out", 2e-2, 2e-3)
