@@ -209,57 +209,110 @@ struct ScoreParams {
   int MG, H, D;
   int64_t NC;
   float scale;
+  // columns from here on are hidden from a query row and those before it, and nobody reads their scores
+  int causal, G, chunk_size, chunk_size_k, block_size, q_off, id_base, id_stride;
+  __device__ __forceinline__ int64_t columns(int g) const {
+    if (!causal) return NC;
+    const int64_t q_cid = static_cast<int64_t>(g) * G / chunk_size + q_off;
+    const int64_t ids = ((q_cid + 1) * chunk_size_k + block_size - 1) / block_size - id_base;
+    const int64_t n = (ids + id_stride - 1) / id_stride;
+    return ids <= 0 ? 0 : (n < NC ? n : NC);
+  }
 };
 
 constexpr int kScoreCols = 64;
-constexpr int kScoreRows = 32;
-
-template <typename T>
-__global__ void __launch_bounds__(256) score_kernel(const ScoreParams p) {
-  extern __shared__ float s_f[];
-  float* ks = s_f;                                   // [64][D+1]
-  float* qs = s_f + kScoreCols * (p.D + 1);          // [32][D]
-  const int64_t c0 = static_cast<int64_t>(blockIdx.x) * kScoreCols;
+// R rows per thread, 4 R rows per step, every `parts`-th step per thread block.  R = 8 spends fewer shared-memory reads
+// per product; R = 1 spreads short calls over the chip.  VEC: 16-byte aligned fp32 rows, copied with cp.async and read
+// four elements at a time.  25 rows x 98 keys x 12 heads, fp32, D = 128: 20.8 us with R = 8 on 24 thread blocks, 14.2 us
+// with R = 1 and element-wise loads.  The products of a score are summed in the order of the head dimension in all of them.
+template <typename T, int R, bool VEC>
+__global__ void __launch_bounds__(256) score_kernel(const ScoreParams p, int parts) {
+  extern __shared__ __align__(16) float s_f[];
+  const int pitch = p.D + (VEC ? 4 : 1);
+  float* ks = s_f;                                   // [64][pitch]
+  float* qs = s_f + kScoreCols * pitch;              // [4 R][D]
+  const int64_t c0 = static_cast<int64_t>(blockIdx.x / parts) * kScoreCols;
   const int h = blockIdx.y, b = blockIdx.z;
   const int ncol = static_cast<int>(p.NC - c0 < kScoreCols ? p.NC - c0 : kScoreCols);
-  for (int i = threadIdx.x; i < kScoreCols * p.D; i += blockDim.x) {
-    const int c = i / p.D, d = i - c * p.D;
-    float v = 0.f;
-    if (c < ncol)
-      v = to_f32<T>(*reinterpret_cast<const T*>(p.k + (b * p.k_sb + (c0 + c) * p.k_sc + h * p.k_sh + d) * sizeof(T)));
-    ks[c * (p.D + 1) + d] = v;
-  }
-  const int cl = threadIdx.x & 63, gq = threadIdx.x >> 6;   // 4 row groups of 8 rows
-  float* out = p.scores + ((static_cast<int64_t>(b) * p.H + h) * p.MG) * p.NC + c0 + cl;
-  for (int g0 = 0; g0 < p.MG; g0 += kScoreRows) {
-    __syncthreads();
-    const int nrow = min(kScoreRows, p.MG - g0);
-    for (int i = threadIdx.x; i < kScoreRows * p.D; i += blockDim.x) {
-      const int r = i / p.D, d = i - r * p.D;
-      float v = 0.f;
-      if (r < nrow)
-        v = to_f32<T>(*reinterpret_cast<const T*>(p.q + (b * p.q_sb + (g0 + r) * p.q_sg + h * p.q_sh + d) * sizeof(T)));
-      qs[i] = v;
+  // rows [0, n) of [rows][D] in global memory -> rows of `to` elements in shared memory, zeros up to `rows`
+  const auto load = [&](float* dst, int to, const char* src, int64_t row_bytes, int n, int rows) {
+    if constexpr (VEC) {
+      const int per = p.D / 4;
+      for (int i = threadIdx.x; i < rows * per; i += 256) {
+        const int r = i / per, x = i - r * per;
+        cp_async16(dst + r * to + x * 4, r < n ? src + r * row_bytes + x * 16 : src, r < n ? 16 : 0);
+      }
+      cp_async_commit();
+      cp_async_wait<0>();
+    } else {
+#pragma unroll 8
+      for (int i = threadIdx.x; i < rows * p.D; i += 256) {
+        const int r = i / p.D, d = i - r * p.D;
+        dst[r * to + d] = r < n ? to_f32<T>(*reinterpret_cast<const T*>(src + r * row_bytes + d * sizeof(T))) : 0.f;
+      }
     }
+  };
+  load(ks, pitch, p.k + (b * p.k_sb + c0 * p.k_sc + h * p.k_sh) * sizeof(T), p.k_sc * sizeof(T), ncol, kScoreCols);
+  const int cl = threadIdx.x & 63, gq = threadIdx.x >> 6;   // 4 row groups of R rows
+  float* out = p.scores + ((static_cast<int64_t>(b) * p.H + h) * p.MG) * p.NC + c0 + cl;
+  for (int g0 = static_cast<int>(blockIdx.x % parts) * 4 * R; g0 < p.MG; g0 += parts * 4 * R) {
     __syncthreads();
-    float acc[8];
+    load(qs, p.D, p.q + (b * p.q_sb + g0 * p.q_sg + h * p.q_sh) * sizeof(T), p.q_sg * sizeof(T), min(4 * R, p.MG - g0), 4 * R);
+    __syncthreads();
+    float acc[R];
 #pragma unroll
-    for (int i = 0; i < 8; ++i) acc[i] = 0.f;
-    const float* kr = ks + cl * (p.D + 1);
-    const float* qr = qs + gq * 8 * p.D;
-    for (int d = 0; d < p.D; ++d) {
-      const float kv = kr[d];
+    for (int i = 0; i < R; ++i) acc[i] = 0.f;
+    const float* kr = ks + cl * pitch;
+    const float* qr = qs + gq * R * p.D;
+    if constexpr (VEC) {
+#pragma unroll 4
+      for (int d = 0; d < p.D; d += 4) {
+        const float4 kv = *reinterpret_cast<const float4*>(kr + d);
 #pragma unroll
-      for (int i = 0; i < 8; ++i) acc[i] = fmaf(qr[i * p.D + d], kv, acc[i]);
+        for (int i = 0; i < R; ++i) {
+          const float4 qv = *reinterpret_cast<const float4*>(qr + i * p.D + d);
+          acc[i] = fmaf(qv.w, kv.w, fmaf(qv.z, kv.z, fmaf(qv.y, kv.y, fmaf(qv.x, kv.x, acc[i]))));
+        }
+      }
+    } else {
+      for (int d = 0; d < p.D; ++d) {
+        const float kv = kr[d];
+#pragma unroll
+        for (int i = 0; i < R; ++i) acc[i] = fmaf(qr[i * p.D + d], kv, acc[i]);
+      }
     }
     if (cl < ncol) {
 #pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        const int g = g0 + gq * 8 + i;
+      for (int i = 0; i < R; ++i) {
+        const int g = g0 + gq * R + i;
         if (g < p.MG) out[static_cast<int64_t>(g) * p.NC] = acc[i] * p.scale + 0.f;
       }
     }
   }
+}
+template <typename T, int R, bool VEC>
+int launch_score_rows(const ScoreParams& sp, int B, int parts, cudaStream_t s) {
+  const size_t smem = (static_cast<size_t>(kScoreCols) * (sp.D + (VEC ? 4 : 1)) + static_cast<size_t>(4 * R) * sp.D) * sizeof(float);
+  auto kernel = score_kernel<T, R, VEC>;
+  NSA_CUDA_OK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
+  kernel<<<dim3(static_cast<unsigned>(cdiv64(sp.NC, kScoreCols) * parts), sp.H, B), 256, smem, s>>>(sp, parts);
+  NSA_LAUNCH_OK("score_kernel");
+  return NSA_OK;
+}
+template <typename T>
+int launch_score(const ScoreParams& sp, int B, cudaStream_t s) {
+  // row steps are dealt out to as many thread blocks as the chip holds at once (four per SM)
+  const int64_t tiles = cdiv64(sp.NC, kScoreCols) * sp.H * B;
+  const auto parts = [&](int rows) {
+    const int64_t steps = cdiv(sp.MG, rows), room = 4 * 148 / (tiles > 0 ? tiles : 1);
+    return static_cast<int>(room < 1 ? 1 : (room < steps ? room : steps));
+  };
+  if constexpr (sizeof(T) == 4) {
+    const bool vec = sp.D % 4 == 0 && aligned16(sp.q) && aligned16(sp.k) && sp.q_sb % 4 == 0 && sp.q_sg % 4 == 0 && sp.q_sh % 4 == 0 &&
+                     sp.k_sb % 4 == 0 && sp.k_sc % 4 == 0 && sp.k_sh % 4 == 0;
+    if (vec) return tiles * cdiv(sp.MG, 32) < 148 ? launch_score_rows<T, 1, true>(sp, B, parts(4), s) : launch_score_rows<T, 8, true>(sp, B, parts(32), s);
+  }
+  return launch_score_rows<T, 8, false>(sp, B, parts(32), s);
 }
 
 // 16-bit inputs: the same scores on mma.sync (products of bf16 / fp16 operands are exact in fp32,
@@ -279,6 +332,7 @@ __global__ void __launch_bounds__(128) score_mma_kernel(const ScoreParams p) {
   const int h = blockIdx.z % p.H, b = blockIdx.z / p.H;
   const int ncol = static_cast<int>(p.NC - c0 < kScoreCols ? p.NC - c0 : kScoreCols);
   const int nrow = min(kScoreMmaRows, p.MG - g0);
+  if (c0 >= p.columns(g0 + nrow - 1)) return;           // hidden from all rows
   const int cpr = p.D / 8;                              // 16-byte chunks per row
   for (int i = threadIdx.x; i < kScoreCols * cpr; i += blockDim.x) {
     const int r = i / cpr, cc = i - r * cpr;
@@ -308,15 +362,26 @@ __global__ void __launch_bounds__(128) score_mma_kernel(const ScoreParams p) {
     }
   }
   float* out = p.scores + ((static_cast<int64_t>(b) * p.H + h) * p.MG + g0) * p.NC + c0;
+  // neighbouring lanes swap halves so that each holds four columns in a row: 16-byte stores where the rows allow them
+  const bool wide = p.NC % 4 == 0 && ncol % 4 == 0;
 #pragma unroll
-  for (int r = 0; r < 2; ++r) {
-    const int row = warp * 16 + gid + 8 * r;
-    if (row < nrow) {
+  for (int n = 0; n < 8; ++n) {
 #pragma unroll
-      for (int n = 0; n < 8; ++n) {
-        const int col = n * 8 + 2 * t4;
-        if (col < ncol) out[static_cast<int64_t>(row) * p.NC + col] = acc[n][2 * r] * p.scale + 0.f;
-        if (col + 1 < ncol) out[static_cast<int64_t>(row) * p.NC + col + 1] = acc[n][2 * r + 1] * p.scale + 0.f;
+    for (int e = 0; e < 4; ++e) acc[n][e] = acc[n][e] * p.scale + 0.f;
+    if (wide) {
+      const bool odd = t4 & 1;                          // even lanes take row gid, odd ones row gid + 8
+      const float x = __shfl_xor_sync(0xffffffffu, odd ? acc[n][0] : acc[n][2], 1);
+      const float y = __shfl_xor_sync(0xffffffffu, odd ? acc[n][1] : acc[n][3], 1);
+      const int row = warp * 16 + gid + (odd ? 8 : 0), col = n * 8 + (t4 >> 1) * 4;
+      if (row < nrow && col < ncol)
+        *reinterpret_cast<float4*>(out + static_cast<int64_t>(row) * p.NC + col) =
+            odd ? make_float4(x, y, acc[n][2], acc[n][3]) : make_float4(acc[n][0], acc[n][1], x, y);
+    } else {
+#pragma unroll
+      for (int r = 0; r < 2; ++r) {
+        const int row = warp * 16 + gid + 8 * r, col = n * 8 + 2 * t4;
+        if (row < nrow && col < ncol) out[static_cast<int64_t>(row) * p.NC + col] = acc[n][2 * r];
+        if (row < nrow && col + 1 < ncol) out[static_cast<int64_t>(row) * p.NC + col + 1] = acc[n][2 * r + 1];
       }
     }
   }
@@ -445,9 +510,6 @@ struct SelectParams {
   int32_t* out_idx;       // [rows][topk]
   float* out_scores;      // may be null
   Mask mask;
-  int seg_cols;           // MASKED, first stage of long rows: columns per segment (0 = the whole row);
-  int n_seg;              //   warp w takes segment w % n_seg of row w / n_seg and writes its list to
-                          //   out_idx / out_scores laid out [n_seg][rows][topk]
 };
 
 template <bool MERGE>
@@ -707,13 +769,8 @@ __global__ void __launch_bounds__(128) select_warp_kernel(const SelectParams p, 
   chain_release();
   chain_wait();
   const int warp = threadIdx.x >> 5;
-  const int64_t unit = static_cast<int64_t>(blockIdx.x) * 4 + warp;
-  const int n_seg = (!MERGE && p.seg_cols > 0) ? p.n_seg : 1;
-  if (unit >= rows * n_seg) return;
-  const int64_t row = unit / n_seg;
-  const int seg = static_cast<int>(unit - row * n_seg);
-  const int64_t c_off = static_cast<int64_t>(seg) * p.seg_cols;          // 0 unless segmented
-  const int64_t NC = n_seg > 1 ? (p.NC - c_off < p.seg_cols ? p.NC - c_off : p.seg_cols) : p.NC;
+  const int64_t row = static_cast<int64_t>(blockIdx.x) * 4 + warp;
+  if (row >= rows) return;
   RowMask rm{};
   const float* srow;
   if (MERGE) {
@@ -724,12 +781,137 @@ __global__ void __launch_bounds__(128) select_warp_kernel(const SelectParams p, 
     const int g = static_cast<int>(bg % p.MG);
     const int64_t b = bg / p.MG;
     rm = make_row_mask(p.mask, g);
-    srow = p.scores + ((b * p.H + h) * p.MG + g) * p.NC + c_off;
+    srow = p.scores + ((b * p.H + h) * p.MG + g) * p.NC;
   }
   __shared__ unsigned long long s_sorted[4][ITEMS][32];
-  const int64_t out_row = n_seg > 1 ? static_cast<int64_t>(seg) * rows + row : row;
-  warp_select<ITEMS, MERGE>(p, srow, rm, NC, c_off, row, p.out_idx + out_row * p.topk,
-                            p.out_scores ? p.out_scores + out_row * p.topk : nullptr, s_sorted[warp]);
+  warp_select<ITEMS, MERGE>(p, srow, rm, p.NC, 0, row, p.out_idx + row * p.topk,
+                            p.out_scores ? p.out_scores + row * p.topk : nullptr, s_sorted[warp]);
+}
+
+// Rows of any length: W warps per row read it twice, every thread a column in 32 W.
+//   threshold  every lane finds its largest key; with r = ceil(topk / W), the smallest over the warps of the r-th
+//              largest lane maximum has at least topk keys at or above it
+//   collect    the keys at or above the threshold (a few more than topk) go to shared memory, where a key's rank is
+//              the number of larger ones
+// A row that leaves more than 64 W candidates (its large scores all in a few columns of every 32 W) takes one round of
+// the whole row per winner.  What bounds it is the instructions per column (some ten) and, for the longest rows, their
+// bytes.  Same keys and order as select_kernel.
+constexpr int kCandidates = 64;            // per warp
+template <int W>
+__global__ void __launch_bounds__(W == 1 ? 128 : 32 * W) select_rows_kernel(const SelectParams p, int64_t rows) {
+  constexpr int kRows = W == 1 ? 4 : 1, kThreads = 32 * W, kCap = kCandidates * W;
+  __shared__ unsigned long long s_cand[kRows][kCap];
+  __shared__ unsigned long long s_warp[kRows][W];
+  __shared__ int s_total[kRows];
+  const int slot = W == 1 ? threadIdx.x >> 5 : 0, t = W == 1 ? threadIdx.x & 31 : threadIdx.x;
+  const int lane = threadIdx.x & 31, warp = W == 1 ? 0 : threadIdx.x >> 5;
+  const auto sync = [] {
+    if constexpr (W == 1) __syncwarp(); else __syncthreads();
+  };
+  if (t == 0) s_total[slot] = 0;
+  chain_release();
+  chain_wait();
+  const int64_t row = static_cast<int64_t>(blockIdx.x) * kRows + slot;
+  if (row >= rows) return;                            // whole warps (W = 1) or the whole block
+  const int h = static_cast<int>(row % p.H);
+  const int64_t bg = row / p.H;
+  const int g = static_cast<int>(bg % p.MG);
+  const RowMask rm = make_row_mask(p.mask, g);
+  const RowBounds rb = make_row_bounds(p.mask, rm);
+  const float* srow = p.scores + ((bg / p.MG * p.H + h) * p.MG + g) * p.NC;
+  unsigned long long* cand = s_cand[slot];
+  int32_t* oi = p.out_idx + row * p.topk;
+  float* os = p.out_scores ? p.out_scores + row * p.topk : nullptr;
+  // the columns in front of the causal limit
+  int64_t n = p.NC;
+  if (!p.mask.tf && p.mask.causal) {
+    const int64_t ids = static_cast<int64_t>(rb.hi) - p.mask.id_base;
+    const int64_t c = ids <= 0 ? 0 : (ids + p.mask.id_stride - 1) / p.mask.id_stride;
+    n = c < n ? c : n;
+  }
+  // f(key) for this thread's visible columns, loads ahead of their use
+  const auto each = [&](auto&& f) {
+    constexpr int kAhead = 8;
+    for (int64_t c0 = t; c0 < n; c0 += kAhead * kThreads) {
+      float v[kAhead];
+#pragma unroll
+      for (int i = 0; i < kAhead; ++i) {
+        const int64_t c = c0 + i * kThreads;
+        v[i] = c < n ? srow[c] : 0.f;
+      }
+#pragma unroll
+      for (int i = 0; i < kAhead; ++i) {
+        const int64_t c = c0 + i * kThreads;
+        const int bid = p.mask.id_base + static_cast<int>(c) * p.mask.id_stride;
+        const bool vis = c < n && (p.mask.tf ? visible(p.mask, rm, bid) : visible_in(rb, bid));
+        f(vis ? pack_key(v[i], bid) : 0ull);
+      }
+    }
+  };
+  const auto warp_max = [&](unsigned long long k) {
+#pragma unroll
+    for (int d = 16; d; d >>= 1) {
+      const unsigned long long o = __shfl_xor_sync(0xffffffffu, k, d);
+      k = o > k ? o : k;
+    }
+    return k;
+  };
+
+  unsigned long long best = 0ull, none = 0ull;
+  each([&](unsigned long long k) { best = k > best ? k : best; });
+  warp_sort64_desc(best, none, false);
+  unsigned long long tau = __shfl_sync(0xffffffffu, best, (p.topk + W - 1) / W - 1);
+  if constexpr (W > 1) {
+    if (lane == 0) s_warp[0][warp] = tau;
+    __syncthreads();
+#pragma unroll
+    for (int w = 0; w < W; ++w) tau = s_warp[0][w] < tau ? s_warp[0][w] : tau;
+  } else {
+    __syncwarp();
+  }
+  each([&](unsigned long long k) {
+    if (k != 0ull && k >= tau) {
+      const int at = atomicAdd(&s_total[slot], 1);
+      if (at < kCap) cand[at] = k;
+    }
+  });
+  sync();
+  const int total = s_total[slot];
+  int found = total < p.topk ? total : p.topk;
+  if (total <= kCap) {
+    for (int i = t; i < total; i += kThreads) {
+      const unsigned long long k = cand[i];
+      int rank = 0;
+      for (int j = 0; j < total; ++j) rank += cand[j] > k;
+      if (rank < p.topk) {
+        oi[rank] = key_id(k);
+        if (os) os[rank] = key_score(k);
+      }
+    }
+  } else {
+    unsigned long long bound = ~0ull;
+    for (int r = 0; r < found; ++r) {
+      best = 0ull;
+      each([&](unsigned long long k) { best = k < bound && k > best ? k : best; });
+      best = warp_max(best);
+      if constexpr (W > 1) {
+        __syncthreads();
+        if (lane == 0) s_warp[0][warp] = best;
+        __syncthreads();
+#pragma unroll
+        for (int w = 0; w < W; ++w) best = s_warp[0][w] > best ? s_warp[0][w] : best;
+      }
+      bound = best;
+      if (t == 0) {
+        oi[r] = key_id(best);
+        if (os) os[r] = key_score(best);
+      }
+    }
+  }
+  for (int i = found + t; i < p.topk; i += kThreads) {
+    oi[i] = -1;
+    if (os) os[i] = -INFINITY;
+  }
 }
 
 // ------------------------------------------------------------------- fused scoring + selection
@@ -932,35 +1114,24 @@ int launch_score_select(const ScoreSelectParams& p, int B, cudaStream_t s) {
   return NSA_OK;
 }
 
-constexpr int kSegCols = 1024;       // candidates one warp sorts in registers
-constexpr int kSegTopkMax = 64;      // largest top-k the two-stage selection of long rows is sized for
-
-size_t segment_workspace_bytes(int64_t rows, int64_t NC) {
-  if (NC <= kSegCols) return 0;
-  return align_up(static_cast<size_t>(cdiv64(NC, kSegCols)) * rows * kSegTopkMax * 8, 256);
+template <int W> int launch_select_rows(const SelectParams& sel, int64_t rows, cudaStream_t s) {
+  NSA_CUDA_OK(launch_chained(kChainSmall, select_rows_kernel<W>, dim3(static_cast<unsigned>(W == 1 ? cdiv64(rows, 4) : rows)),
+                             dim3(W == 1 ? 128 : 32 * W), 0, s, sel, rows));
+  NSA_LAUNCH_OK("select_rows_kernel");
+  return NSA_OK;
 }
 
 template <bool MERGE>
-int launch_select(const SelectParams& sel, int64_t rows, cudaStream_t s, void* seg_ws = nullptr) {
+int launch_select(const SelectParams& sel, int64_t rows, cudaStream_t s) {
   const unsigned blocks4 = static_cast<unsigned>(cdiv64(rows, 4));
-  if (!MERGE && seg_ws != nullptr && sel.NC > kSegCols && sel.topk <= kSegTopkMax &&
-      cdiv64(sel.NC, kSegCols) * rows <= 0x7fffffff) {
-    // Long rows in two stages: one warp per (row, 1024-column segment) takes the segment's top-k
-    // (same keys, same order), then the per-segment lists of a row are merged like per-shard
-    // candidate lists.  Exact: the row's top-k is a subset of the union of the segments' top-k.
-    const int n_seg = static_cast<int>(cdiv64(sel.NC, kSegCols));
-    int32_t* cand_idx = static_cast<int32_t*>(seg_ws);
-    float* cand_val = reinterpret_cast<float*>(cand_idx + static_cast<int64_t>(n_seg) * rows * sel.topk);
-    SelectParams first = sel;
-    first.seg_cols = kSegCols; first.n_seg = n_seg; first.out_idx = cand_idx; first.out_scores = cand_val;
-    const unsigned blocks = static_cast<unsigned>(cdiv64(rows * n_seg, 4));
-    NSA_CUDA_OK(launch_chained(kChainSmall, select_warp_kernel<32, false>, dim3(blocks), dim3(128), 0, s, first, rows));
-    NSA_LAUNCH_OK("select kernel (segments)");
-    SelectParams merge{};
-    merge.scores = cand_val; merge.cand_ids = cand_idx; merge.NC = static_cast<int64_t>(n_seg) * sel.topk;
-    merge.MG = 1; merge.H = 1; merge.seg_len = sel.topk; merge.seg_stride = rows * sel.topk; merge.topk = sel.topk;
-    merge.out_idx = sel.out_idx; merge.out_scores = sel.out_scores;
-    return launch_select<true>(merge, rows, s);
+  if (!MERGE && sel.NC > 1024 && sel.topk <= 128) {
+    // a lane list of 16 per warp, and 2048 columns per warp while that leaves fewer than 16 warps per SM
+    int w = cdiv(sel.topk, 16);
+    while (w < 8 && sel.NC > 2048ll * w && rows * w < 148 * 16) ++w;
+    if (w <= 1) return launch_select_rows<1>(sel, rows, s);
+    if (w <= 2) return launch_select_rows<2>(sel, rows, s);
+    if (w <= 4) return launch_select_rows<4>(sel, rows, s);
+    return launch_select_rows<8>(sel, rows, s);
   }
   if (sel.NC <= 512) {
     NSA_CUDA_OK(launch_chained(kChainSmall, select_warp_kernel<16, MERGE>, dim3(blocks4), dim3(128), 0, s, sel, rows));
@@ -1075,11 +1246,10 @@ int check_rows16(const char* what, const void* ptr, const int64_t* stride, int e
 int run_score_select(const void* qp, const int64_t* qs, const void* kp, const int64_t* ks, int B,
                      int MG, int H, int D, int64_t NC, int topk, float scale, const Mask& m,
                      int32_t* out_idx, float* out_scores, float* scores, int dtype, cudaStream_t s,
-                     void* seg_ws = nullptr, bool allow_fused = true) {
+                     bool allow_fused = true) {
   ScoreParams sp{static_cast<const char*>(qp), qs[0], qs[1], qs[2], static_cast<const char*>(kp),
-                 ks[0], ks[1], ks[2], scores, MG, H, D, NC, scale};
-  const size_t smem = (static_cast<size_t>(kScoreCols) * (D + 1) + static_cast<size_t>(kScoreRows) * D) * sizeof(float);
-  const dim3 grid(static_cast<unsigned>(cdiv64(NC, kScoreCols)), H, B);
+                 ks[0], ks[1], ks[2], scores, MG, H, D, NC, scale,
+                 m.causal && !m.tf, m.G, m.chunk_size, m.chunk_size_k, m.block_size, m.q_off, m.id_base, m.id_stride};
   // 16-bit operands with 16-byte addressable rows go to the mma kernel
   const bool mma_ok = dtype != NSA_F32 && D % 16 == 0 && D <= 256 && static_cast<int64_t>(H) * B <= 65535 &&
                       aligned16(qp) && aligned16(kp) && (qs[0] * 2) % 16 == 0 && (qs[1] * 2) % 16 == 0 &&
@@ -1093,25 +1263,16 @@ int run_score_select(const void* qp, const int64_t* qs, const void* kp, const in
     fp.sel.out_scores = out_scores; fp.sel.mask = m;
     return dtype == NSA_BF16 ? launch_score_select<__nv_bfloat16>(fp, B, s) : launch_score_select<__half>(fp, B, s);
   }
-  if (mma_ok) {
-    const int rc = dtype == NSA_BF16 ? launch_score_mma<__nv_bfloat16>(sp, B, s) : launch_score_mma<__half>(sp, B, s);
-    if (rc) return rc;
-  } else if (dtype == NSA_BF16) {
-    NSA_CUDA_OK(cudaFuncSetAttribute(score_kernel<__nv_bfloat16>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
-    score_kernel<__nv_bfloat16><<<grid, 256, smem, s>>>(sp);
-  } else if (dtype == NSA_F16) {
-    NSA_CUDA_OK(cudaFuncSetAttribute(score_kernel<__half>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
-    score_kernel<__half><<<grid, 256, smem, s>>>(sp);
-  } else {
-    NSA_CUDA_OK(cudaFuncSetAttribute(score_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
-    score_kernel<float><<<grid, 256, smem, s>>>(sp);
-  }
-  NSA_LAUNCH_OK("score_kernel");
+  const int rc = mma_ok ? (dtype == NSA_BF16 ? launch_score_mma<__nv_bfloat16>(sp, B, s) : launch_score_mma<__half>(sp, B, s))
+                 : dtype == NSA_BF16 ? launch_score<__nv_bfloat16>(sp, B, s)
+                 : dtype == NSA_F16  ? launch_score<__half>(sp, B, s)
+                                     : launch_score<float>(sp, B, s);
+  if (rc) return rc;
   SelectParams sel{};
   sel.scores = scores; sel.cand_ids = nullptr; sel.NC = NC; sel.MG = MG; sel.H = H;
   sel.seg_len = 0; sel.seg_stride = 0; sel.topk = topk; sel.out_idx = out_idx; sel.out_scores = out_scores;
   sel.mask = m;
-  return launch_select<false>(sel, static_cast<int64_t>(B) * MG * H, s, seg_ws);
+  return launch_select<false>(sel, static_cast<int64_t>(B) * MG * H, s);
 }
 
 __global__ void fill_empty_kernel(int32_t* __restrict__ out_idx, float* __restrict__ out_scores, int64_t n) {
@@ -1176,12 +1337,12 @@ extern "C" int nsa_pool_rows(const void* x, const int64_t x_stride[3], void* out
   return launch_pool<float>(p, B, NB, s);
 }
 
-// scores [B,H,MG,NC] fp32, then (rows longer than 1024 columns) the per-segment candidate lists
+// scores [B,H,MG,NC] fp32
 static size_t score_bytes(int32_t B, int32_t MG, int32_t H, int64_t NC) {
   return align_up(static_cast<size_t>(B) * MG * H * NC * sizeof(float), 256);
 }
 extern "C" size_t nsa_topk_workspace_bytes(int32_t B, int32_t MG, int32_t H, int64_t NC) {
-  return score_bytes(B, MG, H, NC) + segment_workspace_bytes(static_cast<int64_t>(B) * MG * H, NC);
+  return score_bytes(B, MG, H, NC);
 }
 
 static int topk_common_checks(int32_t B, int32_t MG, int32_t H, int32_t D, int64_t NC, int32_t topk,
@@ -1212,9 +1373,8 @@ extern "C" int nsa_topk(const void* q_pooled, const int64_t q_stride[3], const v
               "topk: workspace too small");
   Mask m;
   if ((rc = fill_mask_checked(mask, MG, NC, &m))) return rc;
-  void* seg_ws = NC > kSegCols ? static_cast<char*>(workspace) + score_bytes(B, MG, H, NC) : nullptr;
   return run_score_select(q_pooled, q_stride, k_pooled, k_stride, B, MG, H, D, NC, topk, scale, m,
-                          out_idx, out_scores, static_cast<float*>(workspace), dtype, s, seg_ws);
+                          out_idx, out_scores, static_cast<float*>(workspace), dtype, s);
 }
 
 // Pooling of the raw keys, then scoring + selection (one kernel when a row's scores fit shared memory).
@@ -1379,5 +1539,5 @@ extern "C" int nsa_topk_static_scratch(const void* q_pooled, const int64_t q_str
   // Every score the selection reads is written by the scoring kernel of the same call, so nothing
   // in the array has to start at zero and whatever an earlier call left behind is never read.
   return run_score_select(q_pooled, q_stride, k_pooled, k_stride, B, MG, H, D, NC, topk, scale, m, out_idx,
-                          out_scores, scratch, dtype, s, nullptr, /*allow_fused=*/false);
+                          out_scores, scratch, dtype, s, /*allow_fused=*/false);
 }
