@@ -7,6 +7,8 @@
 //     bit-reproducible from run to run.
 #include "sel_rows.cuh"
 
+#include <type_traits>
+
 namespace nsa {
 namespace {
 
@@ -632,6 +634,13 @@ int launch_dkv_rows(const RingMaps& maps, const BwdParams& p, int32_t* status, c
 template <typename T, int D>
 int launch_dkv(const BwdParams& p, int32_t* st, cudaStream_t s) {
   const int64_t qs[3] = {p.q_sb, p.q_sm, p.q_sh}, ds[3] = {p.do_sb, p.do_sm, p.do_sh};
+  if (!p.tab.on) {
+    const DkvRowsArgs a{p.q, p.dO, p.dk, p.dv, p.lse, p.delta, p.groups, p.offsets, p.kv, p.B, p.H, p.T, p.block_size, p.chunk_size,
+                        p.causal, p.G, p.MG, 0, p.M, p.NS, p.scale, p.scale_log2};
+    bool launched = false;
+    const int rc = try_launch_sel_bwd_dkv_rows_tc(a, qs, ds, D, std::is_same<T, __half>::value ? NSA_F16 : NSA_BF16, st, s, &launched);
+    if (rc || launched) return rc;
+  }
   RingMaps maps{};
   const bool tma = make_unit_maps(&maps.a, &maps.a_tail, p.q, qs, p.B, p.M, p.H, D, p.G, 16) &&
                    make_unit_maps(&maps.b, &maps.b_tail, p.dO, ds, p.B, p.M, p.H, D, p.G, 16);

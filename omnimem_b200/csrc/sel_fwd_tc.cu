@@ -520,28 +520,29 @@ int make_tile_maps(const void* q, const int64_t* q_stride, const nsa_kv_source* 
 // element the last dimension is the 64-column half, so that one copy brings whole rows.  fp16 travels as bf16: a copy
 // does not look at the values.
 static bool unit_map(CUtensorMap* map, const void* base, int64_t head_stride, int64_t row_stride, int64_t batch_stride, int B,
-                     int H, int D, int64_t unit_rows, int64_t units, int rows) {
+                     int H, int D, int64_t unit_rows, int64_t units, int rows, bool join) {
   // a dimension of size 1 may carry any stride; the map wants a positive multiple of 16 bytes
   auto st = [](int64_t s, int64_t size) { return size > 1 ? static_cast<uint64_t>(s) * 2 : 128ull; };
   if (encode_tiled_fn() == nullptr || unit_rows <= 0 || units <= 0 || unit_rows > 0x7fffffff || units > 0x7fffffff) return false;
   if ((H > 1 && head_stride <= 0) || (unit_rows * units > 1 && row_stride <= 0) || (B > 1 && batch_stride <= 0)) return false;
-  const uint64_t dims[5] = {static_cast<uint64_t>(B > 1 ? D : 64), static_cast<uint64_t>(H), static_cast<uint64_t>(unit_rows),
-                            static_cast<uint64_t>(units), static_cast<uint64_t>(B > 1 ? B : D / 64)};
+  const uint64_t dims[5] = {static_cast<uint64_t>(join ? 64 : D), static_cast<uint64_t>(H), static_cast<uint64_t>(unit_rows),
+                            static_cast<uint64_t>(units), static_cast<uint64_t>(join ? D / 64 : B)};
   const uint64_t s[4] = {st(head_stride, H), st(row_stride, unit_rows), st(row_stride * unit_rows, units),
-                         B > 1 ? static_cast<uint64_t>(batch_stride) * 2 : 128ull};
-  const uint32_t bx[5] = {64, 1, static_cast<uint32_t>(rows), 1, static_cast<uint32_t>(B > 1 ? 1 : D / 64)};
+                         join ? 128ull : st(batch_stride, B)};
+  const uint32_t bx[5] = {64, 1, static_cast<uint32_t>(rows), 1, static_cast<uint32_t>(join ? D / 64 : 1)};
   return tc::encode_16bit_map(map, base, 5, dims, s, bx) == CUDA_SUCCESS;
 }
 bool make_unit_maps(CUtensorMap* whole, CUtensorMap* tail, const void* base, const int64_t* stride, int B, int64_t N, int H,
-                    int D, int unit, int rows) {
+                    int D, int unit, int rows, bool join_halves) {
   if (N > 0x7fffffff) return false;
-  return (N / unit == 0 || unit_map(whole, base, stride[2], stride[1], stride[0], B, H, D, unit, N / unit, rows)) &&
-         (N % unit == 0 || unit_map(tail, base, stride[2], stride[1], stride[0], B, H, D, N, 1, rows));
+  const bool join = join_halves && B == 1;
+  return (N / unit == 0 || unit_map(whole, base, stride[2], stride[1], stride[0], B, H, D, unit, N / unit, rows, join)) &&
+         (N % unit == 0 || unit_map(tail, base, stride[2], stride[1], stride[0], B, H, D, N, 1, rows, join));
 }
 bool make_ring_maps(const nsa_kv_source* kv, int B, int H, int D, int unit, int rows, RingMaps* m) {
   if (kv->mode == NSA_KV_PAGED) {
     const int64_t pages = kv->num_pages > 0 ? kv->num_pages : (1ll << 31) / unit;
-    return unit_map(&m->a, kv->k, 0, D, 0, 1, 1, D, unit, pages, rows) && unit_map(&m->b, kv->v, 0, D, 0, 1, 1, D, unit, pages, rows);
+    return unit_map(&m->a, kv->k, 0, D, 0, 1, 1, D, unit, pages, rows, true) && unit_map(&m->b, kv->v, 0, D, 0, 1, 1, D, unit, pages, rows, true);
   }
   return kv->mode == NSA_KV_DENSE &&
          make_unit_maps(&m->a, &m->a_tail, kv->k, kv->k_stride, B, kv->n_tokens, H, D, unit, rows) &&

@@ -377,10 +377,25 @@ __device__ __forceinline__ RingSource kv_ring_source(const KVSrc& kv, const Ring
 // ---- host side
 // Maps of rows of one dense operand [B,N,H,D] in units of `unit` rows, boxes of `rows` rows x 64 columns; `tail`
 // takes the unit that the end of the tensor cuts off.  False: not describable (the caller loads with cp.async).
+// join_halves: with one batch element the map's last dimension is the 64-column half, so that one copy brings whole rows.
 bool make_unit_maps(CUtensorMap* whole, CUtensorMap* tail, const void* base, const int64_t* stride, int B, int64_t N, int H,
-                    int D, int unit, int rows);
+                    int D, int unit, int rows, bool join_halves = true);
 // The same for the K and V of a source (a pool's units are its pages).
 bool make_ring_maps(const nsa_kv_source* kv, int B, int H, int D, int unit, int rows, RingMaps* maps);
 int device_status_address(int32_t** out);
+
+// dK / dV on the tensor cores (sel_bwd_dkv_rows_tc.cu).
+struct DkvRowsArgs {
+  const char *q, *dO;                    // [B,M,H,D]
+  char *dk, *dv;                         // contiguous [B,N,H,D]
+  const float *lse, *delta;              // [B,H,M]
+  const int32_t *groups, *offsets;       // [B,H,MG*T], [B,H,NS+1]
+  KVSrc kv;
+  int B, H, T, block_size, chunk_size, causal, G, MG, whole;   // whole: query groups in front of a cut-off one
+  int64_t M, NS;
+  float scale, scale_log2;
+};
+int try_launch_sel_bwd_dkv_rows_tc(DkvRowsArgs p, const int64_t* q_stride, const int64_t* do_stride, int D, int dtype,
+                                   int32_t* status, cudaStream_t stream, bool* launched);
 
 }  // namespace nsa
