@@ -464,6 +464,8 @@ int nsa_cache_select_victims(const int32_t* page_owner, const int64_t* page_stam
  *   direction 3 (drain): second half, meant for a stream of its own - staging slot i (passed as
  *                        k_pool / v_pool) -> the host slot of keys[i]; a fetch of those keys must be
  *                        ordered after it (pages and the tables are not used).
+ *   direction 4 (swap):  evict of pages[i] and fetch of keys[1+i] into it in one pass, both directions of the
+ *                        host link at once (a page without an owner is only fetched into).
  * n = *n_dev when n_dev != NULL (grid sized by cap), else n.  `counters` (device int64 [4], may
  * be NULL): counters[2] += pages evicted, counters[3] += pages fetched (bytes moved = pages x
  * 2 x page_bytes).

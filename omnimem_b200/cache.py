@@ -238,8 +238,7 @@ class BlockKVCache:
             self._wait_drain()                   # a missing block may still be on its way to the host tier
             n_dev = miss[:1]
             victims = self._select_victims(0, n_dev, cap, protect_from)
-            self._move(0, victims, None, 0, n_dev, cap)
-            self._move(1, victims, miss, 0, n_dev, cap)
+            self._move(4, victims, miss, 0, n_dev, cap)
         return uniq, miss
 
     def _pages_for(self, first: int, n_touched: int, n_exist: int, n_new: int, protect_from: int):

@@ -644,6 +644,65 @@ __global__ void __launch_bounds__(256) move_pages_kernel(const MoveParams p) {
   }
 }
 
+// Evict and fetch in one: page i goes to the host slot of the key that owns it (if any) while the block of key i comes
+// from its slot, so that both directions of the host link work at the same time (an evict followed by a fetch leaves
+// one idle).  No key is in both lists and no page listed twice.  Some 2100 pages of 32 KB: 2693 us in two passes, 2055 us
+// in one (67 GB/s, both directions together).
+__global__ void __launch_bounds__(256) swap_pages_kernel(const MoveParams p) {
+  const int i = blockIdx.x;
+  const int n = p.n_dev ? *p.n_dev : p.n_host;
+  if (i >= n) return;
+  const int page = p.pages[i];
+  if (page < 0) return;
+  const int key = p.keys[1 + i], old = p.page_owner[page];
+  uint4* const dev[2] = {reinterpret_cast<uint4*>(p.k_pool + static_cast<int64_t>(page) * p.page_bytes),
+                         reinterpret_cast<uint4*>(p.v_pool + static_cast<int64_t>(page) * p.page_bytes)};
+  char* const host[2] = {p.host_k, p.host_v};
+  const int64_t pieces = p.page_bytes / 16;
+  constexpr int kFlight = 4;                    // 16-byte pieces of K and of V per thread on their way
+  for (int64_t c0 = threadIdx.x; c0 < pieces; c0 += 256 * kFlight) {
+    uint4 in[2][kFlight], out[2][kFlight];
+#pragma unroll
+    for (int x = 0; x < 2; ++x) {
+      const uint4* from = reinterpret_cast<const uint4*>(host[x] + static_cast<int64_t>(key) * p.page_bytes);
+#pragma unroll
+      for (int y = 0; y < kFlight; ++y)
+        if (c0 + y * 256 < pieces) in[x][y] = __ldcv(from + c0 + y * 256);
+    }
+    if (old >= 0) {
+#pragma unroll
+      for (int x = 0; x < 2; ++x)
+#pragma unroll
+        for (int y = 0; y < kFlight; ++y)
+          if (c0 + y * 256 < pieces) out[x][y] = dev[x][c0 + y * 256];
+#pragma unroll
+      for (int x = 0; x < 2; ++x) {
+        uint4* to = reinterpret_cast<uint4*>(host[x] + static_cast<int64_t>(old) * p.page_bytes);
+#pragma unroll
+        for (int y = 0; y < kFlight; ++y)
+          if (c0 + y * 256 < pieces) to[c0 + y * 256] = out[x][y];
+      }
+    }
+#pragma unroll
+    for (int x = 0; x < 2; ++x)
+#pragma unroll
+      for (int y = 0; y < kFlight; ++y)
+        if (c0 + y * 256 < pieces) dev[x][c0 + y * 256] = in[x][y];
+  }
+  __threadfence_system();
+  __syncthreads();                              // publish only after the whole page has landed
+  if (threadIdx.x == 0) {
+    if (old >= 0) p.block_table[old] = -1;
+    p.page_owner[page] = key;
+    p.page_stamp[page] = p.epoch;
+    p.block_table[key] = page;
+    if (p.counters) {
+      if (old >= 0) atomicAdd(p.counters + 2, 1ull);
+      atomicAdd(p.counters + 3, 1ull);
+    }
+  }
+}
+
 // Write-behind eviction, first half: like an evict, but the page goes to slot i of a staging
 // buffer in device memory (host_k / host_v hold the staging bases here) and its key to stage_keys[i]
 // (-1: nothing staged); tables are updated at once, so the page is free for the caller.
@@ -970,16 +1029,16 @@ extern "C" int nsa_cache_move_pages(int32_t direction, const int32_t* pages, con
                                     void* v_pool, int64_t page_bytes, void* host_k, void* host_v,
                                     int32_t* block_table, int32_t* page_owner, int64_t* page_stamp,
                                     int64_t epoch, int64_t* counters, void* stream) {
-  NSA_REQUIRE(direction >= 0 && direction <= 3, NSA_ERR_INVALID, "cache_move_pages: direction must be 0 .. 3");
+  NSA_REQUIRE(direction >= 0 && direction <= 4, NSA_ERR_INVALID, "cache_move_pages: direction must be 0 .. 4");
   NSA_REQUIRE(n >= 0 && cap >= 0 && page_bytes > 0 && page_bytes % 16 == 0, NSA_ERR_INVALID, "cache_move_pages: bad size");
   NSA_REQUIRE(k_pool && v_pool, NSA_ERR_INVALID, "cache_move_pages: null pointer");
   NSA_REQUIRE(direction == 3 || (pages && block_table && page_owner && page_stamp), NSA_ERR_INVALID,
               "cache_move_pages: null pointer");
   NSA_REQUIRE(direction == 0 || (keys && host_k && host_v), NSA_ERR_INVALID,
-              "cache_move_pages: fetch, stage and drain need keys and the second set of slots");
+              "cache_move_pages: fetch, stage, drain and swap need keys and the second set of slots");
   const int grid = n_dev ? cap : n;
   if (grid == 0) return NSA_OK;
-  if (direction >= 2) {
+  if (direction == 2 || direction == 3) {
     MoveParams sp{pages, keys, n, n_dev, static_cast<char*>(k_pool), static_cast<char*>(v_pool), page_bytes,
                   static_cast<char*>(host_k), static_cast<char*>(host_v), block_table, page_owner, page_stamp, epoch,
                   reinterpret_cast<unsigned long long*>(counters)};
@@ -992,7 +1051,8 @@ extern "C" int nsa_cache_move_pages(int32_t direction, const int32_t* pages, con
                static_cast<char*>(host_k), static_cast<char*>(host_v), block_table, page_owner, page_stamp, epoch,
                reinterpret_cast<unsigned long long*>(counters)};
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  if (direction == 1) move_pages_kernel<true><<<grid, 256, 0, s>>>(p);
+  if (direction == 4) swap_pages_kernel<<<grid, 256, 0, s>>>(p);
+  else if (direction == 1) move_pages_kernel<true><<<grid, 256, 0, s>>>(p);
   else move_pages_kernel<false><<<grid, 256, 0, s>>>(p);
   NSA_LAUNCH_OK("move_pages_kernel");
   return NSA_OK;
