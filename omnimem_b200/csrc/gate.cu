@@ -57,6 +57,11 @@ __global__ void gate_combine_fwd_kernel(const GateParams p) {
     const uint32_t iu = static_cast<uint32_t>(i);
     const int64_t row = iu / cpr;
     const int cc = static_cast<int>(iu - static_cast<uint32_t>(row) * cpr);
+    // the branches are on their way while the gates are computed: 393120 rows of 128, 96 -> 89 us (403 MB)
+    uint4 v[3];
+#pragma unroll
+    for (int b = 0; b < 3; ++b)
+      if (p.o[b] != nullptr) v[b] = __ldcs(reinterpret_cast<const uint4*>(p.o[b] + (row * p.D) * sizeof(T) + cc * 16));
     float s[3];
     bool inside[3];
     gates_of_row<T>(p, row, s, inside);
@@ -67,8 +72,7 @@ __global__ void gate_combine_fwd_kernel(const GateParams p) {
     for (int b = 0; b < 3; ++b) {
       if (p.o[b] == nullptr) continue;
       const float gb = to_f32<T>(from_f32<T>(s[b]));
-      const uint4 v = *reinterpret_cast<const uint4*>(p.o[b] + (row * p.D) * sizeof(T) + cc * 16);
-      const T* e8 = reinterpret_cast<const T*>(&v);
+      const T* e8 = reinterpret_cast<const T*>(&v[b]);
 #pragma unroll
       for (int e = 0; e < 8; ++e) {
         const float prod = to_f32<T>(from_f32<T>(gb * to_f32<T>(e8[e])));
