@@ -154,8 +154,10 @@ def _fused(x: torch.Tensor) -> bool:
 def _plain(dtype: torch.dtype, *mods: nn.Module) -> bool:
     """Whether the parameters of `mods` may be used without calling them: the layers built here (not something a user
     put in their place), no hooks, parameters of the activations' type."""
-    return all(type(m) in _PLAIN and not m._forward_hooks and not m._forward_pre_hooks and m.weight.dtype == dtype
-               for m in mods)
+    for m in mods:
+        if type(m) not in _PLAIN or m._forward_hooks or m._forward_pre_hooks or m._parameters["weight"].dtype != dtype:
+            return False
+    return True
 
 
 _PLAIN = (nn.Linear, nn.LayerNorm, RMSNorm)
@@ -168,55 +170,48 @@ class _Packed(nn.Module):
     a multiple of 64, so that every row of the output keeps the alignment that fast products want."""
 
     packed: tuple = ()
+    _whole = None                                     # (weight, bias) over the parameters' common storage
 
     def _apply(self, fn, *args, **kwargs):
         super()._apply(fn, *args, **kwargs)
         mods = [getattr(self, n) for n in self.packed]
-        if all(type(m) is nn.Linear and m.weight.is_cuda for m in mods) and self._joined(mods) is None \
+        if all(type(m) is nn.Linear for m in mods) and self._joined(mods) is None and mods[0].weight.is_cuda \
                 and len({(m.weight.dtype, m.weight.device, m.in_features) for m in mods}) == 1:
-            rows = sum(m.out_features for m in mods)
-            weight = mods[0].weight.new_zeros(rows + -rows % 64, mods[0].in_features, requires_grad=False)
-            bias = weight.new_zeros(rows + -rows % 64)
-            at = 0
-            for m in mods:
-                for whole, t in ((weight, m.weight), (bias, m.bias)):
-                    part = whole[at:at + m.out_features]
-                    part.copy_(t.data)
-                    t.data = part
-                at += m.out_features
+            pad = -sum(m.out_features for m in mods) % 64
+            whole = []
+            for name in ("weight", "bias"):
+                parts = [m._parameters[name] for m in mods]
+                t = torch.cat([p.data for p in parts] + [parts[0].data.new_zeros(pad, *parts[0].shape[1:])])
+                at = 0
+                for p in parts:
+                    p.data = t[at:at + p.shape[0]]
+                    at += p.shape[0]
+                whole.append(t)
+            self._whole = tuple(whole)
         return self
 
-    @staticmethod
-    def _joined(mods):
-        """(weight, bias) of the layers as one, padded, or None if they do not lie so."""
-        out = []
-        for ts in ([m.weight for m in mods], [m.bias for m in mods]):
-            first = ts[0]
-            row = first.numel() // first.shape[0]
-            rows = sum(t.shape[0] for t in ts)
-            rows += -rows % 64
-            at, home = first.data_ptr(), first.untyped_storage()
-            if first.storage_offset() + rows * row > home.nbytes() // first.element_size():
-                return None
-            for t in ts:
-                if t.data_ptr() != at or not t.is_contiguous() or t.dtype != first.dtype \
-                        or t.untyped_storage().data_ptr() != home.data_ptr():
+    def _joined(self, mods):
+        """_whole, if the parameters still lie in it (its storage is kept, so an equal address is a view of it)."""
+        if self._whole is None:
+            return None
+        for name, t in zip(("weight", "bias"), self._whole):
+            at = t.data_ptr()
+            for m in mods:
+                p = m._parameters[name]
+                if p.data_ptr() != at or p.dtype != t.dtype or not p.is_contiguous():
+                    self._whole = None
                     return None
-                at += t.numel() * t.element_size()
-            out.append(first.detach().as_strided((rows,) + tuple(first.shape[1:]), first.stride()))
-        return out
+                at += p.nbytes
+        return self._whole
 
     def project(self, x: torch.Tensor):
         """The layers' outputs of x [.., d] (views of one tensor where the weights lie together)."""
-        mods = [getattr(self, n) for n in self.packed]
+        mods = [self._modules[n] for n in self.packed]
         joined = self._joined(mods)
         if joined is None:
             return [F.linear(x, m.weight, m.bias) for m in mods]
-        y, at, out = F.linear(x, *joined), 0, []
-        for m in mods:
-            out.append(y[..., at:at + m.out_features])
-            at += m.out_features
-        return out
+        widths = [m.out_features for m in mods]
+        return F.linear(x, *joined).split_with_sizes(widths + [joined[0].shape[0] - sum(widths)], -1)[:len(mods)]
 
 
 class NSASelfAttention(_Packed):

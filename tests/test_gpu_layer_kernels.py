@@ -95,7 +95,7 @@ def test_packed_projections_follow_their_layers(dev):
     state = {n: t.clone() for n, t in m.state_dict().items()}
     fresh = lambda: torch.nn.Parameter(torch.randn_like(m.v.bias))
     with torch.no_grad():
-        assert m._joined((m.k, m.v)) is not None
+        assert m._joined((m.k, m.v)) is not None and m.k.weight.untyped_storage().data_ptr() == m.v.weight.untyped_storage().data_ptr()
         changes = (lambda: m.k.weight.mul_(2), lambda: m.k.weight.data.copy_(torch.randn_like(m.k.weight)),
                    lambda: m.load_state_dict(state), lambda: setattr(m.v, "bias", fresh()),
                    lambda: m.to(dtype=torch.float32).to(dtype=torch.bfloat16), lambda: setattr(m.v, "bias", fresh()),
