@@ -36,9 +36,10 @@ __device__ __forceinline__ bool pair_bucket(const IdxParams& p, int b, int g, in
   const int32_t bid = p.ids[b * p.i_sb + g * p.i_sg + h * p.i_sh + t * p.i_st];
   if (bid < 0 || bid >= p.NS) return false;
   if (p.causal) {
-    const int64_t kc = (static_cast<int64_t>(bid) * p.block_size) / p.chunk_size;
-    const int64_t qc = (static_cast<int64_t>(g) * p.G) / p.chunk_size;
-    if (kc > qc) return false;
+    // chunk of the block's first token <= chunk of the group's first token; one division, in 32 bits where it fits
+    const int64_t q0 = static_cast<int64_t>(g) * p.G;
+    const int64_t in_chunk = q0 <= 0xffffffffll ? static_cast<uint32_t>(q0) % static_cast<uint32_t>(p.chunk_size) : q0 % p.chunk_size;
+    if (static_cast<int64_t>(bid) * p.block_size >= q0 - in_chunk + p.chunk_size) return false;
   }
   bucket = bid;
   return true;
@@ -47,10 +48,10 @@ __device__ __forceinline__ bool pair_bucket(const IdxParams& p, int b, int g, in
 template <bool SCATTER>
 __global__ void inv_pass_kernel(const IdxParams p, int32_t* __restrict__ counts,
                                 int32_t* __restrict__ groups) {
-  const int64_t pair = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (pair >= static_cast<int64_t>(p.MG) * p.T) return;
+  const uint32_t pair = blockIdx.x * blockDim.x + threadIdx.x;        // (the host keeps them below 2^31)
+  if (pair >= static_cast<uint32_t>(p.MG) * static_cast<uint32_t>(p.T)) return;
   const int h = blockIdx.y, b = blockIdx.z;
-  const int g = static_cast<int>(pair / p.T), t = static_cast<int>(pair % p.T);
+  const int g = static_cast<int>(pair / static_cast<uint32_t>(p.T)), t = static_cast<int>(pair - static_cast<uint32_t>(g) * p.T);
   int bucket;
   if (!pair_bucket(p, b, g, h, t, bucket)) return;
   const int64_t row = static_cast<int64_t>(b) * p.H + h;
@@ -101,40 +102,115 @@ __global__ void inv_scan_kernel(int32_t* __restrict__ counts, int32_t* __restric
   if (threadIdx.x == 0) o[NS] = carry_s;
 }
 
-// One thread per bucket: insertion sort of its group ids (buckets are short; the scatter pass
-// fills them in arrival order), so every consumer sees ascending groups and sums in a fixed order.
-__global__ void inv_sort_kernel(const int32_t* __restrict__ offsets, int32_t* __restrict__ groups, int64_t NS,
-                                int64_t groups_row, int64_t n_buckets, int32_t* __restrict__ slots) {
-  const int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (i >= n_buckets) return;
-  const int64_t row = i / NS, s = i % NS;
-  const int32_t* o = offsets + row * (NS + 1);
-  int32_t* gp = groups + row * groups_row + o[s];
-  const int n = o[s + 1] - o[s];
-  for (int a = 1; a < n; ++a) {
-    const int32_t v = gp[a];
-    int c = a - 1;
-    while (c >= 0 && gp[c] > v) { gp[c + 1] = gp[c]; --c; }
-    gp[c + 1] = v;
+// A warp sorts a bucket of n <= 32 HELD entries in registers (bitonic network, entry e = 32 x + lane in v[x]) and writes
+// it in order; in place is fine.
+constexpr int kHeld = 8;
+template <int HELD>
+__device__ __forceinline__ void sort_held(const int32_t* in, int32_t* out, int32_t* out_slots, int n) {
+  const int lane = threadIdx.x & 31;
+  int32_t v[HELD];
+#pragma unroll
+  for (int x = 0; x < HELD; ++x) v[x] = x * 32 + lane < n ? in[x * 32 + lane] : 0x7fffffff;
+#pragma unroll
+  for (int k = 2; k <= 32 * HELD; k <<= 1)
+#pragma unroll
+    for (int j = k >> 1; j > 0; j >>= 1)
+#pragma unroll
+      for (int x = 0; x < HELD; ++x) {
+        if (j >= 32) {
+          const int y = x ^ (j / 32);
+          if (y > x) {
+            const int32_t lo = min(v[x], v[y]), hi = max(v[x], v[y]);
+            const bool up = ((x * 32) & k) == 0;
+            v[x] = up ? lo : hi;
+            v[y] = up ? hi : lo;
+          }
+        } else {
+          const int32_t o = __shfl_xor_sync(0xffffffffu, v[x], j);
+          const bool up = ((x * 32 + lane) & k) == 0, lower = (lane & j) == 0;
+          v[x] = up == lower ? min(v[x], o) : max(v[x], o);
+        }
+      }
+#pragma unroll
+  for (int x = 0; x < HELD; ++x)
+    if (x * 32 + lane < n) {
+      out[x * 32 + lane] = out_slots != nullptr ? v[x] >> kSlotBits : v[x];
+      if (out_slots != nullptr) out_slots[x * 32 + lane] = v[x] & ((1 << kSlotBits) - 1);
+    }
+}
+__device__ __forceinline__ void warp_sort(const int32_t* in, int32_t* out, int32_t* out_slots, int n) {
+  if (n <= 32) sort_held<1>(in, out, out_slots, n);
+  else if (n <= 64) sort_held<2>(in, out, out_slots, n);
+  else if (n <= 128) sort_held<4>(in, out, out_slots, n);
+  else sort_held<kHeld>(in, out, out_slots, n);
+}
+
+// Puts buckets [i0, i1) of row (b, h) in order, by a block of 32 warps: a warp sorts a bucket of `shortest` to 32 kHeld
+// entries, a longer one is written again by the whole block walking over the row's pairs.  Bucket i is
+// [begin(i), begin(i + 1)) of `in`, `out` and `slots`.
+template <typename Begin>
+__device__ __forceinline__ void inv_order(const IdxParams& p, int b, int h, const int32_t* in, int32_t* out, int32_t* slots,
+                                          int i0, int i1, int shortest, Begin&& begin) {
+  constexpr int longest = 32 * kHeld;
+  __shared__ int found[2][32];
+  __shared__ int any_long;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  if (threadIdx.x == 0) any_long = 0;
+  __syncthreads();
+  for (int i = i0 + warp; i < i1; i += 32) {
+    const int beg = begin(i), n = begin(i + 1) - beg;
+    if (n > longest) {
+      if (lane == 0) any_long = 1;
+    } else if (n >= shortest) {
+      warp_sort(in + beg, out + beg, slots != nullptr ? slots + beg : nullptr, n);
+    }
   }
-  if (slots != nullptr) {
-    int32_t* sp = slots + row * groups_row + o[s];
-    for (int a = 0; a < n; ++a) {
-      const int32_t v = gp[a];
-      gp[a] = v >> kSlotBits;
-      sp[a] = v & ((1 << kSlotBits) - 1);
+  __syncthreads();
+  if (any_long == 0) return;
+  const int pairs = p.MG * p.T;
+  for (int i = i0; i < i1; ++i) {
+    int at = begin(i);
+    if (begin(i + 1) - at <= longest) continue;
+    __syncthreads();                                 // the counters of the bucket before
+    for (int p0 = 0, turn = 0; p0 < pairs; p0 += 1024, turn ^= 1) {
+      const int pr = p0 + threadIdx.x, g = pr / p.T;
+      int bucket = -1;
+      const bool mine = pr < pairs && pair_bucket(p, b, g, h, pr - g * p.T, bucket) && bucket == i;
+      const uint32_t m = __ballot_sync(0xffffffffu, mine);
+      if (lane == 0) found[turn][warp] = __popc(m);
+      __syncthreads();
+      int upto = found[turn][lane];                  // inclusive prefix sum over the warps
+#pragma unroll
+      for (int d = 1; d < 32; d <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, upto, d);
+        if (lane >= d) upto += y;
+      }
+      const int before = __shfl_sync(0xffffffffu, upto, warp > 0 ? warp - 1 : 0);
+      const int to = at + (warp > 0 ? before : 0) + __popc(m & ((1u << lane) - 1));
+      if (mine) {
+        out[to] = g;
+        if (slots != nullptr) slots[to] = pr - g * p.T;
+      }
+      at += __shfl_sync(0xffffffffu, upto, 31);
     }
   }
 }
 
-// The whole index of one (b, h) row in a single thread block when its NS counters fit in shared
-// memory: histogram and cursors in shared memory, scatter, then one thread per bucket sorts it.
-// STAGED: the row's pairs also fit, so scatter and sort run in shared memory and the bucket
-// array is written out once, coalesced.
-template <bool STAGED>
-__global__ void __launch_bounds__(1024) inv_fused_kernel(const IdxParams p, int32_t* __restrict__ groups,
-                                                         int32_t* __restrict__ offsets) {
-  extern __shared__ int s_cnt[];                   // [NS] (+ [pairs] when STAGED)
+// After the scatter pass: a thread block puts 32 buckets of a row in order, where they lie.
+__global__ void __launch_bounds__(1024) inv_sort_kernel(const IdxParams p, const int32_t* __restrict__ offsets, int32_t* groups) {
+  const int h = blockIdx.y, b = blockIdx.z;
+  const int64_t row = static_cast<int64_t>(b) * p.H + h, pairs = static_cast<int64_t>(p.MG) * p.T;
+  const int32_t* o = offsets + row * (p.NS + 1);
+  const int64_t i0 = static_cast<int64_t>(blockIdx.x) * 32, i1 = min64(i0 + 32, p.NS);
+  inv_order(p, b, h, groups + row * pairs, groups + row * pairs, p.slots != nullptr ? p.slots + row * pairs : nullptr,
+            static_cast<int>(i0), static_cast<int>(i1), 1, [&](int i) { return o[i]; });
+}
+
+// The whole index of one (b, h) row in a single thread block: histogram, cursors and buckets in shared memory, scatter,
+// then one thread per bucket sorts it (a warp where it is long) and the bucket array is written out once, coalesced.
+constexpr int kThreadSort = 48;
+__global__ void __launch_bounds__(1024) inv_fused_kernel(const IdxParams p, int32_t* __restrict__ groups, int32_t* __restrict__ offsets) {
+  extern __shared__ int s_cnt[];                   // [NS], then [pairs]
   __shared__ int warp_sums[32];
   __shared__ int carry_s;
   const int h = blockIdx.x % p.H, b = blockIdx.x / p.H;
@@ -143,7 +219,7 @@ __global__ void __launch_bounds__(1024) inv_fused_kernel(const IdxParams p, int3
   const int pairs = p.MG * p.T;
   int32_t* o = offsets + row * (p.NS + 1);
   int32_t* gr_out = groups + row * static_cast<int64_t>(pairs);
-  int32_t* gr = STAGED ? s_cnt + NS : gr_out;
+  int32_t* gr = s_cnt + NS;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
   for (int i = threadIdx.x; i < NS; i += blockDim.x) s_cnt[i] = 0;
   if (threadIdx.x == 0) carry_s = 0;
@@ -187,10 +263,12 @@ __global__ void __launch_bounds__(1024) inv_fused_kernel(const IdxParams p, int3
     const int g = pr / p.T;
     if (pair_bucket(p, b, g, h, pr % p.T, bucket)) gr[atomicAdd(&s_cnt[bucket], 1)] = inv_entry(p, g, pr % p.T);
   }
-  __syncthreads();                                   // scatter (global) visible to the block
+  __syncthreads();                                   // cursors now point one past their bucket
+  bool any = false;
+  const auto begin = [&](int i) { return i > 0 ? s_cnt[i - 1] : 0; };
   for (int sidx = threadIdx.x; sidx < NS; sidx += blockDim.x) {
-    const int end = s_cnt[sidx];                     // cursor now points one past the bucket
-    const int beg = o[sidx];
+    const int end = s_cnt[sidx], beg = begin(sidx);
+    if (end - beg > kThreadSort) { any = true; continue; }
     for (int a = beg + 1; a < end; ++a) {
       const int32_t v = gr[a];
       int c = a - 1;
@@ -198,20 +276,19 @@ __global__ void __launch_bounds__(1024) inv_fused_kernel(const IdxParams p, int3
       gr[c + 1] = v;
     }
   }
-  if (STAGED || p.slots != nullptr) {
-    __syncthreads();
-    const int total = carry_s;                         // pairs that landed in a bucket
-    int32_t* sl_out = p.slots != nullptr ? p.slots + row * static_cast<int64_t>(pairs) : nullptr;
-    for (int i = threadIdx.x; i < total; i += blockDim.x) {
-      const int32_t v = gr[i];
-      if (sl_out != nullptr) {
-        gr_out[i] = v >> kSlotBits;
-        sl_out[i] = v & ((1 << kSlotBits) - 1);
-      } else {
-        gr_out[i] = v;
-      }
+  any = __syncthreads_or(any);
+  const int total = carry_s;                         // pairs that landed in a bucket
+  int32_t* sl_out = p.slots != nullptr ? p.slots + row * static_cast<int64_t>(pairs) : nullptr;
+  for (int i = threadIdx.x; i < total; i += blockDim.x) {
+    const int32_t v = gr[i];
+    if (sl_out != nullptr) {
+      gr_out[i] = v >> kSlotBits;
+      sl_out[i] = v & ((1 << kSlotBits) - 1);
+    } else {
+      gr_out[i] = v;
     }
   }
+  if (any) inv_order(p, b, h, gr, gr_out, sl_out, 0, NS, kThreadSort + 1, begin);        // (its first barrier: after the copies)
 }
 
 // ------------------------------------------------------------------------------------ dQ
@@ -672,15 +749,14 @@ int run_inverted_index(const IdxParams& ip, int32_t* groups, int32_t* offsets, i
     return NSA_OK;
   }
   const int64_t pairs = static_cast<int64_t>(ip.MG) * ip.T;
-  if (ip.NS * 4 <= 160 * 1024 && pairs <= 0x7fffffff && rows <= 0x7fffffff) {
-    const size_t smem_idx = static_cast<size_t>(ip.NS) * 4, smem_all = smem_idx + static_cast<size_t>(pairs) * 4;
-    if (smem_all <= 200 * 1024) {
-      NSA_CUDA_OK(cudaFuncSetAttribute(inv_fused_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem_all)));
-      inv_fused_kernel<true><<<static_cast<unsigned>(rows), 1024, smem_all, stream>>>(ip, groups, offsets);
-    } else {
-      NSA_CUDA_OK(cudaFuncSetAttribute(inv_fused_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem_idx)));
-      inv_fused_kernel<false><<<static_cast<unsigned>(rows), 1024, smem_idx, stream>>>(ip, groups, offsets);
-    }
+  NSA_REQUIRE(pairs <= 0x7fffffff && ip.NS <= 0x7fffffff, NSA_ERR_INVALID, "inverted_index: too many pairs or blocks");
+  // One thread block per row while its pairs and their sort are little work (12 rows of 14208 pairs over 512 buckets:
+  // 7.7 us); else every pass is spread over the chip (12 rows of 34944 pairs over 1092 buckets, causal: 121 us in one, 34 us
+  // spread; 32 rows of 16640 pairs over 130 buckets: 139 and 39 us).
+  const size_t smem = static_cast<size_t>(ip.NS + pairs) * 4;
+  if (pairs <= 16384 && pairs <= kThreadSort * ip.NS && smem <= 200 * 1024 && rows <= 0x7fffffff) {
+    NSA_CUDA_OK(cudaFuncSetAttribute(inv_fused_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
+    inv_fused_kernel<<<static_cast<unsigned>(rows), 1024, smem, stream>>>(ip, groups, offsets);
     NSA_LAUNCH_OK("inv_fused_kernel");
     return NSA_OK;
   }
@@ -695,9 +771,7 @@ int run_inverted_index(const IdxParams& ip, int32_t* groups, int32_t* offsets, i
   if (pairs > 0) {
     inv_pass_kernel<true><<<grid, kIdxThreads, 0, stream>>>(ip, counts, groups);
     NSA_LAUNCH_OK("inv_pass_kernel<scatter>");
-    const int64_t n_buckets = rows * ip.NS;
-    inv_sort_kernel<<<static_cast<unsigned>(cdiv64(n_buckets, 128)), 128, 0, stream>>>(offsets, groups, ip.NS, pairs,
-                                                                                       n_buckets, ip.slots);
+    inv_sort_kernel<<<dim3(static_cast<unsigned>(cdiv64(ip.NS, 32)), ip.H, ip.B), 1024, 0, stream>>>(ip, offsets, groups);
     NSA_LAUNCH_OK("inv_sort_kernel");
   }
   return NSA_OK;
