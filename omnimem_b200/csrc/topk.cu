@@ -87,15 +87,15 @@ __global__ void __launch_bounds__(256) pool_rows_kernel(const PoolParams p) {
 
 // The same pooling for tensors whose rows are contiguous over the heads (x_sh == D, x_sn == H * D):
 // a thread block owns one run of rows for ALL heads and streams it through shared memory with bulk
-// asynchronous copies (cp.async.bulk, kBulkStages stages of up to 16 KiB, whole rows each), so the
-// bytes in flight are set by shared memory - about 45 KiB per thread block, four or five blocks per SM,
-// enough blocks resident for a selection's 586 runs to start together - not
+// asynchronous copies (cp.async.bulk, kBulkStages stages of whole rows each), so the bytes in flight are
+// set by shared memory - about 45 KiB per thread block, four or five blocks per SM, enough blocks resident for a
+// selection's 586 runs to start together; 96 or 192 KiB where there is no more than a block or two per SM - not
 // by registers: with 16-byte register loads these kernels had about 85 KiB per SM in flight and
 // stayed near 0.68 of the copy bandwidth.  Thread i owns 16-byte column piece i of the row, adds the
 // rows in ascending order (fp32) and writes its piece of the pooled row.  A wait that gives up
 // (bounded) raises the sticky device status word.
 constexpr int kBulkStages = 3;
-constexpr int kBulkStageBytes = 16 * 1024;
+constexpr int kBulkStageBytes = 16 * 1024;             // with several thread blocks per SM
 
 struct BulkPlan { int rows_per_stage; int threads; size_t smem; };
 
@@ -483,12 +483,13 @@ __device__ __forceinline__ bool visible_in(const RowBounds& rb, int bid) {
 
 // (score, id) -> 64-bit key; a larger key is a better candidate: higher score first, then the
 // lower id.  0 is reserved for "not a candidate".
-__device__ __forceinline__ unsigned long long pack_key(float s, int id) {
+__device__ __forceinline__ uint32_t score_half(float s) {
   uint32_t u = __float_as_uint(s + 0.f);
   u = (u & 0x80000000u) ? ~u : (u | 0x80000000u);
-  if (s != s) u = 1u;
-  if (u == 0u) u = 1u;
-  return (static_cast<unsigned long long>(u) << 32) | (0xffffffffu - static_cast<uint32_t>(id));
+  return s != s ? 1u : u;                              // (0 would be a NaN)
+}
+__device__ __forceinline__ unsigned long long pack_key(float s, int id) {
+  return (static_cast<unsigned long long>(score_half(s)) << 32) | (0xffffffffu - static_cast<uint32_t>(id));
 }
 __device__ __forceinline__ float key_score(unsigned long long k) {
   uint32_t u = static_cast<uint32_t>(k >> 32);
@@ -829,7 +830,8 @@ __global__ void __launch_bounds__(W == 1 ? 128 : 32 * W) select_rows_kernel(cons
     const int64_t c = ids <= 0 ? 0 : (ids + p.mask.id_stride - 1) / p.mask.id_stride;
     n = c < n ? c : n;
   }
-  // f(key) for this thread's visible columns, loads ahead of their use
+  // f(score half of the key, id) for this thread's columns (0: not visible), loads ahead of their use
+  const bool window = p.mask.tf || rb.lo > 0 || rb.win_hi > rb.win_lo;        // else every column below n is visible
   const auto each = [&](auto&& f) {
     constexpr int kAhead = 8;
     for (int64_t c0 = t; c0 < n; c0 += kAhead * kThreads) {
@@ -843,11 +845,13 @@ __global__ void __launch_bounds__(W == 1 ? 128 : 32 * W) select_rows_kernel(cons
       for (int i = 0; i < kAhead; ++i) {
         const int64_t c = c0 + i * kThreads;
         const int bid = p.mask.id_base + static_cast<int>(c) * p.mask.id_stride;
-        const bool vis = c < n && (p.mask.tf ? visible(p.mask, rm, bid) : visible_in(rb, bid));
-        f(vis ? pack_key(v[i], bid) : 0ull);
+        bool vis = c < n;
+        if (window) vis = vis && (p.mask.tf ? visible(p.mask, rm, bid) : visible_in(rb, bid));
+        f(vis ? score_half(v[i]) : 0u, bid);
       }
     }
   };
+  const auto key = [](uint32_t u, int bid) { return (static_cast<unsigned long long>(u) << 32) | (0xffffffffu - static_cast<uint32_t>(bid)); };
   const auto warp_max = [&](unsigned long long k) {
 #pragma unroll
     for (int d = 16; d; d >>= 1) {
@@ -857,8 +861,12 @@ __global__ void __launch_bounds__(W == 1 ? 128 : 32 * W) select_rows_kernel(cons
     return k;
   };
 
-  unsigned long long best = 0ull, none = 0ull;
-  each([&](unsigned long long k) { best = k > best ? k : best; });
+  uint32_t top = 0u;
+  int top_id = 0;
+  each([&](uint32_t u, int bid) {                      // ids ascend: the first of equal scores is the best key
+    if (u > top) { top = u; top_id = bid; }
+  });
+  unsigned long long best = top != 0u ? key(top, top_id) : 0ull, none = 0ull;
   warp_sort64_desc(best, none, false);
   unsigned long long tau = __shfl_sync(0xffffffffu, best, (p.topk + W - 1) / W - 1);
   if constexpr (W > 1) {
@@ -869,10 +877,11 @@ __global__ void __launch_bounds__(W == 1 ? 128 : 32 * W) select_rows_kernel(cons
   } else {
     __syncwarp();
   }
-  each([&](unsigned long long k) {
-    if (k != 0ull && k >= tau) {
+  const uint32_t tau_half = static_cast<uint32_t>(tau >> 32);
+  each([&](uint32_t u, int bid) {
+    if (u != 0u && u >= tau_half && key(u, bid) >= tau) {
       const int at = atomicAdd(&s_total[slot], 1);
-      if (at < kCap) cand[at] = k;
+      if (at < kCap) cand[at] = key(u, bid);
     }
   });
   sync();
@@ -892,7 +901,10 @@ __global__ void __launch_bounds__(W == 1 ? 128 : 32 * W) select_rows_kernel(cons
     unsigned long long bound = ~0ull;
     for (int r = 0; r < found; ++r) {
       best = 0ull;
-      each([&](unsigned long long k) { best = k < bound && k > best ? k : best; });
+      each([&](uint32_t u, int bid) {
+        const unsigned long long k = u != 0u ? key(u, bid) : 0ull;
+        best = k < bound && k > best ? k : best;
+      });
       best = warp_max(best);
       if constexpr (W > 1) {
         __syncthreads();
@@ -1201,13 +1213,14 @@ int launch_pool(const PoolParams& p, int B, int64_t NB, cudaStream_t s) {
 }
 
 // Whether the bulk-copy pooling kernel can serve p (rows contiguous over the heads, at most 16 KiB
-// each, 16-byte aligned), and how it would be launched.
-bool bulk_plan(const PoolParams& p, int B, int esz, BulkPlan* plan) {
+// each, 16-byte aligned), and how it would be launched among `blocks` thread blocks: the fewer of them, the more each
+// keeps in flight (25 and 98 runs of 393 KB, fp32: 31.6 -> 17.8 us).
+bool bulk_plan(const PoolParams& p, int64_t blocks, int esz, BulkPlan* plan) {
   const int64_t row_bytes = static_cast<int64_t>(p.H) * p.D * esz;
   if (p.x_sh != p.D || p.x_sn != static_cast<int64_t>(p.H) * p.D) return false;
   if (row_bytes % 16 != 0 || row_bytes > 16 * 1024 || !aligned16(p.x) || (p.x_sb * esz) % 16 != 0) return false;
-  (void)B;
-  int rows = static_cast<int>(kBulkStageBytes / row_bytes);
+  const int stage = kBulkStageBytes * (blocks <= 148 ? 4 : (blocks <= 2 * 148 ? 2 : 1));
+  int rows = static_cast<int>(stage / row_bytes);
   if (rows < 1) rows = 1;
   if (rows > p.size) rows = p.size;
   const int items = static_cast<int>(row_bytes / 16);
@@ -1327,7 +1340,7 @@ extern "C" int nsa_pool_rows(const void* x, const int64_t x_stride[3], void* out
   if (B == 0 || N == 0 || H == 0) return NSA_OK;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   BulkPlan plan;
-  if (bulk_plan(p, B, dtype_size(dtype), &plan)) {
+  if (bulk_plan(p, NB * B, dtype_size(dtype), &plan)) {
     if (dtype == NSA_BF16) return launch_pool_bulk<__nv_bfloat16>(p, plan, NB, p, plan, 0, B, s);
     if (dtype == NSA_F16) return launch_pool_bulk<__half>(p, plan, NB, p, plan, 0, B, s);
     return launch_pool_bulk<float>(p, plan, NB, p, plan, 0, B, s);
@@ -1427,7 +1440,8 @@ extern "C" int nsa_select_blocks(const void* q, const int64_t q_stride[3], const
   if (have_q && (rc = make_pool_params("select_blocks q", q, q_stride, q_pooled_out, qs, B, M, H, D, mask->q_group_size, dtype, &pq, &nbq))) return rc;
   if (have_k && (rc = make_pool_params("select_blocks k", k, k_stride, k_pooled_out, ps, B, N, H, D, mask->block_size, dtype, &pk, &nbk))) return rc;
   BulkPlan bq, bk;
-  if (have_q && have_k && bulk_plan(pq, B, dtype_size(dtype), &bq) && bulk_plan(pk, B, dtype_size(dtype), &bk)) {
+  const int64_t blocks = (nbq + nbk) * B;
+  if (have_q && have_k && bulk_plan(pq, blocks, dtype_size(dtype), &bq) && bulk_plan(pk, blocks, dtype_size(dtype), &bk)) {
     // the long tensor first: its thread blocks fill the GPU while the short one's trail behind
     if (dtype == NSA_BF16) rc = launch_pool_bulk<__nv_bfloat16>(pk, bk, nbk, pq, bq, nbq, B, s);
     else if (dtype == NSA_F16) rc = launch_pool_bulk<__half>(pk, bk, nbk, pq, bq, nbq, B, s);
