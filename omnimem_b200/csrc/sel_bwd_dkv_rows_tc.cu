@@ -18,8 +18,8 @@
 // What bounds it: the chain copy -> S, dP -> exponentials -> dV, dK of a thread block against the bytes that shared memory
 // can keep in flight.  32760 queries x 12 heads, D = 128, 16 blocks of 30, groups of 15, bf16: 1106 us on mma.sync, 620 us
 // with tiles of 128 rows and two thread blocks per SM, 549 us as it is.  2 x 3120 queries x 16 heads, D = 64, 64 blocks of
-// 24, groups of 12, fp16: 699 us, 410 us with tiles of 128 rows, 531 us with 64.  (256 threads for the exponentials: 632 /
-// 500 us.)
+// 24, groups of 12, fp16: 699 us, 371 us as it is (410 us with three thread blocks per SM), 531 us with tiles of 64 rows.
+// (256 threads for the exponentials: 632 / 500 us.)
 #include "sel_rows.cuh"
 
 #include <type_traits>
