@@ -344,7 +344,7 @@ __global__ void __launch_bounds__(32 * W * KS, W == 4 && D == 128 ? 3 : 1) sel_b
   int* words = reinterpret_cast<int*>(bars + KS * kRingBars);                          // abort, tile count
   RingSlot* list = reinterpret_cast<RingSlot*>(words + 4);
   if (warp == 0) {
-    const int count = ring_list<ESZ>(list, p.kv, p.ids, b * p.i_sb + g * p.i_sg + h * p.i_sh, p.i_st, p.T, b, h, D,
+    const int count = ring_list<ESZ, TMA>(list, p.kv, p.ids, b * p.i_sb + g * p.i_sg + h * p.i_sh, p.i_st, p.T, b, h, D,
                                      p.block_size, p.chunk_size, p.causal != 0, static_cast<int>(g0 / p.chunk_size));
     if (lane == 0) { words[0] = 0; words[1] = count; }
   }
@@ -355,7 +355,7 @@ __global__ void __launch_bounds__(32 * W * KS, W == 4 && D == 128 ? 3 : 1) sel_b
   ring.count = KS > 1 ? (words[1] - part + KS - 1) / KS : words[1];
   const RingSource src = kv_ring_source<ESZ>(p.kv, maps, p.B, b, h, D, p.block_size);
   const int per_block = (p.block_size + ROWS - 1) / ROWS;
-  const auto tile_of = [&](int i) { return ring_tile(list, part + i * KS, per_block, src); };
+  const auto tile_of = [&](int i) { return ring_tile<TMA>(list, part + i * KS, per_block, src); };
   ring.start(src, tile_of);
 
   // delta = sum_d O * dO of this thread's rows (lo, hi), from the fragments of both
@@ -675,9 +675,10 @@ template <typename T, int D, bool TMA>
 int launch_dq_loader(const RingMaps& maps, const BwdParams& p, int32_t* st, cudaStream_t s) {
   if (p.G <= 16) {
     // as many warps per list as still fit the chip at once (see the forward)
+    const bool short_list = ring_list_bytes(p.T) <= 64 * 1024;                   // (each warp's ring needs its room)
     const int64_t units = static_cast<int64_t>(p.MG) * p.H * p.B, room = 148 * (D == 128 ? 10 : 16);
-    if (units * 4 <= room) return launch_dq_rows<T, D, 1, 4, TMA>(maps, p, st, s);
-    if (units * 2 <= room) return launch_dq_rows<T, D, 1, 2, TMA>(maps, p, st, s);
+    if (units * 4 <= room && short_list) return launch_dq_rows<T, D, 1, 4, TMA>(maps, p, st, s);
+    if (units * 2 <= room && short_list) return launch_dq_rows<T, D, 1, 2, TMA>(maps, p, st, s);
     return launch_dq_rows<T, D, 1, 1, TMA>(maps, p, st, s);
   }
   if (p.G <= 32) return launch_dq_rows<T, D, 2, 1, TMA>(maps, p, st, s);

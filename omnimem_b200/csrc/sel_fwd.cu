@@ -47,7 +47,7 @@ __global__ void __launch_bounds__(32 * W * KS) sel_fwd_rows_kernel(const __grid_
   int* words = reinterpret_cast<int*>(bars + KS * kRingBars);                          // abort, tile count
   RingSlot* list = reinterpret_cast<RingSlot*>(words + 4);
   if (warp == 0) {
-    const int count = ring_list<ESZ>(list, p.kv, p.ids, b * p.i_sb + g * p.i_sg + h * p.i_sh, p.i_st, p.T, b, h, D,
+    const int count = ring_list<ESZ, TMA>(list, p.kv, p.ids, b * p.i_sb + g * p.i_sg + h * p.i_sh, p.i_st, p.T, b, h, D,
                                      p.block_size, p.chunk_size, p.causal != 0, static_cast<int>(g0 / p.chunk_size));
     if (lane == 0) { words[0] = 0; words[1] = count; }
   }
@@ -58,7 +58,7 @@ __global__ void __launch_bounds__(32 * W * KS) sel_fwd_rows_kernel(const __grid_
   ring.count = KS > 1 ? (words[1] - part + KS - 1) / KS : words[1];
   const RingSource src = kv_ring_source<ESZ>(p.kv, maps, p.B, b, h, D, p.block_size);
   const int per_block = (p.block_size + ROWS - 1) / ROWS;
-  const auto tile_of = [&](int i) { return ring_tile(list, part + i * KS, per_block, src); };
+  const auto tile_of = [&](int i) { return ring_tile<TMA>(list, part + i * KS, per_block, src); };
   ring.start(src, tile_of);
 
   float o[D / 8][4];
@@ -209,9 +209,10 @@ int launch_loader(const RingMaps& maps, const FwdParams& p, int MG, int32_t* st,
     // as many warps per list as still fit the chip at once: 12 warps per SM at D = 128 (registers), 16 at D = 64.
     // Measured, D = 128, 16 blocks of 30, one / two / four warps per list: 384 lists 22.7 / 18.5 / 15.5 us,
     // 768 lists 25.9 / 23.0 / 28.0 us, 1248 lists 31.6 / 40.8 / 41.0 us
+    const bool short_list = ring_list_bytes(p.T) <= 64 * 1024;                   // (each warp's ring needs its room)
     const int64_t units = static_cast<int64_t>(MG) * p.H * p.B, room = 148 * (D == 128 ? 12 : 16);
-    if (units * 4 <= room) return launch_rows<T, D, 1, 4, TMA>(maps, p, MG, st, s);
-    if (units * 2 <= room) return launch_rows<T, D, 1, 2, TMA>(maps, p, MG, st, s);
+    if (units * 4 <= room && short_list) return launch_rows<T, D, 1, 4, TMA>(maps, p, MG, st, s);
+    if (units * 2 <= room && short_list) return launch_rows<T, D, 1, 2, TMA>(maps, p, MG, st, s);
     return launch_rows<T, D, 1, 1, TMA>(maps, p, MG, st, s);
   }
   if (p.G <= 32) return launch_rows<T, D, 2, 1, TMA>(maps, p, MG, st, s);

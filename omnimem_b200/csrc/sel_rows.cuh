@@ -298,14 +298,13 @@ struct Ring {
 
 // A visible block of one (batch, group, head) list: its 32-row tiles are tiles [first, first of the next slot).
 struct RingSlot {
-  uint64_t a, b;       // addresses of row 0
-  int unit, n_vis;     // rows that count
-  int there, first;    // rows that a copy brings
+  uint64_t a, b;       // cp.async loader: addresses of row 0 of either operand; TMA: the unit, the rows that a copy brings
+  int n_vis, first;    // rows that count, first tile
 };
 inline size_t ring_list_bytes(int T) { return (static_cast<size_t>(T) + 1) * sizeof(RingSlot); }
 
 // The visible blocks of a list, in list order and with a sentinel at the end, written by one warp; returns their tiles.
-template <int ESZ>
+template <int ESZ, bool TMA>
 __device__ __forceinline__ int ring_list(RingSlot* out, const KVSrc& kv, const int32_t* ids, int64_t ids_off, int64_t ids_st,
                                          int T, int b, int h, int D, int block_size, int chunk_size, bool causal, int q_chunk) {
   constexpr int ROWS = 32;
@@ -342,8 +341,9 @@ __device__ __forceinline__ int ring_list(RingSlot* out, const KVSrc& kv, const i
       // (a cut-off last block of a dense tensor: what follows it is outside the tensor and arrives as zeros)
       const int64_t there = kv.mode == NSA_KV_DENSE ? kv.n_tokens - static_cast<int64_t>(unit) * block_size : block_size;
       out[slots + __popc(some & ((1u << lane) - 1))] =
-          RingSlot{reinterpret_cast<uint64_t>(r.k), reinterpret_cast<uint64_t>(r.v), unit, r.n_vis,
-                   static_cast<int>(there < block_size ? there : block_size), count + upto - mine};
+          RingSlot{TMA ? static_cast<uint64_t>(unit) : reinterpret_cast<uint64_t>(r.k),
+                   TMA ? static_cast<uint64_t>(there < block_size ? there : block_size) : reinterpret_cast<uint64_t>(r.v), r.n_vis,
+                   count + upto - mine};
     }
     slots += __popc(some);
     count += __shfl_sync(0xffffffffu, upto, 31);
@@ -361,10 +361,12 @@ __device__ __forceinline__ const RingSlot& ring_slot(const RingSlot* list, int i
   while (list[s + 1].first <= i) ++s;
   return list[s];
 }
+template <bool TMA>
 __device__ __forceinline__ RingTile ring_tile(const RingSlot* list, int i, int per_block, const RingSource& src) {
   const RingSlot& w = ring_slot(list, i, per_block);
-  const int r0 = (i - w.first) * 32;
-  return RingTile{w.a + r0 * src.a_row, w.b + r0 * src.b_row, w.unit, r0, min(32, w.n_vis - r0), min(32, w.there - r0), 0};
+  const int r0 = (i - w.first) * 32, n = min(32, w.n_vis - r0);
+  if (!TMA) return RingTile{w.a + r0 * src.a_row, w.b + r0 * src.b_row, 0, r0, n, n, 0};
+  return RingTile{0, 0, static_cast<int>(w.a), r0, n, min(32, static_cast<int>(w.b) - r0), 0};
 }
 
 template <int ESZ>
