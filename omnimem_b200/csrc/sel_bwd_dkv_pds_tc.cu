@@ -18,7 +18,7 @@
 //   warp 5   MMA issuer: the two products of every step; accumulators double buffered across items
 //   warps 0-3  epilogue: read dV^T / dK^T from TMEM, transpose into two staging tiles and store them
 //            with TMA; items with an empty bucket are zero-filled here
-#include "sel_common.cuh"
+#include "common.cuh"
 #include "tc_common.cuh"
 
 #include <cstdlib>

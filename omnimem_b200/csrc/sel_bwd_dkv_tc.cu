@@ -21,7 +21,7 @@
 //   warps 4-7  epilogue: read dV^T / dK^T from TMEM, transpose into the ring stage of the item's
 //            last step and store the two tiles with TMA; items with an empty bucket are zero-filled here
 // S/dP, the P/dS tiles and the dV^T/dK^T accumulators are double buffered.
-#include "sel_common.cuh"
+#include "common.cuh"
 #include "tc_common.cuh"
 
 #include <cstdlib>

@@ -26,7 +26,7 @@
 // store into the (group, head, slot) pair's place in the buffer: the dK/dV kernel then needs no S, dP
 // or exponential of its own.  The P tile makes it 112 KiB of tiles: two thread blocks still share an
 // SM because the static variables shrink to half a KiB (lists of at most 64 slots).
-#include "sel_common.cuh"
+#include "common.cuh"
 #include "tc_common.cuh"
 
 #include <cstdlib>

@@ -21,7 +21,7 @@
 // one full wave and one half-empty one), so the launch may cut the range into `splits` spans of
 // steps: the thread block of (tile, span) writes a partial output and its log-sum-exp into a
 // workspace and nsa_merge_partials joins the spans exactly.
-#include "sel_common.cuh"
+#include "common.cuh"
 #include "tc_common.cuh"
 
 #include <cstdlib>

@@ -14,7 +14,7 @@
 // c ^ (r & 7)).  The maps know the units (blocks, query groups): rows past the end of a unit arrive as zeros.
 #pragma once
 
-#include "sel_common.cuh"
+#include "common.cuh"
 #include "tc_common.cuh"
 
 namespace nsa {
