@@ -563,37 +563,52 @@ void cache_touch(const CacheState& c, const Tensor& ids, int64_t T, int64_t epoc
 }
 
 // ------------------------------------------------------------------------------------------- layers
-const float* f32(const Tensor& t, const char* what) {
-  if (!t.defined()) return nullptr;
-  need(t.scalar_type() == at::kFloat && t.is_contiguous(), std::string(what) + ": the fp32 vectors must be contiguous float32");
-  return t.data_ptr<float>();
+// The kernels address every operand by x's rows: an operand that is smaller than it should be would be read past its end.
+void need_like(const Tensor& t, const Tensor& x, at::ScalarType type, const char* what) {
+  need(t.scalar_type() == type, std::string(what) + ": dtype torch." + c10::toString(t.scalar_type()) + ", expected torch." + c10::toString(type));
+  need(t.device() == x.device(), std::string(what) + ": all tensors must be on one device");
+}
+// a contiguous row of d values (undefined: none)
+const Tensor& need_row(const Tensor& t, const Tensor& x, at::ScalarType type, int64_t d, const char* what) {
+  if (!t.defined()) return t;
+  need_like(t, x, type, what);
+  need(t.is_contiguous() && t.numel() == d, std::string(what) + ": a row of shape " + shape(t) + ", expected " + std::to_string(d) + " contiguous values");
+  return t;
+}
+int64_t row_length(const Tensor& x, const char* what) {
+  need(x.dim() > 0 && x.size(-1) > 0, std::string(what) + ": rows of shape " + shape(x));
+  return x.size(-1);
 }
 // (x', h): see nsa_residual_norm.  Each vector is (rows of T, rows of fp32), either missing.
 using Vec = std::pair<OptTensor, OptTensor>;
 std::pair<Tensor, OptTensor> residual_norm(const Tensor& x, const OptTensor& y, const Vec& gate, const Vec& scale, const Vec& shift,
                                            bool modulated, bool norm, double eps) {
+  const char* what = "residual_norm";
+  const int64_t d = row_length(x, what), rows = x.numel() / d;
+  if (y.has_value()) {
+    need(y->sizes() == x.sizes(), std::string(what) + ": x of shape " + shape(x) + " and y of shape " + shape(*y));
+    need_like(*y, x, x.scalar_type(), what);
+  }
+  const auto mod = [&](const Vec& v) -> void* { return ptr(need_row(or_none(v.first), x, x.scalar_type(), d, what)); };
+  const auto f32 = [&](const Vec& v) { return static_cast<const float*>(ptr(need_row(or_none(v.second), x, at::kFloat, d, what))); };
+  const void *gm = mod(gate), *sm = mod(scale), *hm = mod(shift);
+  const float *ge = f32(gate), *se = f32(scale), *he = f32(shift);
   need_cuda({&x});
   const c10::cuda::CUDAGuard guard(x.device());
   const Tensor xc = x.contiguous(), yc = y.has_value() ? y->contiguous() : Tensor();
-  const int64_t d = x.size(-1), rows = x.numel() / d;
-  auto mod = [&](const Vec& v) -> void* {
-    const Tensor& t = or_none(v.first);
-    need(!t.defined() || (t.scalar_type() == x.scalar_type() && t.is_contiguous() && t.numel() == d), "residual_norm: vectors must be contiguous rows of x's dtype");
-    return ptr(t);
-  };
   Tensor x_out = yc.defined() ? at::empty(x.sizes(), x.options()) : xc, h;
   if (norm) h = at::empty(x.sizes(), x.options());
-  check("nsa_residual_norm", nsa_residual_norm(xc.data_ptr(), ptr(yc), mod(gate), f32(or_none(gate.second), "residual_norm"), mod(scale),
-                                               f32(or_none(scale.second), "residual_norm"), mod(shift), f32(or_none(shift.second), "residual_norm"),
-                                               modulated, yc.defined() ? x_out.data_ptr() : nullptr, ptr(h), rows, d, static_cast<float>(eps),
+  check("nsa_residual_norm", nsa_residual_norm(xc.data_ptr(), ptr(yc), gm, ge, sm, se, hm, he, modulated,
+                                               yc.defined() ? x_out.data_ptr() : nullptr, ptr(h), rows, d, static_cast<float>(eps),
                                                dtype_of(x), stream_of(x)));
   return {x_out, norm ? OptTensor(h) : OptTensor()};
 }
 // rows of the last dimension; leading dimensions must lie at one stride
 Tensor rms_rows(const Tensor& x, const Tensor& weight, double eps) {
-  need_cuda({&x, &weight});
+  const int64_t d = row_length(x, "rms_rows"), nd = x.dim();
+  need_row(weight, x, x.scalar_type(), d, "rms_rows");
+  need_cuda({&x});
   const c10::cuda::CUDAGuard guard(x.device());
-  const int64_t d = x.size(-1), nd = x.dim();
   bool regular = nd >= 2 && x.stride(-1) == 1;
   for (int64_t i = nd - 3; regular && i >= 0; --i) regular = x.size(i) == 1 || x.stride(i) == x.stride(i + 1) * x.size(i + 1);
   const Tensor xr = regular && is_rows16(x) ? x : x.contiguous();
@@ -604,10 +619,16 @@ Tensor rms_rows(const Tensor& x, const Tensor& weight, double eps) {
 }
 // q, k [S, H*D] views with a common row stride -> q' [S,H,D]; k is overwritten with k'
 Tensor qk_norm_rope(const Tensor& q, const Tensor& k, const Tensor& qw, const Tensor& kw, double eps, int64_t H, const Rope& rope) {
-  need_cuda({&q, &k});
+  const char* what = "qk_norm_rope";
+  need(q.dim() == 2 && k.sizes() == q.sizes() && H > 0 && q.size(1) % H == 0,
+       std::string(what) + ": q of shape " + shape(q) + " and k of shape " + shape(k) + ", expected [S, " + std::to_string(H) + " * D]");
+  need_like(k, q, q.scalar_type(), what);
+  need_row(qw, q, q.scalar_type(), q.size(1), what);
+  need_row(kw, q, q.scalar_type(), q.size(1), what);
+  need(q.stride(0) == k.stride(0) && q.stride(1) == 1 && k.stride(1) == 1, "qk_norm_rope: q and k must share a row stride");
+  need_cuda({&q, &rope.f, &rope.h, &rope.w});
   const c10::cuda::CUDAGuard guard(q.device());
   const int64_t S = q.size(0), D = q.size(1) / H;
-  need(q.stride(0) == k.stride(0) && q.stride(1) == 1 && k.stride(1) == 1, "qk_norm_rope: q and k must share a row stride");
   Tensor qo = at::empty({S, H, D}, q.options());
   const nsa_rope r = rope.c();
   check("nsa_qk_norm_rope", nsa_qk_norm_rope(q.data_ptr(), k.data_ptr(), q.stride(0), qw.data_ptr(), kw.data_ptr(), static_cast<float>(eps), S, H, D,
