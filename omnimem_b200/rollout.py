@@ -37,7 +37,7 @@ import torch.nn as nn
 import torch.nn.functional as F
 
 from . import ops
-from ._lib import host
+from ._lib import NSABackendError, host
 from .cache import BlockKVCache, RopeSpec, rope_apply
 from .nsa.ops.index_topk import should_use_selection_attention
 
@@ -231,7 +231,9 @@ class NSASelfAttention(_Packed):
 
     def forward(self, x, cache: BlockKVCache, rope: RopeSpec, start_token: int, timer=_NO_TIMER):
         p = self.plan
-        _, S, _ = x.shape
+        B, S, _ = x.shape
+        if B != 1:                                    # before anything is projected or appended
+            raise NSABackendError(f"the block caches serve batch size 1, got activations {tuple(x.shape)}")
         H, D = self.h, self.hd
         scale = D ** -0.5
         if _fused(x) and 32 % (D // 8) == 0 and \
