@@ -59,6 +59,20 @@ bool is_rows16(const Tensor& t) {
 }
 // t or a contiguous copy whose innermost stride is 1 and whose rows are 16-byte aligned
 Tensor rows16(const Tensor& t) { return is_rows16(t) ? t : t.contiguous(); }
+// The one stride between the rows that t's first `dims` dimensions count, if they lie evenly.  A dimension of size 1 says
+// nothing: its own stride is arbitrary.
+c10::optional<int64_t> even_stride(const Tensor& t, int64_t dims) {
+  bool any = false;
+  int64_t stride = 0, next = 0;
+  for (int64_t i = dims - 1; i >= 0; --i) {
+    if (t.size(i) == 1) continue;
+    if (any && t.stride(i) != next) return c10::nullopt;
+    if (!any) stride = t.stride(i);
+    any = true;
+    next = t.stride(i) * t.size(i);
+  }
+  return stride;
+}
 struct Strides {
   int64_t v[4];
   explicit Strides(const Tensor& t) {
@@ -446,10 +460,10 @@ Gated gate_args(const Tensor& g, const Tensor& a, const Tensor& b, const Tensor&
 bool token_logits(const Tensor& g, int64_t* stride, int64_t* H) {
   const int64_t nd = g.dim();
   if (nd < 3 || g.stride(-1) != 1 || g.stride(-2) != 3) return false;
+  const auto tokens = even_stride(g, nd - 2);
+  if (!tokens.has_value()) return false;
   *H = g.size(-2);
-  *stride = g.stride(-3);
-  for (int64_t i = nd - 4; i >= 0; --i)
-    if (g.size(i) != 1 && g.stride(i) != g.stride(i + 1) * g.size(i + 1)) return false;
+  *stride = *tokens;
   return true;
 }
 Tensor gate_combine(const Tensor& g_, const Tensor& a, const Tensor& b, const Tensor& c, bool softmax) {
@@ -609,11 +623,11 @@ Tensor rms_rows(const Tensor& x, const Tensor& weight, double eps) {
   need_row(weight, x, x.scalar_type(), d, "rms_rows");
   need_cuda({&x});
   const c10::cuda::CUDAGuard guard(x.device());
-  bool regular = nd >= 2 && x.stride(-1) == 1;
-  for (int64_t i = nd - 3; regular && i >= 0; --i) regular = x.size(i) == 1 || x.stride(i) == x.stride(i + 1) * x.size(i + 1);
-  const Tensor xr = regular && is_rows16(x) ? x : x.contiguous();
+  const auto stride = even_stride(x, nd - 1);
+  const bool as_is = stride.has_value() && is_rows16(x);
+  const Tensor xr = as_is ? x : x.contiguous();
   Tensor out = at::empty(x.sizes(), x.options().memory_format(c10::nullopt));
-  check("nsa_rms_rows", nsa_rms_rows(xr.data_ptr(), nd >= 2 ? xr.stride(-2) : d, weight.data_ptr(), out.data_ptr(), x.numel() / d, d,
+  check("nsa_rms_rows", nsa_rms_rows(xr.data_ptr(), as_is ? *stride : d, weight.data_ptr(), out.data_ptr(), x.numel() / d, d,
                                      static_cast<float>(eps), dtype_of(x), stream_of(x)));
   return out;
 }
@@ -661,6 +675,7 @@ PYBIND11_MODULE(_host, m) {
     need_cuda({&k, &v});
     return Source{NSA_KV_PTR, k, v, Tensor(), stride_bn, 0};
   });
+  m.def("even_stride", &even_stride);
   m.def("pool_rows", &pool_rows);
   m.def("topk", &topk);
   m.def("select_blocks", &select_blocks);

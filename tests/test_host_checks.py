@@ -50,3 +50,48 @@ def test_rows_of_no_values_are_refused():
         host.residual_norm(_bf16(3, 0), None, NONE, NONE, NONE, True, True, 1e-6)
     with pytest.raises(NSABackendError, match="rows of shape"):
         host.rms_rows(_bf16(3, 0), _bf16(0), 1e-6)
+
+
+def _row_views():
+    """[..., 2, 3] views whose leading dimensions lie in every manner: contiguous, cut, spread, repeated, turned."""
+    base = torch.arange(4000)
+    yield base[:120].view(2, 10, 2, 3)
+    yield base[:120].view(2, 1, 10, 2, 3)[:, :, :4]                      # the middle one says nothing
+    yield base[:120].view(2, 1, 10, 2, 3)[:1, :, :4]
+    yield base[:480].view(2, 10, 24)[..., 6:12].unflatten(-1, (2, 3))      # a view into a wider projection
+    yield base[:480].view(4, 5, 24)[:, 1:2, 6:12].unflatten(-1, (2, 3))
+    yield base[:24].view(4, 2, 3).expand(2, 1, 4, 2, 3)
+    yield base[:6].view(1, 2, 3).expand(2, 4, 2, 3)
+    yield base[:120].view(2, 10, 2, 3).transpose(0, 1)
+    yield base[:6].view(1, 1, 2, 3)
+    yield torch.as_strided(base, (3, 1, 4, 2, 3), (24, 24, 6, 3, 1))
+    yield torch.as_strided(base, (3, 1, 4, 2, 3), (60, 60, 6, 3, 1))
+    yield torch.as_strided(base, (3, 1, 4, 2, 3), (24, 999, 6, 3, 1))
+    yield torch.as_strided(base, (3, 2, 1, 2, 3), (12, 6, 7, 3, 1))
+
+
+def test_even_stride_finds_the_stride_of_rows_that_lie_evenly_and_no_other():
+    for t in _row_views():
+        dims, n = t.dim() - 2, t[..., 0, 0].numel()
+        at = [int(x) for x in t[..., 0, 0].reshape(-1)]                    # (the values are their own positions)
+        steps = {b - a for a, b in zip(at, at[1:])}
+        got = host.even_stride(t, dims)
+        assert (got is not None) == (len(steps) <= 1), (t.shape, t.stride(), got)
+        if got is not None:
+            assert [at[0] + i * got for i in range(n)] == at
+
+
+@pytest.mark.gpu
+def test_gates_and_norms_of_views_equal_those_of_their_copies(dev):
+    from omnimem_b200 import ops
+    g = torch.Generator(device=dev).manual_seed(0)
+    for view in _row_views():
+        # the same view of random values
+        logits = torch.randn(4000, generator=g, device=dev).to(torch.bfloat16).as_strided(view.shape, view.stride(), view.storage_offset())
+        o = [torch.randn(*view.shape[:-1], 8, generator=g, device=dev).to(torch.bfloat16) for _ in range(3)]
+        assert torch.equal(ops.gate_combine(logits, *o), ops.gate_combine(logits.contiguous(), *o))
+        # rows of 16 values at the view's leading strides (16 bytes apart)
+        lead, strides = view.shape[:-2], [s * 8 for s in view.stride()[:-2]]
+        x = torch.randn(40000, generator=g, device=dev).to(torch.bfloat16).as_strided((*lead, 16), (*strides, 1))
+        w = torch.randn(16, generator=g, device=dev).to(torch.bfloat16)
+        assert torch.equal(host.rms_rows(x, w, 1e-6), host.rms_rows(x.contiguous(), w, 1e-6))
