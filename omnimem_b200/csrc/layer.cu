@@ -199,17 +199,16 @@ template <typename T, int C>
 __global__ void __launch_bounds__(kWarpsPerBlock * 32) qk_norm_rope_kernel(const QkParams p) {
   const int lane = threadIdx.x & 31;
   const int64_t t = static_cast<int64_t>(blockIdx.x) * kWarpsPerBlock + (threadIdx.x >> 5);
-  double2 f[4];
-  if (t < p.S) {
-    int fr, hr, wr;
-    rope_position(p, t, fr, hr, wr);
-    const int j0 = lane % (p.D / 8) * 4;
-#pragma unroll
-    for (int i = 0; i < 4; ++i) f[i] = rope_factor(p, j0 + i, fr, hr, wr);
-  }
+  int fr = 0, hr = 0, wr = 0;
+  if (t < p.S) rope_position(p, t, fr, hr, wr);
   chain_release();
   chain_wait();
   if (t >= p.S) return;
+  // (the tables too may have been written by the kernel in front of this one)
+  const int j0 = lane % (p.D / 8) * 4;
+  double2 f[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) f[i] = rope_factor(p, j0 + i, fr, hr, wr);
 #pragma unroll
   for (int which = 0; which < 2; ++which) {
     const char* x = (which ? p.k : p.q) + t * p.row_stride * 2;

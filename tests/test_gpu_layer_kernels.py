@@ -110,3 +110,24 @@ def test_packed_projections_follow_their_layers(dev):
     assert not _plain(torch.bfloat16, m.k)
     m.v = torch.nn.Sequential(m.v)
     assert not _plain(torch.bfloat16, m.v)
+
+
+@pytest.mark.parametrize("H,D", [(2, 128), (4, 64)])
+def test_rotary_tables_built_on_the_device(dev, H, D):
+    """The copies that split a table on the device are the launches directly in front of the kernel that reads them: the
+    results are those of a table that was complete long before."""
+    from omnimem_b200._lib import host
+    from omnimem_b200.cache import RopeSpec
+    from omnimem_b200.rollout import rope_table
+    d, S = H * D, 2 * 3 * 5
+    g = torch.Generator(device=dev).manual_seed(D)
+    freqs = torch.cat([rope_table(64, D - 4 * (D // 6)), rope_table(64, 2 * (D // 6)), rope_table(64, 2 * (D // 6))], 1)
+    w = torch.ones(d, device=dev, dtype=torch.bfloat16)
+    for start in range(8):
+        q, k = torch.randn(2, S, d, generator=g, device=dev).to(torch.bfloat16).unbind(0)
+        got = []
+        for table in (freqs, freqs.to(dev)):
+            kk = k.clone()
+            rope = RopeSpec(table, (3, 5), start)
+            got.append((host.qk_norm_rope(q, kk, w, w, 1e-6, H, rope.native(dev, D)), kk))
+        assert torch.equal(got[0][0], got[1][0]) and torch.equal(got[0][1], got[1][1])
