@@ -58,11 +58,12 @@ class RopeSpec:
         return self._tables
 
     def native(self, device, D: int):
-        """The tables on `device` and the geometry, as the native host path takes them."""
-        if self._native is None or self._tables[0].device != device:
+        """The tables on `device` and the geometry as it is now, as the native host path takes them."""
+        geometry = (D, *self.grid_hw, *self.pool, self.start_frame)
+        if self._native is None or self._native[0] != geometry or self._tables[0].device != device:
             tables = self._split(device, D)
-            self._native = host.Rope(*tables, *self.grid_hw, *self.pool, self.start_frame)
-        return self._native
+            self._native = geometry, host.Rope(*tables, *geometry[1:])
+        return self._native[1]
 
     def struct(self, device, D: int) -> _lib.Rope:
         c = D // 2
