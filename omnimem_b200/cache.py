@@ -30,6 +30,23 @@ from . import _lib, ops
 from ._lib import NSABackendError, call, host
 
 
+class _Tables:
+    """A rotary table split over frame, row and column, on a device.  The copies may serve later calls: those with a table
+    of the same values (compared byte by byte, so whatever changed the table is seen) on the stream they were made on.  A
+    table on the device itself is split anew each time."""
+
+    def __init__(self, freqs: torch.Tensor, device):
+        c = freqs.shape[1]
+        parts = freqs.split([c - 2 * (c // 3), c // 3, c // 3], dim=1)
+        self.device, self.stream = device, torch.cuda.current_stream(device).cuda_stream
+        self.source = freqs.detach().clone() if freqs.device.type == "cpu" else None
+        self.parts = [torch.view_as_real(p.contiguous()).to(device).contiguous() for p in parts]
+
+    def serve(self, freqs: torch.Tensor, device) -> bool:
+        return self.source is not None and self.device == device and host.same_bytes(self.source, freqs) \
+            and self.stream == torch.cuda.current_stream(device).cuda_stream
+
+
 class RopeSpec:
     """Rotary embedding of one chunk: `freqs` is the reference's complex128 table
     [max_len, D/2] (rope_params, wan_model.py:37-43; split D/2 - 2*(D/2//3), D/2//3, D/2//3 over
@@ -37,11 +54,12 @@ class RopeSpec:
     chunk's first frame, `pool` the (f, h, w) pooling window that defines the token order."""
 
     def __init__(self, freqs: torch.Tensor, grid_hw, start_frame: int, pool=(1, 1, 1), like: Optional["RopeSpec"] = None):
-        """`like`: a RopeSpec over the same table, whose copies on the device are shared."""
+        """`like`: a RopeSpec whose copies on the device are taken over if they are those of an equal table."""
         if freqs.dtype != torch.complex128 or freqs.dim() != 2:
             raise NSABackendError("RopeSpec: freqs must be a complex128 [max_len, D/2] table")
         self.freqs, self.grid_hw, self.start_frame, self.pool = freqs, tuple(grid_hw), int(start_frame), tuple(pool)
-        self._tables = like._tables if like is not None and like.freqs is freqs else None
+        self._tables = None                      # _Tables on the device of the last use
+        self._offered = like._tables if like is not None else None
         self._native = None
 
     def _split(self, device, D: int):
@@ -51,16 +69,15 @@ class RopeSpec:
         device = torch.device(device)
         if device.index is None:
             device = torch.device(device.type, torch.cuda.current_device())
-        if self._tables is None or self._tables[0].device != device:
-            parts = self.freqs.split([c - 2 * (c // 3), c // 3, c // 3], dim=1)
-            self._tables = [torch.view_as_real(p.contiguous()).to(device).contiguous() for p in parts]
-            self._native = None
-        return self._tables
+        if self._tables is None or self._tables.device != device:
+            offered, self._offered, self._native = self._offered, None, None
+            self._tables = offered if offered is not None and offered.serve(self.freqs, device) else _Tables(self.freqs, device)
+        return self._tables.parts
 
     def native(self, device, D: int):
         """The tables on `device` and the geometry as it is now, as the native host path takes them."""
         geometry = (D, *self.grid_hw, *self.pool, self.start_frame)
-        if self._native is None or self._native[0] != geometry or self._tables[0].device != device:
+        if self._native is None or self._native[0] != geometry or self._tables.device != device:
             tables = self._split(device, D)
             self._native = geometry, host.Rope(*tables, *geometry[1:])
         return self._native[1]

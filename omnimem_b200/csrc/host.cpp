@@ -73,6 +73,12 @@ c10::optional<int64_t> even_stride(const Tensor& t, int64_t dims) {
   }
   return stride;
 }
+// Whether two contiguous CPU tensors hold the same bytes of the same type and shape.
+bool same_bytes(const Tensor& a, const Tensor& b) {
+  const auto plain = [](const Tensor& t) { return t.device().is_cpu() && t.is_contiguous() && !t.is_conj() && !t.is_neg(); };
+  return plain(a) && plain(b) && a.scalar_type() == b.scalar_type() && a.sizes() == b.sizes() &&
+         (a.numel() == 0 || std::memcmp(a.const_data_ptr(), b.const_data_ptr(), a.nbytes()) == 0);
+}
 struct Strides {
   int64_t v[4];
   explicit Strides(const Tensor& t) {
@@ -676,6 +682,7 @@ PYBIND11_MODULE(_host, m) {
     return Source{NSA_KV_PTR, k, v, Tensor(), stride_bn, 0};
   });
   m.def("even_stride", &even_stride);
+  m.def("same_bytes", &same_bytes, py::call_guard<py::gil_scoped_release>());
   m.def("pool_rows", &pool_rows);
   m.def("topk", &topk);
   m.def("select_blocks", &select_blocks);

@@ -36,3 +36,53 @@ def test_rope_refuses_another_head_dim_after_the_first_use(dev):
     rope_apply(_rand(dev, 24, 2, 128), rope)
     with pytest.raises(RuntimeError, match="head dim 64"):
         rope_apply(_rand(dev, 24, 2, 64), rope)
+
+
+def _model(dev):
+    from omnimem_b200 import rollout as R
+    shape = R.WanShape(dim=256, ffn_dim=512, num_heads=2, num_layers=2, text_dim=64, text_len=16)
+    plan = R.RolloutPlan(latent_frames=6, latent_h=8, latent_w=16, topk=2, window_chunks=2, exclude_window_chunks=2)
+    model, caches = R.build(shape, plan, dev, seed=1)
+    latents, raw = _rand(dev, 1, shape.in_dim, 3, 8, 16), _rand(dev, 1, 16, 64)
+
+    def forward(m=model, start=0):
+        for c in caches:
+            c.reset()
+        with torch.no_grad():
+            return m(latents, 500.0, m.text_embedding(raw), start, caches)
+    return R, model, forward
+
+
+def test_rotary_table_changed_in_place_between_forwards(dev):
+    """However the model's table changes, the next forward is that of a model that never used another one."""
+    R, model, forward = _model(dev)
+    first = forward()
+    assert torch.equal(forward(), first)
+    changes = (lambda f: f.mul_(f), lambda f: f.data.mul_(f), lambda f: f.numpy().__imul__(f.numpy()), lambda f: f.copy_(f * f))
+    for change in changes:
+        model.freqs = torch.cat([R.rope_table(1024, 44), R.rope_table(1024, 42), R.rope_table(1024, 42)], dim=1)
+        forward()
+        change(model.freqs)
+        got, model._rope = forward(), None
+        assert torch.equal(got, forward()) and not torch.equal(got, first)
+    model.freqs = model.freqs.to(dev)
+    on_device = forward()
+    model.freqs.data.mul_(model.freqs)
+    got, model._rope = forward(), None
+    assert torch.equal(got, forward()) and not torch.equal(got, on_device)
+
+
+def test_rotary_tables_stay_on_their_stream(dev):
+    """The copies are taken over by later specs on the stream they were made on; another stream makes its own."""
+    from omnimem_b200.cache import RopeSpec, rope_apply
+    x, freqs, side = _rand(dev, 24, 2, 128), _freqs(), torch.cuda.Stream()
+    first = RopeSpec(freqs, (2, 4), 3)
+    want = rope_apply(x, first)
+    second = RopeSpec(freqs, (2, 4), 3, like=first)
+    assert torch.equal(rope_apply(x, second), want) and second._tables is first._tables
+    third = RopeSpec(freqs, (2, 4), 3, like=second)
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        got = rope_apply(x, third)
+    side.synchronize()
+    assert torch.equal(got, want) and third._tables is not first._tables

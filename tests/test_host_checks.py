@@ -81,6 +81,14 @@ def test_even_stride_finds_the_stride_of_rows_that_lie_evenly_and_no_other():
             assert [at[0] + i * got for i in range(n)] == at
 
 
+def test_same_bytes():
+    a = torch.polar(torch.ones(6, 4, dtype=torch.float64), torch.arange(24, dtype=torch.float64).view(6, 4))
+    assert host.same_bytes(a, a.clone()) and host.same_bytes(a[:0], a[:0].clone())
+    last = a.clone()
+    last[5, 3] += 1e-16j
+    assert not any(host.same_bytes(a, b) for b in (last, a[:5], a.conj(), a.to(torch.complex64), a.t().contiguous().t(), a.view(4, 6)))
+
+
 @pytest.mark.gpu
 def test_gates_and_norms_of_views_equal_those_of_their_copies(dev):
     from omnimem_b200 import ops
