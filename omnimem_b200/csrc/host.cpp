@@ -205,10 +205,11 @@ struct Source {
     return s;
   }
 };
-Source dense(const Tensor& k, const Tensor& v) {
+// n_tokens < 0: as many as k has
+Source dense(const Tensor& k, const Tensor& v, int64_t n_tokens = -1) {
   need_cuda({&k, &v});
   need(k.sizes() == v.sizes(), "k and v must have the same shape");
-  return Source{NSA_KV_DENSE, rows16(k), rows16(v), Tensor(), k.size(1), 0};
+  return Source{NSA_KV_DENSE, rows16(k), rows16(v), Tensor(), n_tokens < 0 ? k.size(1) : n_tokens, 0};
 }
 Tensor output_like(const Tensor& q, const OptTensor& given, const char* what) {
   if (!given.has_value()) return at::empty(q.sizes(), q.options());
@@ -672,7 +673,7 @@ PYBIND11_MODULE(_host, m) {
       .def_readonly("k", &Source::k)
       .def_readonly("v", &Source::v)
       .def_readonly("n_tokens", &Source::n_tokens);
-  m.def("dense", &dense);
+  m.def("dense", &dense, py::arg("k"), py::arg("v"), py::arg("n_tokens") = -1);
   m.def("paged", [](const Tensor& k, const Tensor& v, const Tensor& table, int64_t n_tokens, int64_t page_tokens) {
     need_cuda({&k, &v, &table});
     return Source{NSA_KV_PAGED, k, v, table, n_tokens, page_tokens};

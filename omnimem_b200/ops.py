@@ -157,18 +157,17 @@ def merge_candidates(idx: torch.Tensor, scores: torch.Tensor, topk: int):
 # --------------------------------------------------------------------------------- K/V sources
 class DenseKV:
     """k, v [B,N,H,D] addressed by stride."""
+    mode = _lib.NSA_KV_DENSE
 
     def __init__(self, k: torch.Tensor, v: torch.Tensor):
-        self.native = host.dense(k, v)
+        rows = host.dense(k, v)
+        self.k, self.v = rows.k, rows.v
         self.n_tokens = k.shape[1]
 
     @property
-    def k(self) -> torch.Tensor:
-        return self.native.k
-
-    @property
-    def v(self) -> torch.Tensor:
-        return self.native.v
+    def native(self):
+        """The source as it is now, as the native host path takes it."""
+        return host.dense(self.k, self.v, self.n_tokens)
 
     def struct(self) -> KVSource:
         s = KVSource()
@@ -182,11 +181,16 @@ class DenseKV:
 
 class PagedKV:
     """Fixed-page pool + block table (see omnimem_b200.cache.BlockKVCache)."""
+    mode = _lib.NSA_KV_PAGED
 
     def __init__(self, k_pool, v_pool, block_table, n_tokens: int, page_tokens: int):
-        self.native = host.paged(k_pool, v_pool, block_table, int(n_tokens), int(page_tokens))
+        _require_cuda(k_pool, v_pool, block_table)
         self.k_pool, self.v_pool, self.block_table = k_pool, v_pool, block_table
         self.n_tokens, self.page_tokens = int(n_tokens), int(page_tokens)
+
+    @property
+    def native(self):
+        return host.paged(self.k_pool, self.v_pool, self.block_table, self.n_tokens, self.page_tokens)
 
     def struct(self) -> KVSource:
         s = KVSource()
@@ -203,6 +207,7 @@ class PagedKV:
 class PtrKV:
     """int64 byte-address tables [B,MG,H,T] (0 = skip), whole blocks, `stride_bn` elements
     between tokens - the reference's pointer-table contract."""
+    mode = _lib.NSA_KV_PTR
 
     def __init__(self, ptr_k: torch.Tensor, ptr_v: torch.Tensor, stride_bn: int):
         _require_cuda(ptr_k, ptr_v)
@@ -211,7 +216,10 @@ class PtrKV:
         if ptr_k.shape != ptr_v.shape or ptr_k.stride() != ptr_v.stride():
             raise NSABackendError("ptr_k / ptr_v must be [B,MG,H,T] with identical layout")
         self.ptr_k, self.ptr_v, self.stride_bn = ptr_k, ptr_v, int(stride_bn)
-        self.native = host.pointers(ptr_k, ptr_v, self.stride_bn)
+
+    @property
+    def native(self):
+        return host.pointers(self.ptr_k, self.ptr_v, self.stride_bn)
 
     def struct(self) -> KVSource:
         s = KVSource()
@@ -262,7 +270,7 @@ def stored_probabilities_bytes(q, kv, block_indices, block_size: int, group_size
     """Size of the P / dS buffer when the backward of this call can compute them once (dQ kernel
     stores, dK/dV kernel streams), else 0.  The buffer holds 16 KiB per (query group, head, slot);
     OMNIMEM_B200_BWD_STORED_MB caps it (default 4096, 0 turns the path off)."""
-    return host.stored_bytes(q, kv.native.mode, block_indices.shape[-1], block_size, group_size)
+    return host.stored_bytes(q, kv.mode, block_indices.shape[-1], block_size, group_size)
 
 
 def inverted_index(block_indices: torch.Tensor, NS: int, block_size: int, chunk_size: int, causal: bool,

@@ -86,3 +86,50 @@ def test_rotary_tables_stay_on_their_stream(dev):
         got = rope_apply(x, third)
     side.synchronize()
     assert torch.equal(got, want) and third._tables is not first._tables
+
+
+def test_kv_sources_may_change_between_calls(dev):
+    """The forward, the whole backward and its first half read the same fields, as they are at the call."""
+    from omnimem_b200 import ops
+    H, D, G, n = 2, 128, 64, 192
+    q, k, v, k2, v2 = (_rand(dev, 1, n, H, D, seed=i) for i in range(5))
+    ids = torch.arange(3, dtype=torch.int32, device=dev).expand(1, 3, H, 3).contiguous()
+
+    def results(kv, backward=True):
+        out, lse = ops.sel_fwd(q, kv, None if isinstance(kv, ops.PtrKV) else ids, 64, 1, 0.1, False, G)
+        if not backward:
+            return [out, lse]
+        dq, delta = ops.sel_bwd_dq(q, kv, ids, out, lse, q, 64, 1, 0.1, False, G)
+        return [out, lse, dq, delta, *ops.sel_bwd(q, kv, ids, out, lse, q, 64, 1, 0.1, False, G)]
+
+    def same(a, b):
+        return all(x.shape == y.shape and torch.equal(x, y) for x, y in zip(a, b, strict=True))
+
+    kv = ops.DenseKV(k, v)
+    first = results(kv)
+    kv.n_tokens = 100                                                     # the rest of the tokens is not there
+    assert same(results(kv), results(ops.DenseKV(k[:, :100], v[:, :100]))) and not same(results(kv)[:2], first[:2])
+    kv.k, kv.v, kv.n_tokens = k2, v2, n
+    assert same(results(kv), results(ops.DenseKV(k2, v2)))
+
+    pools = [t.view(3, 64, H, D).permute(2, 0, 1, 3).reshape(3 * H, 64, D).contiguous() for t in (k[0], v[0], k2[0], v2[0])]
+    table = torch.arange(3 * H, dtype=torch.int32, device=dev).view(H, 3)
+    other = table.flip(0).contiguous()
+    kv = ops.PagedKV(*pools[:2], table, n, 64)
+    assert same(results(kv), first)
+    kv.n_tokens = 100
+    assert same(results(kv), results(ops.PagedKV(*pools[:2], table, 100, 64)))
+    kv.n_tokens, kv.block_table = n, other
+    assert same(results(kv), results(ops.PagedKV(*pools[:2], other, n, 64)))
+    kv.k_pool, kv.v_pool, kv.block_table = pools[2], pools[3], table
+    assert same(results(kv), results(ops.DenseKV(k2, v2)))
+
+    def addresses(t):
+        return t.data_ptr() + 2 * (ids.long() * 64 * H * D + torch.arange(H, device=dev).view(1, 1, H, 1) * D)
+
+    kv = ops.PtrKV(addresses(k), addresses(v), H * D)
+    ops.sel_fwd(q, kv, None, 64, 1, 0.1, False, G)
+    kv.ptr_k, kv.ptr_v = addresses(k2), addresses(v2)
+    assert same(results(kv, False), results(ops.PtrKV(addresses(k2), addresses(v2), H * D), False))
+    kv.stride_bn = D                                                      # other rows of the same memory
+    assert same(results(kv, False), results(ops.PtrKV(addresses(k2), addresses(v2), D), False))
