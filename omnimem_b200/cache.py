@@ -22,6 +22,7 @@ for them) are taken by kernels; the host only supplies sizes it knows by constru
 from __future__ import annotations
 
 import ctypes as C
+import operator
 from typing import Optional
 
 import torch
@@ -146,9 +147,7 @@ class BlockKVCache:
         self._evicted_any = False
         self.page_bytes = page_tokens * head_dim * self.k_pool.element_size()
         self._dtype_code = ops._dtype(self.k_pool)
-        self._state = host.CacheState([self.k_pool, self.v_pool, self.block_table, self.page_owner, self.page_stamp,
-                                       self.k_pooled, self.v_pooled, self._stamp32, self.status, self.counters],
-                                      num_heads, head_dim, page_tokens, max_blocks)
+        self._native = None
         self.write_behind = bool(write_behind) and host_tier
         self._stage_k = self._stage_v = self._stage_keys = None
         self._drain_event = None                 # recorded behind the last copy from the staging buffer to the host
@@ -157,6 +156,17 @@ class BlockKVCache:
     @property
     def n_blocks(self) -> int:
         return -(-self.n_tokens // self.page_tokens)
+
+    def _state(self):
+        """The device tensors and sizes as they are now, as the native host path takes them (rebuilt when one of them has
+        been replaced; the tensors held are compared as objects, which live as long as they are held)."""
+        tensors = (self.k_pool, self.v_pool, self.block_table, self.page_owner, self.page_stamp, self.k_pooled,
+                   self.v_pooled, self._stamp32, self.status, self.counters)
+        sizes = (self.H, self.D, self.page_tokens, self.max_blocks)
+        held = self._native
+        if held is None or held[1] != sizes or not all(map(operator.is_, held[0], tensors)):
+            self._native = held = tensors, sizes, host.CacheState(list(tensors), *sizes)
+        return held[2]
 
     def _stream(self) -> int:
         return torch.cuda.current_stream(self.device).cuda_stream
@@ -317,7 +327,7 @@ class BlockKVCache:
         if need or (n_exist and self._evicted_any):
             with torch.cuda.device(self.device):
                 new_pages = self._pages_for(first, n_touched, n_exist, n_new, protect_from)
-        host.cache_append(self._state, k_new, v_new, pos0, self.n_tokens, self.epoch, new_pages,
+        host.cache_append(self._state(), k_new, v_new, pos0, self.n_tokens, self.epoch, new_pages,
                           None if rope is None else rope.native(self.device, self.D))
         self.n_tokens = max(self.n_tokens, pos0 + S)
 
@@ -330,7 +340,7 @@ class BlockKVCache:
         self.epoch += 1
         if not return_lists and not (self._evicted_any and self.host_k is not None):
             # nothing to fetch: stamps and counters only, no lists
-            host.cache_touch(self._state, ids, T, self.epoch)
+            host.cache_touch(self._state(), ids, T, self.epoch)
             return None
         with torch.cuda.device(self.device):
             uniq, miss = self._make_resident(ids, T, count=True)

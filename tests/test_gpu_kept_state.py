@@ -133,3 +133,23 @@ def test_kv_sources_may_change_between_calls(dev):
     assert same(results(kv, False), results(ops.PtrKV(addresses(k2), addresses(v2), H * D), False))
     kv.stride_bn = D                                                      # other rows of the same memory
     assert same(results(kv, False), results(ops.PtrKV(addresses(k2), addresses(v2), D), False))
+
+
+def test_cache_tensors_may_be_replaced(dev):
+    """Appends and touches write the tensors that the cache has now, as the page moves and the attention do."""
+    from omnimem_b200.cache import BlockKVCache
+    H, D = 2, 128
+    k, v = _rand(dev, 200, H, D, seed=1), _rand(dev, 200, H, D, seed=2)
+    ids = torch.arange(4, dtype=torch.int32, device=dev).expand(1, 1, H, 4).contiguous()
+    kept, moved = (BlockKVCache(H, D, 8, 4, device=dev, host_tier=False) for _ in range(2))
+    names = ("k_pool", "v_pool", "block_table", "page_owner", "page_stamp", "k_pooled", "v_pooled", "_stamp32", "status", "counters")
+    for step in range(3):
+        old = [getattr(moved, n) for n in names]
+        for n, t in zip(names, old):
+            setattr(moved, n, t.clone())
+        before = [t.clone() for t in old]
+        for cache in (kept, moved):
+            cache.append(k[step * 60:step * 60 + 80], v[step * 60:step * 60 + 80], pos0=step * 60)
+            cache.touch(ids)
+        assert all(torch.equal(getattr(kept, n), getattr(moved, n)) for n in names)
+        assert all(map(torch.equal, old, before))
