@@ -63,6 +63,9 @@ class RopeSpec:
         self._offered = like._tables if like is not None else None
         self._native = None
 
+    def __getstate__(self):                      # (copies and pickles make their own)
+        return {**self.__dict__, "_tables": None, "_offered": None, "_native": None}
+
     def _split(self, device, D: int):
         c = D // 2
         if self.freqs.shape[1] != c:
@@ -151,6 +154,14 @@ class BlockKVCache:
         self.write_behind = bool(write_behind) and host_tier
         self._stage_k = self._stage_v = self._stage_keys = None
         self._drain_event = None                 # recorded behind the last copy from the staging buffer to the host
+
+    def __getstate__(self):
+        return {**self.__dict__, "_native": None}
+
+    def __setstate__(self, state):
+        self.__dict__.update(state)
+        if self.host_k is not None:              # the device writes to the host tier, and a copy of it is not pinned
+            self.host_k, self.host_v = (t if t.is_pinned() else t.pin_memory() for t in (self.host_k, self.host_v))
 
     # ------------------------------------------------------------------------------ helpers
     @property

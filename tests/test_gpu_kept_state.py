@@ -1,4 +1,7 @@
 """Objects that the native host path keeps something of between calls: what their owner changes is seen by the next call."""
+import copy
+import pickle
+
 import pytest
 import torch
 
@@ -153,3 +156,59 @@ def test_cache_tensors_may_be_replaced(dev):
             cache.touch(ids)
         assert all(torch.equal(getattr(kept, n), getattr(moved, n)) for n in names)
         assert all(map(torch.equal, old, before))
+
+
+COPIES = [copy.copy, copy.deepcopy, lambda x: pickle.loads(pickle.dumps(x))]
+
+
+@pytest.mark.parametrize("duplicate", COPIES)
+def test_used_objects_can_be_copied(dev, duplicate):
+    from omnimem_b200 import ops
+    from omnimem_b200.cache import RopeSpec, rope_apply
+    x = _rand(dev, 1, 128, 2, 128)
+    rope = RopeSpec(_freqs(), (4, 8), 3)
+    want = rope_apply(x[0], rope)
+    other = duplicate(rope)
+    other.start_frame = 5
+    assert torch.equal(rope_apply(x[0], duplicate(rope)), want) and not torch.equal(rope_apply(x[0], other), want)
+    ids = torch.zeros(1, 2, 2, 1, dtype=torch.int32, device=dev)
+    table = torch.arange(4, dtype=torch.int32, device=dev).view(2, 2)
+    pool = _rand(dev, 4, 64, 128)
+    for kv in (ops.DenseKV(x, x), ops.PagedKV(pool, pool, table, 128, 64)):
+        want = ops.sel_fwd(x, kv, ids, 64, 1, 0.1, False, 64)
+        assert all(map(torch.equal, ops.sel_fwd(x, duplicate(kv), ids, 64, 1, 0.1, False, 64), want))
+
+
+@pytest.mark.parametrize("duplicate", COPIES[1:])
+@pytest.mark.parametrize("host_tier", [False, True])
+def test_used_caches_can_be_copied(dev, duplicate, host_tier):
+    """The copy goes its own way, its host tier included, and meets what the original would have met."""
+    from omnimem_b200.cache import BlockKVCache
+    H, D = 2, 128
+    cache = BlockKVCache(H, D, 12 if host_tier else 32, 16, device=dev, host_tier=host_tier, write_behind=False)
+    for i in range(8):
+        cache.append(_rand(dev, 64, H, D, seed=i), _rand(dev, 64, H, D, seed=100 + i))
+    assert (cache.stats()["pages_evicted"] > 0) == host_tier
+    other = duplicate(cache)
+    q = _rand(dev, 1, 64, H, D, seed=9)
+    ids = torch.tensor([0, 1, 6], dtype=torch.int32, device=dev).expand(1, 1, H, 3).contiguous()
+    for i in range(2):
+        outs = [c.selection_attention(q, ids) for c in (cache, other)]
+        assert torch.equal(*outs) and cache.stats() == other.stats() and cache.n_tokens == other.n_tokens
+        for c in (cache, other):
+            c.append(_rand(dev, 64, H, D, seed=50 + i), _rand(dev, 64, H, D, seed=60 + i))
+    other.append(q[0], q[0])
+    assert other.n_tokens == cache.n_tokens + 64
+    for c in (cache, other):
+        c.check_status()
+
+
+@pytest.mark.parametrize("duplicate", COPIES[1:])
+def test_used_models_can_be_copied(dev, duplicate):
+    R, model, forward = _model(dev)
+    want = forward()
+    other = duplicate(model)
+    assert torch.equal(forward(other), want)
+    with torch.no_grad():
+        other.blocks[0].self_attn.q.weight.zero_()
+    assert not torch.equal(forward(other), want) and torch.equal(forward(), want)
