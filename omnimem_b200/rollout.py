@@ -35,6 +35,7 @@ from typing import List, Optional
 import torch
 import torch.nn as nn
 import torch.nn.functional as F
+from torch.nn.modules.module import _has_any_global_hook
 
 from . import ops
 from ._lib import NSABackendError, host
@@ -146,21 +147,31 @@ class RMSNorm(nn.Module):
 
 def _fused(x: torch.Tensor) -> bool:
     """Whether the fused kernels serve activations x [.., d] (layer.cu): 16-bit, no gradients, no autocast, rows they are
-    built for."""
+    built for, and no hook that every module's call has to run."""
     return x.is_cuda and x.dtype in (torch.bfloat16, torch.float16) and not torch.is_grad_enabled() \
-        and not torch.is_autocast_enabled("cuda") and x.shape[-1] in (256, 512, 1024, 1536, 2048)
+        and not torch.is_autocast_enabled("cuda") and x.shape[-1] in (256, 512, 1024, 1536, 2048) \
+        and not _has_any_global_hook()
+
+
+def _untouched(m: nn.Module) -> bool:
+    """Whether calling module m does nothing but what its class does as it is written here: no hooks, no `forward` of its
+    own (offloading and adapter libraries set one), none put on its class, and it is not compiled."""
+    own = _PLAIN.get(type(m))
+    return own is not None and own is type(m).forward and "forward" not in m.__dict__ and not m._forward_hooks \
+        and not m._forward_pre_hooks and m._compiled_call_impl is None
 
 
 def _plain(dtype: torch.dtype, *mods: nn.Module) -> bool:
     """Whether the parameters of `mods` may be used without calling them: the layers built here (not something a user
-    put in their place), no hooks, parameters of the activations' type."""
+    put in their place), untouched, parameters of the activations' type."""
     for m in mods:
-        if type(m) not in _PLAIN or m._forward_hooks or m._forward_pre_hooks or m._parameters["weight"].dtype != dtype:
+        weight = m._parameters.get("weight")
+        if not _untouched(m) or weight is None or weight.dtype != dtype:
             return False
     return True
 
 
-_PLAIN = (nn.Linear, nn.LayerNorm, RMSNorm)
+_PLAIN = {c: c.forward for c in (nn.Linear, nn.LayerNorm, nn.GELU, nn.Sequential, RMSNorm)}     # (and the layers below)
 
 
 class _Packed(nn.Module):
@@ -333,9 +344,10 @@ class Block(nn.Module):
 
     def fusable(self, dtype: torch.dtype) -> bool:
         up, act, down = self.ffn if len(self.ffn) == 3 else (None, None, None)
-        return type(self) is Block and not self._forward_hooks and not self._forward_pre_hooks \
-            and type(act) is nn.GELU and act.approximate == "tanh" and not self.ffn._forward_hooks \
-            and not self.ffn._forward_pre_hooks and self.modulation.dtype == dtype and _plain(dtype, up, down, self.norm3)
+        attn, cross = self.self_attn, self.cross_attn
+        return all(map(_untouched, (self, attn, cross, self.ffn, act))) and type(act) is nn.GELU \
+            and act.approximate == "tanh" and self.modulation.dtype == dtype \
+            and _plain(dtype, up, down, self.norm3, attn.o, cross.o)
 
     def fused(self, x, pending, e, context, cache, rope, start_token, timer=_NO_TIMER):
         """forward() with the residual of the sub-layer in front still `pending` (its output and gate vector, or
@@ -373,6 +385,9 @@ class Block(nn.Module):
             h = (F.layer_norm(x.float(), (d,), eps=self.eps) * (1 + e[4]) + e[3]).to(x.dtype)
             x = x + (self.ffn(h).float() * e[5]).to(x.dtype)
         return x
+
+
+_PLAIN.update((c, c.forward) for c in (NSASelfAttention, CrossAttention, Block))
 
 
 class CausalWanNSA(nn.Module):

@@ -26,3 +26,77 @@ def test_batches_are_refused(dev):
         with pytest.raises(RuntimeError, match="batch size 1"):
             model(torch.randn(2, shape.in_dim, 3, 8, 16, device=dev).to(torch.bfloat16), 500.0, context, 0, caches)
     assert caches[0].n_tokens == 0 and caches[1].n_tokens == 0
+
+
+def _setup(dev):
+    R, shape, plan = _tiny()
+    model, caches = R.build(shape, plan, dev, seed=1)
+    g = torch.Generator(device=dev).manual_seed(2)
+    rand = lambda *s: torch.randn(*s, generator=g, device=dev).to(torch.bfloat16)
+    for p in model.parameters():                       # biases and norm weights that are not 0 and 1
+        with torch.no_grad():
+            p.add_(0.05 * torch.randn(p.shape, generator=g, device=dev))
+    latents, raw = [rand(1, shape.in_dim, 3, 8, 16) for _ in range(2)], rand(1, 16, 64)
+
+    def forward(eager=False):
+        """Two chunks in a row; the layers take their eager form where gradients are on."""
+        for c in caches:
+            c.reset()
+        with torch.set_grad_enabled(eager):
+            context = model.text_embedding(raw)
+            return torch.cat([model(x, 500.0, context, 3 * i, caches).detach() for i, x in enumerate(latents)])
+    return model, forward
+
+
+def _agree(got, want):
+    # two bf16 blocks in a row, their activations rounded at other places: some four roundings of 2^-9 each
+    assert (got.float() - want.float()).norm() <= 1e-2 * want.float().norm()
+
+
+def test_the_fused_model_computes_what_its_eager_form_does(dev):
+    model, forward = _setup(dev)
+    assert all(b.fusable(torch.bfloat16) for b in model.blocks)
+    _agree(forward(), forward(eager=True))
+
+
+LAYERS = ("self_attn", "self_attn.q", "self_attn.k", "self_attn.v", "self_attn.g_proj", "self_attn.norm_q", "self_attn.norm_k",
+          "self_attn.o", "norm3", "cross_attn", "cross_attn.q", "cross_attn.k", "cross_attn.v", "cross_attn.norm_q", "cross_attn.norm_k",
+          "cross_attn.o", "ffn", "ffn.0", "ffn.1", "ffn.2", "")
+
+
+@pytest.mark.parametrize("layer", LAYERS)
+def test_a_layer_with_a_forward_of_its_own_is_called(dev, layer):
+    model, forward = _setup(dev)
+    plain = forward()
+    m = model.blocks[1].get_submodule(layer)
+    own, calls = m.forward, []
+
+    def scaled(*args, **kw):
+        calls.append(layer)
+        return own(*args, **kw) * 0.5
+
+    m.forward = scaled
+    got = forward()
+    assert len(calls) == 2 and not torch.equal(got, plain)
+    _agree(got, forward(eager=True))
+    del m.forward
+    assert torch.equal(forward(), plain)
+
+
+def test_global_hooks_and_patched_classes_are_met(dev):
+    from torch.nn.modules.module import register_module_forward_hook
+    model, forward = _setup(dev)
+    plain, seen = forward(), set()
+    handle = register_module_forward_hook(lambda m, args, out: seen.add(m))
+    forward()
+    handle.remove()
+    assert {m for n, m in model.named_modules() if n.startswith("blocks.")} <= seen
+    own = torch.nn.Linear.forward
+    try:
+        torch.nn.Linear.forward = lambda self, x: 0.5 * own(self, x)
+        got = forward()
+        _agree(got, forward(eager=True))
+        assert not torch.equal(got, plain)
+    finally:
+        torch.nn.Linear.forward = own
+    assert torch.equal(forward(), plain)
