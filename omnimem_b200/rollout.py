@@ -161,16 +161,29 @@ def _untouched(m: nn.Module) -> bool:
         and not m._forward_pre_hooks and m._compiled_call_impl is None
 
 
+def _row(p, dtype: torch.dtype) -> bool:
+    """Whether the row kernels can read vector (or rows of vectors) p as it lies."""
+    return type(p) in _TENSORS and p.dtype == dtype and p.is_contiguous() and p.data_ptr() % 16 == 0
+
+
 def _plain(dtype: torch.dtype, *mods: nn.Module) -> bool:
     """Whether the parameters of `mods` may be used without calling them: the layers built here (not something a user
-    put in their place), untouched, parameters of the activations' type."""
+    put in their place), untouched, parameters of the activations' type.  A linear layer may lack its bias, a norm has to
+    have all that it is built with."""
     for m in mods:
-        weight = m._parameters.get("weight")
-        if not _untouched(m) or weight is None or weight.dtype != dtype:
+        if not _untouched(m):
+            return False
+        weight, bias = m._parameters.get("weight"), m._parameters.get("bias")
+        if type(m) is nn.Linear:
+            if type(weight) not in _TENSORS or weight.dtype != dtype or \
+                    bias is not None and (type(bias) not in _TENSORS or bias.dtype != dtype):
+                return False
+        elif not _row(weight, dtype) or type(m) is nn.LayerNorm and not _row(bias, dtype):
             return False
     return True
 
 
+_TENSORS = (nn.Parameter, torch.Tensor)              # (not subclasses, which may keep their values elsewhere)
 _PLAIN = {c: c.forward for c in (nn.Linear, nn.LayerNorm, nn.GELU, nn.Sequential, RMSNorm)}     # (and the layers below)
 
 
@@ -186,20 +199,26 @@ class _Packed(nn.Module):
     def _apply(self, fn, *args, **kwargs):
         super()._apply(fn, *args, **kwargs)
         mods = [getattr(self, n) for n in self.packed]
-        if all(type(m) is nn.Linear for m in mods) and self._joined(mods) is None and mods[0].weight.is_cuda \
-                and len({(m.weight.dtype, m.weight.device, m.in_features) for m in mods}) == 1:
-            pad = -sum(m.out_features for m in mods) % 64
-            whole = []
-            for name in ("weight", "bias"):
-                parts = [m._parameters[name] for m in mods]
-                t = torch.cat([p.data for p in parts] + [parts[0].data.new_zeros(pad, *parts[0].shape[1:])])
-                at = 0
-                for p in parts:
-                    p.data = t[at:at + p.shape[0]]
-                    at += p.shape[0]
-                whole.append(t)
-            self._whole = tuple(whole)
+        if all(type(m) is nn.Linear for m in mods):
+            params = [m._parameters.get(n) for n in ("weight", "bias") for m in mods]
+            if all(type(p) is nn.Parameter and p.is_cuda for p in params) and len(set(map(id, params))) == len(params) \
+                    and len({(p.dtype, p.device) for p in params}) == 1 and len({m.in_features for m in mods}) == 1 \
+                    and self._joined(mods) is None:
+                self._pack(params[:len(mods)], params[len(mods):])
         return self
+
+    def _pack(self, *kinds):
+        """Moves the weights, and the biases, one below the other."""
+        whole = []
+        for parts in kinds:
+            pad = -sum(p.shape[0] for p in parts) % 64
+            t = torch.cat([p.data for p in parts] + [parts[0].data.new_zeros(pad, *parts[0].shape[1:])])
+            at = 0
+            for p in parts:
+                p.data = t[at:at + p.shape[0]]
+                at += p.shape[0]
+            whole.append(t)
+        self._whole = tuple(whole)
 
     def _joined(self, mods):
         """_whole, if the parameters still lie in it (its storage is kept, so an equal address is a view of it)."""
@@ -208,8 +227,8 @@ class _Packed(nn.Module):
         for name, t in zip(("weight", "bias"), self._whole):
             at = t.data_ptr()
             for m in mods:
-                p = m._parameters[name]
-                if p.data_ptr() != at or p.dtype != t.dtype or not p.is_contiguous():
+                p = m._parameters.get(name)
+                if type(p) not in _TENSORS or p.data_ptr() != at or p.dtype != t.dtype or not p.is_contiguous():
                     self._whole = None
                     return None
                 at += p.nbytes
@@ -346,8 +365,8 @@ class Block(nn.Module):
         up, act, down = self.ffn if len(self.ffn) == 3 else (None, None, None)
         attn, cross = self.self_attn, self.cross_attn
         return all(map(_untouched, (self, attn, cross, self.ffn, act))) and type(act) is nn.GELU \
-            and act.approximate == "tanh" and self.modulation.dtype == dtype \
-            and _plain(dtype, up, down, self.norm3, attn.o, cross.o)
+            and act.approximate == "tanh" and _row(self.modulation, dtype) \
+            and _plain(dtype, up, down, self.norm3, attn.o, cross.o) and up.bias is not None
 
     def fused(self, x, pending, e, context, cache, rope, start_token, timer=_NO_TIMER):
         """forward() with the residual of the sub-layer in front still `pending` (its output and gate vector, or
@@ -421,7 +440,7 @@ class CausalWanNSA(nn.Module):
         e0 = self.time_projection(e).float().view(1, 6, sh.dim)
         rope = self._rope = RopeSpec(self.freqs, (gh, gw), start_frame, (1, 1, 1), like=self._rope)
         start_token = start_frame * gh * gw
-        if _fused(x) and self.head_modulation.dtype == x.dtype and all(b.fusable(x.dtype) for b in self.blocks):
+        if _fused(x) and _row(self.head_modulation, x.dtype) and all(b.fusable(x.dtype) for b in self.blocks):
             pending, e_rows = None, e0[0].unbind(0)
             for blk, cache in zip(self.blocks, caches):
                 x, pending = blk.fused(x, pending, e_rows, context_embedded, cache, rope, start_token, timer)

@@ -100,3 +100,80 @@ def test_global_hooks_and_patched_classes_are_met(dev):
     finally:
         torch.nn.Linear.forward = own
     assert torch.equal(forward(), plain)
+
+
+def _without(layer, name):
+    def change(model):
+        for b in model.blocks:
+            b.get_submodule(layer).register_parameter(name, None)
+    return pytest.param(change, id=f"{layer} without {name}")
+
+
+def _replaced(layer, make, what):
+    def change(model):
+        for b in model.blocks:
+            path, _, name = layer.rpartition(".")
+            old = b.get_submodule(layer)
+            new = make(old).to(device=next(model.parameters()).device, dtype=torch.bfloat16)
+            setattr(b.get_submodule(path), name, new)
+    return pytest.param(change, id=f"{layer}: {what}")
+
+
+def _parameter(layer, name, make, what):
+    def change(model):
+        for b in model.blocks:
+            m = b.get_submodule(layer)
+            setattr(m, name, torch.nn.Parameter(make(getattr(m, name).data)))
+    return pytest.param(change, id=f"{layer}.{name}: {what}")
+
+
+def _spread(t):
+    return torch.stack([t, t], -1)[..., 0]                        # not contiguous
+
+
+def _shifted(t):
+    return torch.cat([t.new_zeros(1), t.flatten()])[1:].view_as(t)  # not aligned to 16 bytes
+
+
+def _no_bias(old):
+    return torch.nn.Linear(old.in_features, old.out_features, bias=False)
+
+
+def _no_affine(old):
+    return torch.nn.LayerNorm(old.normalized_shape, eps=old.eps, elementwise_affine=False)
+
+
+VARIANTS = [_without(l, "bias") for l in ("self_attn.q", "self_attn.g_proj", "self_attn.o", "cross_attn.k", "cross_attn.o", "ffn.0", "ffn.2",
+                                          "norm3")]
+VARIANTS += [_replaced(l, _no_bias, "no bias") for l in ("self_attn.k", "cross_attn.v", "ffn.0", "ffn.2")]
+VARIANTS += [_replaced("norm3", _no_affine, "no affine")]
+VARIANTS += [_parameter(l, "weight", f, f.__name__) for l in ("self_attn.norm_q", "self_attn.norm_k", "cross_attn.norm_k", "norm3", "self_attn.v")
+             for f in (_spread, _shifted)]
+VARIANTS += [_parameter("", "modulation", f, f.__name__) for f in (_spread, _shifted)]
+VARIANTS += [_parameter("self_attn.norm_q", "weight", torch.Tensor.float, "fp32")]
+
+
+@pytest.mark.parametrize("moved", [False, True])
+@pytest.mark.parametrize("change", VARIANTS)
+def test_ordinary_variants_of_the_layers(dev, change, moved):
+    """Layers without a bias, norms without a weight, parameters that lie otherwise: the eager form's result, also after
+    the model has been moved (where the weights of the projections are laid together)."""
+    model, forward = _setup(dev)
+    plain = forward()
+    change(model)
+    if moved:
+        model.to(dtype=torch.float32).to(dtype=torch.bfloat16)
+    got = forward()
+    _agree(got, forward(eager=True))
+    assert got.shape == plain.shape and torch.isfinite(got.float()).all()
+
+
+def test_moved_models_keep_types_and_ties(dev):
+    """Laying weights together changes neither a parameter's type nor which layers share one."""
+    model, forward = _setup(dev)
+    attn, cross = model.blocks[0].self_attn, model.blocks[0].cross_attn
+    attn.q.bias = torch.nn.Parameter(attn.q.bias.data.float())
+    cross.k.weight = cross.v.weight
+    model.to(dev)
+    assert attn.q.bias.dtype == torch.float32 and attn.k.bias.dtype == torch.bfloat16 and attn.q.weight.dtype == torch.bfloat16
+    assert cross.k.weight is cross.v.weight and cross.k.weight.data_ptr() == cross.v.weight.data_ptr()
