@@ -266,8 +266,10 @@ class NSASelfAttention(_Packed):
             raise NSABackendError(f"the block caches serve batch size 1, got activations {tuple(x.shape)}")
         H, D = self.h, self.hd
         scale = D ** -0.5
-        if _fused(x) and 32 % (D // 8) == 0 and \
-                _plain(x.dtype, self.q, self.k, self.v, self.g_proj, self.norm_q, self.norm_k):
+        # (one eps serves both norms)
+        if _fused(x) and D % 8 == 0 and 32 % (D // 8) == 0 and \
+                _plain(x.dtype, self.q, self.k, self.v, self.g_proj, self.norm_q, self.norm_k) and \
+                self.norm_q.eps == self.norm_k.eps:
             with timer("qkv_gate_proj"):
                 q, k, v, g = self.project(x[0])
                 g = g.view(1, S, H, 3)

@@ -177,3 +177,14 @@ def test_moved_models_keep_types_and_ties(dev):
     model.to(dev)
     assert attn.q.bias.dtype == torch.float32 and attn.k.bias.dtype == torch.bfloat16 and attn.q.weight.dtype == torch.bfloat16
     assert cross.k.weight is cross.v.weight and cross.k.weight.data_ptr() == cross.v.weight.data_ptr()
+
+
+@pytest.mark.parametrize("layer", ["self_attn.norm_q", "self_attn.norm_k", "cross_attn.norm_k", "norm3"])
+def test_each_norm_has_an_eps_of_its_own(dev, layer):
+    model, forward = _setup(dev)
+    plain = forward()
+    for b in model.blocks:
+        b.get_submodule(layer).eps = 4.0
+    got = forward()
+    _agree(got, forward(eager=True))
+    assert not torch.equal(got, plain)
