@@ -183,6 +183,10 @@ def _plain(dtype: torch.dtype, *mods: nn.Module) -> bool:
     return True
 
 
+def _are(kind, *mods: nn.Module) -> bool:
+    return all(type(m) is kind for m in mods)
+
+
 _TENSORS = (nn.Parameter, torch.Tensor)              # (not subclasses, which may keep their values elsewhere)
 _PLAIN = {c: c.forward for c in (nn.Linear, nn.LayerNorm, nn.GELU, nn.Sequential, RMSNorm)}     # (and the layers below)
 
@@ -268,6 +272,7 @@ class NSASelfAttention(_Packed):
         scale = D ** -0.5
         # (one eps serves both norms)
         if _fused(x) and D % 8 == 0 and 32 % (D // 8) == 0 and \
+                _are(nn.Linear, self.q, self.k, self.v, self.g_proj) and _are(RMSNorm, self.norm_q, self.norm_k) and \
                 _plain(x.dtype, self.q, self.k, self.v, self.g_proj, self.norm_q, self.norm_k) and \
                 self.norm_q.eps == self.norm_k.eps:
             with timer("qkv_gate_proj"):
@@ -335,7 +340,8 @@ class CrossAttention(_Packed):
     def forward(self, x, context):
         B, S, d = x.shape
         L = context.shape[1]
-        if _fused(x) and _plain(x.dtype, self.k, self.v, self.norm_q, self.norm_k) and context.dtype == x.dtype:
+        if _fused(x) and context.dtype == x.dtype and _are(nn.Linear, self.k, self.v) and _are(RMSNorm, self.norm_q, self.norm_k) \
+                and _plain(x.dtype, self.k, self.v, self.norm_q, self.norm_k):
             heads = lambda t: t.unflatten(-1, (self.h, self.hd)).transpose(1, 2)
             k, v = self.project(context)
             q = heads(host.rms_rows(self.q(x), self.norm_q.weight, self.norm_q.eps))
@@ -364,9 +370,12 @@ class Block(nn.Module):
         self.modulation = nn.Parameter(torch.randn(1, 6, d) / d ** 0.5)
 
     def fusable(self, dtype: torch.dtype) -> bool:
-        up, act, down = self.ffn if len(self.ffn) == 3 else (None, None, None)
-        attn, cross = self.self_attn, self.cross_attn
-        return all(map(_untouched, (self, attn, cross, self.ffn, act))) and type(act) is nn.GELU \
+        attn, cross, ffn = self.self_attn, self.cross_attn, self.ffn
+        if not (_are(NSASelfAttention, attn) and _are(CrossAttention, cross) and _are(nn.LayerNorm, self.norm3)
+                and _are(nn.Sequential, ffn) and all(map(_untouched, (self, attn, cross, ffn))) and len(ffn) == 3):
+            return False
+        up, act, down = ffn
+        return _are(nn.Linear, up, down, attn.o, cross.o) and _are(nn.GELU, act) and _untouched(act) \
             and act.approximate == "tanh" and _row(self.modulation, dtype) \
             and _plain(dtype, up, down, self.norm3, attn.o, cross.o) and up.bias is not None
 
@@ -442,7 +451,7 @@ class CausalWanNSA(nn.Module):
         e0 = self.time_projection(e).float().view(1, 6, sh.dim)
         rope = self._rope = RopeSpec(self.freqs, (gh, gw), start_frame, (1, 1, 1), like=self._rope)
         start_token = start_frame * gh * gw
-        if _fused(x) and _row(self.head_modulation, x.dtype) and all(b.fusable(x.dtype) for b in self.blocks):
+        if _fused(x) and _row(self.head_modulation, x.dtype) and all(_are(Block, b) and b.fusable(x.dtype) for b in self.blocks):
             pending, e_rows = None, e0[0].unbind(0)
             for blk, cache in zip(self.blocks, caches):
                 x, pending = blk.fused(x, pending, e_rows, context_embedded, cache, rope, start_token, timer)

@@ -188,3 +188,43 @@ def test_each_norm_has_an_eps_of_its_own(dev, layer):
     got = forward()
     _agree(got, forward(eager=True))
     assert not torch.equal(got, plain)
+
+
+class _Wrapped(torch.nn.Module):
+    def __init__(self, inner):
+        super().__init__()
+        self.inner = inner
+
+    def forward(self, *args, **kw):
+        return self.inner(*args, **kw)
+
+
+def _layer_norm(old):
+    return torch.nn.LayerNorm(old.weight.numel())
+
+
+def _rms_norm(old):
+    from omnimem_b200.rollout import RMSNorm
+    return RMSNorm(old.weight.numel(), old.eps)
+
+
+KINDS = [_replaced(l, _layer_norm, "layer norm") for l in ("self_attn.norm_q", "self_attn.norm_k", "cross_attn.norm_q", "cross_attn.norm_k")]
+KINDS += [_replaced("norm3", _rms_norm, "rms norm")]
+KINDS += [_replaced(l, _Wrapped, "wrapped") for l in ("ffn", "ffn.0", "ffn.1", "self_attn", "cross_attn", "self_attn.q", "self_attn.o", "norm3")]
+KINDS += [_replaced("ffn.1", lambda old: torch.nn.GELU(), "exact gelu"),
+          _replaced("ffn", lambda old: torch.nn.Sequential(*old, torch.nn.Identity()), "longer")]
+
+
+@pytest.mark.parametrize("change", KINDS)
+def test_layers_of_another_kind(dev, change):
+    """What a user puts in a layer's place is what runs there, also where it is one of the kinds that the fused form knows."""
+    model, forward = _setup(dev)
+    change(model)
+    _agree(forward(), forward(eager=True))
+
+
+def test_blocks_of_another_kind(dev):
+    model, forward = _setup(dev)
+    plain = forward(eager=True)
+    model.blocks[1] = _Wrapped(model.blocks[1])
+    _agree(forward(), plain)
