@@ -372,12 +372,7 @@ struct IdCheck {
   }
   bool bad() {
     if (!live) return false;
-    cudaError_t e;
-    {
-      py::gil_scoped_release release;
-      e = cudaEventSynchronize(flag.event);
-    }
-    C10_CUDA_CHECK(e);
+    C10_CUDA_CHECK(cudaEventSynchronize(flag.event));
     waited = true;
     return *static_cast<volatile int32_t*>(flag.word) != 0;
   }
@@ -660,6 +655,8 @@ Tensor qk_norm_rope(const Tensor& q, const Tensor& k, const Tensor& qw, const Te
 }  // namespace
 
 PYBIND11_MODULE(_host, m) {
+  // a launch may block on a full queue, and the id check waits: other Python threads run meanwhile
+  using nogil = py::call_guard<py::gil_scoped_release>;
   m.def("set_error", [](py::object e) { g_error = e.release().ptr(); });
   py::register_exception_translator([](std::exception_ptr p) {
     try {
@@ -673,7 +670,7 @@ PYBIND11_MODULE(_host, m) {
       .def_readonly("k", &Source::k)
       .def_readonly("v", &Source::v)
       .def_readonly("n_tokens", &Source::n_tokens);
-  m.def("dense", &dense, py::arg("k"), py::arg("v"), py::arg("n_tokens") = -1);
+  m.def("dense", &dense, nogil(), py::arg("k"), py::arg("v"), py::arg("n_tokens") = -1);
   m.def("paged", [](const Tensor& k, const Tensor& v, const Tensor& table, int64_t n_tokens, int64_t page_tokens) {
     need_cuda({&k, &v, &table});
     return Source{NSA_KV_PAGED, k, v, table, n_tokens, page_tokens};
@@ -683,35 +680,35 @@ PYBIND11_MODULE(_host, m) {
     return Source{NSA_KV_PTR, k, v, Tensor(), stride_bn, 0};
   });
   m.def("even_stride", &even_stride);
-  m.def("same_bytes", &same_bytes, py::call_guard<py::gil_scoped_release>());
-  m.def("pool_rows", &pool_rows);
-  m.def("topk", &topk);
-  m.def("select_blocks", &select_blocks);
-  m.def("sel_fwd", &sel_fwd, py::arg("q"), py::arg("kv"), py::arg("ids"), py::arg("block_size"), py::arg("chunk_size"), py::arg("scale"),
+  m.def("same_bytes", &same_bytes, nogil());
+  m.def("pool_rows", &pool_rows, nogil());
+  m.def("topk", &topk, nogil());
+  m.def("select_blocks", &select_blocks, nogil());
+  m.def("sel_fwd", &sel_fwd, nogil(), py::arg("q"), py::arg("kv"), py::arg("ids"), py::arg("block_size"), py::arg("chunk_size"), py::arg("scale"),
         py::arg("causal"), py::arg("group_size"), py::arg("out") = py::none());
-  m.def("range_fwd", &range_fwd);
+  m.def("range_fwd", &range_fwd, nogil());
   m.def("stored_bytes", &stored_bytes);
-  m.def("sel_bwd", &sel_bwd);
-  m.def("selection_attention", &selection_attention);
+  m.def("sel_bwd", &sel_bwd, nogil());
+  m.def("selection_attention", &selection_attention, nogil());
   m.def("gate_combine", [](const Tensor& g, const OptTensor& a, const OptTensor& b, const OptTensor& c, bool softmax) {
     return gate_combine(g, or_none(a), or_none(b), or_none(c), softmax);
-  });
+  }, nogil());
   m.def("gate_combine_bwd", [](const Tensor& g, const OptTensor& a, const OptTensor& b, const OptTensor& c, const Tensor& dx, bool softmax) {
     return gate_combine_bwd(g, or_none(a), or_none(b), or_none(c), dx, softmax);
-  });
+  }, nogil());
   m.def("gated_sum", [](const Tensor& g, const OptTensor& a, const OptTensor& b, const OptTensor& c, bool softmax) {
     return GateFunction::apply(g, a, b, c, softmax);
-  });
+  }, nogil());
   py::class_<Rope>(m, "Rope").def(py::init([](const Tensor& f, const Tensor& h, const Tensor& w, int64_t gh, int64_t gw, int64_t pf, int64_t ph,
                                               int64_t pw, int64_t start) { return Rope{f, h, w, gh, gw, pf, ph, pw, start}; }));
-  m.def("rope_apply", &rope_apply);
+  m.def("rope_apply", &rope_apply, nogil());
   py::class_<CacheState>(m, "CacheState").def(py::init([](std::vector<Tensor> t, int64_t H, int64_t D, int64_t page_tokens, int64_t max_blocks) {
     need(t.size() == 10, "CacheState: ten tensors are expected");
     return CacheState{t[0], t[1], t[2], t[3], t[4], t[5], t[6], t[7], t[8], t[9], H, D, page_tokens, max_blocks};
   }));
-  m.def("cache_append", &cache_append);
-  m.def("cache_touch", &cache_touch);
-  m.def("residual_norm", &residual_norm);
-  m.def("rms_rows", &rms_rows);
-  m.def("qk_norm_rope", &qk_norm_rope);
+  m.def("cache_append", &cache_append, nogil());
+  m.def("cache_touch", &cache_touch, nogil());
+  m.def("residual_norm", &residual_norm, nogil());
+  m.def("rms_rows", &rms_rows, nogil());
+  m.def("qk_norm_rope", &qk_norm_rope, nogil());
 }
