@@ -384,6 +384,16 @@ struct IdCheck {
 };
 
 // ----------------------------------------------------------------------------------------- autograd
+// The autograd engine hands a C++ exception to Python as a RuntimeError: a backward raises the package's own instead.
+template <typename F> auto in_backward(F&& f) -> decltype(f()) {
+  try {
+    return f();
+  } catch (const BackendError& e) {
+    py::gil_scoped_acquire gil;
+    PyErr_SetString(g_error != nullptr ? g_error : PyExc_RuntimeError, e.what());
+    throw py::error_already_set();
+  }
+}
 struct SelectionFunction : torch::autograd::Function<SelectionFunction> {
   // fp32 tensors are computed on bf16 operands with fp32 accumulation (the kernels are 16-bit; the reference's
   // default for fp32 is TF32, also a reduced-precision product) and the results are returned in fp32
@@ -411,9 +421,11 @@ struct SelectionFunction : torch::autograd::Function<SelectionFunction> {
     const auto s = ctx->get_saved_variables();
     const Tensor &q = s[0], &k = s[1], &v = s[2], &ids = s[3], &out = s[4], &lse = s[5];
     const auto io = static_cast<at::ScalarType>(ctx->saved_data["io"].toInt());
-    auto g = sel_bwd(q, dense(k, v), ids, out, lse, grads[0].to(q.scalar_type()), ctx->saved_data["bs"].toInt(),
+    auto g = in_backward([&] {
+      return sel_bwd(q, dense(k, v), ids, out, lse, grads[0].to(q.scalar_type()), ctx->saved_data["bs"].toInt(),
                      ctx->saved_data["chunk"].toInt(), ctx->saved_data["scale"].toDouble(), ctx->saved_data["causal"].toBool(),
                      ctx->saved_data["G"].toInt());
+    });
     const Tensor none;
     return {std::get<0>(g).to(io), std::get<1>(g).to(io), std::get<2>(g).to(io), none, none, none, none, none, none};
   }
@@ -507,7 +519,7 @@ struct GateFunction : torch::autograd::Function<GateFunction> {
   }
   static variable_list backward(AutogradContext* ctx, const variable_list& grads) {
     const auto s = ctx->get_saved_variables();
-    auto r = gate_combine_bwd(s[0], s[1], s[2], s[3], grads[0], ctx->saved_data["softmax"].toBool());
+    auto r = in_backward([&] { return gate_combine_bwd(s[0], s[1], s[2], s[3], grads[0], ctx->saved_data["softmax"].toBool()); });
     variable_list out;
     for (auto& t : r) out.push_back(or_none(t));
     out.emplace_back();
