@@ -21,6 +21,20 @@ from ... import ops
 from ..._lib import host
 
 
+class _GatedSum(torch.autograd.Function):
+    """The same operator where a trace or a functorch transform has to see the function itself."""
+
+    @staticmethod
+    def forward(ctx, g_logits, o_cmp, o_slc, o_swa, gate_mode):
+        ctx.gate_mode = gate_mode
+        ctx.save_for_backward(g_logits, o_cmp, o_slc, o_swa)
+        return ops.gate_combine(g_logits, o_cmp, o_slc, o_swa, gate_mode)
+
+    @staticmethod
+    def backward(ctx, dx):
+        return *ops.gate_combine_bwd(*ctx.saved_tensors, dx, ctx.gate_mode), None
+
+
 def gated_branch_sum(g_logits: torch.Tensor, o_cmp: Optional[torch.Tensor], o_slc: Optional[torch.Tensor],
                      o_swa: Optional[torch.Tensor], gate_mode: str = "sigmoid",
                      skip_module: Optional[str] = None) -> torch.Tensor:
@@ -29,4 +43,6 @@ def gated_branch_sum(g_logits: torch.Tensor, o_cmp: Optional[torch.Tensor], o_sl
         o_cmp = None
     elif skip_module == "slc":
         o_slc = None
+    if torch._C._is_tracing() or torch._C._are_functorch_transforms_active():
+        return _GatedSum.apply(g_logits, o_cmp, o_slc, o_swa, gate_mode)
     return host.gated_sum(g_logits, o_cmp, o_slc, o_swa, ops._softmax_gates(gate_mode))
