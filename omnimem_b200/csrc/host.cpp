@@ -101,8 +101,19 @@ int32_t i32(int64_t x, const char* what) {
 }
 int64_t ceil_div(int64_t a, int64_t b) { return (a + b - 1) / b; }
 
+std::string shape(const Tensor& t) {
+  std::string s = "(";
+  for (int64_t i = 0; i < t.dim(); ++i) s += (i ? ", " : "") + std::to_string(t.size(i));
+  return s + ")";
+}
+// (the callers unpack four sizes: a fifth dimension would be dropped)
+void need_4d(const Tensor& t, const char* what) {
+  if (t.dim() != 4) throw py::value_error(std::string(what) + ": a tensor of four dimensions is expected, got " + shape(t));
+}
+
 // ----------------------------------------------------------------------------------------- pooling
 Tensor pool_rows(const Tensor& x_, int64_t size) {
+  need_4d(x_, "pool_rows x");
   need_cuda({&x_});
   const Tensor x = rows16(x_);
   const c10::cuda::CUDAGuard guard(x.device());
@@ -126,14 +137,11 @@ nsa_topk_mask mask_of(const MaskArgs& a) {
   for (int i = 0; i < 12; ++i) v[i] = i32(a[i], names[i]);
   return nsa_topk_mask{v[0], v[1], v[2], v[3], v[4], v[5], v[6], v[7] != 0, v[8] != 0, v[9] != 0, v[10], v[11]};
 }
-std::string shape(const Tensor& t) {
-  std::string s = "(";
-  for (int64_t i = 0; i < t.dim(); ++i) s += (i ? ", " : "") + std::to_string(t.size(i));
-  return s + ")";
-}
 Tensor unit_inner(const Tensor& t) { return t.stride(-1) == 1 ? t : t.contiguous(); }
 
 std::pair<Tensor, OptTensor> topk(const Tensor& q_, const Tensor& k_, int64_t T, double scale, const MaskArgs& mask, bool scores) {
+  need_4d(q_, "topk q");
+  need_4d(k_, "topk k");
   need_cuda({&q_, &k_});
   need(q_.scalar_type() == k_.scalar_type(), std::string("topk: q and k must share a dtype, got torch.") + c10::toString(q_.scalar_type()) +
                                                  " vs torch." + c10::toString(k_.scalar_type()));
@@ -153,6 +161,8 @@ std::pair<Tensor, OptTensor> topk(const Tensor& q_, const Tensor& k_, int64_t T,
 
 std::tuple<Tensor, Tensor, Tensor, OptTensor> select_blocks(const Tensor& q_, const Tensor& k_, int64_t T, double scale, const MaskArgs& mask,
                                                             bool scores) {
+  need_4d(q_, "select_blocks q");
+  need_4d(k_, "select_blocks k");
   need_cuda({&q_, &k_});
   need(q_.scalar_type() == k_.scalar_type(), std::string("select_blocks: q and k must share a dtype, got torch.") +
                                                  c10::toString(q_.scalar_type()) + " vs torch." + c10::toString(k_.scalar_type()));
@@ -207,6 +217,7 @@ struct Source {
 };
 // n_tokens < 0: as many as k has
 Source dense(const Tensor& k, const Tensor& v, int64_t n_tokens = -1) {
+  need_4d(k, "k");
   need_cuda({&k, &v});
   need(k.sizes() == v.sizes(), "k and v must have the same shape");
   return Source{NSA_KV_DENSE, rows16(k), rows16(v), Tensor(), n_tokens < 0 ? k.size(1) : n_tokens, 0};
@@ -220,6 +231,7 @@ Tensor output_like(const Tensor& q, const OptTensor& given, const char* what) {
 
 std::pair<Tensor, Tensor> sel_fwd(const Tensor& q_, const Source& kv, const OptTensor& ids_, int64_t bs, int64_t chunk, double scale, bool causal,
                                   int64_t G, const OptTensor& out_) {
+  need_4d(q_, "sel_fwd q");
   const Tensor& ids = or_none(ids_);
   need_cuda({&q_, &ids});
   const Tensor q = rows16(q_);
@@ -240,6 +252,7 @@ std::pair<Tensor, Tensor> sel_fwd(const Tensor& q_, const Source& kv, const OptT
 // None: the shape is not one of the range kernel's (the caller lists the blocks)
 c10::optional<std::pair<Tensor, Tensor>> range_fwd(const Tensor& q_, const Source& kv, int64_t first, int64_t n, int64_t bs, double scale,
                                                    const OptTensor& out_) {
+  need_4d(q_, "range_fwd q");
   need_cuda({&q_});
   const char* hook = std::getenv("OMNIMEM_B200_RANGE_KERNEL");          // test hook "listed": always list the blocks
   const int64_t B = q_.size(0), M = q_.size(1), H = q_.size(2), D = q_.size(3);
@@ -274,6 +287,7 @@ int64_t stored_bytes(const Tensor& q, int mode, int64_t T, int64_t bs, int64_t G
 
 std::tuple<Tensor, Tensor, Tensor> sel_bwd(const Tensor& q_, const Source& kv, const Tensor& ids, const Tensor& out_, const Tensor& lse_,
                                            const Tensor& do_, int64_t bs, int64_t chunk, double scale_, bool causal, int64_t G) {
+  for (const Tensor* t : {&q_, &ids, &out_, &do_}) need_4d(*t, "sel_bwd q, ids, out, d_out");
   need_cuda({&q_, &ids, &out_, &lse_, &do_});
   const Tensor q = rows16(q_), out = rows16(out_), d_out = rows16(do_), lse = lse_.contiguous();
   need(ids.scalar_type() == at::kInt, "block_indices must be int32");

@@ -81,6 +81,20 @@ def test_even_stride_finds_the_stride_of_rows_that_lie_evenly_and_no_other():
             assert [at[0] + i * got for i in range(n)] == at
 
 
+@pytest.mark.parametrize("sizes", [(1, 64, 2), (1, 64, 2, 64, 2), (64,)])
+def test_operators_refuse_other_ranks(sizes):
+    """A fifth dimension used to be an error of the unpacking; the native path would read its first slice."""
+    from omnimem_b200 import ops
+    x, good, ids = _bf16(*sizes), _bf16(1, 64, 2, 64), torch.zeros(1, 1, 2, 1, dtype=torch.int32)
+    mask = (64, 64, 64, 1, 0, 0, 0, False, False, False, 0, 1)
+    calls = [lambda: ops.pool_rows(x, 4), lambda: host.topk(x, good, 1, 1.0, mask, False), lambda: host.topk(good, x, 1, 1.0, mask, False),
+             lambda: host.select_blocks(x, good, 1, 1.0, mask, False), lambda: host.select_blocks(good, x, 1, 1.0, mask, False),
+             lambda: ops.DenseKV(x, x)]
+    for call in calls:
+        with pytest.raises(ValueError, match="four dimensions"):
+            call()
+
+
 def test_same_bytes():
     a = torch.polar(torch.ones(6, 4, dtype=torch.float64), torch.arange(24, dtype=torch.float64).view(6, 4))
     assert host.same_bytes(a, a.clone()) and host.same_bytes(a[:0], a[:0].clone())
@@ -103,3 +117,19 @@ def test_gates_and_norms_of_views_equal_those_of_their_copies(dev):
         x = torch.randn(40000, generator=g, device=dev).to(torch.bfloat16).as_strided((*lead, 16), (*strides, 1))
         w = torch.randn(16, generator=g, device=dev).to(torch.bfloat16)
         assert torch.equal(host.rms_rows(x, w, 1e-6), host.rms_rows(x.contiguous(), w, 1e-6))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("sizes", [(1, 64, 2), (1, 64, 2, 64, 2)])
+def test_attention_refuses_other_ranks(dev, sizes):
+    from omnimem_b200 import ops
+    good, x = (torch.zeros(*s, device=dev, dtype=torch.bfloat16) for s in ((1, 64, 2, 64), sizes))
+    ids, lse = torch.zeros(1, 1, 2, 1, dtype=torch.int32, device=dev), torch.zeros(1, 2, 64, device=dev)
+    kv = ops.DenseKV(good, good)
+    ops.sel_fwd(good, kv, ids, 64, 1, 0.1, False, 64)
+    for call in (lambda: ops.sel_fwd(x, kv, ids, 64, 1, 0.1, False, 64), lambda: ops.range_fwd(x, kv, 0, 1, 64, 0.1),
+                 lambda: ops.sel_bwd(good, kv, ids, x, lse, good, 64, 1, 0.1, False, 64),
+                 lambda: ops.sel_bwd(good, kv, ids, good, lse, x, 64, 1, 0.1, False, 64),
+                 lambda: ops.sel_bwd(good, kv, ids[None], good, lse, good, 64, 1, 0.1, False, 64)):
+        with pytest.raises((ValueError, RuntimeError)):
+            call()
