@@ -446,13 +446,16 @@ __global__ void __launch_bounds__(32 * W * KS, W == 4 && D == 128 ? 3 : 1) sel_b
 // --------------------------------------------------------------------------------- dK / dV
 // A thread block of TW warps owns at most 16 TW tokens of one (batch, head, block) tile, 16 per warp, keeps their K and
 // V rows in shared memory as A operands and streams the Q and dO rows (and LSE and delta) of the block's bucket, in
-// ascending group order, through the ring, 16 query rows at a time: S^T = K Q^T and dP^T = V dO^T, then dV += P^T dO
+// ascending group order, through the ring, QR query rows at a time: S^T = K Q^T and dP^T = V dO^T, then dV += P^T dO
 // and dK += dS^T Q.  No atomics: results are bit-reproducible.  What bounds it is the length of a step (products,
-// exponentials, and the issue of the next copies: 3.5 k cycles, of them 1.8 k products) times the 12 warps per SM that
-// two accumulators of 16 x 128 allow.  32760 queries x 12 heads, 15-query groups, 16 blocks of 30: 971 us (3847 us with
-// 64-row tiles; two query tiles per step with 8 warps per SM: 1096 us).
-template <typename T, int D, int TW, bool TMA>
-__global__ void __launch_bounds__(32 * TW, (D == 128 ? 12 : 16) / TW)
+// exponentials, and the issue of the next copies: 3.5 k cycles at 16 rows, of them 1.8 k products) times the 12 warps
+// per SM that two accumulators of 16 x 128 allow; with more rows a step there are 8 warps (12 at D = 64) but the K and V
+// operands, the barriers and the exponentials' latency serve them all.
+// 3120 queries x 12 heads, 16 of 98 blocks of 64, groups of 64, D = 128, 16 / 32 / 64 rows: 224 / 187 / 177 us; groups of
+// 32: 213 / 178 / 234 us; of 80: 223 / 205 / 218 us; of 16: 207 / 270 / 359 us.  D = 64, groups of 64: 126 / 121 / 95 us; of
+// 80, blocks of 64 and 128: 133 / 142 / 125 and 225 / 240 / 230 us.
+template <typename T, int D, int TW, int QR, bool TMA>
+__global__ void __launch_bounds__(32 * TW, (D == 128 ? (QR == 16 ? 12 : 8) : (QR == 64 ? 12 : 16)) / TW)
 sel_bwd_dkv_rows_kernel(const __grid_constant__ RingMaps maps, const BwdParams p, const int tiles_per_block, const int stages,
                         int32_t* status) {
   constexpr int ESZ = sizeof(T), TROWS = 16 * TW, kList = 64;
@@ -519,23 +522,23 @@ sel_bwd_dkv_rows_kernel(const __grid_constant__ RingMaps maps, const BwdParams p
 
   const uint32_t k_tile = smem_u32(smem), v_tile = k_tile + kRingTile<D, TROWS>;
   const uint32_t ring_mem = v_tile + kRingTile<D, TROWS>;
-  const uint32_t ring_bytes = static_cast<uint32_t>(stages) * 2 * kRingTile<D, 16>;
+  const uint32_t ring_bytes = static_cast<uint32_t>(stages) * 2 * kRingTile<D, QR>;
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + 2 * kRingTile<D, TROWS> + ring_bytes);
   int* words = reinterpret_cast<int*>(bars + kRingBars);
-  const float* rows32 = reinterpret_cast<const float*>(words + 4);         // [stage][LSE, delta][16]
-  int4* list = reinterpret_cast<int4*>(words + 4 + stages * 32);           // [2 kList] tiles: group, first row, rows, visible tokens
+  const float* rows32 = reinterpret_cast<const float*>(words + 4);         // [stage][LSE, delta][QR]
+  int4* list = reinterpret_cast<int4*>(words + 4 + stages * 2 * QR);       // [2 kList] tiles: group, first row, rows, visible tokens
 
-  const int subs = (p.G + 15) / 16;                         // ring tiles per group
-  Ring<D, 16, TMA, true> ring{ring_mem, bars, words, n_ent * subs, stages, warp, TW, p.lse, p.delta, smem_u32(rows32)};
+  const int subs = (p.G + QR - 1) / QR;                     // ring tiles per group
+  Ring<D, QR, TMA, true> ring{ring_mem, bars, words, n_ent * subs, stages, warp, TW, p.lse, p.delta, smem_u32(rows32)};
   if (threadIdx.x == 0) words[0] = 0;
   ring.init();
   // tiles [from, from + kList) of the bucket
   const auto list_tiles = [&](int from) {
     for (int i = from + threadIdx.x; i < from + kList && i < ring.count; i += 32 * TW) {
-      const int e = i / subs, r0 = (i - e * subs) * 16, g = bucket[e];
+      const int e = i / subs, r0 = (i - e * subs) * QR, g = bucket[e];
       const int64_t g0 = static_cast<int64_t>(g) * p.G;
       // rows of the tile (a short last group may leave one empty); rows of this block that the group may see
-      const int n = max(0, min(16, static_cast<int>(min64(p.G, p.M - g0)) - r0));
+      const int n = max(0, min(QR, static_cast<int>(min64(p.G, p.M - g0)) - r0));
       int vis = n_rows;
       if (p.causal) vis = static_cast<int>(min64(vis, (g0 / p.chunk_size + 1) * p.chunk_size - tok0));
       list[i % (2 * kList)] = make_int4(g, r0, n, n > 0 ? vis : 0);
@@ -597,19 +600,21 @@ sel_bwd_dkv_rows_kernel(const __grid_constant__ RingMaps maps, const BwdParams p
     ok = ok && ring.template wait<0>();
     if (ok && vis > 0) {
       const uint32_t qt = ring.tile(0), dt = ring.tile(1);
-      float st[2][4], dp[2][4];
+      constexpr int C = QR / 8;
+      const int n16 = (n + 15) >> 4;
+      float st[C][4], dp[C][4];
 #pragma unroll
-      for (int j = 0; j < 2; ++j) {
+      for (int j = 0; j < C; ++j) {
         st[j][0] = st[j][1] = st[j][2] = st[j][3] = 0.f;
         dp[j][0] = dp[j][1] = dp[j][2] = dp[j][3] = 0.f;
       }
-      mma_rows_t2<T, D, TROWS>(st, k_tile, qt, dp, v_tile, dt, warp * 16);
-      const float2* lse = reinterpret_cast<const float2*>(rows32 + ring.stage * 32) + t4;
-      uint32_t pa[1][4], ds[1][4];
+      mma_rows_t2<T, D, TROWS, QR>(st, k_tile, qt, dp, v_tile, dt, warp * 16, n16);
+      const float2* lse = reinterpret_cast<const float2*>(rows32 + ring.stage * 2 * QR) + t4;
+      uint32_t pa[QR / 16][4], ds[QR / 16][4];
 #pragma unroll
-      for (int j = 0; j < 2; ++j) {
+      for (int j = 0; j < C; ++j) {
         const int q0 = 8 * j + 2 * t4;                         // this thread's columns: query rows q0, q0 + 1
-        const float2 l = lse[j * 4], dl = lse[8 + j * 4];
+        const float2 l = lse[j * 4], dl = lse[QR / 2 + j * 4];
         const float dls[2] = {dl.x, dl.y};
         // rows past the group's end: exp2(-inf) = 0
         const float l2[2] = {q0 < n ? l.x * kLog2e : INFINITY, q0 + 1 < n ? l.y * kLog2e : INFINITY};
@@ -618,13 +623,14 @@ sel_bwd_dkv_rows_kernel(const __grid_constant__ RingMaps maps, const BwdParams p
           st[j][y] = fast_exp2(st[j][y] * p.scale_log2 - l2[y & 1]);
           if (gid + 8 * (y >> 1) >= vis) st[j][y] = 0.f;
         }
-        pa[0][j * 2] = pack2<T>(st[j][0], st[j][1]);
-        pa[0][j * 2 + 1] = pack2<T>(st[j][2], st[j][3]);
-        ds[0][j * 2] = pack2<T>(st[j][0] * (dp[j][0] - dls[0]) * p.scale, st[j][1] * (dp[j][1] - dls[1]) * p.scale);
-        ds[0][j * 2 + 1] = pack2<T>(st[j][2] * (dp[j][2] - dls[0]) * p.scale, st[j][3] * (dp[j][3] - dls[1]) * p.scale);
+        const int at = (j & 1) * 2;
+        pa[j >> 1][at] = pack2<T>(st[j][0], st[j][1]);
+        pa[j >> 1][at + 1] = pack2<T>(st[j][2], st[j][3]);
+        ds[j >> 1][at] = pack2<T>(st[j][0] * (dp[j][0] - dls[0]) * p.scale, st[j][1] * (dp[j][1] - dls[1]) * p.scale);
+        ds[j >> 1][at + 1] = pack2<T>(st[j][2] * (dp[j][2] - dls[0]) * p.scale, st[j][3] * (dp[j][3] - dls[1]) * p.scale);
       }
-      mma_rows<T, D, 16>(dv, pa, dt, 1);
-      mma_rows<T, D, 16>(dk, ds, qt, 1);
+      mma_rows<T, D, QR>(dv, pa, dt, n16);
+      mma_rows<T, D, QR>(dk, ds, qt, n16);
     }
     ok = ok && ring.template release<1>(i, src, tile_of);
     ring.step();
@@ -693,20 +699,28 @@ int launch_dq(const nsa_kv_source* kv, const BwdParams& p, int32_t* st, cudaStre
                                                           : launch_dq_loader<T, D, false>(maps, p, st, s);
 }
 
-template <typename T, int D, int TW, bool TMA>
+template <typename T, int D, int TW, int QR, bool TMA>
 int launch_dkv_rows(const RingMaps& maps, const BwdParams& p, int32_t* status, cudaStream_t stream) {
   const int tpb = cdiv(p.block_size, 16 * TW);
-  constexpr int stages = TW == 2 && D == 128 ? 1 : 2;   // where registers leave the room (measured 971 / 1008 us at TW = 2, D = 128; 653 / 642 us at D = 64)
-  constexpr size_t smem = 2 * kRingTile<D, 16 * TW> + static_cast<size_t>(stages) * (2 * kRingTile<D, 16> + 128) + kRingBars * 8 + 16 + 2 * 64 * 16;
+  constexpr int stages = TW == 2 && D == 128 ? 1 : 2;   // where registers leave the room
+  constexpr size_t smem = 2 * kRingTile<D, 16 * TW> + static_cast<size_t>(stages) * (2 * kRingTile<D, QR> + 8 * QR) + kRingBars * 8 + 16 + 2 * 64 * 16;
   static_assert(TW * 16 * (D * 2 + 16) <= 2 * kRingTile<D, 16 * TW>, "the epilogue stages its rows in the K and V tiles");
   const int64_t nblk = p.NS * tpb;
   NSA_REQUIRE(nblk <= 0x7fffffff, NSA_ERR_INVALID, "sel_bwd: too many K/V tiles");
   if (nblk == 0) return NSA_OK;
-  auto kernel = sel_bwd_dkv_rows_kernel<T, D, TW, TMA>;
+  auto kernel = sel_bwd_dkv_rows_kernel<T, D, TW, QR, TMA>;
   NSA_CUDA_OK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
   kernel<<<dim3(static_cast<unsigned>(nblk), p.H, p.B), 32 * TW, smem, stream>>>(maps, p, tpb, stages, status);
   NSA_LAUNCH_OK("sel_bwd_dkv_rows_kernel");
   return NSA_OK;
+}
+
+template <typename T, int D, int TW, int QR>
+int launch_dkv_loader(const BwdParams& p, const int64_t* qs, const int64_t* ds, int32_t* st, cudaStream_t s) {
+  RingMaps maps{};
+  const bool tma = make_unit_maps(&maps.a, &maps.a_tail, p.q, qs, p.B, p.M, p.H, D, p.G, QR) &&
+                   make_unit_maps(&maps.b, &maps.b_tail, p.dO, ds, p.B, p.M, p.H, D, p.G, QR);
+  return tma ? launch_dkv_rows<T, D, TW, QR, true>(maps, p, st, s) : launch_dkv_rows<T, D, TW, QR, false>(maps, p, st, s);
 }
 
 template <typename T, int D>
@@ -719,13 +733,13 @@ int launch_dkv(const BwdParams& p, int32_t* st, cudaStream_t s) {
     const int rc = try_launch_sel_bwd_dkv_rows_tc(a, qs, ds, D, std::is_same<T, __half>::value ? NSA_F16 : NSA_BF16, st, s, &launched);
     if (rc || launched) return rc;
   }
-  RingMaps maps{};
-  const bool tma = make_unit_maps(&maps.a, &maps.a_tail, p.q, qs, p.B, p.M, p.H, D, p.G, 16) &&
-                   make_unit_maps(&maps.b, &maps.b_tail, p.dO, ds, p.B, p.M, p.H, D, p.G, 16);
-  // a block of more than 32 tokens is one tile of four warps: its bucket's rows are fetched once, not per 32 tokens
-  if (p.block_size > 32)
-    return tma ? launch_dkv_rows<T, D, 4, true>(maps, p, st, s) : launch_dkv_rows<T, D, 4, false>(maps, p, st, s);
-  return tma ? launch_dkv_rows<T, D, 2, true>(maps, p, st, s) : launch_dkv_rows<T, D, 2, false>(maps, p, st, s);
+  if (p.block_size <= 32) return launch_dkv_loader<T, D, 2, 16>(p, qs, ds, st, s);
+  // a block of more than 32 tokens is one tile of four warps: its bucket's rows are fetched once, not per 32 tokens.  The
+  // rows per step are those that fill their tiles (the figures are at the kernel).
+  if (p.G <= 16) return launch_dkv_loader<T, D, 4, 16>(p, qs, ds, st, s);
+  if (p.G <= 32) return launch_dkv_loader<T, D, 4, 32>(p, qs, ds, st, s);
+  if (p.G <= 64 || p.G > 96) return launch_dkv_loader<T, D, 4, 64>(p, qs, ds, st, s);
+  return launch_dkv_loader<T, D, 4, D == 128 ? 32 : 16>(p, qs, ds, st, s);
 }
 
 // kv: the source of the dQ kernel's K/V; nullptr: dK / dV

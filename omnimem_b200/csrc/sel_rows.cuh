@@ -95,22 +95,28 @@ __device__ __forceinline__ void mma_rows_t(float (&acc)[ROWS / 8][4], const uint
         mma16816<T>(acc[2 * j + 1], a[kk], b[2], b[3]);
       }
 }
-// two such products with one 16-row tile each, A being 16 rows (from a_row0) of a tile each: their chains of dependent
+// two such products with tiles of ROWS rows, A being 16 rows (from a_row0) of a tile each: their chains of dependent
 // products interleave
-template <typename T, int D, int AROWS>
-__device__ __forceinline__ void mma_rows_t2(float (&x)[2][4], uint32_t ax, uint32_t bx, float (&y)[2][4], uint32_t ay,
-                                            uint32_t by, int a_row0) {
+template <typename T, int D, int AROWS, int ROWS>
+__device__ __forceinline__ void mma_rows_t2(float (&x)[ROWS / 8][4], uint32_t ax, uint32_t bx, float (&y)[ROWS / 8][4], uint32_t ay,
+                                            uint32_t by, int a_row0, int n16) {
 #pragma unroll
   for (int kk = 0; kk < D / 16; ++kk) {
-    uint32_t a0[4], a1[4], b0[4], b1[4];
+    uint32_t a0[4], a1[4];
     ldsm_a<AROWS>(a0, ax, a_row0, kk);
-    ldsm_b<16>(b0, bx, 0, kk);
     ldsm_a<AROWS>(a1, ay, a_row0, kk);
-    ldsm_b<16>(b1, by, 0, kk);
-    mma16816<T>(x[0], a0, b0[0], b0[1]);
-    mma16816<T>(x[1], a0, b0[2], b0[3]);
-    mma16816<T>(y[0], a1, b1[0], b1[1]);
-    mma16816<T>(y[1], a1, b1[2], b1[3]);
+#pragma unroll
+    for (int j = 0; j < ROWS / 16; ++j) {
+      if (ROWS == 16 || j < n16) {
+        uint32_t b0[4], b1[4];
+        ldsm_b<ROWS>(b0, bx, j, kk);
+        ldsm_b<ROWS>(b1, by, j, kk);
+        mma16816<T>(x[2 * j], a0, b0[0], b0[1]);
+        mma16816<T>(x[2 * j + 1], a0, b0[2], b0[3]);
+        mma16816<T>(y[2 * j], a1, b1[0], b1[1]);
+        mma16816<T>(y[2 * j + 1], a1, b1[2], b1[3]);
+      }
+    }
   }
 }
 
