@@ -5,6 +5,7 @@
 //   * dK/dV kernel: one thread block OWNS a tile of at most 32 tokens of one (b, h, block) and walks the
 //     block's bucket of query groups in ascending group order - no atomics, results are
 //     bit-reproducible from run to run.
+#include "sel_packed.cuh"
 #include "sel_rows.cuh"
 
 #include <type_traits>
@@ -305,6 +306,7 @@ struct BwdParams {
   const int32_t* offsets;                // [B,H,NS+1]
   KVSrc kv;
   int B, H, T, block_size, chunk_size, causal, G, MG;
+  int parts;                             // dQ: thread blocks that share a group's rows
   int64_t M, NS;
   float scale, scale_log2;
   // dK/dV kernel only, pointer mode (selection_bwd.cu:1409-1527, bwd_common.cuh:64-121): K/V blocks
@@ -322,22 +324,27 @@ struct BwdParams {
   } tab;
 };
 
-// W warps of 16 query rows share one ring of K/V tiles; with W = 1 the list may be dealt out to KS warps.  Bounds as in
-// the forward, with 9 warps per SM (registers: Q and dO fragments and the accumulator).  32760 queries x 12 heads,
-// 15-query groups, 16 blocks of 30: 623 us (10142 us with one warp per thread block).
+// W warps of 16 query rows share one ring of K/V tiles; p.parts such thread blocks take a group and walk the list each for
+// itself; with W = 1 the list may be dealt out to KS warps.  Bounds as in the forward, with 9 warps per SM (registers: Q and dO fragments and the
+// accumulator).  32760 queries x 12 heads, 15-query groups, 16 blocks of 30: 623 us (10142 us with packed tiles).
+// 3120 queries x 12 heads, 16 blocks of 64, D = 128, groups of 32 / 64 / 128: 130 / 131 / 173 us; 151 / 152 / 184 us with two warps per
+// ring, 417 / 294 / 294 us with four, 506 / 259 / 203 us with eight.
 template <typename T, int D, int W, int KS, bool TMA>
-__global__ void __launch_bounds__(32 * W * KS, W == 4 && D == 128 ? 3 : 1) sel_bwd_dq_rows_kernel(
+__global__ void __launch_bounds__(32 * W * KS, 1) sel_bwd_dq_rows_kernel(
     const __grid_constant__ RingMaps maps, const BwdParams p, const int stages, int32_t* status) {
   static_assert(W == 1 || KS == 1, "only single-warp groups are split");
   constexpr int ESZ = sizeof(T), ROWS = 32;
   extern __shared__ __align__(1024) uint8_t smem[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int gid = lane >> 2, t4 = lane & 3;
-  const int g = blockIdx.x, h = blockIdx.y, b = blockIdx.z;
+  const int g = p.parts == 1 ? blockIdx.x : blockIdx.x / p.parts, first_row = (blockIdx.x - g * p.parts) * (16 * W);
+  const int h = blockIdx.y, b = blockIdx.z;
   const int64_t g0 = static_cast<int64_t>(g) * p.G;
   const int row_warp = W > 1 ? warp : 0, part = KS > 1 ? warp : 0;
-  const int n_q = static_cast<int>(p.M - g0 < p.G ? p.M - g0 : p.G) - row_warp * 16;
-  const int64_t m0 = g0 + row_warp * 16;
+  const int block_rows = static_cast<int>(p.M - g0 < p.G ? p.M - g0 : p.G) - first_row;
+  if (block_rows <= 0) return;                                     // (a short last group)
+  const int n_q = block_rows - row_warp * 16;                      // rows of this warp (may be <= 0)
+  const int64_t m0 = g0 + first_row + row_warp * 16;
 
   const uint32_t ring_bytes = static_cast<uint32_t>(stages) * 2 * kRingTile<D, ROWS>;
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + KS * ring_bytes);
@@ -441,6 +448,174 @@ __global__ void __launch_bounds__(32 * W * KS, W == 4 && D == 128 ? 3 : 1) sel_b
   if (n_q > 0)
     store_rows<T, D>(dq, 1.f, 1.f, smem_u32(smem) + row_warp * 16 * (D * 2 + 16),
                      p.dq + (b * p.dq_sb + m0 * p.dq_sm + h * p.dq_sh) * ESZ, p.dq_sm * ESZ, n_q);
+}
+
+// ------------------------------------------------------------------------- dQ, packed tiles
+template <typename T, int D>
+__global__ void __launch_bounds__(256) sel_bwd_dq_packed_kernel(const BwdParams p) {
+  constexpr int PITCH = D + 8;
+  constexpr int ESZ = sizeof(T);
+  constexpr int KK = D / 16;
+  constexpr int DN = D / 8;
+  extern __shared__ __align__(1024) uint8_t smem[];
+
+  const int g = blockIdx.x, h = blockIdx.y, b = blockIdx.z;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int gid = lane >> 2, t4 = lane & 3;
+  const int rows_pad = (blockDim.x >> 5) * 16;
+  const int64_t m0 = static_cast<int64_t>(g) * p.G;
+  const int n_q = static_cast<int>(p.M - m0 < p.G ? p.M - m0 : p.G);
+  const int q_chunk = static_cast<int>(m0 / p.chunk_size);
+
+  T* tiles = reinterpret_cast<T*>(smem);                         // [2][2][64][PITCH]
+  T* sQ = tiles + 4 * kPackedRows * PITCH;                          // [rows_pad][PITCH]
+  T* sdO = sQ + rows_pad * PITCH;
+  float* s_lse = reinterpret_cast<float*>(sdO + rows_pad * PITCH);
+  float* s_delta = s_lse + rows_pad;
+  const SlotTable st = carve_slot_table(reinterpret_cast<char*>(s_delta + rows_pad), p.T);
+  auto stageK = [&](int s) { return tiles + (s * 2) * kPackedRows * PITCH; };
+  auto stageV = [&](int s) { return tiles + (s * 2 + 1) * kPackedRows * PITCH; };
+
+  const int total = build_slot_table<ESZ>(st, p.kv, p.ids, b * p.i_sb + g * p.i_sg + h * p.i_sh, p.i_st,
+                                          p.T, b, h, D, p.block_size, p.chunk_size, p.causal != 0, q_chunk);
+
+  const char* q_base = p.q + (b * p.q_sb + m0 * p.q_sm + h * p.q_sh) * ESZ;
+  const char* o_base = p.o + (b * p.o_sb + m0 * p.o_sm + h * p.o_sh) * ESZ;
+  const char* do_base = p.dO + (b * p.do_sb + m0 * p.do_sm + h * p.do_sh) * ESZ;
+  char* dq_base = p.dq + (b * p.dq_sb + m0 * p.dq_sm + h * p.dq_sh) * ESZ;
+  const int64_t bhm = (static_cast<int64_t>(b) * p.H + h) * p.M + m0;
+
+  // delta = sum_d O * dO (one warp per row), kept in shared memory and stored for dK/dV
+  for (int r = warp; r < rows_pad; r += (blockDim.x >> 5)) {
+    float acc = 0.f;
+    if (r < n_q) {
+      const T* orow = reinterpret_cast<const T*>(o_base + r * p.o_sm * ESZ);
+      const T* drow = reinterpret_cast<const T*>(do_base + r * p.do_sm * ESZ);
+      for (int d = lane * 2; d < D; d += 64) {
+        const float2 a = unpack2<T>(*reinterpret_cast<const uint32_t*>(orow + d));
+        const float2 c = unpack2<T>(*reinterpret_cast<const uint32_t*>(drow + d));
+        acc += a.x * c.x + a.y * c.y;
+      }
+    }
+#pragma unroll
+    for (int d = 16; d; d >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, d);
+    if (lane == 0) {
+      s_delta[r] = acc;
+      s_lse[r] = r < n_q ? p.lse[bhm + r] * kLog2e : INFINITY;
+      if (r < n_q) p.delta[bhm + r] = acc;
+    }
+  }
+
+  if (total == 0) {
+    for (int i = threadIdx.x; i < n_q * (D / 8); i += blockDim.x) {
+      const int r = i / (D / 8), c = i % (D / 8);
+      *reinterpret_cast<uint4*>(dq_base + r * p.dq_sm * ESZ + c * 16) = make_uint4(0, 0, 0, 0);
+    }
+    return;
+  }
+
+  const int64_t k_row_bytes = kv_row_bytes(p.kv, false, D, ESZ);
+  const int64_t v_row_bytes = kv_row_bytes(p.kv, true, D, ESZ);
+  const int ntiles = (total + kPackedRows - 1) / kPackedRows;
+
+  issue_rows<T, D, PITCH>(sQ, q_base, p.q_sm * ESZ, n_q, rows_pad);
+  issue_rows<T, D, PITCH>(sdO, do_base, p.do_sm * ESZ, n_q, rows_pad);
+  issue_kv_tile<T, D, PITCH>(stageK(0), stageV(0), st, p.T, 0, total, k_row_bytes, v_row_bytes, p.q);
+  cp_async_commit();
+
+  float dq[DN][4];
+#pragma unroll
+  for (int n = 0; n < DN; ++n) { dq[n][0] = dq[n][1] = dq[n][2] = dq[n][3] = 0.f; }
+  const bool warp_active = warp * 16 < n_q;
+  const T* qa = sQ + (warp * 16 + (lane & 15)) * PITCH + (lane >> 4) * 8;
+  const T* da = sdO + (warp * 16 + (lane & 15)) * PITCH + (lane >> 4) * 8;
+
+  for (int i = 0; i < ntiles; ++i) {
+    if (i + 1 < ntiles) {
+      issue_kv_tile<T, D, PITCH>(stageK((i + 1) & 1), stageV((i + 1) & 1), st, p.T,
+                                 (i + 1) * kPackedRows, total, k_row_bytes, v_row_bytes, p.q);
+      cp_async_commit();
+      cp_async_wait<1>();
+    } else {
+      cp_async_wait<0>();
+    }
+    __syncthreads();
+    if (warp_active) {
+      const T* sK = stageK(i & 1);
+      const T* sV = stageV(i & 1);
+      const int nvalid = min(kPackedRows, total - i * kPackedRows);
+      const int nb_off = ((lane & 7) + ((lane >> 4) << 3)) * PITCH + ((lane >> 3) & 1) * 8;
+      float s[8][4], dp[8][4];
+#pragma unroll
+      for (int n = 0; n < 8; ++n) {
+        s[n][0] = s[n][1] = s[n][2] = s[n][3] = 0.f;
+        dp[n][0] = dp[n][1] = dp[n][2] = dp[n][3] = 0.f;
+      }
+#pragma unroll
+      for (int kk = 0; kk < KK; ++kk) {
+        uint32_t aq[4], ad[4];
+        ldmatrix_x4(aq, qa + kk * 16);
+        ldmatrix_x4(ad, da + kk * 16);
+#pragma unroll
+        for (int n16 = 0; n16 < 4; ++n16) {
+          if (n16 * 16 < nvalid) {
+            uint32_t bf[4];
+            ldmatrix_x4(bf, sK + nb_off + n16 * 16 * PITCH + kk * 16);
+            mma16816<T>(s[2 * n16], aq, bf[0], bf[1]);
+            mma16816<T>(s[2 * n16 + 1], aq, bf[2], bf[3]);
+            ldmatrix_x4(bf, sV + nb_off + n16 * 16 * PITCH + kk * 16);
+            mma16816<T>(dp[2 * n16], ad, bf[0], bf[1]);
+            mma16816<T>(dp[2 * n16 + 1], ad, bf[2], bf[3]);
+          }
+        }
+      }
+      const float lse0 = s_lse[warp * 16 + gid], lse1 = s_lse[warp * 16 + gid + 8];
+      const float dl0 = s_delta[warp * 16 + gid], dl1 = s_delta[warp * 16 + gid + 8];
+      uint32_t dsa[4][4];
+#pragma unroll
+      for (int n = 0; n < 8; ++n) {
+        float ds[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const int col = n * 8 + 2 * t4 + (e & 1);
+          const float l = (e >> 1) ? lse1 : lse0;
+          const float dl = (e >> 1) ? dl1 : dl0;
+          const float pe = (col < nvalid) ? fast_exp2(s[n][e] * p.scale_log2 - l) : 0.f;
+          ds[e] = pe * (dp[n][e] - dl) * p.scale;
+        }
+        dsa[n >> 1][(n & 1) * 2] = pack2<T>(ds[0], ds[1]);
+        dsa[n >> 1][(n & 1) * 2 + 1] = pack2<T>(ds[2], ds[3]);
+      }
+      const T* kb = sK + ((lane & 7) + ((lane >> 3) & 1) * 8) * PITCH + (lane >> 4) * 8;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        if (j * 16 < nvalid) {
+#pragma unroll
+          for (int d16 = 0; d16 < D / 16; ++d16) {
+            uint32_t bf[4];
+            ldmatrix_x4_trans(bf, kb + j * 16 * PITCH + d16 * 16);
+            mma16816<T>(dq[2 * d16], dsa[j], bf[0], bf[1]);
+            mma16816<T>(dq[2 * d16 + 1], dsa[j], bf[2], bf[3]);
+          }
+        }
+      }
+    }
+    __syncthreads();
+  }
+
+  if (warp_active) {
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
+      const int row = warp * 16 + gid + 8 * r;
+      if (row < n_q) {
+        char* drow = dq_base + row * p.dq_sm * ESZ;
+#pragma unroll
+        for (int n = 0; n < DN; ++n)
+          *reinterpret_cast<uint32_t*>(drow + (n * 8 + 2 * t4) * ESZ) =
+              pack2<T>(dq[n][2 * r], dq[n][2 * r + 1]);
+      }
+    }
+  }
 }
 
 // --------------------------------------------------------------------------------- dK / dV
@@ -663,7 +838,7 @@ sel_bwd_dkv_rows_kernel(const __grid_constant__ RingMaps maps, const BwdParams p
 }
 
 template <typename T, int D, int W, int KS, bool TMA>
-int launch_dq_rows(const RingMaps& maps, const BwdParams& p, int32_t* status, cudaStream_t stream) {
+int launch_dq_rows(const RingMaps& maps, BwdParams p, int32_t* status, cudaStream_t stream) {
   constexpr int stages = W <= 2 ? 1 : 3;                    // as in the forward
   static_assert(W * 16 * (D * 2 + 16) <= stages * 2 * kRingTile<D, 32>, "the epilogue stages its rows in the ring");
   static_assert((KS - 1) * (D / 8 * 512) <= KS * 2 * kRingTile<D, 32>, "the partial results are summed in the ring");
@@ -672,31 +847,60 @@ int launch_dq_rows(const RingMaps& maps, const BwdParams& p, int32_t* status, cu
   NSA_REQUIRE(smem <= 226 * 1024, NSA_ERR_UNSUPPORTED, "sel_bwd: T=%d needs too much shared memory", p.T);
   auto kernel = sel_bwd_dq_rows_kernel<T, D, W, KS, TMA>;
   NSA_CUDA_OK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
-  kernel<<<dim3(p.MG, p.H, p.B), 32 * W * KS, smem, stream>>>(maps, p, stages, status);
+  p.parts = cdiv(p.G, 16 * W);
+  kernel<<<dim3(static_cast<unsigned>(p.MG) * p.parts, p.H, p.B), 32 * W * KS, smem, stream>>>(maps, p, stages, status);
   NSA_LAUNCH_OK("sel_bwd_dq_rows_kernel");
   return NSA_OK;
 }
 
 template <typename T, int D, bool TMA>
 int launch_dq_loader(const RingMaps& maps, const BwdParams& p, int32_t* st, cudaStream_t s) {
-  if (p.G <= 16) {
-    // as many warps per list as still fit the chip at once (see the forward)
-    const bool short_list = ring_list_bytes(p.T) <= 64 * 1024;                   // (each warp's ring needs its room)
-    const int64_t units = static_cast<int64_t>(p.MG) * p.H * p.B, room = 148 * (D == 128 ? 10 : 16);
-    if (units * 4 <= room && short_list) return launch_dq_rows<T, D, 1, 4, TMA>(maps, p, st, s);
-    if (units * 2 <= room && short_list) return launch_dq_rows<T, D, 1, 2, TMA>(maps, p, st, s);
-    return launch_dq_rows<T, D, 1, 1, TMA>(maps, p, st, s);
-  }
-  if (p.G <= 32) return launch_dq_rows<T, D, 2, 1, TMA>(maps, p, st, s);
-  if (p.G <= 64) return launch_dq_rows<T, D, 4, 1, TMA>(maps, p, st, s);
-  return launch_dq_rows<T, D, 8, 1, TMA>(maps, p, st, s);
+  // four warps share a ring where they fill it and a thread block of one has no better use for its registers: 4680 queries x
+  // 12 heads, 16 blocks of 64, D = 64, groups of 64: 116 us, 121 us with a warp per ring; 3120 of D = 128: 294 and 131 us
+  if constexpr (TMA && D == 64)
+    if (p.G > 48 && p.G <= 64) return launch_dq_rows<T, D, 4, 1, TMA>(maps, p, st, s);
+  if constexpr (!TMA)                       // (a warp's own cp.async loads: two share them)
+    if (p.G > 16 && p.G <= 32) return launch_dq_rows<T, D, 2, 1, TMA>(maps, p, st, s);
+  // a warp per 16 rows, and as many warps per list as still fit the chip at once (see the forward; two of them need more
+  // registers each and pay only for the smallest groups: 624 units at D = 128, 16 blocks of 64, one / two warps: 62 / 83 us)
+  const bool short_list = ring_list_bytes(p.T) <= 64 * 1024;                   // (each warp's ring needs its room)
+  const int64_t units = static_cast<int64_t>(p.MG) * cdiv(p.G, 16) * p.H * p.B, room = 148 * (D == 128 ? 10 : 16);
+  if (units * 4 <= room && short_list) return launch_dq_rows<T, D, 1, 4, TMA>(maps, p, st, s);
+  if (units * 2 <= room && short_list && p.G <= 16) return launch_dq_rows<T, D, 1, 2, TMA>(maps, p, st, s);
+  return launch_dq_rows<T, D, 1, 1, TMA>(maps, p, st, s);
+}
+
+size_t packed_dq_smem(int G, int D, int T) {
+  const int rows = cdiv(G, 16) * 16;
+  return static_cast<size_t>(4 * kPackedRows + 2 * rows) * (D + 8) * 2 + 2 * rows * 4 + slot_table_bytes(T);
+}
+template <typename T, int D>
+int launch_dq_packed(const BwdParams& p, cudaStream_t stream) {
+  const size_t smem = packed_dq_smem(p.G, D, p.T);
+  NSA_CUDA_OK(cudaFuncSetAttribute(sel_bwd_dq_packed_kernel<T, D>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   static_cast<int>(smem)));
+  sel_bwd_dq_packed_kernel<T, D><<<dim3(p.MG, p.H, p.B), cdiv(p.G, 16) * 32, smem, stream>>>(p);
+  NSA_LAUNCH_OK("sel_bwd_dq_packed_kernel");
+  return NSA_OK;
+}
+// Where the packed tiles are the faster ones.  3120 queries x 12 heads, 16 blocks each, packed / row kernel: D = 128, blocks
+// of 1, groups of 17 / 64: 101 / 99, 37 / 56 us; of 8, groups of 48 / 65: 84 / 59, 54 / 75 us; D = 64, blocks of 8, groups of 32 / 64: 37 / 43,
+// 35 / 43 us.  With cp.async loads, D = 128, blocks of 16, groups of 65 / 128: 84 / 110, 70 / 78 us; D = 64, blocks of 64, groups of
+// 64 / 128: 134 / 122, 106 / 122 us.
+bool packed_dq_is_better(bool tma, int G, int block_size, int D) {
+  if (block_size < 4) return G > 16 || D == 64;
+  if (block_size < 16) return G > (D == 64 ? 16 : tma ? 48 : 32);
+  if (block_size < 24) return !tma && D == 128 && G > 64;
+  if (!tma) return D == 64 && block_size >= 48 && G > 112;
+  return D == 64 && G > 48 && G <= 64 && block_size > 32 && block_size <= 36;    // (whose second tile is hardly filled: 97 / 110 us)
 }
 
 template <typename T, int D>
 int launch_dq(const nsa_kv_source* kv, const BwdParams& p, int32_t* st, cudaStream_t s) {
   RingMaps maps{};
-  return make_ring_maps(kv, p.B, p.H, D, p.block_size, 32, &maps) ? launch_dq_loader<T, D, true>(maps, p, st, s)
-                                                          : launch_dq_loader<T, D, false>(maps, p, st, s);
+  const bool tma = make_ring_maps(kv, p.B, p.H, D, p.block_size, 32, &maps);
+  if (packed_dq_is_better(tma, p.G, p.block_size, D) && packed_dq_smem(p.G, D, p.T) <= 220 * 1024) return launch_dq_packed<T, D>(p, s);
+  return tma ? launch_dq_loader<T, D, true>(maps, p, st, s) : launch_dq_loader<T, D, false>(maps, p, st, s);
 }
 
 template <typename T, int D, int TW, int QR, bool TMA>

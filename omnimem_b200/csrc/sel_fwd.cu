@@ -2,6 +2,7 @@
 // a thread block is one (batch, query group, head); each of its warps owns 16 query rows and all of them read the
 // same ring of K/V tiles (sel_rows.cuh); S = Q K^T and O += P V run on mma.sync m16n8k16 with fp32 accumulation
 // and an online softmax in the exp2 domain.
+#include "sel_packed.cuh"
 #include "sel_rows.cuh"
 
 namespace nsa {
@@ -17,17 +18,21 @@ struct FwdParams {
   int64_t i_sb, i_sg, i_sh, i_st;
   KVSrc kv;
   int B, H, T, block_size, chunk_size, causal, G;
+  int parts;                // thread blocks that share a group's rows
   int64_t M;
   float scale_log2;
 };
 
-// W warps of 16 query rows each share one ring; with W = 1 the tiles of the list may be dealt out to KS warps
+// W warps of 16 query rows each share one ring; p.parts such thread blocks take a group; with W = 1 the tiles of the list may be dealt out to KS warps
 // with rings of their own, whose partial results are merged at the end (few groups on many SMs).
 // What bounds it for small groups: the gathered K/V rows, which every list fetches for itself, through the L2 to SM
 // path.  32760 queries x 12 heads, 15-query groups, 16 blocks of 30 tokens: 397 us = 16 TB/s of rows against the
 // 18 TB/s that bulk copies reach here (5911 us with one warp per 70 KB thread block, 124 TF -> 243 TF of products).
 // One K/V stage and 12 warps per SM: 397 us; two stages and 7 warps: 661 us; 16- or 32-byte loads straight into
 // fragments, no shared memory: 780 us.
+// A group of more than 64 queries is dealt out to thread blocks of one warp that walk the list each for itself: 3120 queries
+// x 12 heads, 16 blocks of 64, D = 128, groups of 48 / 64 / 128: 117 / 116 / 117 us; with four warps per ring 131 / 131 / 131 us,
+// with eight 470 / 320 / 247 us.  9360 queries, causal, groups of 64 / 128: 201 / 200 us; with four warps 193 / 196 us.
 template <typename T, int D, int W, int KS, bool TMA>
 __global__ void __launch_bounds__(32 * W * KS) sel_fwd_rows_kernel(const __grid_constant__ RingMaps maps, const FwdParams p,
                                                                    const int stages, int32_t* status) {
@@ -36,11 +41,14 @@ __global__ void __launch_bounds__(32 * W * KS) sel_fwd_rows_kernel(const __grid_
   extern __shared__ __align__(1024) uint8_t smem[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int gid = lane >> 2, t4 = lane & 3;
-  const int g = blockIdx.x, h = blockIdx.y, b = blockIdx.z;
+  const int g = p.parts == 1 ? blockIdx.x : blockIdx.x / p.parts, first_row = (blockIdx.x - g * p.parts) * (16 * W);
+  const int h = blockIdx.y, b = blockIdx.z;
   const int64_t g0 = static_cast<int64_t>(g) * p.G;
   const int row_warp = W > 1 ? warp : 0, part = KS > 1 ? warp : 0;
-  const int n_q = static_cast<int>(p.M - g0 < p.G ? p.M - g0 : p.G) - row_warp * 16;   // rows of this warp (may be <= 0)
-  const int64_t m0 = g0 + row_warp * 16;
+  const int block_rows = static_cast<int>(p.M - g0 < p.G ? p.M - g0 : p.G) - first_row;
+  if (block_rows <= 0) return;                                     // (a short last group)
+  const int n_q = block_rows - row_warp * 16;                      // rows of this warp (may be <= 0)
+  const int64_t m0 = g0 + first_row + row_warp * 16;
 
   const uint32_t ring_bytes = static_cast<uint32_t>(stages) * 2 * kRingTile<D, ROWS>;
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + KS * ring_bytes);
@@ -186,38 +194,232 @@ __global__ void __launch_bounds__(32 * W * KS) sel_fwd_rows_kernel(const __grid_
   }
 }
 
+// ------------------------------------------------------------------------------ packed tiles
+template <typename T, int D>
+__global__ void __launch_bounds__(256) sel_fwd_packed_kernel(const FwdParams p) {
+  constexpr int PITCH = D + 8;
+  constexpr int ESZ = sizeof(T);
+  constexpr int KK = D / 16;     // k-steps of S = Q K^T
+  constexpr int DN = D / 8;      // n8 tiles of O
+  extern __shared__ __align__(1024) uint8_t smem[];
+
+  const int g = blockIdx.x, h = blockIdx.y, b = blockIdx.z;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int gid = lane >> 2, t4 = lane & 3;
+  const int64_t m0 = static_cast<int64_t>(g) * p.G;
+  const int n_q = static_cast<int>(p.M - m0 < p.G ? p.M - m0 : p.G);
+  const int q_chunk = static_cast<int>(m0 / p.chunk_size);
+
+  T* tiles = reinterpret_cast<T*>(smem);                       // [2][2][64][PITCH]
+  const SlotTable st = carve_slot_table(reinterpret_cast<char*>(smem) + 4 * kPackedRows * PITCH * ESZ, p.T);
+  auto stageK = [&](int s) { return tiles + (s * 2) * kPackedRows * PITCH; };
+  auto stageV = [&](int s) { return tiles + (s * 2 + 1) * kPackedRows * PITCH; };
+
+  const int total = build_slot_table<ESZ>(st, p.kv, p.ids, b * p.i_sb + g * p.i_sg + h * p.i_sh, p.i_st,
+                                          p.T, b, h, D, p.block_size, p.chunk_size, p.causal != 0, q_chunk);
+
+  char* out_row0 = p.out + (b * p.o_sb + m0 * p.o_sm + h * p.o_sh) * ESZ;
+  float* lse_row0 = p.lse + (static_cast<int64_t>(b) * p.H + h) * p.M + m0;
+  if (total == 0) {  // no visible key: O = 0, LSE = -inf
+    for (int i = threadIdx.x; i < n_q * (D / 8); i += blockDim.x) {
+      const int r = i / (D / 8), c = i % (D / 8);
+      *reinterpret_cast<uint4*>(out_row0 + r * p.o_sm * ESZ + c * 16) = make_uint4(0, 0, 0, 0);
+    }
+    for (int r = threadIdx.x; r < n_q; r += blockDim.x) lse_row0[r] = -INFINITY;
+    return;
+  }
+
+  const int64_t k_row_bytes = kv_row_bytes(p.kv, false, D, ESZ);
+  const int64_t v_row_bytes = kv_row_bytes(p.kv, true, D, ESZ);
+  const char* q_base = p.q + (b * p.q_sb + m0 * p.q_sm + h * p.q_sh) * ESZ;
+  const int ntiles = (total + kPackedRows - 1) / kPackedRows;
+  const int rows_pad = (blockDim.x >> 5) * 16;
+
+  // Q goes through stage 1 (128 rows) while tile 0 lands in stage 0.
+  issue_rows<T, D, PITCH>(stageK(1), q_base, p.q_sm * ESZ, n_q, rows_pad);
+  cp_async_commit();
+  issue_kv_tile<T, D, PITCH>(stageK(0), stageV(0), st, p.T, 0, total, k_row_bytes, v_row_bytes, p.q);
+  cp_async_commit();
+  cp_async_wait<1>();
+  __syncthreads();
+
+  uint32_t qf[KK][4];
+  {
+    const T* sQ = stageK(1) + (warp * 16 + (lane & 15)) * PITCH + (lane >> 4) * 8;
+#pragma unroll
+    for (int kk = 0; kk < KK; ++kk) ldmatrix_x4(qf[kk], sQ + kk * 16);
+  }
+  __syncthreads();
+
+  float o[DN][4];
+#pragma unroll
+  for (int n = 0; n < DN; ++n) { o[n][0] = o[n][1] = o[n][2] = o[n][3] = 0.f; }
+  float m_i[2] = {-INFINITY, -INFINITY};
+  float l_i[2] = {0.f, 0.f};
+  const bool warp_active = warp * 16 < n_q;
+
+  for (int i = 0; i < ntiles; ++i) {
+    if (i + 1 < ntiles) {
+      issue_kv_tile<T, D, PITCH>(stageK((i + 1) & 1), stageV((i + 1) & 1), st, p.T,
+                                 (i + 1) * kPackedRows, total, k_row_bytes, v_row_bytes, p.q);
+      cp_async_commit();
+      cp_async_wait<1>();
+    } else {
+      cp_async_wait<0>();
+    }
+    __syncthreads();
+    if (warp_active) {
+      const T* sK = stageK(i & 1);
+      const T* sV = stageV(i & 1);
+      const int nvalid = min(kPackedRows, total - i * kPackedRows);
+      float s[8][4];
+#pragma unroll
+      for (int n = 0; n < 8; ++n) { s[n][0] = s[n][1] = s[n][2] = s[n][3] = 0.f; }
+      const T* kb = sK + ((lane & 7) + ((lane >> 4) << 3)) * PITCH + ((lane >> 3) & 1) * 8;
+#pragma unroll
+      for (int kk = 0; kk < KK; ++kk) {
+#pragma unroll
+        for (int n16 = 0; n16 < 4; ++n16) {
+          if (n16 * 16 < nvalid) {
+            uint32_t bf[4];
+            ldmatrix_x4(bf, kb + n16 * 16 * PITCH + kk * 16);
+            mma16816<T>(s[2 * n16], qf[kk], bf[0], bf[1]);
+            mma16816<T>(s[2 * n16 + 1], qf[kk], bf[2], bf[3]);
+          }
+        }
+      }
+      // mask + online softmax (rows gid and gid + 8), exp2 domain
+      float mx[2] = {-INFINITY, -INFINITY};
+#pragma unroll
+      for (int n = 0; n < 8; ++n) {
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const int col = n * 8 + 2 * t4 + (e & 1);
+          const float v = (col < nvalid) ? s[n][e] * p.scale_log2 : -INFINITY;
+          s[n][e] = v;
+          mx[e >> 1] = fmaxf(mx[e >> 1], v);
+        }
+      }
+#pragma unroll
+      for (int r = 0; r < 2; ++r) {
+        mx[r] = fmaxf(mx[r], __shfl_xor_sync(0xffffffffu, mx[r], 1));
+        mx[r] = fmaxf(mx[r], __shfl_xor_sync(0xffffffffu, mx[r], 2));
+        const float m_new = fmaxf(m_i[r], mx[r]);   // finite: every tile has a valid column
+        const float corr = fast_exp2(m_i[r] - m_new);
+        m_i[r] = m_new;
+        l_i[r] *= corr;
+#pragma unroll
+        for (int n = 0; n < DN; ++n) { o[n][2 * r] *= corr; o[n][2 * r + 1] *= corr; }
+      }
+      uint32_t pa[4][4];
+#pragma unroll
+      for (int n = 0; n < 8; ++n) {
+        const float p0 = fast_exp2(s[n][0] - m_i[0]);
+        const float p1 = fast_exp2(s[n][1] - m_i[0]);
+        const float p2 = fast_exp2(s[n][2] - m_i[1]);
+        const float p3 = fast_exp2(s[n][3] - m_i[1]);
+        l_i[0] += p0 + p1;
+        l_i[1] += p2 + p3;
+        pa[n >> 1][(n & 1) * 2] = pack2<T>(p0, p1);
+        pa[n >> 1][(n & 1) * 2 + 1] = pack2<T>(p2, p3);
+      }
+      const T* vb = sV + ((lane & 7) + ((lane >> 3) & 1) * 8) * PITCH + (lane >> 4) * 8;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        if (j * 16 < nvalid) {
+#pragma unroll
+          for (int d16 = 0; d16 < D / 16; ++d16) {
+            uint32_t bf[4];
+            ldmatrix_x4_trans(bf, vb + j * 16 * PITCH + d16 * 16);
+            mma16816<T>(o[2 * d16], pa[j], bf[0], bf[1]);
+            mma16816<T>(o[2 * d16 + 1], pa[j], bf[2], bf[3]);
+          }
+        }
+      }
+    }
+    __syncthreads();
+  }
+
+  if (warp_active) {
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
+      l_i[r] += __shfl_xor_sync(0xffffffffu, l_i[r], 1);
+      l_i[r] += __shfl_xor_sync(0xffffffffu, l_i[r], 2);
+      const int row = warp * 16 + gid + 8 * r;
+      if (row < n_q) {
+        const float inv = l_i[r] > 0.f ? 1.f / l_i[r] : 0.f;
+        char* orow = out_row0 + row * p.o_sm * ESZ;
+#pragma unroll
+        for (int n = 0; n < DN; ++n)
+          *reinterpret_cast<uint32_t*>(orow + (n * 8 + 2 * t4) * ESZ) =
+              pack2<T>(o[n][2 * r] * inv, o[n][2 * r + 1] * inv);
+        if (t4 == 0)
+          lse_row0[row] = l_i[r] > 0.f ? (m_i[r] + log2f(l_i[r])) * kLn2 : -INFINITY;
+      }
+    }
+  }
+}
+
+size_t packed_fwd_smem(int D, int T) { return 4 * kPackedRows * (D + 8) * 2 + slot_table_bytes(T); }
+template <typename T, int D>
+int launch_packed(const FwdParams& p, int MG, cudaStream_t stream) {
+  const size_t smem = packed_fwd_smem(D, p.T);
+  NSA_CUDA_OK(cudaFuncSetAttribute(sel_fwd_packed_kernel<T, D>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   static_cast<int>(smem)));
+  sel_fwd_packed_kernel<T, D><<<dim3(MG, p.H, p.B), cdiv(p.G, 16) * 32, smem, stream>>>(p);
+  NSA_LAUNCH_OK("sel_fwd_packed_kernel");
+  return NSA_OK;
+}
+// Where the packed tiles are the faster ones.  3120 queries x 12 heads, 16 blocks each, packed / row kernel: D = 128, blocks
+// of 1 and groups of 8 / 64: 50 / 50, 15 / 50 us; blocks of 8, groups of 32 / 64 / 128: 53 / 50, 29 / 50, 33 / 51 us; of 16: 98 / 50,
+// 51 / 50, 55 / 51 us; D = 64, blocks of 16, groups of 48 / 64: 33 / 27, 21 / 27 us.  With cp.async loads, D = 128, blocks of 16, groups
+// of 32 / 64: 99 / 65, 50 / 60 us; of 64, groups of 64 / 128: 174 / 148, 131 / 143 us; D = 64: 64 / 63, 54 / 63 us.
+bool packed_fwd_is_better(bool tma, int G, int block_size, int D) {
+  if (block_size < 4) return G >= 8 || D == 64 || !tma;
+  if (block_size < 16) return G > (tma && D == 128 ? 32 : 16);
+  if (block_size < 24) return tma ? D == 64 && G > 48 : G > (D == 64 ? 32 : 48);
+  if (!tma) return G >= (D == 64 ? 60 : 113);
+  // by the rows that a block leaves free in its last tile: blocks of 33, D = 64, groups of 64: 65 / 99 us; D = 128, groups of
+  // 128: 112 / 180 us
+  const int rows = cdiv(block_size, 32) * 32;
+  if (D == 128) return G > 96 && rows * 5 >= block_size * 8;
+  return rows * 5 >= block_size * 6 ? G > 48 && (G <= 72 || G > 96) : G > 112 && block_size > 32;   // (64, 128: 80 / 93 us)
+}
+
+// -------------------------------------------------------------------------------------- launch
 template <typename T, int D, int W, int KS, bool TMA>
-int launch_rows(const RingMaps& maps, const FwdParams& p, int MG, int32_t* status, cudaStream_t stream) {
-  // stages: two per ring of a single warp (the thread blocks that share an SM are the depth), three where several
-  // warps wait for the same ring; never less than the epilogue's staging needs
-  const int stages = W <= 2 ? 1 : 3;
-  static_assert(W * 16 * (D * 2 + 16) <= (W <= 2 ? 1 : 3) * 2 * kRingTile<D, 32>, "the epilogue stages its rows in the ring");
+int launch_rows(const RingMaps& maps, FwdParams p, int MG, int32_t* status, cudaStream_t stream) {
+  // stages: one for a single warp (the thread blocks that share an SM are the depth), three where several warps wait for
+  // the same ring; never less than the epilogue's staging needs
+  constexpr int stages = W <= 2 ? 1 : 3;
+  static_assert(W * 16 * (D * 2 + 16) <= stages * 2 * kRingTile<D, 32>, "the epilogue stages its rows in the ring");
   static_assert((KS - 1) * (D / 8 * 128 + 128) * 4 <= KS * 2 * kRingTile<D, 32>, "the partial results are merged in the ring");
   const size_t smem = static_cast<size_t>(KS) * stages * 2 * kRingTile<D, 32> + KS * kRingBars * 8 + 16 +
                       ring_list_bytes(p.T);
   NSA_REQUIRE(smem <= 226 * 1024, NSA_ERR_UNSUPPORTED, "sel_fwd: T=%d needs too much shared memory", p.T);
   auto kernel = sel_fwd_rows_kernel<T, D, W, KS, TMA>;
   NSA_CUDA_OK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
-  kernel<<<dim3(MG, p.H, p.B), 32 * W * KS, smem, stream>>>(maps, p, stages, status);
+  p.parts = cdiv(p.G, 16 * W);
+  kernel<<<dim3(static_cast<unsigned>(MG) * p.parts, p.H, p.B), 32 * W * KS, smem, stream>>>(maps, p, stages, status);
   NSA_LAUNCH_OK("sel_fwd_rows_kernel");
   return NSA_OK;
 }
 
 template <typename T, int D, bool TMA>
 int launch_loader(const RingMaps& maps, const FwdParams& p, int MG, int32_t* st, cudaStream_t s) {
-  if (p.G <= 16) {
-    // as many warps per list as still fit the chip at once: 12 warps per SM at D = 128 (registers), 16 at D = 64.
-    // Measured, D = 128, 16 blocks of 30, one / two / four warps per list: 384 lists 22.7 / 18.5 / 15.5 us,
-    // 768 lists 25.9 / 23.0 / 28.0 us, 1248 lists 31.6 / 40.8 / 41.0 us
-    const bool short_list = ring_list_bytes(p.T) <= 64 * 1024;                   // (each warp's ring needs its room)
-    const int64_t units = static_cast<int64_t>(MG) * p.H * p.B, room = 148 * (D == 128 ? 12 : 16);
-    if (units * 4 <= room && short_list) return launch_rows<T, D, 1, 4, TMA>(maps, p, MG, st, s);
-    if (units * 2 <= room && short_list) return launch_rows<T, D, 1, 2, TMA>(maps, p, MG, st, s);
-    return launch_rows<T, D, 1, 1, TMA>(maps, p, MG, st, s);
+  // A warp per 16 rows, and as many warps per list as still fit the chip at once: 12 warps per SM at D = 128 (registers),
+  // 16 at D = 64.  Measured, D = 128, 16 blocks of 30, one / two / four warps per list: 384 lists 22.7 / 18.5 / 15.5 us,
+  // 768 lists 25.9 / 23.0 / 28.0 us, 1248 lists 31.6 / 40.8 / 41.0 us.  With more lists than that two or four warps share a
+  // ring where they fill it, and always where the loads are a warp's own (cp.async).
+  const bool short_list = ring_list_bytes(p.T) <= 64 * 1024;                   // (each warp's ring needs its room)
+  const int64_t units = static_cast<int64_t>(MG) * cdiv(p.G, 16) * p.H * p.B, room = 148 * (D == 128 ? 12 : 16);
+  if (!TMA || units * 2 > room || !short_list) {
+    if (p.G > 16 && p.G <= 32) return launch_rows<T, D, 2, 1, TMA>(maps, p, MG, st, s);
+    if (TMA ? p.G > 48 && p.G <= 64 : p.G > 32) return launch_rows<T, D, 4, 1, TMA>(maps, p, MG, st, s);
   }
-  if (p.G <= 32) return launch_rows<T, D, 2, 1, TMA>(maps, p, MG, st, s);
-  if (p.G <= 64) return launch_rows<T, D, 4, 1, TMA>(maps, p, MG, st, s);
-  return launch_rows<T, D, 8, 1, TMA>(maps, p, MG, st, s);
+  if (units * 4 <= room && short_list) return launch_rows<T, D, 1, 4, TMA>(maps, p, MG, st, s);
+  if (units * 2 <= room && short_list) return launch_rows<T, D, 1, 2, TMA>(maps, p, MG, st, s);
+  return launch_rows<T, D, 1, 1, TMA>(maps, p, MG, st, s);
 }
 
 template <typename T, int D>
@@ -226,8 +428,9 @@ int launch(const nsa_kv_source* kv, const FwdParams& p, int MG, cudaStream_t s) 
   int rc = device_status_address(&st);
   if (rc) return rc;
   RingMaps maps{};
-  return make_ring_maps(kv, p.B, p.H, D, p.block_size, 32, &maps) ? launch_loader<T, D, true>(maps, p, MG, st, s)
-                                                              : launch_loader<T, D, false>(maps, p, MG, st, s);
+  const bool tma = make_ring_maps(kv, p.B, p.H, D, p.block_size, 32, &maps);
+  if (packed_fwd_is_better(tma, p.G, p.block_size, D) && packed_fwd_smem(D, p.T) <= 200 * 1024) return launch_packed<T, D>(p, MG, s);
+  return tma ? launch_loader<T, D, true>(maps, p, MG, st, s) : launch_loader<T, D, false>(maps, p, MG, st, s);
 }
 
 }  // namespace
