@@ -213,9 +213,13 @@ struct ScoreParams {
   int causal, G, chunk_size, chunk_size_k, block_size, q_off, id_base, id_stride;
   __device__ __forceinline__ int64_t columns(int g) const {
     if (!causal) return NC;
-    const int64_t q_cid = static_cast<int64_t>(g) * G / chunk_size + q_off;
-    const int64_t ids = ((q_cid + 1) * chunk_size_k + block_size - 1) / block_size - id_base;
-    const int64_t n = (ids + id_stride - 1) / id_stride;
+    // (64-bit divisions took a sixth of a kernel that scores one row against a long memory)
+    const auto div = [](int64_t a, int b) -> int64_t {
+      return static_cast<uint64_t>(a) <= 0xffffffffull ? static_cast<uint32_t>(a) / static_cast<uint32_t>(b) : a / b;
+    };
+    const int64_t q_cid = div(static_cast<int64_t>(g) * G, chunk_size) + q_off;
+    const int64_t ids = div((q_cid + 1) * chunk_size_k + block_size - 1, block_size) - id_base;
+    const int64_t n = id_stride == 1 ? ids : div(ids + id_stride - 1, id_stride);
     return ids <= 0 ? 0 : (n < NC ? n : NC);
   }
 };
@@ -345,6 +349,7 @@ __global__ void __launch_bounds__(128) score_mma_kernel(const ScoreParams p) {
   cp_async_wait<0>();
   __syncthreads();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, gid = lane >> 2, t4 = lane & 3;
+  if (warp * 16 >= nrow) return;
   float acc[8][4];
 #pragma unroll
   for (int n = 0; n < 8; ++n) { acc[n][0] = acc[n][1] = acc[n][2] = acc[n][3] = 0.f; }
@@ -765,13 +770,17 @@ __device__ __forceinline__ void warp_select(const SelectParams& p, const float* 
   warp_take_topk<ITEMS>(keys, p.topk, oi, os, sorted);
 }
 
-template <int ITEMS, bool MERGE>
-__global__ void __launch_bounds__(128) select_warp_kernel(const SelectParams p, int64_t rows) {
+// SEGS: warp w takes columns [32 ITEMS s, 32 ITEMS (s + 1)) of row w / n_seg, s = w % n_seg, and writes its list to
+// out_idx / out_scores laid out [n_seg][rows][topk]
+template <int ITEMS, bool MERGE, bool SEGS = false>
+__global__ void __launch_bounds__(128) select_warp_kernel(const SelectParams p, int64_t rows, int n_seg) {
   chain_release();
   chain_wait();
   const int warp = threadIdx.x >> 5;
-  const int64_t row = static_cast<int64_t>(blockIdx.x) * 4 + warp;
+  const int64_t unit = static_cast<int64_t>(blockIdx.x) * 4 + warp, row = SEGS ? unit / n_seg : unit;
   if (row >= rows) return;
+  const int64_t seg = unit - row * n_seg, c_off = SEGS ? seg * (32 * ITEMS) : 0, out_row = SEGS ? seg * rows + row : row;
+  const int64_t NC = SEGS && p.NC - c_off > 32 * ITEMS ? 32 * ITEMS : p.NC - c_off;
   RowMask rm{};
   const float* srow;
   if (MERGE) {
@@ -782,11 +791,11 @@ __global__ void __launch_bounds__(128) select_warp_kernel(const SelectParams p, 
     const int g = static_cast<int>(bg % p.MG);
     const int64_t b = bg / p.MG;
     rm = make_row_mask(p.mask, g);
-    srow = p.scores + ((b * p.H + h) * p.MG + g) * p.NC;
+    srow = p.scores + ((b * p.H + h) * p.MG + g) * p.NC + c_off;
   }
   __shared__ unsigned long long s_sorted[4][ITEMS][32];
-  warp_select<ITEMS, MERGE>(p, srow, rm, p.NC, 0, row, p.out_idx + row * p.topk,
-                            p.out_scores ? p.out_scores + row * p.topk : nullptr, s_sorted[warp]);
+  warp_select<ITEMS, MERGE>(p, srow, rm, NC, c_off, row, p.out_idx + out_row * p.topk,
+                            p.out_scores ? p.out_scores + out_row * p.topk : nullptr, s_sorted[warp]);
 }
 
 // Rows of any length: W warps per row read it twice, every thread a column in 32 W.
@@ -1126,6 +1135,15 @@ int launch_score_select(const ScoreSelectParams& p, int B, cudaStream_t s) {
   return NSA_OK;
 }
 
+// Fewer long rows than SMs: a thread block per row leaves the chip idle, so a warp sorts the keys of each 1024 columns and
+// the lists of a row are merged like those of several ranks (exact: a row's best are among its segments' best, with the
+// same keys).  12 rows of 60000 / 200000, top-8: 78 / 215 us; with 32 warps per row 99 / 296 us, with eight 131 / 414 us.
+constexpr int kSegCols = 1024, kSegRows = 148, kSegTopk = 16;
+bool in_segments(int64_t rows, int64_t NC) { return rows <= kSegRows && NC > 8 * kSegCols; }
+size_t segment_bytes(int64_t rows, int64_t NC) {
+  return in_segments(rows, NC) ? align_up(static_cast<size_t>(cdiv64(NC, kSegCols)) * rows * kSegTopk * 8, 256) : 0;
+}
+
 template <int W> int launch_select_rows(const SelectParams& sel, int64_t rows, cudaStream_t s) {
   NSA_CUDA_OK(launch_chained(kChainSmall, select_rows_kernel<W>, dim3(static_cast<unsigned>(W == 1 ? cdiv64(rows, 4) : rows)),
                              dim3(W == 1 ? 128 : 32 * W), 0, s, sel, rows));
@@ -1134,21 +1152,37 @@ template <int W> int launch_select_rows(const SelectParams& sel, int64_t rows, c
 }
 
 template <bool MERGE>
-int launch_select(const SelectParams& sel, int64_t rows, cudaStream_t s) {
+int launch_select(const SelectParams& sel, int64_t rows, cudaStream_t s, void* seg_ws = nullptr) {
   const unsigned blocks4 = static_cast<unsigned>(cdiv64(rows, 4));
+  if (!MERGE && seg_ws != nullptr && in_segments(rows, sel.NC) && sel.topk <= kSegTopk) {
+    const int64_t n_seg = cdiv64(sel.NC, kSegCols);
+    NSA_REQUIRE(n_seg * rows <= 0x7fffffff, NSA_ERR_INVALID, "topk: rows too long");
+    SelectParams first = sel, merge{};
+    first.out_idx = static_cast<int32_t*>(seg_ws);
+    first.out_scores = reinterpret_cast<float*>(first.out_idx + n_seg * rows * sel.topk);
+    NSA_CUDA_OK(launch_chained(kChainSmall, select_warp_kernel<kSegCols / 32, false, true>, dim3(static_cast<unsigned>(cdiv64(rows * n_seg, 4))),
+                               dim3(128), 0, s, first, rows, static_cast<int>(n_seg)));
+    NSA_LAUNCH_OK("select kernel (segments)");
+    merge.scores = first.out_scores; merge.cand_ids = first.out_idx; merge.NC = n_seg * sel.topk;
+    merge.MG = 1; merge.H = 1; merge.seg_len = sel.topk; merge.seg_stride = rows * sel.topk; merge.topk = sel.topk;
+    merge.out_idx = sel.out_idx; merge.out_scores = sel.out_scores;
+    return launch_select<true>(merge, rows, s);
+  }
   if (!MERGE && sel.NC > 1024 && sel.topk <= 128) {
     // a lane list of 16 per warp, and 2048 columns per warp while that leaves fewer than 16 warps per SM
     int w = cdiv(sel.topk, 16);
-    while (w < 8 && sel.NC > 2048ll * w && rows * w < 148 * 16) ++w;
+    while (w < 32 && sel.NC > 1024ll * w && rows * w < 148 * 16) ++w;
     if (w <= 1) return launch_select_rows<1>(sel, rows, s);
     if (w <= 2) return launch_select_rows<2>(sel, rows, s);
     if (w <= 4) return launch_select_rows<4>(sel, rows, s);
-    return launch_select_rows<8>(sel, rows, s);
+    if (w <= 8) return launch_select_rows<8>(sel, rows, s);
+    if (w <= 16) return launch_select_rows<16>(sel, rows, s);
+    return launch_select_rows<32>(sel, rows, s);
   }
   if (sel.NC <= 512) {
-    NSA_CUDA_OK(launch_chained(kChainSmall, select_warp_kernel<16, MERGE>, dim3(blocks4), dim3(128), 0, s, sel, rows));
+    NSA_CUDA_OK(launch_chained(kChainSmall, select_warp_kernel<16, MERGE>, dim3(blocks4), dim3(128), 0, s, sel, rows, 1));
   } else if (sel.NC <= 1024) {
-    NSA_CUDA_OK(launch_chained(kChainSmall, select_warp_kernel<32, MERGE>, dim3(blocks4), dim3(128), 0, s, sel, rows));
+    NSA_CUDA_OK(launch_chained(kChainSmall, select_warp_kernel<32, MERGE>, dim3(blocks4), dim3(128), 0, s, sel, rows, 1));
   } else {
     const size_t ksmem = sel.NC * 8 <= 64 * 1024 ? static_cast<size_t>(sel.NC) * 8 : 0;
     NSA_CUDA_OK(cudaFuncSetAttribute(select_kernel<MERGE>, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024));
@@ -1259,7 +1293,7 @@ int check_rows16(const char* what, const void* ptr, const int64_t* stride, int e
 int run_score_select(const void* qp, const int64_t* qs, const void* kp, const int64_t* ks, int B,
                      int MG, int H, int D, int64_t NC, int topk, float scale, const Mask& m,
                      int32_t* out_idx, float* out_scores, float* scores, int dtype, cudaStream_t s,
-                     bool allow_fused = true) {
+                     void* seg_ws = nullptr, bool allow_fused = true) {
   ScoreParams sp{static_cast<const char*>(qp), qs[0], qs[1], qs[2], static_cast<const char*>(kp),
                  ks[0], ks[1], ks[2], scores, MG, H, D, NC, scale,
                  m.causal && !m.tf, m.G, m.chunk_size, m.chunk_size_k, m.block_size, m.q_off, m.id_base, m.id_stride};
@@ -1285,7 +1319,7 @@ int run_score_select(const void* qp, const int64_t* qs, const void* kp, const in
   sel.scores = scores; sel.cand_ids = nullptr; sel.NC = NC; sel.MG = MG; sel.H = H;
   sel.seg_len = 0; sel.seg_stride = 0; sel.topk = topk; sel.out_idx = out_idx; sel.out_scores = out_scores;
   sel.mask = m;
-  return launch_select<false>(sel, static_cast<int64_t>(B) * MG * H, s);
+  return launch_select<false>(sel, static_cast<int64_t>(B) * MG * H, s, seg_ws);
 }
 
 __global__ void fill_empty_kernel(int32_t* __restrict__ out_idx, float* __restrict__ out_scores, int64_t n) {
@@ -1350,12 +1384,12 @@ extern "C" int nsa_pool_rows(const void* x, const int64_t x_stride[3], void* out
   return launch_pool<float>(p, B, NB, s);
 }
 
-// scores [B,H,MG,NC] fp32
+// scores [B,H,MG,NC] fp32, then (a few long rows) the lists of their segments
 static size_t score_bytes(int32_t B, int32_t MG, int32_t H, int64_t NC) {
   return align_up(static_cast<size_t>(B) * MG * H * NC * sizeof(float), 256);
 }
 extern "C" size_t nsa_topk_workspace_bytes(int32_t B, int32_t MG, int32_t H, int64_t NC) {
-  return score_bytes(B, MG, H, NC);
+  return score_bytes(B, MG, H, NC) + segment_bytes(static_cast<int64_t>(B) * MG * H, NC);
 }
 
 static int topk_common_checks(int32_t B, int32_t MG, int32_t H, int32_t D, int64_t NC, int32_t topk,
@@ -1387,7 +1421,8 @@ extern "C" int nsa_topk(const void* q_pooled, const int64_t q_stride[3], const v
   Mask m;
   if ((rc = fill_mask_checked(mask, MG, NC, &m))) return rc;
   return run_score_select(q_pooled, q_stride, k_pooled, k_stride, B, MG, H, D, NC, topk, scale, m,
-                          out_idx, out_scores, static_cast<float*>(workspace), dtype, s);
+                          out_idx, out_scores, static_cast<float*>(workspace), dtype, s,
+                          static_cast<char*>(workspace) + score_bytes(B, MG, H, NC));
 }
 
 // Pooling of the raw keys, then scoring + selection (one kernel when a row's scores fit shared memory).
@@ -1553,5 +1588,5 @@ extern "C" int nsa_topk_static_scratch(const void* q_pooled, const int64_t q_str
   // Every score the selection reads is written by the scoring kernel of the same call, so nothing
   // in the array has to start at zero and whatever an earlier call left behind is never read.
   return run_score_select(q_pooled, q_stride, k_pooled, k_stride, B, MG, H, D, NC, topk, scale, m, out_idx,
-                          out_scores, scratch, dtype, s, /*allow_fused=*/false);
+                          out_scores, scratch, dtype, s, nullptr, /*allow_fused=*/false);
 }

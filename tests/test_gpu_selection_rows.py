@@ -90,3 +90,18 @@ def test_inverted_index(dev, MG, T, NS, causal, slots):
         assert torch.equal(groups.cpu().view(H, -1)[h, :len(order)].long(), g_of[ok][order])
         if slots:
             assert torch.equal(slot.cpu().view(H, -1)[h, :len(order)].long(), t_of[ok][order])
+
+
+@pytest.mark.parametrize("case", [
+    (3, 8192, 64, 16, "random", False, torch.bfloat16),      # eight segments: still a thread block per row
+    (3, 8193, 64, 16, "ties", True, torch.bfloat16),         # segments, the last one of one column
+    (74, 9001, 64, 16, "random", True, torch.float16),       # the most rows that are split
+    (75, 9001, 64, 16, "ties", False, torch.bfloat16),       # one more
+    (1, 20000, 64, 1, "random", False, torch.bfloat16),
+    (2, 17500, 64, 8, "few lanes", True, torch.float32),
+    (3, 33000, 64, 17, "few lanes", False, torch.bfloat16),  # 32 warps per row
+    (20, 17000, 64, 128, "ties", True, torch.bfloat16),      # 16
+    (17, 1000, 64, 8, "random", True, torch.bfloat16),       # scores of 17 rows: warps with none
+], ids=lambda c: f"{c[0]}x{c[1]}_t{c[3]}")
+def test_few_long_rows(dev, case):
+    test_long_rows(dev, case)
