@@ -25,8 +25,13 @@ struct GateParams {
 template <typename T>
 __device__ __forceinline__ void gates_of_row(const GateParams& p, int64_t row, float (&s)[3], bool (&inside)[3]) {
   float z[3];
-  const uint32_t token = static_cast<uint32_t>(row) / static_cast<uint32_t>(p.H);
-  const T* g = reinterpret_cast<const T*>(p.g) + token * p.g_stride + (static_cast<uint32_t>(row) - token * p.H) * 3;
+  const T* g = reinterpret_cast<const T*>(p.g);
+  if (p.H == 1) {
+    g += row * p.g_stride;
+  } else {
+    const uint32_t token = static_cast<uint32_t>(row) / static_cast<uint32_t>(p.H);
+    g += token * p.g_stride + (static_cast<uint32_t>(row) - token * p.H) * 3;
+  }
 #pragma unroll
   for (int i = 0; i < 3; ++i) {
     const float raw = to_f32<T>(g[i]);
@@ -57,11 +62,12 @@ __global__ void gate_combine_fwd_kernel(const GateParams p) {
     const uint32_t iu = static_cast<uint32_t>(i);
     const int64_t row = iu / cpr;
     const int cc = static_cast<int>(iu - static_cast<uint32_t>(row) * cpr);
-    // the branches are on their way while the gates are computed: 393120 rows of 128, 96 -> 89 us (403 MB)
+    // the branches are on their way while the gates are computed: 393120 rows of 128, 96 -> 89 us (403 MB).  (They are loaded
+    // the ordinary way: evict-first loads take as long there, and lose the L2's copies of branches that fit it.)
     uint4 v[3];
 #pragma unroll
     for (int b = 0; b < 3; ++b)
-      if (p.o[b] != nullptr) v[b] = __ldcs(reinterpret_cast<const uint4*>(p.o[b] + (row * p.D) * sizeof(T) + cc * 16));
+      if (p.o[b] != nullptr) v[b] = *reinterpret_cast<const uint4*>(p.o[b] + (row * p.D) * sizeof(T) + cc * 16);
     float s[3];
     bool inside[3];
     gates_of_row<T>(p, row, s, inside);
@@ -168,6 +174,11 @@ extern "C" int nsa_gate_combine_strided(const void* g_logits, int64_t g_token_st
                                         const void* o_swa, void* x, int64_t tokens, int32_t H, int32_t D, int32_t softmax,
                                         int32_t dtype, void* stream) {
   NSA_REQUIRE(H > 0 && tokens >= 0, NSA_ERR_INVALID, "gate_combine: bad size");
+  if (g_token_stride == 3 * static_cast<int64_t>(H)) {           // the logits lie row by row
+    tokens *= H;
+    H = 1;
+    g_token_stride = 3;
+  }
   const int64_t rows = tokens * H;
   int rc;
   if ((rc = check_common("gate_combine", g_logits, o_cmp, o_slc, o_swa, rows, D, dtype))) return rc;
