@@ -197,12 +197,12 @@ __device__ __forceinline__ void inv_order(const IdxParams& p, int b, int h, cons
   }
 }
 
-// After the scatter pass: a thread block puts 32 buckets of a row in order, where they lie.
-__global__ void __launch_bounds__(1024) inv_sort_kernel(const IdxParams p, const int32_t* __restrict__ offsets, int32_t* groups) {
+// After the scatter pass: a thread block puts `per` buckets of a row in order, where they lie.
+__global__ void __launch_bounds__(1024) inv_sort_kernel(const IdxParams p, const int32_t* __restrict__ offsets, int32_t* groups, int per) {
   const int h = blockIdx.y, b = blockIdx.z;
   const int64_t row = static_cast<int64_t>(b) * p.H + h, pairs = static_cast<int64_t>(p.MG) * p.T;
   const int32_t* o = offsets + row * (p.NS + 1);
-  const int64_t i0 = static_cast<int64_t>(blockIdx.x) * 32, i1 = min64(i0 + 32, p.NS);
+  const int64_t i0 = static_cast<int64_t>(blockIdx.x) * per, i1 = min64(i0 + per, p.NS);
   inv_order(p, b, h, groups + row * pairs, groups + row * pairs, p.slots != nullptr ? p.slots + row * pairs : nullptr,
             static_cast<int>(i0), static_cast<int>(i1), 1, [&](int i) { return o[i]; });
 }
@@ -990,7 +990,9 @@ int run_inverted_index(const IdxParams& ip, int32_t* groups, int32_t* offsets, i
   if (pairs > 0) {
     inv_pass_kernel<true><<<grid, kIdxThreads, 0, stream>>>(ip, counts, groups);
     NSA_LAUNCH_OK("inv_pass_kernel<scatter>");
-    inv_sort_kernel<<<dim3(static_cast<unsigned>(cdiv64(ip.NS, 32)), ip.H, ip.B), 1024, 0, stream>>>(ip, offsets, groups);
+    // a bucket that a warp cannot hold takes its thread block a walk over the row: one such bucket per block, side by side
+    const int per = pairs > ip.NS * (24 * kHeld) ? 1 : 32;
+    inv_sort_kernel<<<dim3(static_cast<unsigned>(cdiv64(ip.NS, per)), ip.H, ip.B), 1024, 0, stream>>>(ip, offsets, groups, per);
     NSA_LAUNCH_OK("inv_sort_kernel");
   }
   return NSA_OK;
