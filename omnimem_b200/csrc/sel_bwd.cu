@@ -1,10 +1,11 @@
 // Selection attention backward, general geometry (bf16 / fp16, D in {64,128}):
-//   * inverted (block -> query groups) CSR index: histogram, per-(b,h) scan, scatter;
-//   * dQ kernel: one thread block per (b, group, h), the same ring of K/V tiles as the forward (sel_rows.cuh);
-//     computes delta = sum(O*dO) in its prologue and stores it for the dK/dV kernel;
-//   * dK/dV kernel: one thread block OWNS a tile of at most 32 tokens of one (b, h, block) and walks the
+//   * inverted (block -> query groups) CSR index: histogram, per-(b,h) scan, scatter, sort;
+//   * dQ: the forward's two forms, a ring of K/V tiles per warp (sel_rows.cuh) or packed tiles per group
+//     (sel_packed.cuh); computes delta = sum(O*dO) in its prologue and stores it for the dK/dV kernel;
+//   * dK/dV kernel: one thread block OWNS a tile of at most 32 or 64 tokens of one (b, h, block) and walks the
 //     block's bucket of query groups in ascending group order - no atomics, results are
-//     bit-reproducible from run to run.
+//     bit-reproducible from run to run.  (Blocks of at most 32 tokens take sel_bwd_dkv_rows_tc.cu where tensor maps
+//     describe the query rows.)
 #include "sel_packed.cuh"
 #include "sel_rows.cuh"
 

@@ -1,7 +1,7 @@
 // Selection attention forward, general geometry (any block size, group size <= 128, D in {64, 128}, bf16 / fp16):
-// a thread block is one (batch, query group, head); each of its warps owns 16 query rows and all of them read the
-// same ring of K/V tiles (sel_rows.cuh); S = Q K^T and O += P V run on mma.sync m16n8k16 with fp32 accumulation
-// and an online softmax in the exp2 domain.
+// a thread block is one (batch, query group, head) or a part of its rows; a warp owns 16 query rows; the K/V rows come in
+// tiles of one block each through a ring (sel_rows.cuh) or packed into tiles of 64 (sel_packed.cuh); S = Q K^T and
+// O += P V run on mma.sync m16n8k16 with fp32 accumulation and an online softmax in the exp2 domain.
 #include "sel_packed.cuh"
 #include "sel_rows.cuh"
 

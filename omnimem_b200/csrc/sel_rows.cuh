@@ -4,7 +4,7 @@
 // A query group of this path is often far smaller than a tensor-core tile (15 queries against 30-token
 // blocks), and every group reads its own blocks, so what bounds these kernels is how fast the gathered rows
 // reach shared memory and how many warps hide each other's chains of small products, not the products
-// themselves.  Hence: a warp works on 16 rows by itself, the gathered rows come in tiles of 16 or 32 rows through a
+// themselves.  Hence: a warp works on 16 rows by itself, the gathered rows come in tiles of 16 to 64 rows through a
 // ring that one thread fills with TMA copies (one instruction per operand and tile), and as many small thread
 // blocks as registers allow share an SM, each with its own ring: one stage is enough, depth only costs warps.
 // Operands that the tensor maps cannot describe (address tables, zero strides) go through the same ring with
