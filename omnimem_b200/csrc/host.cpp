@@ -33,9 +33,11 @@ void check(const char* name, int rc) {
   if (rc == 0) return;
   throw BackendError(std::string(name) + " failed (" + std::to_string(rc) + "): " + nsa_last_error());
 }
-void need(bool ok, const std::string& text) {
-  if (!ok) throw BackendError(text);
-}
+// (the text is put together only where it is needed: a call checks some twenty conditions)
+#define NEED(ok, text)                    \
+  do {                                    \
+    if (!(ok)) throw BackendError(text);  \
+  } while (0)
 
 // ----------------------------------------------------------------------------------------- tensors
 int dtype_of(const Tensor& t) {
@@ -96,7 +98,7 @@ const Tensor& or_none(const OptTensor& t) {
 }
 void* ptr(const Tensor& t) { return t.defined() ? t.data_ptr() : nullptr; }
 int32_t i32(int64_t x, const char* what) {
-  need(x >= INT32_MIN && x <= INT32_MAX, std::string(what) + "=" + std::to_string(x) + " does not fit in int32");
+  NEED(x >= INT32_MIN && x <= INT32_MAX, std::string(what) + "=" + std::to_string(x) + " does not fit in int32");
   return static_cast<int32_t>(x);
 }
 int64_t ceil_div(int64_t a, int64_t b) { return (a + b - 1) / b; }
@@ -132,7 +134,7 @@ using MaskArgs = std::vector<int64_t>;
 nsa_topk_mask mask_of(const MaskArgs& a) {
   static const char* names[12] = {"block_size", "chunk_size", "chunk_size_k", "q_group_size", "q_chunk_offset", "ex_win", "ex_sink",
                                   "causal", "tf_mask", "prog_excl", "id_base", "id_stride"};
-  need(a.size() == 12, "topk: 12 mask values are expected");
+  NEED(a.size() == 12, "topk: 12 mask values are expected");
   int32_t v[12];
   for (int i = 0; i < 12; ++i) v[i] = i32(a[i], names[i]);
   return nsa_topk_mask{v[0], v[1], v[2], v[3], v[4], v[5], v[6], v[7] != 0, v[8] != 0, v[9] != 0, v[10], v[11]};
@@ -143,10 +145,10 @@ std::pair<Tensor, OptTensor> topk(const Tensor& q_, const Tensor& k_, int64_t T,
   need_4d(q_, "topk q");
   need_4d(k_, "topk k");
   need_cuda({&q_, &k_});
-  need(q_.scalar_type() == k_.scalar_type(), std::string("topk: q and k must share a dtype, got torch.") + c10::toString(q_.scalar_type()) +
+  NEED(q_.scalar_type() == k_.scalar_type(), std::string("topk: q and k must share a dtype, got torch.") + c10::toString(q_.scalar_type()) +
                                                  " vs torch." + c10::toString(k_.scalar_type()));
   const int64_t B = q_.size(0), MG = q_.size(1), H = q_.size(2), D = q_.size(3), NC = k_.size(1);
-  need(k_.size(0) == B && k_.size(2) == H && k_.size(3) == D, "topk: incompatible shapes q=" + shape(q_) + " k=" + shape(k_));
+  NEED(k_.size(0) == B && k_.size(2) == H && k_.size(3) == D, "topk: incompatible shapes q=" + shape(q_) + " k=" + shape(k_));
   const Tensor q = unit_inner(q_), k = unit_inner(k_);
   const c10::cuda::CUDAGuard guard(q.device());
   Tensor out = at::empty({B, MG, H, T}, q.options().dtype(at::kInt)), sc;
@@ -164,7 +166,7 @@ std::tuple<Tensor, Tensor, Tensor, OptTensor> select_blocks(const Tensor& q_, co
   need_4d(q_, "select_blocks q");
   need_4d(k_, "select_blocks k");
   need_cuda({&q_, &k_});
-  need(q_.scalar_type() == k_.scalar_type(), std::string("select_blocks: q and k must share a dtype, got torch.") +
+  NEED(q_.scalar_type() == k_.scalar_type(), std::string("select_blocks: q and k must share a dtype, got torch.") +
                                                  c10::toString(q_.scalar_type()) + " vs torch." + c10::toString(k_.scalar_type()));
   const Tensor q = rows16(q_), k = rows16(k_);
   const c10::cuda::CUDAGuard guard(k.device());
@@ -219,12 +221,12 @@ struct Source {
 Source dense(const Tensor& k, const Tensor& v, int64_t n_tokens = -1) {
   need_4d(k, "k");
   need_cuda({&k, &v});
-  need(k.sizes() == v.sizes(), "k and v must have the same shape");
+  NEED(k.sizes() == v.sizes(), "k and v must have the same shape");
   return Source{NSA_KV_DENSE, rows16(k), rows16(v), Tensor(), n_tokens < 0 ? k.size(1) : n_tokens, 0};
 }
 Tensor output_like(const Tensor& q, const OptTensor& given, const char* what) {
   if (!given.has_value()) return at::empty(q.sizes(), q.options());
-  need(given->sizes() == q.sizes() && given->scalar_type() == q.scalar_type() && is_rows16(*given),
+  NEED(given->sizes() == q.sizes() && given->scalar_type() == q.scalar_type() && is_rows16(*given),
        std::string(what) + ": `out` must have q's shape and dtype, unit innermost stride and 16-byte aligned rows");
   return *given;
 }
@@ -240,8 +242,8 @@ std::pair<Tensor, Tensor> sel_fwd(const Tensor& q_, const Source& kv, const OptT
   Tensor out = output_like(q, out_, "sel_fwd");
   Tensor lse = at::empty({B, H, M}, q.options().dtype(at::kFloat));
   const Tensor& layout = kv.mode == NSA_KV_PTR ? kv.k : ids;
-  need(layout.defined() && layout.dim() == 4, "block_indices must be [B,MG,H,T]");
-  need(!ids.defined() || ids.scalar_type() == at::kInt, "block_indices must be int32");
+  NEED(layout.defined() && layout.dim() == 4, "block_indices must be [B,MG,H,T]");
+  NEED(!ids.defined() || ids.scalar_type() == at::kInt, "block_indices must be int32");
   const nsa_kv_source s = kv.c();
   check("nsa_sel_fwd", nsa_sel_fwd(q.data_ptr(), Strides(q), &s, static_cast<const int32_t*>(ptr(ids)), Strides(layout), out.data_ptr(),
                                    Strides(out), lse.data_ptr<float>(), B, M, H, D, layout.size(-1), i32(bs, "block_size"),
@@ -290,7 +292,7 @@ std::tuple<Tensor, Tensor, Tensor> sel_bwd(const Tensor& q_, const Source& kv, c
   for (const Tensor* t : {&q_, &ids, &out_, &do_}) need_4d(*t, "sel_bwd q, ids, out, d_out");
   need_cuda({&q_, &ids, &out_, &lse_, &do_});
   const Tensor q = rows16(q_), out = rows16(out_), d_out = rows16(do_), lse = lse_.contiguous();
-  need(ids.scalar_type() == at::kInt, "block_indices must be int32");
+  NEED(ids.scalar_type() == at::kInt, "block_indices must be int32");
   const c10::cuda::CUDAGuard guard(q.device());
   const int64_t B = q.size(0), M = q.size(1), H = q.size(2), D = q.size(3), N = kv.n_tokens, T = ids.size(-1), MG = ids.size(1);
   const int32_t block = i32(bs, "block_size"), chunk32 = i32(chunk, "chunk_size"), group = i32(G, "group_size");
@@ -559,7 +561,7 @@ struct Rope {
 };
 
 Tensor rope_apply(const Tensor& x_, const Rope& rope) {
-  need(x_.is_cuda() && x_.dim() == 3, "rope_apply: x must be a CUDA tensor [S,H,D]");
+  NEED(x_.is_cuda() && x_.dim() == 3, "rope_apply: x must be a CUDA tensor [S,H,D]");
   const Tensor x = rows16(x_);
   const c10::cuda::CUDAGuard guard(x.device());
   Tensor out = at::empty(x.sizes(), x.options());
@@ -607,18 +609,18 @@ void cache_touch(const CacheState& c, const Tensor& ids, int64_t T, int64_t epoc
 // ------------------------------------------------------------------------------------------- layers
 // The kernels address every operand by x's rows: an operand that is smaller than it should be would be read past its end.
 void need_like(const Tensor& t, const Tensor& x, at::ScalarType type, const char* what) {
-  need(t.scalar_type() == type, std::string(what) + ": dtype torch." + c10::toString(t.scalar_type()) + ", expected torch." + c10::toString(type));
-  need(t.device() == x.device(), std::string(what) + ": all tensors must be on one device");
+  NEED(t.scalar_type() == type, std::string(what) + ": dtype torch." + c10::toString(t.scalar_type()) + ", expected torch." + c10::toString(type));
+  NEED(t.device() == x.device(), std::string(what) + ": all tensors must be on one device");
 }
 // a contiguous row of d values (undefined: none)
 const Tensor& need_row(const Tensor& t, const Tensor& x, at::ScalarType type, int64_t d, const char* what) {
   if (!t.defined()) return t;
   need_like(t, x, type, what);
-  need(t.is_contiguous() && t.numel() == d, std::string(what) + ": a row of shape " + shape(t) + ", expected " + std::to_string(d) + " contiguous values");
+  NEED(t.is_contiguous() && t.numel() == d, std::string(what) + ": a row of shape " + shape(t) + ", expected " + std::to_string(d) + " contiguous values");
   return t;
 }
 int64_t row_length(const Tensor& x, const char* what) {
-  need(x.dim() > 0 && x.size(-1) > 0, std::string(what) + ": rows of shape " + shape(x));
+  NEED(x.dim() > 0 && x.size(-1) > 0, std::string(what) + ": rows of shape " + shape(x));
   return x.size(-1);
 }
 // (x', h): see nsa_residual_norm.  Each vector is (rows of T, rows of fp32), either missing.
@@ -628,7 +630,7 @@ std::pair<Tensor, OptTensor> residual_norm(const Tensor& x, const OptTensor& y, 
   const char* what = "residual_norm";
   const int64_t d = row_length(x, what), rows = x.numel() / d;
   if (y.has_value()) {
-    need(y->sizes() == x.sizes(), std::string(what) + ": x of shape " + shape(x) + " and y of shape " + shape(*y));
+    NEED(y->sizes() == x.sizes(), std::string(what) + ": x of shape " + shape(x) + " and y of shape " + shape(*y));
     need_like(*y, x, x.scalar_type(), what);
   }
   const auto mod = [&](const Vec& v) -> void* { return ptr(need_row(or_none(v.first), x, x.scalar_type(), d, what)); };
@@ -662,12 +664,12 @@ Tensor rms_rows(const Tensor& x, const Tensor& weight, double eps) {
 // q, k [S, H*D] views with a common row stride -> q' [S,H,D]; k is overwritten with k'
 Tensor qk_norm_rope(const Tensor& q, const Tensor& k, const Tensor& qw, const Tensor& kw, double eps, int64_t H, const Rope& rope) {
   const char* what = "qk_norm_rope";
-  need(q.dim() == 2 && k.sizes() == q.sizes() && H > 0 && q.size(1) % H == 0,
+  NEED(q.dim() == 2 && k.sizes() == q.sizes() && H > 0 && q.size(1) % H == 0,
        std::string(what) + ": q of shape " + shape(q) + " and k of shape " + shape(k) + ", expected [S, " + std::to_string(H) + " * D]");
   need_like(k, q, q.scalar_type(), what);
   need_row(qw, q, q.scalar_type(), q.size(1), what);
   need_row(kw, q, q.scalar_type(), q.size(1), what);
-  need(q.stride(0) == k.stride(0) && q.stride(1) == 1 && k.stride(1) == 1, "qk_norm_rope: q and k must share a row stride");
+  NEED(q.stride(0) == k.stride(0) && q.stride(1) == 1 && k.stride(1) == 1, "qk_norm_rope: q and k must share a row stride");
   need_cuda({&q, &rope.f, &rope.h, &rope.w});
   const c10::cuda::CUDAGuard guard(q.device());
   const int64_t S = q.size(0), D = q.size(1) / H;
@@ -676,6 +678,82 @@ Tensor qk_norm_rope(const Tensor& q, const Tensor& k, const Tensor& qw, const Te
   check("nsa_qk_norm_rope", nsa_qk_norm_rope(q.data_ptr(), k.data_ptr(), q.stride(0), qw.data_ptr(), kw.data_ptr(), static_cast<float>(eps), S, H, D,
                                              qo.data_ptr(), k.data_ptr(), k.stride(0), &r, dtype_of(q), stream_of(q)));
   return qo;
+}
+
+// ------------------------------------------------------------------------- what a module's call would do
+// The fused rollout layers use their sub-layers' parameters without calling them.  Two questions about that, asked for some
+// thirty modules per transformer block, which costs Python 80 us and this code a few.
+PyObject* dict_of(PyObject* o) {
+  PyObject** d = _PyObject_GetDictPtr(o);
+  return d != nullptr ? *d : nullptr;
+}
+const Tensor* tensor_of(PyObject* o, PyObject* parameter) {            // (not of subclasses, which may keep their values elsewhere)
+  return o != nullptr && (reinterpret_cast<PyObject*>(Py_TYPE(o)) == parameter || reinterpret_cast<PyObject*>(Py_TYPE(o)) == THPVariableClass)
+             ? &THPVariable_Unpack(o) : nullptr;
+}
+bool has_entries(PyObject* dict, PyObject* name) {
+  PyObject* v = PyDict_GetItem(dict, name);
+  return v != nullptr && v != Py_None && (PyDict_Check(v) ? PyDict_Size(v) != 0 : PyObject_IsTrue(v) != 0);
+}
+struct Names {
+  PyObject *forward = PyUnicode_InternFromString("forward"), *hooks = PyUnicode_InternFromString("_forward_hooks"),
+           *pre_hooks = PyUnicode_InternFromString("_forward_pre_hooks"), *compiled = PyUnicode_InternFromString("_compiled_call_impl"),
+           *params = PyUnicode_InternFromString("_parameters"), *weight = PyUnicode_InternFromString("weight"),
+           *bias = PyUnicode_InternFromString("bias");
+};
+const Names& names() {
+  static const Names n;
+  return n;
+}
+// Whether every module is exactly of its kind, untouched (no hooks, no forward of its own, its class's forward is the one in
+// `table`, not compiled) and has the parameters its kind is built with, of type `dtype`.  table: {class: (forward, kind of
+// parameters)}: 0 none, 1 a weight and perhaps a bias, 2 a weight that the row kernels can read as it lies, 3 and a bias.
+bool plain(const py::tuple& mods, const py::tuple& kinds, const py::dict& table, py::handle parameter, at::ScalarType dtype) {
+  const Names& n = names();
+  const auto row = [&](const Tensor* t) {
+    return t != nullptr && t->scalar_type() == dtype && t->is_contiguous() && reinterpret_cast<uintptr_t>(t->const_data_ptr()) % 16 == 0;
+  };
+  for (size_t i = 0; i < mods.size(); ++i) {
+    PyObject *m = mods[i].ptr(), *type = reinterpret_cast<PyObject*>(Py_TYPE(m)), *entry = PyDict_GetItem(table.ptr(), type);
+    if (type != kinds[i].ptr() || entry == nullptr) return false;
+    const py::object now = py::reinterpret_steal<py::object>(PyObject_GetAttr(type, n.forward));
+    PyObject* d = dict_of(m);
+    if (!now || now.ptr() != PyTuple_GET_ITEM(entry, 0) || d == nullptr || PyDict_Contains(d, n.forward) != 0) {
+      PyErr_Clear();
+      return false;
+    }
+    if (has_entries(d, n.hooks) || has_entries(d, n.pre_hooks) || has_entries(d, n.compiled)) return false;
+    const long kind = PyLong_AsLong(PyTuple_GET_ITEM(entry, 1));
+    if (kind == 0) continue;
+    PyObject* params = PyDict_GetItem(d, n.params);
+    if (params == nullptr) return false;
+    PyObject *w = PyDict_GetItem(params, n.weight), *b = PyDict_GetItem(params, n.bias);
+    const Tensor* weight = tensor_of(w, parameter.ptr());
+    if (kind == 1) {
+      const Tensor* bias = tensor_of(b, parameter.ptr());
+      if (weight == nullptr || weight->scalar_type() != dtype) return false;
+      if (b != nullptr && b != Py_None && (bias == nullptr || bias->scalar_type() != dtype)) return false;
+    } else if (!row(weight) || (kind == 3 && !row(tensor_of(b, parameter.ptr())))) {
+      return false;
+    }
+  }
+  return true;
+}
+// Whether the modules' weights and biases still lie one below the other in the two tensors of `whole` (whose storage is
+// kept, so that an equal address is a view of it).
+bool joined(const py::tuple& mods, const py::tuple& whole, py::handle parameter) {
+  for (int k = 0; k < 2; ++k) {
+    const Tensor& t = THPVariable_Unpack(whole[k].ptr());
+    const char* at = static_cast<const char*>(t.const_data_ptr());
+    for (const py::handle m : mods) {
+      PyObject* d = dict_of(m.ptr());
+      PyObject* params = d != nullptr ? PyDict_GetItem(d, names().params) : nullptr;
+      const Tensor* p = params != nullptr ? tensor_of(PyDict_GetItem(params, k == 0 ? names().weight : names().bias), parameter.ptr()) : nullptr;
+      if (p == nullptr || p->const_data_ptr() != at || p->scalar_type() != t.scalar_type() || !p->is_contiguous()) return false;
+      at += p->nbytes();
+    }
+  }
+  return true;
 }
 
 }  // namespace
@@ -729,11 +807,13 @@ PYBIND11_MODULE(_host, m) {
                                               int64_t pw, int64_t start) { return Rope{f, h, w, gh, gw, pf, ph, pw, start}; }));
   m.def("rope_apply", &rope_apply, nogil());
   py::class_<CacheState>(m, "CacheState").def(py::init([](std::vector<Tensor> t, int64_t H, int64_t D, int64_t page_tokens, int64_t max_blocks) {
-    need(t.size() == 10, "CacheState: ten tensors are expected");
+    NEED(t.size() == 10, "CacheState: ten tensors are expected");
     return CacheState{t[0], t[1], t[2], t[3], t[4], t[5], t[6], t[7], t[8], t[9], H, D, page_tokens, max_blocks};
   }));
   m.def("cache_append", &cache_append, nogil());
   m.def("cache_touch", &cache_touch, nogil());
+  m.def("plain", &plain);
+  m.def("joined", &joined);
   m.def("residual_norm", &residual_norm, nogil());
   m.def("rms_rows", &rms_rows, nogil());
   m.def("qk_norm_rope", &qk_norm_rope, nogil());

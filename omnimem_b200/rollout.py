@@ -153,42 +153,27 @@ def _fused(x: torch.Tensor) -> bool:
         and not _has_any_global_hook()
 
 
-def _untouched(m: nn.Module) -> bool:
-    """Whether calling module m does nothing but what its class does as it is written here: no hooks, no `forward` of its
-    own (offloading and adapter libraries set one), none put on its class, and it is not compiled."""
-    own = _PLAIN.get(type(m))
-    return own is not None and own is type(m).forward and "forward" not in m.__dict__ and not m._forward_hooks \
-        and not m._forward_pre_hooks and m._compiled_call_impl is None
-
-
 def _row(p, dtype: torch.dtype) -> bool:
     """Whether the row kernels can read vector (or rows of vectors) p as it lies."""
-    return type(p) in _TENSORS and p.dtype == dtype and p.is_contiguous() and p.data_ptr() % 16 == 0
+    return type(p) in (nn.Parameter, torch.Tensor) and p.dtype == dtype and p.is_contiguous() and p.data_ptr() % 16 == 0
+
+
+def _are(kinds: tuple, dtype: torch.dtype, mods: tuple) -> bool:
+    """Whether the fused form may use the parameters of `mods` without calling them: modules exactly of these kinds (not
+    something a user put in their place), whose call does nothing but what their class does as it is written here (no hooks,
+    no `forward` of their own: offloading and adapter libraries set one; none put on the class; not compiled), with
+    parameters of the activations' type.  A linear layer may lack its bias, a norm has to have all that it is built with."""
+    return host.plain(mods, kinds, _PLAIN, nn.Parameter, dtype)
 
 
 def _plain(dtype: torch.dtype, *mods: nn.Module) -> bool:
-    """Whether the parameters of `mods` may be used without calling them: the layers built here (not something a user
-    put in their place), untouched, parameters of the activations' type.  A linear layer may lack its bias, a norm has to
-    have all that it is built with."""
-    for m in mods:
-        if not _untouched(m):
-            return False
-        weight, bias = m._parameters.get("weight"), m._parameters.get("bias")
-        if type(m) is nn.Linear:
-            if type(weight) not in _TENSORS or weight.dtype != dtype or \
-                    bias is not None and (type(bias) not in _TENSORS or bias.dtype != dtype):
-                return False
-        elif not _row(weight, dtype) or type(m) is nn.LayerNorm and not _row(bias, dtype):
-            return False
-    return True
+    kinds = tuple(map(type, mods))
+    return all(k in (nn.Linear, nn.LayerNorm, RMSNorm) for k in kinds) and _are(kinds, dtype, mods)
 
 
-def _are(kind, *mods: nn.Module) -> bool:
-    return all(type(m) is kind for m in mods)
-
-
-_TENSORS = (nn.Parameter, torch.Tensor)              # (not subclasses, which may keep their values elsewhere)
-_PLAIN = {c: c.forward for c in (nn.Linear, nn.LayerNorm, nn.GELU, nn.Sequential, RMSNorm)}     # (and the layers below)
+# the kinds' own forward, and which parameters they have (host.plain)
+_PLAIN = {nn.Sequential: (nn.Sequential.forward, 0), nn.GELU: (nn.GELU.forward, 0), nn.Linear: (nn.Linear.forward, 1),
+          RMSNorm: (RMSNorm.forward, 2), nn.LayerNorm: (nn.LayerNorm.forward, 3)}     # (and the layers below)
 
 
 class _Packed(nn.Module):
@@ -225,17 +210,9 @@ class _Packed(nn.Module):
         self._whole = tuple(whole)
 
     def _joined(self, mods):
-        """_whole, if the parameters still lie in it (its storage is kept, so an equal address is a view of it)."""
-        if self._whole is None:
-            return None
-        for name, t in zip(("weight", "bias"), self._whole):
-            at = t.data_ptr()
-            for m in mods:
-                p = m._parameters.get(name)
-                if type(p) not in _TENSORS or p.data_ptr() != at or p.dtype != t.dtype or not p.is_contiguous():
-                    self._whole = None
-                    return None
-                at += p.nbytes
+        """_whole, if the parameters still lie in it."""
+        if self._whole is not None and not host.joined(tuple(mods), self._whole, nn.Parameter):
+            self._whole = None
         return self._whole
 
     def project(self, x: torch.Tensor):
@@ -246,6 +223,10 @@ class _Packed(nn.Module):
             return [F.linear(x, m.weight, m.bias) for m in mods]
         widths = [m.out_features for m in mods]
         return F.linear(x, *joined).split_with_sizes(widths + [joined[0].shape[0] - sum(widths)], -1)[:len(mods)]
+
+
+_ATTN = (nn.Linear,) * 4 + (RMSNorm,) * 2
+_CROSS = (nn.Linear,) * 2 + (RMSNorm,) * 2
 
 
 class NSASelfAttention(_Packed):
@@ -270,11 +251,10 @@ class NSASelfAttention(_Packed):
             raise NSABackendError(f"the block caches serve batch size 1, got activations {tuple(x.shape)}")
         H, D = self.h, self.hd
         scale = D ** -0.5
+        norms = self._modules["norm_q"], self._modules["norm_k"]
         # (one eps serves both norms)
         if _fused(x) and D % 8 == 0 and 32 % (D // 8) == 0 and \
-                _are(nn.Linear, self.q, self.k, self.v, self.g_proj) and _are(RMSNorm, self.norm_q, self.norm_k) and \
-                _plain(x.dtype, self.q, self.k, self.v, self.g_proj, self.norm_q, self.norm_k) and \
-                self.norm_q.eps == self.norm_k.eps:
+                _are(_ATTN, x.dtype, (*(self._modules[n] for n in self.packed), *norms)) and norms[0].eps == norms[1].eps:
             with timer("qkv_gate_proj"):
                 q, k, v, g = self.project(x[0])
                 g = g.view(1, S, H, 3)
@@ -340,8 +320,8 @@ class CrossAttention(_Packed):
     def forward(self, x, context):
         B, S, d = x.shape
         L = context.shape[1]
-        if _fused(x) and context.dtype == x.dtype and _are(nn.Linear, self.k, self.v) and _are(RMSNorm, self.norm_q, self.norm_k) \
-                and _plain(x.dtype, self.k, self.v, self.norm_q, self.norm_k):
+        if _fused(x) and context.dtype == x.dtype and \
+                _are(_CROSS, x.dtype, tuple(self._modules[n] for n in ("k", "v", "norm_q", "norm_k"))):
             heads = lambda t: t.unflatten(-1, (self.h, self.hd)).transpose(1, 2)
             k, v = self.project(context)
             q = heads(host.rms_rows(self.q(x), self.norm_q.weight, self.norm_q.eps))
@@ -370,14 +350,13 @@ class Block(nn.Module):
         self.modulation = nn.Parameter(torch.randn(1, 6, d) / d ** 0.5)
 
     def fusable(self, dtype: torch.dtype) -> bool:
-        attn, cross, ffn = self.self_attn, self.cross_attn, self.ffn
-        if not (_are(NSASelfAttention, attn) and _are(CrossAttention, cross) and _are(nn.LayerNorm, self.norm3)
-                and _are(nn.Sequential, ffn) and all(map(_untouched, (self, attn, cross, ffn))) and len(ffn) == 3):
+        own = self._modules
+        attn, cross, ffn = own["self_attn"], own["cross_attn"], own["ffn"]
+        if len(ffn._modules) != 3:
             return False
-        up, act, down = ffn
-        return _are(nn.Linear, up, down, attn.o, cross.o) and _are(nn.GELU, act) and _untouched(act) \
-            and act.approximate == "tanh" and _row(self.modulation, dtype) \
-            and _plain(dtype, up, down, self.norm3, attn.o, cross.o) and up.bias is not None
+        up, act, down = ffn._modules.values()
+        return _are(_BLOCK, dtype, (self, attn, cross, ffn, act, up, down, own["norm3"], attn._modules.get("o"), cross._modules.get("o"))) \
+            and act.approximate == "tanh" and up._parameters.get("bias") is not None and _row(self.modulation, dtype)
 
     def fused(self, x, pending, e, context, cache, rope, start_token, timer=_NO_TIMER):
         """forward() with the residual of the sub-layer in front still `pending` (its output and gate vector, or
@@ -417,7 +396,8 @@ class Block(nn.Module):
         return x
 
 
-_PLAIN.update((c, c.forward) for c in (NSASelfAttention, CrossAttention, Block))
+_PLAIN.update((c, (c.forward, 0)) for c in (NSASelfAttention, CrossAttention, Block))
+_BLOCK = (Block, NSASelfAttention, CrossAttention, nn.Sequential, nn.GELU, nn.Linear, nn.Linear, nn.LayerNorm, nn.Linear, nn.Linear)
 
 
 class CausalWanNSA(nn.Module):
@@ -451,7 +431,7 @@ class CausalWanNSA(nn.Module):
         e0 = self.time_projection(e).float().view(1, 6, sh.dim)
         rope = self._rope = RopeSpec(self.freqs, (gh, gw), start_frame, (1, 1, 1), like=self._rope)
         start_token = start_frame * gh * gw
-        if _fused(x) and _row(self.head_modulation, x.dtype) and all(_are(Block, b) and b.fusable(x.dtype) for b in self.blocks):
+        if _fused(x) and _row(self.head_modulation, x.dtype) and all(type(b) is Block and b.fusable(x.dtype) for b in self.blocks):
             pending, e_rows = None, e0[0].unbind(0)
             for blk, cache in zip(self.blocks, caches):
                 x, pending = blk.fused(x, pending, e_rows, context_embedded, cache, rope, start_token, timer)
