@@ -1137,7 +1137,8 @@ int launch_score_select(const ScoreSelectParams& p, int B, cudaStream_t s) {
 
 // Fewer long rows than SMs: a thread block per row leaves the chip idle, so a warp sorts the keys of each 1024 columns and
 // the lists of a row are merged like those of several ranks (exact: a row's best are among its segments' best, with the
-// same keys).  12 rows of 60000 / 200000, top-8: 78 / 215 us; with 32 warps per row 99 / 296 us, with eight 131 / 414 us.
+// same keys).  12 rows of 60000 / 200000, top-8, scores included: 74 / 205 us;
+// with 32 warps per row 99 / 296 us, with eight 131 / 414 us.
 constexpr int kSegCols = 1024, kSegRows = 148, kSegTopk = 16;
 bool in_segments(int64_t rows, int64_t NC) { return rows <= kSegRows && NC > 8 * kSegCols; }
 size_t segment_bytes(int64_t rows, int64_t NC) {
